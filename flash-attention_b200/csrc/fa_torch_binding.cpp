@@ -10,12 +10,24 @@
 // Things the reference's positional lists have no slot for arrive as trailing arguments from the
 // Python wrapper: the status buffer of the device, the head-shard pair of the dropout mask, the
 // deterministic-dQ switch, an explicit Philox pair for the backward.
+//
+// The differentiable functions (flash_attn_interface.py, flash_blocksparse_attn_interface.py) are
+// here too, as one autograd node over the same calls: what bounds a training step at short sequences
+// is the host, and a Python autograd function costs several times what its kernels do (see AttnNode).
 #include <torch/extension.h>
 
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAGeneratorImpl.h>
 #include <c10/cuda/CUDAGuard.h>
 
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+
+#include <array>
+#include <cmath>
+#include <limits>
+#include <atomic>
 #include <mutex>
 #include <string>
 
@@ -36,48 +48,82 @@ void check_rc(int rc) {
     throw std::runtime_error(std::string("fa_b200: ") + fa_status_string(rc) + ": " + fa_last_error());
 }
 
+// One operand of the attention call: a (rows, heads, d) view of a tensor.  The packed layouts are cut
+// into views by pointer arithmetic; making the three tensors qkv[:, i] would cost more than the checks.
+struct View {
+  char* ptr;
+  int64_t dim, rows, heads, d, row_stride, head_stride, last_stride;
+  at::ScalarType dtype;
+  bool cuda;
+};
+
+View view_of(const at::Tensor& t) {
+  View v{};
+  v.ptr = static_cast<char*>(t.data_ptr());
+  v.dim = t.dim();
+  v.dtype = t.scalar_type();
+  v.cuda = t.is_cuda();
+  if (v.dim == 3) {
+    v.rows = t.size(0); v.heads = t.size(1); v.d = t.size(2);
+    v.row_stride = t.stride(0); v.head_stride = t.stride(1); v.last_stride = t.stride(2);
+  }
+  return v;
+}
+
+// packed[:, i] of a (rows, n, heads, d) tensor
+View view_of(const at::Tensor& packed, int64_t i) {
+  if (packed.dim() != 4 || packed.size(1) <= i) return view_of(packed.select(1, i));
+  View v{};
+  v.ptr = static_cast<char*>(packed.data_ptr()) + i * packed.stride(1) * packed.element_size();
+  v.dim = 3;
+  v.dtype = packed.scalar_type();
+  v.cuda = packed.is_cuda();
+  v.rows = packed.size(0); v.heads = packed.size(2); v.d = packed.size(3);
+  v.row_stride = packed.stride(0); v.head_stride = packed.stride(2); v.last_stride = packed.stride(3);
+  return v;
+}
+
 // Argument checks of mha_fwd / mha_bwd (fmha_api.cpp:199-230), same messages as the Python binding.
-Dims check_qkv(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& cu_q,
-               const at::Tensor& cu_k) {
-  require(q.is_cuda() && k.is_cuda() && v.is_cuda(), "q, k, v must be CUDA tensors");
-  const auto dt = q.scalar_type();
+Dims check_qkv(const View& q, const View& k, const View& v, const at::Tensor& cu_q, const at::Tensor& cu_k) {
+  require(q.cuda && k.cuda && v.cuda, "q, k, v must be CUDA tensors");
+  const auto dt = q.dtype;
   require(dt == at::kHalf || dt == at::kBFloat16, "q must be fp16 or bf16");
-  require(k.scalar_type() == dt && v.scalar_type() == dt, "q, k, v must have the same dtype");
+  require(k.dtype == dt && v.dtype == dt, "q, k, v must have the same dtype");
   require(cu_q.scalar_type() == at::kInt && cu_k.scalar_type() == at::kInt, "cu_seqlens must be int32");
   require(cu_q.is_cuda() && cu_k.is_cuda(), "cu_seqlens must be CUDA tensors");
   require(cu_q.is_contiguous() && cu_k.is_contiguous(), "cu_seqlens must be contiguous");
-  require(q.dim() == 3 && k.dim() == 3 && v.dim() == 3, "q, k, v must be (total, heads, d)");
-  require(q.stride(2) == 1 && k.stride(2) == 1 && v.stride(2) == 1,
+  require(q.dim == 3 && k.dim == 3 && v.dim == 3, "q, k, v must be (total, heads, d)");
+  require(q.last_stride == 1 && k.last_stride == 1 && v.last_stride == 1,
           "q, k, v must have a contiguous last dimension");
   Dims s;
   s.batch = cu_q.size(0) - 1;
   require(s.batch > 0, "batch size must be positive");
   require(cu_k.size(0) == s.batch + 1, "cu_seqlens_q / cu_seqlens_k size mismatch");
-  s.total_q = q.size(0);
-  s.heads = q.size(1);
-  s.d = q.size(2);
-  s.total_k = k.size(0);
+  s.total_q = q.rows;
+  s.heads = q.heads;
+  s.d = q.d;
+  s.total_k = k.rows;
   require(s.d == 16 || s.d == 32 || s.d == 64 || s.d == 128, "head_dim must be 16, 32, 64 or 128");
-  require(k.size(1) == s.heads && k.size(2) == s.d, "k has the wrong shape");
-  require(v.size(0) == s.total_k && v.size(1) == s.heads && v.size(2) == s.d, "v has the wrong shape");
+  require(k.heads == s.heads && k.d == s.d, "k has the wrong shape");
+  require(v.rows == s.total_k && v.heads == s.heads && v.d == s.d, "v has the wrong shape");
   return s;
 }
 
-void fill_fwd(fa_fwd_params& p, const Dims& s, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
+void fill_fwd(fa_fwd_params& p, const Dims& s, const View& q, const View& k, const View& v,
               const at::Tensor& o, const at::Tensor& lse, const at::Tensor& cu_q, const at::Tensor& cu_k,
               int64_t max_q, int64_t max_k, double p_dropout, double scale, bool causal, uint64_t seed,
               uint64_t offset, int64_t mask_heads_total, int64_t mask_head_offset, int64_t status_ptr) {
   p = fa_fwd_params{};
-  p.q = q.data_ptr();
-  p.k = k.data_ptr();
-  p.v = v.data_ptr();
+  p.q = q.ptr;
+  p.k = k.ptr;
+  p.v = v.ptr;
   p.o = o.data_ptr();
   p.softmax_lse = static_cast<float*>(lse.data_ptr());
   p.cu_seqlens_q = static_cast<const int32_t*>(cu_q.data_ptr());
   p.cu_seqlens_k = static_cast<const int32_t*>(cu_k.data_ptr());
-  p.q_row_stride = q.stride(0); p.q_head_stride = q.stride(1);
-  p.k_row_stride = k.stride(0); p.k_head_stride = k.stride(1);
-  p.v_row_stride = v.stride(0); p.v_head_stride = v.stride(1);
+  p.q_row_stride = q.row_stride; p.q_head_stride = q.head_stride;
+  p.k_row_stride = k.row_stride; p.k_head_stride = k.head_stride;
+  p.v_row_stride = v.row_stride; p.v_head_stride = v.head_stride;
   p.o_row_stride = o.stride(0); p.o_head_stride = o.stride(1);
   p.lse_stride = lse.size(2);
   p.batch = static_cast<int32_t>(s.batch);
@@ -90,7 +136,7 @@ void fill_fwd(fa_fwd_params& p, const Dims& s, const at::Tensor& q, const at::Te
   p.p_dropout = static_cast<float>(p_dropout);
   p.softmax_scale = static_cast<float>(scale);
   p.is_causal = causal ? 1 : 0;
-  p.is_bf16 = q.scalar_type() == at::kBFloat16 ? 1 : 0;
+  p.is_bf16 = q.dtype == at::kBFloat16 ? 1 : 0;
   p.philox_seed = seed;
   p.philox_offset = offset;
   if (mask_heads_total != 0 || mask_head_offset != 0) {
@@ -118,7 +164,7 @@ int64_t round_up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
 // per-sequence block-visit table.  The reference checks for exactly (ceil(max_k / 256), ceil16(max_q) /
 // 16) (:515); its own module passes a mask cut at a multiple of 256 rows' worth of slots, so a larger
 // mask is accepted and its real row length is used.
-void check_blockmask(const at::Tensor& blockmask, const at::Tensor& q, int64_t max_q, int64_t max_k) {
+void check_blockmask(const at::Tensor& blockmask, const View& q, int64_t max_q, int64_t max_k) {
   require(blockmask.is_cuda() && blockmask.scalar_type() == at::kInt && blockmask.is_contiguous(),
           "blockmask must be a contiguous int32 CUDA tensor");
   const int64_t want0 = round_up(max_k, 256) / 256, want1 = round_up(max_q, 16) / 16;
@@ -129,14 +175,14 @@ void check_blockmask(const at::Tensor& blockmask, const at::Tensor& q, int64_t m
     throw std::runtime_error("blockmask must have at least shape (" + std::to_string(want0) + ", " +
                              std::to_string(want1) + "), got " + got + ")");
   }
-  require(q.scalar_type() == at::kHalf, "block-sparse attention is fp16 only");
-  require(q.size(2) == 16 || q.size(2) == 32 || q.size(2) == 64, "block-sparse attention supports head_dim 16, 32, 64");
+  require(q.dtype == at::kHalf, "block-sparse attention is fp16 only");
+  require(q.d == 16 || q.d == 32 || q.d == 64, "block-sparse attention supports head_dim 16, 32, 64");
 }
 
-at::Tensor attach_blockmask(fa_fwd_params& p, const at::Tensor& blockmask, const at::Tensor& q, int64_t batch) {
+at::Tensor attach_blockmask(fa_fwd_params& p, const at::Tensor& blockmask, int64_t batch) {
   const size_t nbytes = fa_blocksparse_workspace_bytes(static_cast<int32_t>(batch), static_cast<int32_t>(blockmask.size(0)),
                                                        static_cast<int32_t>(blockmask.size(1)));
-  at::Tensor ws = at::empty({static_cast<int64_t>(nbytes < 4 ? 4 : nbytes)}, q.options().dtype(at::kByte));
+  at::Tensor ws = at::empty({static_cast<int64_t>(nbytes < 4 ? 4 : nbytes)}, blockmask.options().dtype(at::kByte));
   p.blockmask = static_cast<const int32_t*>(blockmask.data_ptr());
   p.blockmask_rows = static_cast<int32_t>(blockmask.size(0));
   p.blockmask_cols = static_cast<int32_t>(blockmask.size(1));
@@ -145,53 +191,117 @@ at::Tensor attach_blockmask(fa_fwd_params& p, const at::Tensor& blockmask, const
   return ws;
 }
 
+struct FwdCall {
+  int64_t max_q, max_k;
+  double p_dropout, scale;
+  bool zero_tensors, causal, return_softmax;
+  int64_t mask_heads_total, mask_head_offset, status_ptr;
+};
+
+struct FwdResult {
+  at::Tensor o, lse, s_dmask;
+  uint64_t seed = 0, offset = 0;
+};
+
+// One forward call: outputs allocated, Philox pair taken, kernels launched on the current stream.
+FwdResult run_fwd(const View& q, const View& k, const View& v, const at::TensorOptions& opts, const at::Tensor& cu_q,
+                  const at::Tensor& cu_k, const at::Tensor* blockmask, const FwdCall& c,
+                  const c10::optional<at::Generator>& gen) {
+  const Dims s = check_qkv(q, k, v, cu_q, cu_k);
+  require(c.p_dropout < 1.0, "p_dropout must be < 1");
+  const bool sparse = blockmask != nullptr;
+  if (sparse) check_blockmask(*blockmask, q, c.max_q, c.max_k);
+  c10::cuda::CUDAGuard guard(opts.device());
+  const int64_t lse_len = round_up(c.max_q, 16);
+  FwdResult r;
+  // the block-sparse entry always starts from o = 0 (:519)
+  r.o = (c.zero_tensors || sparse) ? at::zeros({s.total_q, s.heads, s.d}, opts)
+                                   : at::empty({s.total_q, s.heads, s.d}, opts);
+  r.lse = c.zero_tensors
+              ? at::full({s.batch, s.heads, lse_len}, -std::numeric_limits<float>::infinity(), opts.dtype(at::kFloat))
+              : at::empty({s.batch, s.heads, lse_len}, opts.dtype(at::kFloat));
+  if (c.p_dropout > 0)
+    philox_state(gen, fa_philox_increment(static_cast<int32_t>(s.d), static_cast<int32_t>(c.max_q),
+                                          static_cast<int32_t>(c.max_k), sparse ? 1 : 0), r.seed, r.offset);
+  fa_fwd_params p;
+  fill_fwd(p, s, q, k, v, r.o, r.lse, cu_q, cu_k, c.max_q, c.max_k, c.p_dropout, c.scale, c.causal, r.seed, r.offset,
+           c.mask_heads_total, c.mask_head_offset, c.status_ptr);
+  at::Tensor bs_ws;
+  if (c.return_softmax) {
+    // (batch, heads, seqlen_q rounded to 16, seqlen_k rounded as the reference does, :232-240, :253);
+    // zero outside the sequences
+    const int64_t base = sparse ? 256 : ((s.d == 128 && c.p_dropout > 0) ? 128 : 256);
+    const int64_t sk_r = (c.max_k <= 128 && !sparse) ? 128 : (c.max_k <= 256 ? 256 : round_up(c.max_k, base));
+    r.s_dmask = at::zeros({s.batch, s.heads, lse_len, sk_r}, opts);
+    p.s_dmask = r.s_dmask.data_ptr();
+    p.s_rows = lse_len;
+    p.s_cols = sk_r;
+  }
+  if (sparse) bs_ws = attach_blockmask(p, *blockmask, s.batch);
+  check_rc(fa_fwd(&p, at::cuda::getCurrentCUDAStream().stream()));
+  return r;
+}
+
 py::list fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& cu_q,
              const at::Tensor& cu_k, int64_t max_q, int64_t max_k, double p_dropout, double scale,
              bool zero_tensors, bool causal, bool return_softmax, c10::optional<at::Generator> gen,
              c10::optional<at::Tensor> blockmask, bool return_philox, int64_t mask_heads_total,
              int64_t mask_head_offset, int64_t status_ptr) {
-  const Dims s = check_qkv(q, k, v, cu_q, cu_k);
-  require(p_dropout < 1.0, "p_dropout must be < 1");
-  const bool sparse = blockmask.has_value();
-  if (sparse) check_blockmask(*blockmask, q, max_q, max_k);
-  c10::cuda::CUDAGuard guard(q.device());
-  const auto opts = q.options();
-  const int64_t lse_len = round_up(max_q, 16);
-  // the block-sparse entry always starts from o = 0 (:519)
-  at::Tensor o = (zero_tensors || sparse) ? at::zeros({s.total_q, s.heads, s.d}, opts)
-                                          : at::empty({s.total_q, s.heads, s.d}, opts);
-  at::Tensor lse = zero_tensors
-                       ? at::full({s.batch, s.heads, lse_len}, -std::numeric_limits<float>::infinity(), opts.dtype(at::kFloat))
-                       : at::empty({s.batch, s.heads, lse_len}, opts.dtype(at::kFloat));
-  uint64_t seed = 0, offset = 0;
-  if (p_dropout > 0)
-    philox_state(gen, fa_philox_increment(static_cast<int32_t>(s.d), static_cast<int32_t>(max_q),
-                                          static_cast<int32_t>(max_k), sparse ? 1 : 0), seed, offset);
-  fa_fwd_params p;
-  fill_fwd(p, s, q, k, v, o, lse, cu_q, cu_k, max_q, max_k, p_dropout, scale, causal, seed, offset,
-           mask_heads_total, mask_head_offset, status_ptr);
-  at::Tensor s_dmask, bs_ws;
-  if (return_softmax) {
-    // (batch, heads, seqlen_q rounded to 16, seqlen_k rounded as the reference does, :232-240, :253);
-    // zero outside the sequences
-    const int64_t base = sparse ? 256 : ((s.d == 128 && p_dropout > 0) ? 128 : 256);
-    const int64_t sk_r = (max_k <= 128 && !sparse) ? 128 : (max_k <= 256 ? 256 : round_up(max_k, base));
-    s_dmask = at::zeros({s.batch, s.heads, lse_len, sk_r}, opts);
-    p.s_dmask = s_dmask.data_ptr();
-    p.s_rows = lse_len;
-    p.s_cols = sk_r;
-  }
-  if (sparse) bs_ws = attach_blockmask(p, *blockmask, q, s.batch);
-  check_rc(fa_fwd(&p, at::cuda::getCurrentCUDAStream().stream()));
+  const FwdCall c{max_q, max_k, p_dropout, scale, zero_tensors, causal, return_softmax,
+                  mask_heads_total, mask_head_offset, status_ptr};
+  const FwdResult r = run_fwd(view_of(q), view_of(k), view_of(v), q.options(), cu_q, cu_k,
+                              blockmask.has_value() ? &*blockmask : nullptr, c, gen);
   py::list res;
-  res.append(o);
-  res.append(lse);
-  if (return_softmax) res.append(s_dmask);
+  res.append(r.o);
+  res.append(r.lse);
+  if (return_softmax) res.append(r.s_dmask);
   if (return_philox) {
-    res.append(py::int_(seed));
-    res.append(py::int_(offset));
+    res.append(py::int_(r.seed));
+    res.append(py::int_(r.offset));
   }
   return res;
+}
+
+struct BwdCall {
+  int64_t max_q, max_k;
+  double p_dropout, scale;
+  bool causal, deterministic;
+  int64_t stage_mask;
+  uint64_t seed, offset;
+  int64_t mask_heads_total, mask_head_offset, status_ptr;
+};
+
+// One backward call on the current stream; the device of the tensors is current.
+void run_bwd(const Dims& s, const View& q, const View& k, const View& v, const at::Tensor& dout, const at::Tensor& out,
+             const at::Tensor& lse, const View& dq, const View& dk, const View& dv, float* softmax_d,
+             const at::Tensor& cu_q, const at::Tensor& cu_k, const at::Tensor* blockmask, const BwdCall& c) {
+  // fp32 dQ accumulator (and the ticket words of the deterministic mode) from the caching allocator,
+  // per call, like the reference's dq_tmp (:402-404)
+  const size_t nbytes = fa_bwd_workspace_bytes_ex(static_cast<int32_t>(s.total_q), static_cast<int32_t>(s.heads),
+                                                  static_cast<int32_t>(s.d), static_cast<int32_t>(s.batch),
+                                                  static_cast<int32_t>(c.max_q), c.deterministic ? 1 : 0);
+  at::Tensor ws = at::empty({static_cast<int64_t>(nbytes < 16 ? 16 : nbytes)}, lse.options().dtype(at::kByte));
+  fa_bwd_params p = {};
+  fill_fwd(p.fwd, s, q, k, v, out, lse, cu_q, cu_k, c.max_q, c.max_k, c.p_dropout, c.scale, c.causal, c.seed, c.offset,
+           c.mask_heads_total, c.mask_head_offset, c.status_ptr);
+  p.dout = dout.data_ptr();
+  p.dq = dq.ptr;
+  p.dk = dk.ptr;
+  p.dv = dv.ptr;
+  p.softmax_d = softmax_d;
+  p.dq_row_stride = dq.row_stride; p.dq_head_stride = dq.head_stride;
+  p.dk_row_stride = dk.row_stride; p.dk_head_stride = dk.head_stride;
+  p.dv_row_stride = dv.row_stride; p.dv_head_stride = dv.head_stride;
+  p.workspace = ws.data_ptr();
+  p.workspace_bytes = static_cast<size_t>(ws.numel());
+  p.stage_mask = static_cast<int32_t>(c.stage_mask);
+  p.deterministic = c.deterministic ? 1 : 0;
+  at::Tensor bs_ws;
+  if (blockmask != nullptr) {
+    check_blockmask(*blockmask, q, c.max_q, c.max_k);
+    bs_ws = attach_blockmask(p.fwd, *blockmask, s.batch);
+  }
+  check_rc(fa_bwd(&p, at::cuda::getCurrentCUDAStream().stream()));
 }
 
 py::list bwd(const at::Tensor& dout, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
@@ -201,7 +311,8 @@ py::list bwd(const at::Tensor& dout, const at::Tensor& q, const at::Tensor& k, c
              c10::optional<at::Tensor> blockmask, int64_t stage_mask, bool has_philox, uint64_t philox_seed,
              uint64_t philox_offset, bool deterministic,
              int64_t mask_heads_total, int64_t mask_head_offset, int64_t status_ptr) {
-  const Dims s = check_qkv(q, k, v, cu_q, cu_k);
+  const View qv = view_of(q), kv = view_of(k), vv = view_of(v);
+  const Dims s = check_qkv(qv, kv, vv, cu_q, cu_k);
   const auto dt = q.scalar_type();
   require(dout.scalar_type() == dt && out.scalar_type() == dt, "dout / out dtype mismatch");
   require(dq.scalar_type() == dt && dk.scalar_type() == dt && dv.scalar_type() == dt, "dq / dk / dv dtype mismatch");
@@ -222,44 +333,20 @@ py::list bwd(const at::Tensor& dout, const at::Tensor& q, const at::Tensor& k, c
     dv.zero_();
   }
   at::Tensor softmax_d = at::empty_like(lse);
-  uint64_t seed = 0, offset = 0;
+  BwdCall c{max_q, max_k, p_dropout, scale, causal, deterministic, stage_mask, 0, 0,
+            mask_heads_total, mask_head_offset, status_ptr};
   if (p_dropout > 0) {
     // The caller restores the generator state saved before the forward, so reading the state here
     // yields the forward's pair; the reference then advances it by a dummy amount (:437-445).
     if (has_philox) {
-      seed = philox_seed;
-      offset = philox_offset;
+      c.seed = philox_seed;
+      c.offset = philox_offset;
     } else {
-      philox_state(gen, 4, seed, offset);
+      philox_state(gen, 4, c.seed, c.offset);
     }
   }
-  // fp32 dQ accumulator (and the ticket words of the deterministic mode) from the caching allocator,
-  // per call, like the reference's dq_tmp (:402-404)
-  const size_t nbytes = fa_bwd_workspace_bytes_ex(static_cast<int32_t>(s.total_q), static_cast<int32_t>(s.heads),
-                                                  static_cast<int32_t>(s.d), static_cast<int32_t>(s.batch),
-                                                  static_cast<int32_t>(max_q), deterministic ? 1 : 0);
-  at::Tensor ws = at::empty({static_cast<int64_t>(nbytes < 16 ? 16 : nbytes)}, q.options().dtype(at::kByte));
-  fa_bwd_params p = {};
-  fill_fwd(p.fwd, s, q, k, v, out, lse, cu_q, cu_k, max_q, max_k, p_dropout, scale, causal, seed, offset,
-           mask_heads_total, mask_head_offset, status_ptr);
-  p.dout = dout.data_ptr();
-  p.dq = dq.data_ptr();
-  p.dk = dk.data_ptr();
-  p.dv = dv.data_ptr();
-  p.softmax_d = static_cast<float*>(softmax_d.data_ptr());
-  p.dq_row_stride = dq.stride(0); p.dq_head_stride = dq.stride(1);
-  p.dk_row_stride = dk.stride(0); p.dk_head_stride = dk.stride(1);
-  p.dv_row_stride = dv.stride(0); p.dv_head_stride = dv.stride(1);
-  p.workspace = ws.data_ptr();
-  p.workspace_bytes = static_cast<size_t>(ws.numel());
-  p.stage_mask = static_cast<int32_t>(stage_mask);
-  p.deterministic = deterministic ? 1 : 0;
-  at::Tensor bs_ws;
-  if (blockmask.has_value()) {
-    check_blockmask(*blockmask, q, max_q, max_k);
-    bs_ws = attach_blockmask(p.fwd, *blockmask, q, s.batch);
-  }
-  check_rc(fa_bwd(&p, at::cuda::getCurrentCUDAStream().stream()));
+  run_bwd(s, qv, kv, vv, dout, out, lse, view_of(dq), view_of(dk), view_of(dv),
+          static_cast<float*>(softmax_d.data_ptr()), cu_q, cu_k, blockmask.has_value() ? &*blockmask : nullptr, c);
   py::list res;
   res.append(dq);
   res.append(dk);
@@ -268,10 +355,171 @@ py::list bwd(const at::Tensor& dout, const at::Tensor& q, const at::Tensor& k, c
   return res;
 }
 
+// ---------------------------------------------------------------------------------------------
+// Differentiable entry points (flash_attn/flash_attn_interface.py:39-148 and
+// flash_attn/flash_blocksparse_attn_interface.py:64-96 of the reference).
+
+// Process-wide options of the Python binding (flash_attn_cuda.options), mirrored here by its setters:
+// the backward runs on an autograd thread that does not hold the interpreter.
+std::atomic<bool> g_deterministic{false};
+std::atomic<int64_t> g_mask_heads_total{0}, g_mask_head_offset{0};
+// Per-device status buffer of the kernels (owned by the Python module, lives as long as the process).
+constexpr int kMaxDevices = 64;
+std::atomic<int64_t> g_status[kMaxDevices];
+
+int64_t status_of(const c10::Device& dev) {
+  const int i = dev.index();
+  return i >= 0 && i < kMaxDevices ? g_status[i].load(std::memory_order_acquire) : 0;
+}
+
+// How the inputs of a call are cut into q, k, v.
+enum Layout { kQkvPacked = 1, kKvPacked = 2, kSeparate = 3 };  // value = number of input tensors
+
+struct Operands { View q, k, v; };
+
+Operands cut(const at::Tensor* x, int layout) {
+  if (layout == kQkvPacked) return {view_of(x[0], 0), view_of(x[0], 1), view_of(x[0], 2)};
+  if (layout == kKvPacked) return {view_of(x[0]), view_of(x[1], 0), view_of(x[1], 1)};
+  return {view_of(x[0]), view_of(x[1]), view_of(x[2])};
+}
+
+// Gradient of one attention call.  What a training step at short sequences pays for is host time: a
+// Python autograd function, the generator states it saves and restores (two 16-byte host tensors per
+// call, each copied under the generator's lock) and the views of the packed tensors took 100-110 us of
+// host time per forward + backward at batch 8 x 12 heads x 128 tokens, whose kernels run 23 us.  Here
+// the node keeps the Philox pair itself, so the generator is read once, in the forward; after the
+// backward it stands where it stood before, as with the saved and restored states.
+struct AttnNode : public torch::autograd::Node {
+  std::array<torch::autograd::SavedVariable, 3> inputs;
+  torch::autograd::SavedVariable out, lse, cu_q, cu_k, blockmask;
+  int layout = 0;
+  int64_t max_q = 0, max_k = 0;
+  double p_dropout = 0, scale = 0;
+  bool causal = false, sparse = false, released = false;
+  uint64_t seed = 0, offset = 0;
+
+  std::string name() const override { return sparse ? "FlashBlocksparseAttnBackward" : "FlashAttnBackward"; }
+
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    for (auto& v : inputs) v.reset_data();
+    out.reset_data(); lse.reset_data(); cu_q.reset_data(); cu_k.reset_data(); blockmask.reset_data();
+    released = true;
+  }
+
+  torch::autograd::variable_list apply(torch::autograd::variable_list&& grads) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
+    at::Tensor x[3];
+    for (int i = 0; i < layout; ++i) x[i] = inputs[i].unpack();
+    const at::Tensor o = out.unpack(shared_from_this());
+    const at::Tensor l = lse.unpack(), cq = cu_q.unpack(), ck = cu_k.unpack(), bm = blockmask.unpack();
+    c10::NoGradGuard no_grad;
+    at::AutoDispatchBelowADInplaceOrView below;
+    c10::cuda::CUDAGuard guard(o.device());
+    const at::Tensor dout = grads[0].defined() ? grads[0].contiguous() : at::zeros_like(o, at::MemoryFormat::Contiguous);
+    const Operands v = cut(x, layout);
+    const Dims s = check_qkv(v.q, v.k, v.v, cq, ck);
+    require(dout.scalar_type() == o.scalar_type(), "dout / out dtype mismatch");
+    require(dout.sizes() == o.sizes(), "out / dout have the wrong shape");
+    torch::autograd::variable_list result(layout);
+    at::Tensor dx[3];
+    for (int i = 0; i < layout; ++i) result[i] = dx[i] = at::empty_like(x[i]);
+    const Operands g = cut(dx, layout);
+    require(g.q.last_stride == 1 && g.k.last_stride == 1 && g.v.last_stride == 1,
+            "dq, dk, dv must have a contiguous last dimension");
+    at::Tensor softmax_d = at::empty_like(l);
+    const BwdCall c{max_q, max_k, p_dropout, scale, causal, g_deterministic.load(), 0, seed, offset,
+                    g_mask_heads_total.load(), g_mask_head_offset.load(), status_of(o.device())};
+    run_bwd(s, v.q, v.k, v.v, dout, o, l, g.q, g.k, g.v, static_cast<float*>(softmax_d.data_ptr()), cq, ck,
+            sparse ? &bm : nullptr, c);
+    return result;
+  }
+};
+
+at::Tensor attention(const at::Tensor* x, int layout, const at::Tensor& cu_q, const at::Tensor& cu_k, int64_t max_q,
+                     int64_t max_k, double p_dropout, c10::optional<double> softmax_scale, bool causal,
+                     const at::Tensor* blockmask) {
+  const double scale = softmax_scale.has_value() ? *softmax_scale : 1.0 / std::sqrt(static_cast<double>(x[0].size(-1)));
+  bool needs_grad = false;
+  if (c10::GradMode::is_enabled())
+    for (int i = 0; i < layout; ++i) needs_grad = needs_grad || x[i].requires_grad();
+  FwdResult r;
+  {
+    c10::NoGradGuard no_grad;
+    at::AutoDispatchBelowADInplaceOrView below;
+    const Operands v = cut(x, layout);
+    const FwdCall c{max_q, max_k, p_dropout, scale, false, causal, false,
+                    g_mask_heads_total.load(), g_mask_head_offset.load(), status_of(x[0].device())};
+    r = run_fwd(v.q, v.k, v.v, x[0].options(), cu_q, cu_k, blockmask, c, c10::nullopt);
+  }
+  if (needs_grad) {
+    auto node = std::shared_ptr<AttnNode>(new AttnNode(), torch::autograd::deleteNode);
+    torch::autograd::edge_list edges;
+    edges.reserve(layout);
+    for (int i = 0; i < layout; ++i) edges.push_back(torch::autograd::impl::gradient_edge(x[i]));
+    node->set_next_edges(std::move(edges));
+    for (int i = 0; i < layout; ++i) node->inputs[i] = torch::autograd::SavedVariable(x[i], false);
+    node->lse = torch::autograd::SavedVariable(r.lse, false);
+    node->cu_q = torch::autograd::SavedVariable(cu_q, false);
+    node->cu_k = torch::autograd::SavedVariable(cu_k, false);
+    if (blockmask != nullptr) node->blockmask = torch::autograd::SavedVariable(*blockmask, false);
+    node->layout = layout;
+    node->max_q = max_q; node->max_k = max_k;
+    node->p_dropout = p_dropout; node->scale = scale;
+    node->causal = causal; node->sparse = blockmask != nullptr;
+    node->seed = r.seed; node->offset = r.offset;
+    torch::autograd::set_history(r.o, node);
+    node->out = torch::autograd::SavedVariable(r.o, true);
+  }
+  return r.o;
+}
+
+at::Tensor attn_qkvpacked(const at::Tensor& qkv, const at::Tensor& cu, int64_t max_s, double p_dropout,
+                          c10::optional<double> scale, bool causal) {
+  return attention(&qkv, kQkvPacked, cu, cu, max_s, max_s, p_dropout, scale, causal, nullptr);
+}
+
+at::Tensor attn_kvpacked(const at::Tensor& q, const at::Tensor& kv, const at::Tensor& cu_q, const at::Tensor& cu_k,
+                         int64_t max_q, int64_t max_k, double p_dropout, c10::optional<double> scale, bool causal) {
+  const at::Tensor x[2] = {q, kv};
+  return attention(x, kKvPacked, cu_q, cu_k, max_q, max_k, p_dropout, scale, causal, nullptr);
+}
+
+at::Tensor attn(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& cu_q,
+                const at::Tensor& cu_k, int64_t max_q, int64_t max_k, double p_dropout, c10::optional<double> scale,
+                bool causal) {
+  const at::Tensor x[3] = {q, k, v};
+  return attention(x, kSeparate, cu_q, cu_k, max_q, max_k, p_dropout, scale, causal, nullptr);
+}
+
+at::Tensor attn_sparse_qkvpacked(const at::Tensor& qkv, const at::Tensor& cu, const at::Tensor& blockmask,
+                                 double p_dropout, int64_t max_s, c10::optional<double> scale, bool causal) {
+  require(qkv.dim() == 4 && qkv.size(1) == 3, "qkv must be (total, 3, heads, head_dim)");
+  return attention(&qkv, kQkvPacked, cu, cu, max_s, max_s, p_dropout, scale, causal, &blockmask);
+}
+
+void set_options(bool deterministic, int64_t mask_heads_total, int64_t mask_head_offset) {
+  g_deterministic = deterministic;
+  g_mask_heads_total = mask_heads_total;
+  g_mask_head_offset = mask_head_offset;
+}
+
+void set_status(int64_t device_index, int64_t ptr) {
+  if (device_index >= 0 && device_index < kMaxDevices) g_status[device_index].store(ptr, std::memory_order_release);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
-  m.doc() = "compiled binding of libfa_b200.so: fwd / bwd with the reference extension's argument lists (+ optional block mask)";
+  m.doc() = "compiled binding of libfa_b200.so: fwd / bwd with the reference extension's argument lists (+ optional block mask), "
+            "and the differentiable attention functions";
   m.def("fwd", &fwd);
   m.def("bwd", &bwd);
+  m.def("attn_qkvpacked", &attn_qkvpacked);
+  m.def("attn_kvpacked", &attn_kvpacked);
+  m.def("attn", &attn);
+  m.def("attn_sparse_qkvpacked", &attn_sparse_qkvpacked);
+  m.def("set_options", &set_options);
+  m.def("set_status", &set_status);
 }

@@ -35,6 +35,7 @@ def binding_in_use():
 
 _status = {}
 _status_ptr = {}
+_status_known = set()   # indices of the devices compiled_attention() has set up
 
 
 class _Options:
@@ -47,11 +48,35 @@ class _Options:
                    [head_offset, head_offset + heads) of a model with heads_total heads draws the
                    dropout mask of the unsharded call (fa_fwd_params.mask_heads_total / _offset).
     """
-    __slots__ = ("deterministic", "mask_heads")
+    __slots__ = ("_deterministic", "_mask_heads")
 
     def __init__(self):
-        self.deterministic = False
-        self.mask_heads = None
+        self._deterministic = False
+        self._mask_heads = None
+
+    def _tell_binding(self):
+        # the compiled autograd node reads its own copy: it runs without the interpreter
+        if _binding is not None:
+            total, offset = self._mask_heads or (0, 0)
+            _binding.set_options(bool(self._deterministic), total, offset)
+
+    @property
+    def deterministic(self):
+        return self._deterministic
+
+    @deterministic.setter
+    def deterministic(self, value):
+        self._deterministic = value
+        self._tell_binding()
+
+    @property
+    def mask_heads(self):
+        return self._mask_heads
+
+    @mask_heads.setter
+    def mask_heads(self, value):
+        self._mask_heads = value
+        self._tell_binding()
 
 
 options = _Options()
@@ -82,7 +107,20 @@ def _status_buffer(device):
         buf = torch.zeros(128, dtype=torch.int32, device=device)
         _status[device] = buf
         _status_ptr[device] = buf.data_ptr()
+        if _binding is not None and device.index is not None:
+            _binding.set_status(device.index, buf.data_ptr())
     return buf
+
+
+def compiled_attention(x):
+    """The compiled module when the differentiable functions can run through it for input `x` (its
+    device's status buffer exists afterwards), else None."""
+    if _binding is not None:
+        i = x.get_device()
+        if i >= 0 and i not in _status_known:
+            _status_buffer(x.device)
+            _status_known.add(i)
+    return _binding
 
 
 def check_device_status(device=None):

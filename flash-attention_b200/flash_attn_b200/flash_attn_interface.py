@@ -5,6 +5,10 @@ The three tensor layouts (packed qkv, q + packed kv, separate q/k/v) share one f
 backward helper; the autograd classes only differ in how they slice their inputs and in which
 gradient buffers they allocate, so gradients of packed inputs are written straight into one
 packed tensor through strided views, as the reference does (:64-68, :100-106).
+
+With the compiled binding the same functions run through one C++ autograd node instead
+(csrc/fa_torch_binding.cpp, AttnNode): a forward + backward at batch 8 x 12 heads x 128 tokens with
+dropout is bound by the host.  The classes here serve return_attn_probs and the ctypes route.
 """
 import torch
 
@@ -172,6 +176,10 @@ def flash_attn_unpadded_qkvpacked_func(qkv, cu_seqlens, max_seqlen, dropout_p, s
     Returns out (total, heads, head_dim); with return_attn_probs also softmax_lse
     (batch, heads, seqlen) fp32 = log-sum-exp of each row of softmax_scale * Q K^T, and S_dmask.
     """
+    native = flash_attn_cuda.compiled_attention(qkv)
+    if native is not None and not return_attn_probs:
+        return native.attn_qkvpacked(qkv, cu_seqlens, int(max_seqlen), float(dropout_p),
+                                     softmax_scale, bool(causal))
     return FlashAttnQKVPackedFunc.apply(qkv, cu_seqlens, max_seqlen, dropout_p, softmax_scale,
                                         causal, return_attn_probs)
 
@@ -183,6 +191,10 @@ def flash_attn_unpadded_kvpacked_func(q, kv, cu_seqlens_q, cu_seqlens_k, max_seq
     Query and key sequences have their own cu_seqlens / max_seqlen; other arguments and returns as
     in flash_attn_unpadded_qkvpacked_func.  With `causal`, key j is visible to query i when
     j <= i (both counted from the start of their sequence)."""
+    native = flash_attn_cuda.compiled_attention(q)
+    if native is not None and not return_attn_probs:
+        return native.attn_kvpacked(q, kv, cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q), int(max_seqlen_k),
+                                    float(dropout_p), softmax_scale, bool(causal))
     return FlashAttnKVPackedFunc.apply(q, kv, cu_seqlens_q, cu_seqlens_k, max_seqlen_q,
                                        max_seqlen_k, dropout_p, softmax_scale, causal,
                                        return_attn_probs)
@@ -192,6 +204,10 @@ def flash_attn_unpadded_func(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, 
                              dropout_p, softmax_scale=None, causal=False, return_attn_probs=False):
     """Variable-length attention with separate q (total_q, heads, d) and k, v (total_k, heads, d).
     Arguments and returns as in flash_attn_unpadded_kvpacked_func."""
+    native = flash_attn_cuda.compiled_attention(q)
+    if native is not None and not return_attn_probs:
+        return native.attn(q, k, v, cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q), int(max_seqlen_k),
+                           float(dropout_p), softmax_scale, bool(causal))
     return FlashAttnFunc.apply(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k,
                                dropout_p, softmax_scale, causal, return_attn_probs)
 

@@ -1,0 +1,69 @@
+"""The C++ autograd node behind the functional API and the Python autograd classes give the same outputs,
+the same gradients and leave the generator in the same place."""
+import pytest
+import torch
+
+from tests import _util as U
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("layout,p,only_kv", [("qkv", 0.0, False), ("qkv", 0.2, False), ("kv", 0.2, True),
+                                              ("separate", 0.1, False), ("sparse", 0.1, False)])
+def test_native_node_matches_the_python_classes(layout, p, only_kv):
+    from flash_attn_b200 import flash_attn_cuda as fc
+    from flash_attn_b200 import flash_attn_interface as fi
+    from flash_attn_b200.flash_blocksparse_attn_interface import flash_blocksparse_attn_func
+    if fc.binding_in_use() != "compiled":
+        pytest.skip("compiled binding not built")
+    sq = [150, 1, 77]
+    sk = sq if layout in ("qkv", "sparse") else [260, 40, 5]
+    q, k, v, dout, cu_q, cu_k = U.make_varlen(sq, sk, 2, 64, torch.float16, seed=41)
+    mq, mk = max(sq), max(sk)
+    block = torch.ones(16, 1, dtype=torch.int32, device="cuda")
+
+    def run():
+        torch.cuda.manual_seed(17)
+        if layout in ("qkv", "sparse"):
+            x = [torch.stack([q, k, v], dim=1)]
+        elif layout == "kv":
+            x = [q.clone(), torch.stack([k, v], dim=1)]
+        else:
+            x = [q.clone(), k.clone(), v.clone()]
+        for i, t in enumerate(x):
+            t.requires_grad_(not (only_kv and i == 0))
+        if layout == "qkv":
+            out = fi.flash_attn_unpadded_qkvpacked_func(x[0], cu_q, mq, p, causal=True)
+        elif layout == "sparse":
+            out = flash_blocksparse_attn_func(x[0], cu_q, block, p, mq)
+        elif layout == "kv":
+            out = fi.flash_attn_unpadded_kvpacked_func(*x, cu_q, cu_k, mq, mk, p)
+        else:
+            out = fi.flash_attn_unpadded_func(*x, cu_q, cu_k, mq, mk, p, softmax_scale=0.2)
+        between = torch.rand(1, device="cuda")  # the mask of the backward is the forward's all the same
+        out.backward(dout)
+        return out.detach(), [t.grad for t in x], between, torch.rand(1, device="cuda")
+
+    fc.options.deterministic = True
+    try:
+        a = run()
+        saved, fc._binding = fc._binding, None
+        try:
+            b = run()
+        finally:
+            fc._binding = saved
+    finally:
+        fc.options.deterministic = False
+    assert torch.equal(a[0], b[0]) and torch.equal(a[2], b[2]) and torch.equal(a[3], b[3])
+    for x, y in zip(a[1], b[1]):
+        assert (x is None and y is None) or torch.equal(x, y)
+
+
+def test_backward_twice_is_refused():
+    from flash_attn_b200.flash_attn_interface import flash_attn_unpadded_qkvpacked_func
+    q, k, v, dout, cu, _ = U.make_varlen([33], [33], 1, 64, torch.float16, seed=42)
+    qkv = torch.stack([q, k, v], dim=1).requires_grad_()
+    out = flash_attn_unpadded_qkvpacked_func(qkv, cu, 33, 0.0)
+    out.backward(dout)
+    with pytest.raises(RuntimeError, match="second time"):
+        out.backward(dout)
