@@ -171,8 +171,8 @@ void fill_dropout(const fa_fwd_params* p, fa::KernelArgs* a) {
 }
 
 // Block-sparse: check the scratch, build the block-visit table on the stream, point the kernel
-// arguments at it.
-int setup_blocksparse(const fa_fwd_params* p, fa::KernelArgs* a, cudaStream_t stream) {
+// arguments at it.  `forward`: also zero the rows of o that no attention CTA writes.
+int setup_blocksparse(const fa_fwd_params* p, fa::KernelArgs* a, bool forward, cudaStream_t stream) {
   const int nk = p->blockmask_rows;
   const int nr = p->blockmask_cols;
   FA_REQUIRE(nk >= round_up(p->max_seqlen_k, 256) / 256, "blockmask has too few key-block rows");
@@ -185,7 +185,11 @@ int setup_blocksparse(const fa_fwd_params* p, fa::KernelArgs* a, cudaStream_t st
     return fail(FA_ERR_WORKSPACE, "bs_workspace must hold " + std::to_string(need) + " bytes");
   FA_REQUIRE(nk <= 4096, "block-sparse attention supports at most 4096 key blocks");
   int32_t* table = static_cast<int32_t*>(p->bs_workspace);
-  FA_CUDA(fa::launch_bs_table(table, p->blockmask, p->cu_seqlens_q, p->cu_seqlens_k, p->batch, nk, nr, stream));
+  // a caller with its own row stride keeps what lies between its rows
+  const int64_t row = static_cast<int64_t>(p->heads) * p->head_dim;
+  const bool zero = forward && p->o_head_stride == p->head_dim && p->o_row_stride == row;
+  FA_CUDA(fa::launch_bs_table(table, p->blockmask, p->cu_seqlens_q, p->cu_seqlens_k, p->batch, nk, nr,
+                              zero ? p->o : nullptr, row * 2, p->total_q, p->max_seqlen_q, stream));
   a->bs_iter = table;
   a->bs_kblocks = nk;
   a->bs_rows16 = nr;
@@ -260,6 +264,20 @@ int fa_rotary_qkv(const void* qkv, void* out, const float* cos_table, const floa
   return FA_OK;
 }
 
+int fa_convert_blockmask(const void* layout, int32_t elem_bytes, int32_t is_float, int64_t row_stride,
+                         int64_t col_stride, int32_t rows, int32_t cols, int32_t causal, int32_t* out,
+                         void* cuda_stream) {
+  FA_REQUIRE(rows >= 0 && cols >= 0, "negative size");
+  if (rows == 0 || cols == 0) return FA_OK;
+  FA_REQUIRE(layout && out, "layout and out must be non-null");
+  FA_REQUIRE(elem_bytes == 1 || elem_bytes == 2 || elem_bytes == 4 || elem_bytes == 8,
+             "layout elements must have 1, 2, 4 or 8 bytes");
+  FA_REQUIRE(rows < (1 << 24) && cols < (1 << 20), "layout too large");
+  FA_CUDA(fa::launch_convert_blockmask(out, layout, elem_bytes, is_float != 0, row_stride, col_stride, rows, cols,
+                                       causal != 0, static_cast<cudaStream_t>(cuda_stream)));
+  return FA_OK;
+}
+
 const char* fa_status_string(int status) {
   switch (status) {
     case FA_OK: return "ok";
@@ -318,7 +336,7 @@ int fa_fwd(const fa_fwd_params* p, void* cuda_stream) {
   std::memset(&l, 0, sizeof(l));
   fill_args(p, &l.args);
   if (p->blockmask)
-    if (int rc = setup_blocksparse(p, &l.args, static_cast<cudaStream_t>(cuda_stream))) return rc;
+    if (int rc = setup_blocksparse(p, &l.args, true, static_cast<cudaStream_t>(cuda_stream))) return rc;
   l.dpad = p->head_dim <= 64 ? 64 : 128;
   l.is_bf16 = p->is_bf16 != 0;
   l.is_causal = p->is_causal != 0;
@@ -347,7 +365,7 @@ int fa_debug_dropout_mask(uint8_t* mask_out, int32_t batch_idx, int32_t head_idx
   std::memset(&a, 0, sizeof(a));
   fill_dropout(p, &a);
   if (p->blockmask)
-    if (int rc = setup_blocksparse(p, &a, static_cast<cudaStream_t>(cuda_stream))) return rc;
+    if (int rc = setup_blocksparse(p, &a, false, static_cast<cudaStream_t>(cuda_stream))) return rc;
   FA_CUDA(fa::launch_dropout_mask(mask_out, batch_idx, head_idx, a.drop, p->is_causal != 0, seqlen_q,
                                   seqlen_k, a.bs_iter, a.bs_kblocks, a.bs_rows16,
                                   static_cast<cudaStream_t>(cuda_stream)));
@@ -395,7 +413,7 @@ int run_bwd(const fa_bwd_params* p, float* accum, int stage_mask, bool bind_cont
   std::memset(&l, 0, sizeof(l));
   fill_args(f, &l.args.k);
   if (f->blockmask)
-    if (int rc = setup_blocksparse(f, &l.args.k, stream)) return rc;
+    if (int rc = setup_blocksparse(f, &l.args.k, false, stream)) return rc;
   l.dpad = f->head_dim <= 64 ? 64 : 128;
   l.is_bf16 = f->is_bf16 != 0;
   l.is_causal = f->is_causal != 0;

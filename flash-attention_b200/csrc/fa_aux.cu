@@ -35,41 +35,111 @@ __global__ void dropout_mask_kernel(uint8_t* out, int b, int h, DropoutParams dp
 // reaches a row block at or beyond the sequence's query length
 // (csrc/flash_attn/src/fmha_block_fprop_kernel_1xN.h:90-100, :209, :486); key blocks at or beyond
 // the key length are not visited at all (:88).  table[b][kb][rb] = number of blocks visited
-// before (kb, rb), or -1 when (kb, rb) is not visited.  One CTA per batch entry.
-__global__ void bs_table_kernel(int32_t* table, const int32_t* blockmask, const int32_t* cu_q,
-                                const int32_t* cu_k, int nk, int nr) {
-  extern __shared__ int32_t cnt[];  // nk + 1 entries
-  const int b = blockIdx.x;
+// before (kb, rb), or -1 when (kb, rb) is not visited.
+//
+// One CTA per (key block, batch entry).  It is a few KB of integers, bound by latency: a warp finds the
+// end of a list with coalesced 32-entry reads and a ballot, the CTA's eight warps share the lists in
+// front of its own, and nothing is serial but that sum.  (One CTA per batch entry with a thread per list
+// walked 256 dependent loads: 28 us at 4 x 4096 tokens, 6 us now.)
+constexpr int kTableThreads = 256;
+
+// Length of the visited prefix of one list (all lanes return it).
+__device__ __forceinline__ int visited_prefix(const int32_t* row, int nr, int sq, int lane) {
+  for (int c = 0; c < nr; c += 32) {
+    const int32_t v = c + lane < nr ? row[c + lane] : -1;
+    const unsigned stop = __ballot_sync(0xffffffffu, v < 0 || (v >> 2) * 16 >= sq);
+    if (stop != 0u) return c + __ffs(stop) - 1;
+  }
+  return nr;
+}
+
+// Output rows no attention CTA writes (rows outside every sequence, and rows at or beyond the 256-row
+// tiles that max_seqlen_q covers) are zero in a block-sparse call (fmha_api.cpp:519 starts from
+// o = 0); zeroing the few there are replaces a pass over the whole tensor.
+struct ZeroRows {
+  uint4* o;          // nullptr: nothing to zero
+  int64_t row_vecs;  // 16-byte units per (contiguous) row
+  int32_t total_q, max_q_tiles;  // rows per sequence that the attention grid covers
+};
+
+__device__ __forceinline__ void zero_rows(const ZeroRows& z, int64_t first, int64_t last) {
+  for (int64_t i = first * z.row_vecs + threadIdx.x; i < last * z.row_vecs; i += blockDim.x)
+    z.o[i] = make_uint4(0, 0, 0, 0);
+}
+
+__global__ void __launch_bounds__(kTableThreads)
+bs_table_kernel(int32_t* table, const int32_t* blockmask, const int32_t* cu_q, const int32_t* cu_k, int nk, int nr,
+                int batch, ZeroRows z) {
+  __shared__ int sum[kTableThreads / 32];
+  const int kb = blockIdx.x, b = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sq = cu_q[b + 1] - cu_q[b];
   const int sk = cu_k[b + 1] - cu_k[b];
-  int32_t* tb = table + static_cast<int64_t>(b) * nk * nr;
-  for (int i = threadIdx.x; i < nk * nr; i += blockDim.x) tb[i] = -1;
-  for (int kb = threadIdx.x; kb < nk; kb += blockDim.x) {
-    int c = 0;
-    if (kb * 256 < sk) {
-      const int32_t* row = blockmask + static_cast<int64_t>(kb) * nr;
-      while (c < nr) {
-        const int32_t v = row[c];
-        if (v < 0 || (v >> 2) * 16 >= sq) break;
-        ++c;
-      }
+  if (z.o != nullptr && kb == 0) {
+    if (b == 0) zero_rows(z, 0, min(cu_q[0], z.total_q));
+    zero_rows(z, static_cast<int64_t>(cu_q[b]) + min(sq, z.max_q_tiles), min(cu_q[b + 1], z.total_q));
+    if (b == batch - 1) zero_rows(z, max(cu_q[batch], 0), z.total_q);
+  }
+  int32_t* trow = table + (static_cast<int64_t>(b) * nk + kb) * nr;
+  for (int i = threadIdx.x; i < nr; i += kTableThreads) trow[i] = -1;
+  if (kb * 256 >= sk) return;
+  int before = 0;
+  for (int k = warp; k < kb; k += kTableThreads / 32)
+    before += visited_prefix(blockmask + static_cast<int64_t>(k) * nr, nr, sq, lane);
+  if (lane == 0) sum[warp] = before;
+  __syncthreads();  // also orders the -1 fill before the entries below
+  before = 0;
+#pragma unroll
+  for (int w = 0; w < kTableThreads / 32; ++w) before += sum[w];
+  const int32_t* row = blockmask + static_cast<int64_t>(kb) * nr;
+  const int n = visited_prefix(row, nr, sq, lane);
+  for (int c = threadIdx.x; c < n; c += kTableThreads) {
+    const int rb = row[c] >> 2;
+    if (rb < nr) trow[rb] = before + c;
+  }
+}
+
+// 0/1 layout (nrow, ncol) -> per-column visit lists (flash_blocksparse_attn_interface.py:8-40 of the
+// reference): out[c] lists 4 * r in ascending order for every set (r, c), plus 1 when c is the first set
+// column of row r and plus 2 when it is the last, then -1.  causal drops the blocks that lie entirely
+// above the diagonal first.  One CTA per column; rows are compacted 256 at a time with ballots.  Latency
+// bound like the table above (it replaces two dozen framework launches, 400 us of host time).
+template <typename T>
+__device__ __forceinline__ bool layout_set(const T* m, int64_t row_stride, int64_t col_stride, int r, int c, T value_bits,
+                                           bool causal) {
+  return (m[r * row_stride + c * col_stride] & value_bits) != 0 && !(causal && 256 * c > 16 * r + 15);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kTableThreads)
+convert_blockmask_kernel(int32_t* out, const T* m, int64_t row_stride, int64_t col_stride, int nrow, int ncol,
+                         T value_bits, bool causal) {
+  __shared__ int warp_count[2][kTableThreads / 32];
+  const int c = blockIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int32_t* dst = out + static_cast<int64_t>(c) * nrow;
+  int done = 0, buf = 0;
+  for (int r0 = 0; r0 < nrow; r0 += kTableThreads, buf ^= 1) {
+    const int r = r0 + threadIdx.x;
+    const bool on = r < nrow && layout_set(m, row_stride, col_stride, r, c, value_bits, causal);
+    const unsigned bits = __ballot_sync(0xffffffffu, on);
+    if (lane == 0) warp_count[buf][warp] = __popc(bits);
+    __syncthreads();  // double-buffered counts: one barrier per chunk
+    int pos = done;
+#pragma unroll
+    for (int w = 0; w < kTableThreads / 32; ++w) {
+      const int n = warp_count[buf][w];
+      if (w < warp) pos += n;
+      done += n;
     }
-    cnt[kb + 1] = c;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    cnt[0] = 0;
-    for (int kb = 0; kb < nk; ++kb) cnt[kb + 1] += cnt[kb];
-  }
-  __syncthreads();
-  for (int kb = threadIdx.x; kb < nk; kb += blockDim.x) {
-    const int32_t* row = blockmask + static_cast<int64_t>(kb) * nr;
-    const int n = cnt[kb + 1] - cnt[kb];
-    for (int c = 0; c < n; ++c) {
-      const int rb = row[c] >> 2;
-      if (rb >= 0 && rb < nr) tb[static_cast<int64_t>(kb) * nr + rb] = cnt[kb] + c;
+    if (on) {
+      int first = 0, last = ncol - 1;
+      while (!layout_set(m, row_stride, col_stride, r, first, value_bits, causal)) ++first;  // ends at c at the latest
+      while (!layout_set(m, row_stride, col_stride, r, last, value_bits, causal)) --last;
+      dst[pos + __popc(bits & ((1u << lane) - 1u))] = 4 * r + (first == c ? 1 : 0) + (last == c ? 2 : 0);
     }
   }
+  for (int i = done + threadIdx.x; i < nrow; i += kTableThreads) dst[i] = -1;
 }
 
 // return_softmax output (test aid): s[b, h, i, j] = softmax probability of key j for query i,
@@ -188,8 +258,28 @@ cudaError_t launch_philox_probe(uint32_t* out, int n, unsigned long long seed, u
 }
 
 cudaError_t launch_bs_table(int32_t* table, const int32_t* blockmask, const int32_t* cu_q,
-                            const int32_t* cu_k, int batch, int nk, int nr, cudaStream_t stream) {
-  bs_table_kernel<<<batch, 256, (nk + 1) * sizeof(int32_t), stream>>>(table, blockmask, cu_q, cu_k, nk, nr);
+                            const int32_t* cu_k, int batch, int nk, int nr, void* o, int64_t o_row_bytes,
+                            int total_q, int max_seqlen_q, cudaStream_t stream) {
+  const ZeroRows z{static_cast<uint4*>(o), o_row_bytes / 16, total_q, (max_seqlen_q + 255) / 256 * 256};
+  bs_table_kernel<<<dim3(nk, batch), kTableThreads, 0, stream>>>(table, blockmask, cu_q, cu_k, nk, nr, batch, z);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_convert_blockmask(int32_t* out, const void* layout, int elem_bytes, bool is_float, int64_t row_stride,
+                                     int64_t col_stride, int nrow, int ncol, bool causal, cudaStream_t stream) {
+  if (nrow <= 0 || ncol <= 0) return cudaSuccess;
+  // an element is set when it differs from zero: any bit, without the sign of a floating-point zero
+#define FA_CONVERT(T)                                                                                             \
+  convert_blockmask_kernel<T><<<ncol, kTableThreads, 0, stream>>>(                                                 \
+      out, static_cast<const T*>(layout), row_stride, col_stride, nrow, ncol,                                      \
+      static_cast<T>(is_float ? static_cast<T>(~T(0)) >> 1 : static_cast<T>(~T(0))), causal)
+  switch (elem_bytes) {
+    case 1: FA_CONVERT(uint8_t); break;
+    case 2: FA_CONVERT(uint16_t); break;
+    case 4: FA_CONVERT(uint32_t); break;
+    default: FA_CONVERT(uint64_t); break;
+  }
+#undef FA_CONVERT
   return cudaGetLastError();
 }
 

@@ -75,7 +75,10 @@ cudaError_t launch_sdmask(void* s_out, int64_t s_rows, int64_t s_cols, const voi
 cudaError_t launch_philox_probe(uint32_t* out, int n, unsigned long long seed, unsigned long long offset,
                                 int rounds, int mode, cudaStream_t stream);
 cudaError_t launch_bs_table(int32_t* table, const int32_t* blockmask, const int32_t* cu_q,
-                            const int32_t* cu_k, int batch, int nk, int nr, cudaStream_t stream);
+                            const int32_t* cu_k, int batch, int nk, int nr, void* o, int64_t o_row_bytes,
+                            int total_q, int max_seqlen_q, cudaStream_t stream);
+cudaError_t launch_convert_blockmask(int32_t* out, const void* layout, int elem_bytes, bool is_float, int64_t row_stride,
+                                     int64_t col_stride, int nrow, int ncol, bool causal, cudaStream_t stream);
 cudaError_t launch_dropout_mask(uint8_t* out, int b, int h, const DropoutParams& dp, bool causal,
                                 int sq, int sk, const int32_t* bs_iter, int bs_kblocks,
                                 int bs_rows16, cudaStream_t stream);

@@ -214,9 +214,8 @@ FwdResult run_fwd(const View& q, const View& k, const View& v, const at::TensorO
   c10::cuda::CUDAGuard guard(opts.device());
   const int64_t lse_len = round_up(c.max_q, 16);
   FwdResult r;
-  // the block-sparse entry always starts from o = 0 (:519)
-  r.o = (c.zero_tensors || sparse) ? at::zeros({s.total_q, s.heads, s.d}, opts)
-                                   : at::empty({s.total_q, s.heads, s.d}, opts);
+  // (the library zeroes the rows a block-sparse call leaves out, :519)
+  r.o = c.zero_tensors ? at::zeros({s.total_q, s.heads, s.d}, opts) : at::empty({s.total_q, s.heads, s.d}, opts);
   r.lse = c.zero_tensors
               ? at::full({s.batch, s.heads, lse_len}, -std::numeric_limits<float>::infinity(), opts.dtype(at::kFloat))
               : at::empty({s.batch, s.heads, lse_len}, opts.dtype(at::kFloat));
@@ -499,6 +498,20 @@ at::Tensor attn_sparse_qkvpacked(const at::Tensor& qkv, const at::Tensor& cu, co
   return attention(&qkv, kQkvPacked, cu, cu, max_s, max_s, p_dropout, scale, causal, &blockmask);
 }
 
+// convert_blockmask on a CUDA layout (flash_blocksparse_attn_interface.py)
+at::Tensor convert_blockmask(const at::Tensor& layout, bool causal) {
+  require(layout.is_cuda() && layout.dim() == 2 && !layout.is_complex(), "layout must be a 2-D CUDA tensor of real numbers");
+  c10::cuda::CUDAGuard guard(layout.device());
+  at::AutoDispatchBelowADInplaceOrView below;
+  at::Tensor out = at::empty({layout.size(1), layout.size(0)}, layout.options().dtype(at::kInt));
+  check_rc(fa_convert_blockmask(layout.data_ptr(), static_cast<int32_t>(layout.element_size()),
+                                layout.is_floating_point() ? 1 : 0, layout.stride(0), layout.stride(1),
+                                static_cast<int32_t>(layout.size(0)), static_cast<int32_t>(layout.size(1)),
+                                causal ? 1 : 0, static_cast<int32_t*>(out.data_ptr()),
+                                at::cuda::getCurrentCUDAStream().stream()));
+  return out;
+}
+
 void set_options(bool deterministic, int64_t mask_heads_total, int64_t mask_head_offset) {
   g_deterministic = deterministic;
   g_mask_heads_total = mask_heads_total;
@@ -520,6 +533,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attn_kvpacked", &attn_kvpacked);
   m.def("attn", &attn);
   m.def("attn_sparse_qkvpacked", &attn_sparse_qkvpacked);
+  m.def("convert_blockmask", &convert_blockmask);
   m.def("set_options", &set_options);
   m.def("set_status", &set_status);
 }

@@ -30,6 +30,7 @@ EXPORTED_SYMBOLS = (
     "fa_gather_rows",
     "fa_scatter_rows",
     "fa_rotary_qkv",
+    "fa_convert_blockmask",
     "fa_status_string",
     "fa_last_error",
     "fa_device_supported",
@@ -143,6 +144,10 @@ def _load():
                                   ctypes.c_int64, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,
                                   ctypes.c_int32, ctypes.c_int32, ctypes.c_void_p]
     lib.fa_rotary_qkv.restype = ctypes.c_int
+    lib.fa_convert_blockmask.argtypes = [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32, ctypes.c_int64,
+                                         ctypes.c_int64, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,
+                                         ctypes.c_void_p, ctypes.c_void_p]
+    lib.fa_convert_blockmask.restype = ctypes.c_int
     lib.fa_status_string.argtypes = [ctypes.c_int]
     lib.fa_status_string.restype = ctypes.c_char_p
     lib.fa_last_error.argtypes = []

@@ -22,6 +22,10 @@ def convert_blockmask(blockmask, causal):
     iteration index follows the visit lists alone (csrc/flash_attn/src/
     fmha_block_fprop_kernel_1xN.h:205-232 takes its loop bounds from the block mask, with no
     causal start row)."""
+    if blockmask.is_cuda and blockmask.dim() == 2 and not blockmask.is_complex():
+        native = flash_attn_cuda.compiled_attention(blockmask)
+        if native is not None:   # one launch instead of two dozen
+            return native.convert_blockmask(blockmask, bool(causal))
     mask = blockmask != 0
     nrow, ncol = mask.shape
     device = mask.device

@@ -114,7 +114,8 @@ typedef struct fa_bwd_params {
 } fa_bwd_params;
 
 /* mha_fwd (csrc/flash_attn/fmha_api.cpp:173-299) and, with blockmask != NULL, mha_fwd_block
- * (:451-573).  Writes o and softmax_lse. */
+ * (:451-573).  Writes o and softmax_lse.  A block-sparse call with a contiguous o also zeroes the rows
+ * of o that lie outside the sequences (the reference starts from o = 0, :519). */
 int fa_fwd(const fa_fwd_params* params, void* cuda_stream);
 
 /* mha_bwd (csrc/flash_attn/fmha_api.cpp:302-449) and, with blockmask != NULL, mha_bwd_block
@@ -206,6 +207,16 @@ int fa_scatter_rows(const void* src, const int64_t* indices, void* dst, int64_t 
 int fa_rotary_qkv(const void* qkv, void* out, const float* cos_table, const float* sin_table,
                   int64_t rows, int32_t seqlen, int32_t heads, int32_t head_dim, int32_t is_bf16,
                   int32_t conjugate, void* cuda_stream);
+
+/* 0/1 layout over (16-row query blocks, 256-column key blocks) -> the converted block mask of
+ * fa_fwd_params: out[c] (one row of `rows` int32 per layout column) lists 4 * r in ascending order for
+ * every non-zero layout[r][c], plus 1 / plus 2 when c is the first / last non-zero column of row r,
+ * followed by -1.  Replaces flash_attn/flash_blocksparse_attn_interface.py:8-40 (convert_blockmask).
+ * Elements of `elem_bytes` bytes (is_float != 0: floating point), strides in elements.  causal != 0
+ * first removes the blocks entirely above the diagonal. */
+int fa_convert_blockmask(const void* layout, int32_t elem_bytes, int32_t is_float, int64_t row_stride,
+                         int64_t col_stride, int32_t rows, int32_t cols, int32_t causal, int32_t* out,
+                         void* cuda_stream);
 
 const char* fa_status_string(int status);
 const char* fa_last_error(void);

@@ -1,0 +1,43 @@
+"""The layout conversion and block-visit table kernels: list lengths around the 32-entry and 256-row steps they work
+in, every element type, strided layouts, and the zero rows outside the sequences."""
+import pytest
+import torch
+
+from tests import _util as U
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("rows,cols,density", [(1, 1, 1.0), (16, 1, 0.5), (31, 3, 0.5), (256, 16, 0.25), (257, 17, 0.9),
+                                               (1024, 64, 0.05), (520, 33, 0.0)])
+def test_convert_blockmask_matches_the_framework_version(rows, cols, density, causal):
+    from flash_attn_b200.flash_blocksparse_attn_interface import convert_blockmask
+    torch.manual_seed(rows + cols)
+    layout = (torch.rand(rows, cols) < density).to(torch.int32)
+    want = convert_blockmask(layout, causal)   # CPU: framework operations
+    for dt in (torch.bool, torch.int32, torch.int64, torch.float32, torch.float16, torch.uint8):
+        assert torch.equal(convert_blockmask(layout.to(dt).cuda(), causal).cpu(), want), dt
+    wide = torch.full((rows, 2 * cols), -0.0, device="cuda")
+    wide[:, ::2] = layout.cuda().float() * -3.0
+    assert torch.equal(convert_blockmask(wide[:, ::2], causal).cpu(), want)
+
+
+@pytest.mark.parametrize("lens", [[1, 256, 257], [500, 31], [1000]])
+def test_rows_outside_the_sequences_are_zero(lens):
+    """A token buffer with rows in front of the first and behind the last sequence."""
+    from flash_attn_b200 import flash_attn_cuda as fc
+    from flash_attn_b200.flash_blocksparse_attn_interface import convert_blockmask
+    s = max(lens)
+    kb = (s + 255) // 256
+    torch.manual_seed(1)
+    layout = ((torch.rand(kb, kb) < 0.5) | torch.eye(kb, dtype=torch.bool)).repeat_interleave(16, dim=0).cuda()
+    conv = convert_blockmask(layout, False)
+    q, k, v, _, cu, _ = U.make_varlen(lens, lens, 2, 64, torch.float16, seed=5)
+    pad = [torch.cat([torch.full_like(t[:1], 3.0).expand(7, -1, -1), t, t[:1].expand(9, -1, -1)]) for t in (q, k, v)]
+    garbage = torch.full((1 << 20,), float("nan"), device="cuda", dtype=torch.float16)  # what the allocator hands out next
+    del garbage
+    out = fc.fwd_block(*pad, cu + 7, cu + 7, conv, s, s, 0.0, 0.125, False, False, None)[0]
+    want = fc.fwd_block(q, k, v, cu, cu, conv, s, s, 0.0, 0.125, False, False, None)[0]
+    assert torch.equal(out[7:7 + sum(lens)], want)
+    assert not out[:7].any() and not out[7 + sum(lens):].any()
