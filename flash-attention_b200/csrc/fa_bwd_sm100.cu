@@ -142,7 +142,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   __shared__ BwdShared sh;
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // known to be the same in all lanes
   const int lane = tid & 31;
   const int b = blockIdx.z;
   const int h = blockIdx.y;
@@ -278,29 +278,29 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   constexpr uint32_t idesc_s = make_idesc(BF16, false, false, 128, 128);   // Q K^T, dO V^T
   constexpr uint32_t idesc_tt = make_idesc(BF16, true, true, 128, D);      // P~^T dO, dS^T Q
   constexpr uint32_t idesc_dq = make_idesc(BF16, false, true, 128, D);     // dS K
+  // Called by one elected lane of an issuing warp whose lanes all run the surrounding loop (see mma_ss).
   auto issue_kk = [&](uint32_t dst, uint32_t a_base, uint32_t b_base) {  // both K-major, K = D
+    const uint64_t da = make_smem_desc(a_base, 16, 1024), db = make_smem_desc(b_base, 16, 1024);
 #pragma unroll
     for (int ks = 0; ks < D / 16; ++ks) {
       const uint32_t off = (ks >> 2) * 16384 + (ks & 3) * 32;
-      mma_ss(dst, make_smem_desc(a_base + off, 16, 1024), make_smem_desc(b_base + off, 16, 1024),
-             idesc_s, ks > 0);
+      mma_ss(dst, desc_at(da, off), desc_at(db, off), idesc_s, ks > 0);
     }
   };
   auto issue_tt = [&](uint32_t dst, uint32_t a_base, uint32_t b_base, bool acc) {
     // A = [q][kv] read as M = kv (MN-major); B = [q][d] read as N = d (MN-major); K = q rows
+    const uint64_t da = make_smem_desc(a_base, 16384, 1024), db = make_smem_desc(b_base, 16384, 1024);
 #pragma unroll
-    for (int ks = 0; ks < kBM / 16; ++ks) {
-      mma_ss(dst, make_smem_desc(a_base + ks * 2048, 16384, 1024),
-             make_smem_desc(b_base + ks * 2048, 16384, 1024), idesc_tt, acc || ks > 0);
-    }
+    for (int ks = 0; ks < kBM / 16; ++ks)
+      mma_ss(dst, desc_at(da, ks * 2048), desc_at(db, ks * 2048), idesc_tt, acc || ks > 0);
   };
   auto issue_dq = [&](uint32_t dst, uint32_t a_base, uint32_t b_base) {
     // A = dS [q][kv] K-major; B = K [kv][d] read as N = d (MN-major); K = kv
+    const uint64_t da = make_smem_desc(a_base, 16, 1024), db = make_smem_desc(b_base, 16384, 1024);
 #pragma unroll
     for (int ks = 0; ks < kBN / 16; ++ks) {
       const uint32_t off = (ks >> 2) * 16384 + (ks & 3) * 32;
-      mma_ss(dst, make_smem_desc(a_base + off, 16, 1024),
-             make_smem_desc(b_base + ks * 2048, 16384, 1024), idesc_dq, ks > 0);
+      mma_ss(dst, desc_at(da, off), desc_at(db, ks * 2048), idesc_dq, ks > 0);
     }
   };
   const uint32_t tS_ = tmem + Cfg::kTmemS, tDP_ = tmem + Cfg::kTmemDP;
@@ -308,9 +308,10 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   const uint32_t tDS_ = tmem + Cfg::kTmemDS;
   auto issue_dq_t = [&](uint32_t dst, uint32_t a_tmem, uint32_t b_base) {
     // A = dS from tensor memory (16 keys = 8 columns per step); B = K [kv][d] read as N = d; K = kv
+    const uint64_t db = make_smem_desc(b_base, 16384, 1024);
 #pragma unroll
     for (int ks = 0; ks < kBN / 16; ++ks)
-      mma_ts(dst, a_tmem + ks * 8, make_smem_desc(b_base + ks * 2048, 16384, 1024), idesc_dq, ks > 0);
+      mma_ts(dst, a_tmem + ks * 8, desc_at(db, ks * 2048), idesc_dq, ks > 0);
   };
 
   if (warp >= 12) {
@@ -361,10 +362,10 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           }
         }
       }
-    } else if (warp == 13 && lane == 0) {
+    } else if (warp == 13) {
       // -------------------------------------------------------------- MMA issuer 1
-      bool ok = mbar_wait(smem_u32(&sh.kv_full), 0, abort_flag);
-      if (ok) ok = mbar_wait(smem_u32(&sh.q_full[0]), 0, abort_flag);
+      bool ok = mbar_wait_warp(smem_u32(&sh.kv_full), 0, abort_flag);
+      if (ok) ok = mbar_wait_warp(smem_u32(&sh.q_full[0]), 0, abort_flag);
       if constexpr (Cfg::kTwoPhase) {
         // d = 128: every product, issued by this thread in the order
         //   dV(t) | dK(t), dQ(t) | S(t+1) | dP(t+1)
@@ -374,57 +375,69 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         // out of the columns it shares with dP.
         if (ok) {
           tc_fence_after();
-          issue_kk(tS_, smem_q, smem_k);
-          mma_commit(smem_u32(&sh.s_full));
-          ok = mbar_wait(smem_u32(&sh.do_full), 0, abort_flag);
+          if (elect_one()) {
+            issue_kk(tS_, smem_q, smem_k);
+            mma_commit(smem_u32(&sh.s_full));
+          }
+          ok = mbar_wait_warp(smem_u32(&sh.do_full), 0, abort_flag);
         }
         if (ok) {
           tc_fence_after();
-          issue_kk(tDP_, smem_do, smem_v);
-          mma_commit(smem_u32(&sh.sdp_full));
+          if (elect_one()) {
+            issue_kk(tDP_, smem_do, smem_v);
+            mma_commit(smem_u32(&sh.sdp_full));
+          }
         }
         FA_PROF_DECL
         for (int t = 0; t < nm && ok; ++t) {
           const bool has_next = t + 1 < nm;
           FA_PROF(0)
-          ok = mbar_wait(smem_u32(&sh.p_ready), t & 1, abort_flag);
+          ok = mbar_wait_warp(smem_u32(&sh.p_ready), t & 1, abort_flag);
           if (!ok) break;
           FA_PROF(1)
           tc_fence_after();
-          issue_tt(tDV_, smem_p, smem_do, t > 0);
-          mma_commit(smem_u32(&sh.pds_free));
-          mma_commit(smem_u32(&sh.do_empty));
+          if (elect_one()) {
+            issue_tt(tDV_, smem_p, smem_do, t > 0);
+            mma_commit(smem_u32(&sh.pds_free));
+            mma_commit(smem_u32(&sh.do_empty));
+          }
           FA_STAMP(t, 11)
-          ok = mbar_wait(smem_u32(&sh.pds_ready), t & 1, abort_flag);
+          ok = mbar_wait_warp(smem_u32(&sh.pds_ready), t & 1, abort_flag);
           if (!ok) break;
           FA_PROF(2)
           FA_STAMP(t, 9)
           tc_fence_after();
-          issue_tt(tDK_, smem_ds, smem_q, t > 0);
-          mma_commit(smem_u32(&sh.q_empty[0]));
-          issue_dq(tDQ_, smem_ds, smem_k);
-          mma_commit(smem_u32(&sh.dq_full));
-          mma_commit(smem_u32(&sh.ds_free));
+          if (elect_one()) {
+            issue_tt(tDK_, smem_ds, smem_q, t > 0);
+            mma_commit(smem_u32(&sh.q_empty[0]));
+            issue_dq(tDQ_, smem_ds, smem_k);
+            mma_commit(smem_u32(&sh.dq_full));
+            mma_commit(smem_u32(&sh.ds_free));
+          }
           FA_STAMP(t, 10)
           FA_PROF(3)
           if (has_next) {
             FA_STAMP(t, 5)
-            ok = mbar_wait(smem_u32(&sh.q_full[0]), (t + 1) & 1, abort_flag);
+            ok = mbar_wait_warp(smem_u32(&sh.q_full[0]), (t + 1) & 1, abort_flag);
             FA_STAMP(t, 6)
-            if (ok) ok = mbar_wait(smem_u32(&sh.sdp_consumed), t & 1, abort_flag);
+            if (ok) ok = mbar_wait_warp(smem_u32(&sh.sdp_consumed), t & 1, abort_flag);
             if (!ok) break;
             tc_fence_after();
-            issue_kk(tS_, smem_q, smem_k);
-            mma_commit(smem_u32(&sh.s_full));
+            if (elect_one()) {
+              issue_kk(tS_, smem_q, smem_k);
+              mma_commit(smem_u32(&sh.s_full));
+            }
             FA_STAMP(t, 12)
             FA_PROF(4)
-            ok = mbar_wait(smem_u32(&sh.do_full), (t + 1) & 1, abort_flag);
-            if (ok) ok = mbar_wait(smem_u32(&sh.dq_consumed), t & 1, abort_flag);
+            ok = mbar_wait_warp(smem_u32(&sh.do_full), (t + 1) & 1, abort_flag);
+            if (ok) ok = mbar_wait_warp(smem_u32(&sh.dq_consumed), t & 1, abort_flag);
             if (!ok) break;
             FA_STAMP(t, 7)
             tc_fence_after();
-            issue_kk(tDP_, smem_do, smem_v);
-            mma_commit(smem_u32(&sh.sdp_full));
+            if (elect_one()) {
+              issue_kk(tDP_, smem_do, smem_v);
+              mma_commit(smem_u32(&sh.sdp_full));
+            }
             FA_STAMP(t, 8)
             FA_PROF(5)
           }
@@ -434,9 +447,11 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         // d = 64: S, dP and dQ (dV, dK go through issuer 2)
         if (ok) {
           tc_fence_after();
-          issue_kk(tS_, smem_q, smem_k);
-          issue_kk(tDP_, smem_do, smem_v);
-          mma_commit(smem_u32(&sh.sdp_full));
+          if (elect_one()) {
+            issue_kk(tS_, smem_q, smem_k);
+            issue_kk(tDP_, smem_do, smem_v);
+            mma_commit(smem_u32(&sh.sdp_full));
+          }
         }
         FA_PROF_DECL
         for (int t = 0; t < nm && ok; ++t) {
@@ -445,41 +460,45 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           FA_PROF(0)
           if (has_next) {
             FA_STAMP(t, 5)
-            ok = mbar_wait(smem_u32(&sh.q_full[sn]), ((t + 1) / Cfg::kQStages) & 1, abort_flag);
+            ok = mbar_wait_warp(smem_u32(&sh.q_full[sn]), ((t + 1) / Cfg::kQStages) & 1, abort_flag);
             FA_STAMP(t, 6)
-            if (ok) ok = mbar_wait(smem_u32(&sh.sdp_consumed), t & 1, abort_flag);
+            if (ok) ok = mbar_wait_warp(smem_u32(&sh.sdp_consumed), t & 1, abort_flag);
             FA_STAMP(t, 7)
             if (!ok) break;
             FA_PROF(1)
             tc_fence_after();
-            issue_kk(tS_, smem_q + sn * Cfg::kTileBytes, smem_k);
-            issue_kk(tDP_, smem_do + sn * Cfg::kTileBytes, smem_v);
-            mma_commit(smem_u32(&sh.sdp_full));
+            if (elect_one()) {
+              issue_kk(tS_, smem_q + sn * Cfg::kTileBytes, smem_k);
+              issue_kk(tDP_, smem_do + sn * Cfg::kTileBytes, smem_v);
+              mma_commit(smem_u32(&sh.sdp_full));
+            }
             FA_PROF(2)
             FA_STAMP(t, 8)
           }
-          ok = mbar_wait(smem_u32(&sh.pds_ready), t & 1, abort_flag);
+          ok = mbar_wait_warp(smem_u32(&sh.pds_ready), t & 1, abort_flag);
           if (!ok) break;
           FA_PROF(3)
           FA_STAMP(t, 9)
           tc_fence_after();
           if (t > 0) {
-            ok = mbar_wait(smem_u32(&sh.dq_consumed), (t - 1) & 1, abort_flag);
+            ok = mbar_wait_warp(smem_u32(&sh.dq_consumed), (t - 1) & 1, abort_flag);
             if (!ok) break;
             tc_fence_after();
           }
           FA_PROF(4)
           // its tile is read out of tensor memory while dV / dK are still running
-          if constexpr (kDsInTmem) issue_dq_t(tDQ_, tDS_, smem_k);
-          else issue_dq(tDQ_, smem_ds, smem_k);
-          mma_commit(smem_u32(&sh.dq_full));
-          FA_STAMP(t, 10)
-          mma_commit(smem_u32(&sh.pds_free));
+          if (elect_one()) {
+            if constexpr (kDsInTmem) issue_dq_t(tDQ_, tDS_, smem_k);
+            else issue_dq(tDQ_, smem_ds, smem_k);
+            mma_commit(smem_u32(&sh.dq_full));
+            FA_STAMP(t, 10)
+            mma_commit(smem_u32(&sh.pds_free));
+          }
           FA_PROF(5)
         }
         FA_PROF_FLUSH(16, nm)
       }
-    } else if (warp == 14 && lane == 0 && Cfg::kDualIssue) {
+    } else if (warp == 14 && Cfg::kDualIssue) {
       // -------------------------------------------------------------- MMA issuer 2: dV
       // dV and dK have a thread each: an issuing thread gets an instruction out every ~130 clk
       // (it shares its scheduler with two compute warps), so the 16 instructions of the two products
@@ -489,30 +508,34 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       for (int t = 0; t < nm && ok; ++t) {
         const int s = t % Cfg::kQStages;
         FA_PROF(0)
-        ok = mbar_wait(smem_u32(&sh.pds_ready), t & 1, abort_flag);
+        ok = mbar_wait_warp(smem_u32(&sh.pds_ready), t & 1, abort_flag);
         if (!ok) break;
         FA_PROF(1)
         FA_STAMP(t, 11)
         tc_fence_after();
-        issue_tt(tDV_, smem_p, smem_do + s * Cfg::kTileBytes, t > 0);
-        FA_STAMP(t, 12)
-        mma_commit(smem_u32(&sh.pds_free));
-        mma_commit(smem_u32(&sh.q_empty[s]));
+        if (elect_one()) {
+          issue_tt(tDV_, smem_p, smem_do + s * Cfg::kTileBytes, t > 0);
+          FA_STAMP(t, 12)
+          mma_commit(smem_u32(&sh.pds_free));
+          mma_commit(smem_u32(&sh.q_empty[s]));
+        }
         FA_PROF(2)
       }
       FA_PROF_FLUSH(24, nm)
-    } else if (warp == 15 && lane == 0 && Cfg::kDualIssue) {
+    } else if (warp == 15 && Cfg::kDualIssue) {
       // -------------------------------------------------------------- MMA issuer 3: dK
       bool ok = true;
       for (int t = 0; t < nm && ok; ++t) {
         const int s = t % Cfg::kQStages;
-        ok = mbar_wait(smem_u32(&sh.pds_ready), t & 1, abort_flag);
+        ok = mbar_wait_warp(smem_u32(&sh.pds_ready), t & 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
-        issue_tt(tDK_, smem_ds, smem_q + s * Cfg::kTileBytes, t > 0);
-        FA_STAMP(t, 13)
-        mma_commit(smem_u32(&sh.pds_free));
-        mma_commit(smem_u32(&sh.q_empty[s]));
+        if (elect_one()) {
+          issue_tt(tDK_, smem_ds, smem_q + s * Cfg::kTileBytes, t > 0);
+          FA_STAMP(t, 13)
+          mma_commit(smem_u32(&sh.pds_free));
+          mma_commit(smem_u32(&sh.q_empty[s]));
+        }
       }
     }
   } else if (warp < 8) {

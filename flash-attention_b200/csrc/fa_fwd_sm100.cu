@@ -150,7 +150,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   __shared__ int tile_count;
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // known to be the same in all lanes
   const int lane = tid & 31;
 
   const int b = blockIdx.z;
@@ -284,43 +284,49 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     }
   } else if (warp == 9) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    // all 32 lanes run the loop, one elected lane issues (see mma_ss)
+    {
       constexpr uint32_t idesc_qk = make_idesc(BF16, false, false, kBlockM, kBlockN);
       constexpr uint32_t idesc_pv = make_idesc(BF16, false, true, kBlockM, D);
-      const uint32_t tS[2] = {tmem + Cfg::kTmemS0, tmem + Cfg::kTmemS1};
-      const uint32_t tO[2] = {tmem + Cfg::kTmemO0, tmem + Cfg::kTmemO1};
-      const uint32_t tP[2] = {tmem + Cfg::kTmemP0, tmem + Cfg::kTmemP1};
+      const uint64_t desc_q = make_smem_desc(smem_q, 16, 1024);
+      const uint64_t desc_k = make_smem_desc(smem_k, 16, 1024);
+      const uint64_t desc_v = make_smem_desc(smem_v, 16384, 1024);
       auto issue_qk = [&](int g, int stage) {
-        const uint32_t qa = smem_q + g * Cfg::kTileBytes;
-        const uint32_t ka = smem_k + stage * Cfg::kTileBytes;
+        const uint64_t qa = desc_at(desc_q, g * Cfg::kTileBytes);
+        const uint64_t ka = desc_at(desc_k, stage * Cfg::kTileBytes);
+        const uint32_t tS = tmem + (g == 0 ? Cfg::kTmemS0 : Cfg::kTmemS1);
+        if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks) {
-          const uint32_t off = (ks >> 2) * 16384 + (ks & 3) * 32;
-          mma_ss(tS[g], make_smem_desc(qa + off, 16, 1024), make_smem_desc(ka + off, 16, 1024),
-                 idesc_qk, ks > 0);
+          for (int ks = 0; ks < D / 16; ++ks) {
+            const uint32_t off = (ks >> 2) * 16384 + (ks & 3) * 32;
+            mma_ss(tS, desc_at(qa, off), desc_at(ka, off), idesc_qk, ks > 0);
+          }
+          mma_commit(smem_u32(&sh.s_full[g]));
         }
-        mma_commit(smem_u32(&sh.s_full[g]));
       };
       auto issue_pv = [&](int g, int stage, bool accumulate) {
-        const uint32_t va = smem_v + stage * Cfg::kTileBytes;
+        const uint64_t va = desc_at(desc_v, stage * Cfg::kTileBytes);
+        const uint32_t tO = tmem + (g == 0 ? Cfg::kTmemO0 : Cfg::kTmemO1);
+        const uint32_t tP = tmem + (g == 0 ? Cfg::kTmemP0 : Cfg::kTmemP1);
+        if (elect_one()) {
 #pragma unroll
-        for (int ks = 0; ks < kBlockN / 16; ++ks) {
-          mma_ts(tO[g], tP[g] + ks * 8, make_smem_desc(va + ks * 2048, 16384, 1024), idesc_pv,
-                 accumulate || ks > 0);
+          for (int ks = 0; ks < kBlockN / 16; ++ks)
+            mma_ts(tO, tP + ks * 8, desc_at(va, ks * 2048), idesc_pv, accumulate || ks > 0);
+          mma_commit(smem_u32(&sh.o_full[g]));
         }
-        mma_commit(smem_u32(&sh.o_full[g]));
       };
 
       bool ok = true;
       for (int g = 0; g < 2 && ok; ++g)
-        if (n_tiles[g] > 0) ok = mbar_wait(smem_u32(&sh.q_full[g]), 0, abort_flag);
+        if (n_tiles[g] > 0) ok = mbar_wait_warp(smem_u32(&sh.q_full[g]), 0, abort_flag);
       if (ok && n_max > 0) {
-        ok = mbar_wait(smem_u32(&sh.k_full[0]), 0, abort_flag);
+        ok = mbar_wait_warp(smem_u32(&sh.k_full[0]), 0, abort_flag);
         if (ok) {
           tc_fence_after();
+#pragma unroll
           for (int g = 0; g < 2; ++g)
             if (n_tiles[g] > 0) issue_qk(g, 0);
-          mma_commit(smem_u32(&sh.k_empty[0]));
+          if (elect_one()) mma_commit(smem_u32(&sh.k_empty[0]));
         }
       }
       FA_PROF_DECL
@@ -329,73 +335,83 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         const int sn = (j + 1) % Cfg::kStages;
         const bool has_next = j + 1 < n_max;
         FA_PROF(0)
-        if (!Cfg::kSeparateP) ok = mbar_wait(smem_u32(&sh.v_full[s]), (j / Cfg::kStages) & 1, abort_flag);
+        if (!Cfg::kSeparateP) ok = mbar_wait_warp(smem_u32(&sh.v_full[s]), (j / Cfg::kStages) & 1, abort_flag);
         if (ok && has_next)
-          ok = mbar_wait(smem_u32(&sh.k_full[sn]), ((j + 1) / Cfg::kStages) & 1, abort_flag);
+          ok = mbar_wait_warp(smem_u32(&sh.k_full[sn]), ((j + 1) / Cfg::kStages) & 1, abort_flag);
         if (!ok) break;
         FA_PROF(1)
         if constexpr (Cfg::kSeparateP) {
           // this warp issues only the score products; warp 10 issues P*V
+#pragma unroll
           for (int g = 0; g < 2; ++g) {
-            if (j + 1 < n_tiles[g]) {
-              ok = mbar_wait(smem_u32(&sh.s_free[g]), j & 1, abort_flag);
-              if (!ok) break;
-              tc_fence_after();
-              FA_STAMP(j, 16 + g * 2)
-              issue_qk(g, sn);
-              FA_STAMP(j, 17 + g * 2)
+            if (ok && j + 1 < n_tiles[g]) {
+              ok = mbar_wait_warp(smem_u32(&sh.s_free[g]), j & 1, abort_flag);
+              if (ok) {
+                tc_fence_after();
+                FA_STAMP(j, 16 + g * 2)
+                issue_qk(g, sn);
+                FA_STAMP(j, 17 + g * 2)
+              }
             }
           }
           if (!ok) break;
           FA_PROF(5)
         } else {
+#pragma unroll
           for (int g = 0; g < 2; ++g) {
-            if (j < n_tiles[g]) {
-              ok = mbar_wait(smem_u32(&sh.p_full[g]), j & 1, abort_flag);
-              if (!ok) break;
-              FA_PROF(2 + g)
-              tc_fence_after();
-              issue_pv(g, s, j > 0);
-              FA_PROF(4)
-              if (j + 1 < n_tiles[g]) issue_qk(g, sn);
-              FA_PROF(5)
+            if (ok && j < n_tiles[g]) {
+              ok = mbar_wait_warp(smem_u32(&sh.p_full[g]), j & 1, abort_flag);
+              if (ok) {
+                FA_PROF(2 + g)
+                tc_fence_after();
+                issue_pv(g, s, j > 0);
+                FA_PROF(4)
+                if (j + 1 < n_tiles[g]) issue_qk(g, sn);
+                FA_PROF(5)
+              }
             }
           }
         }
         if (!ok) break;
-        if (!Cfg::kSeparateP) mma_commit(smem_u32(&sh.v_empty[s]));
-        if (has_next) mma_commit(smem_u32(&sh.k_empty[sn]));
+        if (elect_one()) {
+          if (!Cfg::kSeparateP) mma_commit(smem_u32(&sh.v_empty[s]));
+          if (has_next) mma_commit(smem_u32(&sh.k_empty[sn]));
+        }
       }
       FA_PROF_FLUSH(16, n_max)
     }
   } else if (warp == 10) {
     // ------------------------------------------------------------------ second MMA issuer (d = 64): P*V
-    if (Cfg::kSeparateP && lane == 0) {
+    if constexpr (Cfg::kSeparateP) {
       constexpr uint32_t idesc_pv = make_idesc(BF16, false, true, kBlockM, D);
-      const uint32_t tO[2] = {tmem + Cfg::kTmemO0, tmem + Cfg::kTmemO1};
-      const uint32_t tP[2] = {tmem + Cfg::kTmemP0, tmem + Cfg::kTmemP1};
+      const uint64_t desc_v = make_smem_desc(smem_v, 16384, 1024);
       bool ok = true;
       for (int j = 0; j < n_max && ok; ++j) {
         const int s = j % Cfg::kStages;
-        ok = mbar_wait(smem_u32(&sh.v_full[s]), (j / Cfg::kStages) & 1, abort_flag);
+        ok = mbar_wait_warp(smem_u32(&sh.v_full[s]), (j / Cfg::kStages) & 1, abort_flag);
         if (!ok) break;
-        for (int g = 0; g < 2; ++g) {
-          if (j < n_tiles[g]) {
-            ok = mbar_wait(smem_u32(&sh.p_full[g]), j & 1, abort_flag);
-            if (!ok) break;
-            tc_fence_after();
-            FA_STAMP(j, 20 + g * 2)
-            const uint32_t va = smem_v + s * Cfg::kTileBytes;
+        const uint64_t va = desc_at(desc_v, s * Cfg::kTileBytes);
 #pragma unroll
-            for (int ks = 0; ks < kBlockN / 16; ++ks)
-              mma_ts(tO[g], tP[g] + ks * 8, make_smem_desc(va + ks * 2048, 16384, 1024), idesc_pv,
-                     j > 0 || ks > 0);
-            mma_commit(smem_u32(&sh.o_full[g]));
-            FA_STAMP(j, 21 + g * 2)
+        for (int g = 0; g < 2; ++g) {
+          if (ok && j < n_tiles[g]) {
+            ok = mbar_wait_warp(smem_u32(&sh.p_full[g]), j & 1, abort_flag);
+            if (ok) {
+              tc_fence_after();
+              FA_STAMP(j, 20 + g * 2)
+              const uint32_t tO = tmem + (g == 0 ? Cfg::kTmemO0 : Cfg::kTmemO1);
+              const uint32_t tP = tmem + (g == 0 ? Cfg::kTmemP0 : Cfg::kTmemP1);
+              if (elect_one()) {
+#pragma unroll
+                for (int ks = 0; ks < kBlockN / 16; ++ks)
+                  mma_ts(tO, tP + ks * 8, desc_at(va, ks * 2048), idesc_pv, j > 0 || ks > 0);
+                mma_commit(smem_u32(&sh.o_full[g]));
+              }
+              FA_STAMP(j, 21 + g * 2)
+            }
           }
         }
         if (!ok) break;
-        mma_commit(smem_u32(&sh.v_empty[s]));
+        if (elect_one()) mma_commit(smem_u32(&sh.v_empty[s]));
       }
     }
   } else if (warp < 8 && DROPOUT) {

@@ -75,6 +75,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
 }
 
+// The same wait by all 32 lanes of a warp, with one result for the warp.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
+
 // ---------------------------------------------------------------------------------------------
 // TMA (no multicast anywhere)
 // ---------------------------------------------------------------------------------------------
@@ -228,6 +233,12 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, uint32_t lbo_
   return d;
 }
 
+// The descriptor `bytes` (a multiple of 16) further on: only the address field of the low word moves.
+__device__ __forceinline__ uint64_t desc_at(uint64_t desc, uint32_t bytes) {
+  const uint32_t lo = static_cast<uint32_t>(desc) + (bytes >> 4);
+  return (desc & 0xFFFFFFFF00000000ull) | lo;
+}
+
 // Instruction descriptor for kind::f16 with fp32 accumulation.
 //   [4,6) D format 1 = f32; [7,10) A format, [10,13) B format (0 = f16, 1 = bf16);
 //   bit 15 A is MN-major; bit 16 B is MN-major; [17,23) N >> 3; [24,29) M >> 4.
@@ -238,6 +249,13 @@ __host__ __device__ constexpr uint32_t make_idesc(bool bf16, bool a_mn_major, bo
          (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
 }
 
+// tcgen05.mma takes its descriptors and addresses from uniform registers.  The issuing warps
+// therefore run their loops with all 32 lanes (uniform trip counts, waits joined by a vote) and only
+// the instruction itself sits in an `if (elect_one())` block: the operands then live in uniform
+// registers.  With the whole loop under `if (lane == 0)` every operand was moved over from a
+// per-thread register, instruction by instruction, and an issuing thread got one out every 77-130 clk
+// where a 128 x 128 x 16 product takes 64.
+//
 // D[tmem] (+)= A[smem] * B[smem]; one thread issues.
 __device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
                                        uint32_t idesc, uint32_t accumulate) {
