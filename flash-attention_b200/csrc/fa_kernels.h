@@ -48,9 +48,18 @@ struct BwdArgs {
   float p_keep;
 };
 
+// Plain pointers of the decoding kernel (the tile kernels read through tensor maps).
+constexpr int kDecodeMaxRows = 4;  // query rows per sequence it serves
+struct DecodeArgs {
+  const void* q; const void* k; const void* v;
+  int64_t q_row_stride, q_head_stride, k_row_stride, k_head_stride, v_row_stride, v_head_stride;
+  int32_t total_q, total_k;
+};
+
 struct FwdLaunch {
   CUtensorMap tm_q, tm_k, tm_v;
   KernelArgs args;
+  DecodeArgs decode;
   int32_t max_seqlen_q, max_seqlen_k;
   bool is_bf16, is_causal, is_dropout;
   int32_t dpad;  // 64 or 128
@@ -67,6 +76,7 @@ struct BwdLaunch {
 };
 
 cudaError_t launch_fwd(const FwdLaunch& l, cudaStream_t stream);
+cudaError_t launch_decode(const FwdLaunch& l, cudaStream_t stream);
 cudaError_t launch_bwd(const BwdLaunch& l, cudaStream_t stream);
 cudaError_t launch_sdmask(void* s_out, int64_t s_rows, int64_t s_cols, const void* q, const void* k,
                           int64_t q_row_stride, int64_t q_head_stride, int64_t k_row_stride,
