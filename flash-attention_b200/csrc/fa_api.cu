@@ -247,6 +247,16 @@ int fa_scatter_rows(const void* src, const int64_t* indices, void* dst, int64_t 
   return FA_OK;
 }
 
+int fa_mask_index(const uint8_t* mask, int32_t batch, int32_t seqlen, int32_t* counts, int32_t* cu_seqlens,
+                  int64_t* indices, int32_t* summary, void* cuda_stream) {
+  FA_REQUIRE(batch > 0 && seqlen > 0, "sizes must be positive");
+  FA_REQUIRE(static_cast<int64_t>(batch) * seqlen <= 0x7fffffffLL, "mask too large");
+  FA_REQUIRE(mask && counts && cu_seqlens && indices && summary, "null pointer");
+  FA_CUDA(fa::launch_mask_index(mask, batch, seqlen, counts, cu_seqlens, indices, summary,
+                                static_cast<cudaStream_t>(cuda_stream)));
+  return FA_OK;
+}
+
 int fa_rotary_qkv(const void* qkv, void* out, const float* cos_table, const float* sin_table,
                   int64_t rows, int32_t seqlen, int32_t heads, int32_t head_dim, int32_t is_bf16,
                   int32_t conjugate, void* cuda_stream) {

@@ -99,6 +99,9 @@ cudaError_t launch_scatter_rows(const void* src, const int64_t* indices, void* d
                                 int64_t n_dst_rows, int64_t row_bytes, int32_t* inverse,
                                 cudaStream_t stream);
 
+cudaError_t launch_mask_index(const uint8_t* mask, int batch, int seqlen, int32_t* counts, int32_t* cu_seqlens,
+                              int64_t* indices, int32_t* summary, cudaStream_t stream);
+
 cudaError_t launch_rotary_qkv(const void* qkv, void* out, const float* cos_t, const float* sin_t,
                               int64_t rows, int seqlen, int heads, int d, bool bf16, bool conj,
                               cudaStream_t stream);

@@ -17,36 +17,32 @@ namespace {
 
 constexpr int kRowThreads = 256;
 
-constexpr int kRowsPerStep = 4;  // rows a CTA moves together: four independent 16-byte loads per thread in flight
+// One row by a group of lanes (a power of two, a whole warp for rows of 512 bytes and more): four
+// independent 16-byte loads per lane in flight, 64 warps per SM.  (A CTA per row left most of it idle
+// in the last pass over a row: 288 units of 16 bytes are 256 + 32.)
+__device__ __forceinline__ void copy_row(const uint4* __restrict__ from, bool ok, uint4* __restrict__ to, int vec,
+                                         int lane, int lanes) {
+  constexpr int kUnroll = 4;
+  for (int c0 = lane; c0 < vec; c0 += lanes * kUnroll) {
+    uint4 v[kUnroll];
+#pragma unroll
+    for (int j = 0; j < kUnroll; ++j)
+      v[j] = (ok && c0 + j * lanes < vec) ? __ldg(from + c0 + j * lanes) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int j = 0; j < kUnroll; ++j)
+      if (c0 + j * lanes < vec) to[c0 + j * lanes] = v[j];
+  }
+}
 
 // dst[r, :] = src[indices[r], :] (zeros when the index is out of range); vec = 16-byte units per row
 __global__ void __launch_bounds__(kRowThreads)
 gather_rows_kernel(const uint4* __restrict__ src, const int64_t* __restrict__ indices,
-                   uint4* __restrict__ dst, int64_t n_rows, int64_t src_rows, int vec) {
-  for (int64_t r0 = static_cast<int64_t>(blockIdx.x) * kRowsPerStep; r0 < n_rows;
-       r0 += static_cast<int64_t>(gridDim.x) * kRowsPerStep) {
-    const uint4* from[kRowsPerStep];
-    bool ok[kRowsPerStep];
-#pragma unroll
-    for (int j = 0; j < kRowsPerStep; ++j) {
-      const int64_t s = (r0 + j < n_rows) ? indices[r0 + j] : -1;
-      ok[j] = s >= 0 && s < src_rows;
-      from[j] = src + (ok[j] ? s : 0) * vec;
-    }
-    for (int c = threadIdx.x; c < vec; c += kRowThreads) {
-      uint4 v[kRowsPerStep];
-#pragma unroll
-      for (int j = 0; j < kRowsPerStep; ++j) v[j] = ok[j] ? __ldg(from[j] + c) : make_uint4(0, 0, 0, 0);
-#pragma unroll
-      for (int j = 0; j < kRowsPerStep; ++j)
-        if (r0 + j < n_rows) dst[(r0 + j) * vec + c] = v[j];
-    }
-  }
-}
-
-__global__ void fill_i32_kernel(int32_t* p, int64_t n, int32_t value) {
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < n) p[i] = value;
+                   uint4* __restrict__ dst, int64_t n_rows, int64_t src_rows, int vec, int lanes) {
+  const int64_t r = static_cast<int64_t>(blockIdx.x) * (kRowThreads / lanes) + threadIdx.x / lanes;
+  if (r >= n_rows) return;
+  const int64_t s = indices[r];
+  const bool ok = s >= 0 && s < src_rows;
+  copy_row(src + (ok ? s : 0) * vec, ok, dst + r * vec, vec, threadIdx.x % lanes, lanes);
 }
 
 // inverse[indices[r]] = r
@@ -59,38 +55,117 @@ __global__ void invert_indices_kernel(const int64_t* __restrict__ indices, int32
   }
 }
 
-// one pass over the destination: a row is either copied from its source row or zero-filled
+// One pass over the destination: a row is either copied from its source row or zero-filled.  `inverse`
+// was never cleared: an entry counts only when the source row it names points back at this row.
 __global__ void __launch_bounds__(kRowThreads)
-scatter_rows_kernel(const uint4* __restrict__ src, const int32_t* __restrict__ inverse,
-                    uint4* __restrict__ dst, int64_t n_dst_rows, int vec) {
-  for (int64_t d0 = static_cast<int64_t>(blockIdx.x) * kRowsPerStep; d0 < n_dst_rows;
-       d0 += static_cast<int64_t>(gridDim.x) * kRowsPerStep) {
-    const uint4* from[kRowsPerStep];
-    bool ok[kRowsPerStep];
-#pragma unroll
-    for (int j = 0; j < kRowsPerStep; ++j) {
-      const int32_t s = (d0 + j < n_dst_rows) ? inverse[d0 + j] : -1;
-      ok[j] = s >= 0;
-      from[j] = src + static_cast<int64_t>(ok[j] ? s : 0) * vec;
-    }
-    for (int c = threadIdx.x; c < vec; c += kRowThreads) {
-      uint4 v[kRowsPerStep];
-#pragma unroll
-      for (int j = 0; j < kRowsPerStep; ++j) v[j] = ok[j] ? __ldg(from[j] + c) : make_uint4(0, 0, 0, 0);
-#pragma unroll
-      for (int j = 0; j < kRowsPerStep; ++j)
-        if (d0 + j < n_dst_rows) dst[(d0 + j) * vec + c] = v[j];
-    }
-  }
+scatter_rows_kernel(const uint4* __restrict__ src, const int64_t* __restrict__ indices,
+                    const int32_t* __restrict__ inverse, uint4* __restrict__ dst, int64_t n_src_rows,
+                    int64_t n_dst_rows, int vec, int lanes) {
+  const int64_t d = static_cast<int64_t>(blockIdx.x) * (kRowThreads / lanes) + threadIdx.x / lanes;
+  if (d >= n_dst_rows) return;
+  const int32_t s = inverse[d];
+  const bool ok = s >= 0 && s < n_src_rows && indices[s] == d;
+  copy_row(src + static_cast<int64_t>(ok ? s : 0) * vec, ok, dst + d * vec, vec, threadIdx.x % lanes, lanes);
 }
 
-// a few CTAs per SM, rows handed out in a grid-stride loop
-int row_grid(int64_t rows) {
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int64_t cap = static_cast<int64_t>(sms) * 8;
-  const int64_t steps = (rows + kRowsPerStep - 1) / kRowsPerStep;
-  return static_cast<int>(steps < cap ? steps : cap);
+// lanes that share a row of `vec` 16-byte units
+int row_lanes(int vec) {
+  int lanes = 1;
+  while (lanes < 32 && lanes < vec) lanes *= 2;
+  return lanes;
+}
+unsigned row_grid(int64_t rows, int lanes) {
+  const int64_t per = kRowThreads / lanes;
+  return static_cast<unsigned>((rows + per - 1) / per);
+}
+
+// ------------------------------------------------------------------------------------------------
+// Index lists of a boolean validity mask [batch, seqlen], in two launches and no host involvement: what
+// unpad_input needs before its gather.  Latency bound (a few KB of mask).
+constexpr int kMaskThreads = 256;
+
+// counts[b] = valid tokens of sequence b
+__global__ void __launch_bounds__(kMaskThreads)
+mask_count_kernel(const uint8_t* __restrict__ mask, int seqlen, int32_t* __restrict__ counts) {
+  const uint8_t* row = mask + static_cast<int64_t>(blockIdx.x) * seqlen;
+  int n = 0;
+  for (int c0 = 0; c0 < seqlen; c0 += kMaskThreads)
+    n += __syncthreads_count(c0 + static_cast<int>(threadIdx.x) < seqlen && row[c0 + threadIdx.x] != 0);
+  if (threadIdx.x == 0) counts[blockIdx.x] = n;
+}
+
+// CTA b: positions of the valid tokens of sequence b in the flattened mask, behind those of the sequences
+// before it.  CTA 0 also writes cu_seqlens and summary = (total, longest).
+__global__ void __launch_bounds__(kMaskThreads)
+mask_index_kernel(const uint8_t* __restrict__ mask, int batch, int seqlen, const int32_t* __restrict__ counts,
+                  int32_t* __restrict__ cu_seqlens, int64_t* __restrict__ indices, int32_t* __restrict__ summary) {
+  __shared__ int warp_sum[kMaskThreads / 32];
+  const int b = blockIdx.x, tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
+  // sum over the CTA of one value per thread (every thread gets it)
+  auto cta_sum = [&](int v) -> int {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    __syncthreads();
+    if (lane == 0) warp_sum[warp] = v;
+    __syncthreads();
+    int t = 0;
+#pragma unroll
+    for (int w = 0; w < kMaskThreads / 32; ++w) t += warp_sum[w];
+    return t;
+  };
+  int before = 0;
+  for (int i = tid; i < b; i += kMaskThreads) before += counts[i];
+  int base = cta_sum(before);
+  const uint8_t* row = mask + static_cast<int64_t>(b) * seqlen;
+  for (int c0 = 0; c0 < seqlen; c0 += kMaskThreads) {
+    const bool valid = c0 + tid < seqlen && row[c0 + tid] != 0;
+    const unsigned ballot = __ballot_sync(0xffffffffu, valid);
+    __syncthreads();
+    if (lane == 0) warp_sum[warp] = __popc(ballot);
+    __syncthreads();
+    int off = base + __popc(ballot & ((1u << lane) - 1u));
+#pragma unroll
+    for (int w = 0; w < kMaskThreads / 32; ++w) {
+      if (w < warp) off += warp_sum[w];
+      base += warp_sum[w];
+    }
+    if (valid) indices[off] = static_cast<int64_t>(b) * seqlen + c0 + tid;
+  }
+  if (b == 0) {
+    // running sum over the sequences, 256 at a time
+    int run = 0, longest = 0;
+    if (tid == 0) cu_seqlens[0] = 0;
+    for (int i0 = 0; i0 < batch; i0 += kMaskThreads) {
+      const int v = i0 + tid < batch ? counts[i0 + tid] : 0;
+      int incl = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += up;
+      }
+      __syncthreads();
+      if (lane == 31) warp_sum[warp] = incl;
+      __syncthreads();
+      int off = run;
+#pragma unroll
+      for (int w = 0; w < kMaskThreads / 32; ++w) {
+        if (w < warp) off += warp_sum[w];
+        run += warp_sum[w];
+      }
+      if (i0 + tid < batch) cu_seqlens[i0 + tid + 1] = off + incl;
+      longest = max(longest, v);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
+    if (lane == 0) warp_sum[warp] = longest;
+    __syncthreads();
+    if (tid == 0) {
+      for (int w = 1; w < kMaskThreads / 32; ++w) longest = max(longest, warp_sum[w]);
+      summary[0] = run;
+      summary[1] = longest;
+    }
+  }
 }
 
 }  // namespace
@@ -98,9 +173,9 @@ int row_grid(int64_t rows) {
 cudaError_t launch_gather_rows(const void* src, const int64_t* indices, void* dst, int64_t n_rows,
                                int64_t src_rows, int64_t row_bytes, cudaStream_t stream) {
   if (n_rows <= 0 || row_bytes <= 0) return cudaSuccess;
-  gather_rows_kernel<<<row_grid(n_rows), kRowThreads, 0, stream>>>(
-      static_cast<const uint4*>(src), indices, static_cast<uint4*>(dst), n_rows, src_rows,
-      static_cast<int>(row_bytes / 16));
+  const int vec = static_cast<int>(row_bytes / 16), lanes = row_lanes(vec);
+  gather_rows_kernel<<<row_grid(n_rows, lanes), kRowThreads, 0, stream>>>(
+      static_cast<const uint4*>(src), indices, static_cast<uint4*>(dst), n_rows, src_rows, vec, lanes);
   return cudaGetLastError();
 }
 
@@ -108,13 +183,19 @@ cudaError_t launch_scatter_rows(const void* src, const int64_t* indices, void* d
                                 int64_t n_dst_rows, int64_t row_bytes, int32_t* inverse,
                                 cudaStream_t stream) {
   if (n_dst_rows <= 0 || row_bytes <= 0) return cudaSuccess;
-  fill_i32_kernel<<<static_cast<unsigned>((n_dst_rows + 255) / 256), 256, 0, stream>>>(inverse, n_dst_rows, -1);
+  const int vec = static_cast<int>(row_bytes / 16), lanes = row_lanes(vec);
   if (n_src_rows > 0)
     invert_indices_kernel<<<static_cast<unsigned>((n_src_rows + 255) / 256), 256, 0, stream>>>(
         indices, inverse, n_src_rows, n_dst_rows);
-  scatter_rows_kernel<<<row_grid(n_dst_rows), kRowThreads, 0, stream>>>(
-      static_cast<const uint4*>(src), inverse, static_cast<uint4*>(dst), n_dst_rows,
-      static_cast<int>(row_bytes / 16));
+  scatter_rows_kernel<<<row_grid(n_dst_rows, lanes), kRowThreads, 0, stream>>>(
+      static_cast<const uint4*>(src), indices, inverse, static_cast<uint4*>(dst), n_src_rows, n_dst_rows, vec, lanes);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_mask_index(const uint8_t* mask, int batch, int seqlen, int32_t* counts, int32_t* cu_seqlens,
+                              int64_t* indices, int32_t* summary, cudaStream_t stream) {
+  mask_count_kernel<<<batch, kMaskThreads, 0, stream>>>(mask, seqlen, counts);
+  mask_index_kernel<<<batch, kMaskThreads, 0, stream>>>(mask, batch, seqlen, counts, cu_seqlens, indices, summary);
   return cudaGetLastError();
 }
 
@@ -160,28 +241,50 @@ __device__ __forceinline__ void rotate8(const uint4& in, const float4& c, const 
   out = make_uint4(r[0], r[1], r[2], r[3]);
 }
 
+// A warp handles kRotaryUnits 16-byte units of one token's q and the same units of its k and v, six loads in
+// flight per lane; the token and its position are found once per warp (a flat loop over 16-byte units
+// spent two 64-bit divisions on each of them).
+constexpr int kRotaryUnits = 128;
+
 template <bool BF16>
 __global__ void __launch_bounds__(256)
 rotary_qkv_kernel(const uint4* __restrict__ qkv, uint4* __restrict__ out, const float* __restrict__ cos_t,
-                  const float* __restrict__ sin_t, int64_t n_vec, int seqlen, int heads, int d, float sin_sign) {
-  const int vec_per_head = d / 8;
-  const int vec_per_part = heads * vec_per_head;   // one of q / k / v of one token
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n_vec;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int64_t tok_part = i / vec_per_part;      // token * 3 + part
-    const int part = static_cast<int>(tok_part % 3);
-    uint4 v = __ldg(qkv + i);
-    if (part < 2) {
-      const int pos = static_cast<int>((tok_part / 3) % seqlen);
-      const int pair0 = static_cast<int>(i % vec_per_head) * 4;   // first of the four channel pairs
-      const float4 c = __ldg(reinterpret_cast<const float4*>(cos_t + static_cast<int64_t>(pos) * (d / 2) + pair0));
-      float4 s = __ldg(reinterpret_cast<const float4*>(sin_t + static_cast<int64_t>(pos) * (d / 2) + pair0));
-      s.x *= sin_sign; s.y *= sin_sign; s.z *= sin_sign; s.w *= sin_sign;
-      uint4 r;
-      rotate8<BF16>(v, c, s, r);
-      v = r;
+                  const float* __restrict__ sin_t, int64_t n_items, int seqlen, int vec_per_head, int vec_per_part,
+                  int items_per_token, int d, float sin_sign) {
+  const int64_t item = static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  if (item >= n_items) return;
+  const int64_t token = item / items_per_token;
+  const int begin = static_cast<int>(item - token * items_per_token) * kRotaryUnits;
+  const int end = min(begin + kRotaryUnits, vec_per_part);
+  const int64_t pos = token % seqlen;
+  const uint4* src = qkv + token * 3 * vec_per_part;
+  uint4* dst = out + token * 3 * vec_per_part;
+  const float* cos_p = cos_t + pos * (d / 2);
+  const float* sin_p = sin_t + pos * (d / 2);
+  constexpr int kUnroll = 2;
+  for (int c0 = begin + static_cast<int>(threadIdx.x & 31); c0 < end; c0 += 32 * kUnroll) {
+    uint4 v[kUnroll][3];
+#pragma unroll
+    for (int j = 0; j < kUnroll; ++j)
+#pragma unroll
+      for (int part = 0; part < 3; ++part)
+        if (c0 + 32 * j < end) v[j][part] = __ldg(src + part * vec_per_part + c0 + 32 * j);
+#pragma unroll
+    for (int j = 0; j < kUnroll; ++j) {
+      const int c = c0 + 32 * j;
+      if (c >= end) break;
+      const int pair0 = (c % vec_per_head) * 4;   // first of the four channel pairs
+      const float4 cs = __ldg(reinterpret_cast<const float4*>(cos_p + pair0));
+      float4 sn = __ldg(reinterpret_cast<const float4*>(sin_p + pair0));
+      sn.x *= sin_sign; sn.y *= sin_sign; sn.z *= sin_sign; sn.w *= sin_sign;
+#pragma unroll
+      for (int part = 0; part < 2; ++part) {
+        uint4 r;
+        rotate8<BF16>(v[j][part], cs, sn, r);
+        dst[part * vec_per_part + c] = r;
+      }
+      dst[2 * vec_per_part + c] = v[j][2];
     }
-    out[i] = v;
   }
 }
 
@@ -190,19 +293,20 @@ rotary_qkv_kernel(const uint4* __restrict__ qkv, uint4* __restrict__ out, const 
 cudaError_t launch_rotary_qkv(const void* qkv, void* out, const float* cos_t, const float* sin_t,
                               int64_t rows, int seqlen, int heads, int d, bool bf16, bool conj,
                               cudaStream_t stream) {
-  const int64_t n_vec = rows * 3 * heads * (d / 8);
-  if (n_vec <= 0) return cudaSuccess;
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int64_t want = (n_vec + 255) / 256;
-  const int grid = static_cast<int>(want < static_cast<int64_t>(sms) * 16 ? want : static_cast<int64_t>(sms) * 16);
+  const int vec_per_head = d / 8, vec_per_part = heads * vec_per_head;
+  if (rows <= 0 || vec_per_part <= 0) return cudaSuccess;
+  const int items_per_token = (vec_per_part + kRotaryUnits - 1) / kRotaryUnits;
+  const int64_t n_items = rows * items_per_token;
   const float sign = conj ? -1.f : 1.f;
+  const unsigned grid = static_cast<unsigned>((n_items + 7) / 8);
+  const uint4* src = static_cast<const uint4*>(qkv);
+  uint4* dst = static_cast<uint4*>(out);
   if (bf16)
-    rotary_qkv_kernel<true><<<grid, 256, 0, stream>>>(static_cast<const uint4*>(qkv), static_cast<uint4*>(out),
-                                                      cos_t, sin_t, n_vec, seqlen, heads, d, sign);
+    rotary_qkv_kernel<true><<<grid, 256, 0, stream>>>(src, dst, cos_t, sin_t, n_items, seqlen, vec_per_head,
+                                                      vec_per_part, items_per_token, d, sign);
   else
-    rotary_qkv_kernel<false><<<grid, 256, 0, stream>>>(static_cast<const uint4*>(qkv), static_cast<uint4*>(out),
-                                                       cos_t, sin_t, n_vec, seqlen, heads, d, sign);
+    rotary_qkv_kernel<false><<<grid, 256, 0, stream>>>(src, dst, cos_t, sin_t, n_items, seqlen, vec_per_head,
+                                                       vec_per_part, items_per_token, d, sign);
   return cudaGetLastError();
 }
 

@@ -29,6 +29,7 @@ EXPORTED_SYMBOLS = (
     "fa_debug_philox",
     "fa_gather_rows",
     "fa_scatter_rows",
+    "fa_mask_index",
     "fa_rotary_qkv",
     "fa_convert_blockmask",
     "fa_status_string",
@@ -140,6 +141,9 @@ def _load():
     lib.fa_scatter_rows.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int64,
                                     ctypes.c_int64, ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p]
     lib.fa_scatter_rows.restype = ctypes.c_int
+    lib.fa_mask_index.argtypes = [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32, ctypes.c_void_p,
+                                  ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
+    lib.fa_mask_index.restype = ctypes.c_int
     lib.fa_rotary_qkv.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
                                   ctypes.c_int64, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,
                                   ctypes.c_int32, ctypes.c_int32, ctypes.c_void_p]

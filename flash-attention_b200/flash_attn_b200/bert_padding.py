@@ -91,10 +91,34 @@ class IndexPutFirstAxis(torch.autograd.Function):
 index_put_first_axis = IndexPutFirstAxis.apply
 
 
+def _mask_kernel_path(mask):
+    """Boolean masks only: with integer masks the lengths are the sums of the values."""
+    return (mask.is_cuda and mask.dtype is torch.bool and mask.dim() == 2 and mask.is_contiguous()
+            and 0 < mask.numel() < 2 ** 31)
+
+
+def _mask_lists(mask):
+    """(indices, cu_seqlens, longest) of a boolean mask: two launches and one synchronisation."""
+    batch, seqlen = mask.shape
+    counts = torch.empty(batch + 2, dtype=torch.int32, device=mask.device)  # lengths, then (total, longest)
+    cu_seqlens = torch.empty(batch + 1, dtype=torch.int32, device=mask.device)
+    indices = torch.empty(mask.numel(), dtype=torch.int64, device=mask.device)
+    summary = counts[batch:batch + 2]
+    with torch.cuda.device(mask.device):
+        check(lib.fa_mask_index(mask.data_ptr(), batch, seqlen, counts.data_ptr(), cu_seqlens.data_ptr(),
+                                indices.data_ptr(), summary.data_ptr(), _stream(mask.device)))
+    total, longest = summary.tolist()
+    return indices[:total], cu_seqlens, longest
+
+
 def unpad_input(hidden_states, attention_mask):
     """hidden_states (batch, seqlen, dim); attention_mask (batch, seqlen) bool / int, non-zero =
     valid token.  Returns (packed (total, dim), indices (total,), cu_seqlens (batch + 1,) int32,
     max_seqlen_in_batch int) (reference :60-80)."""
+    flat = hidden_states.reshape(-1, hidden_states.shape[-1])
+    if _mask_kernel_path(attention_mask):
+        indices, cu_seqlens, max_seqlen_in_batch = _mask_lists(attention_mask)
+        return index_first_axis(flat, indices), indices, cu_seqlens, max_seqlen_in_batch
     seqlens_in_batch = attention_mask.sum(dim=-1, dtype=torch.int32)
     # One synchronisation, which the API cannot avoid (the packed size and max_seqlen are host values):
     # the lengths come to the host once and both are read from them; the index list is then built
@@ -105,7 +129,6 @@ def unpad_input(hidden_states, attention_mask):
     max_seqlen_in_batch = int(seqlens_host.max()) if seqlens_host.numel() else 0
     indices = torch.nonzero_static(attention_mask.flatten(), size=total).flatten()
     cu_seqlens = F.pad(torch.cumsum(seqlens_in_batch, dim=0, dtype=torch.int32), (1, 0))
-    flat = hidden_states.reshape(-1, hidden_states.shape[-1])
     return index_first_axis(flat, indices), indices, cu_seqlens, max_seqlen_in_batch
 
 

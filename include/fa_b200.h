@@ -197,6 +197,14 @@ int fa_gather_rows(const void* src, const int64_t* indices, void* dst, int64_t n
 int fa_scatter_rows(const void* src, const int64_t* indices, void* dst, int64_t n_src_rows,
                     int64_t n_dst_rows, int64_t row_bytes, int32_t* workspace, void* cuda_stream);
 
+/* Index lists of a validity mask (batch x seqlen bytes, non-zero = valid token, contiguous): cu_seqlens
+ * (batch + 1), indices = positions of the valid tokens in the flattened mask, ascending (room for
+ * batch * seqlen), summary = (number of valid tokens, longest sequence); counts (batch) is scratch and
+ * holds the sequence lengths afterwards.  Replaces the framework operations of
+ * flash_attn/bert_padding.py:69-74 (unpad_input). */
+int fa_mask_index(const uint8_t* mask, int32_t batch, int32_t seqlen, int32_t* counts, int32_t* cu_seqlens,
+                  int64_t* indices, int32_t* summary, void* cuda_stream);
+
 /* Rotary position embedding on a packed qkv tensor (rows, 3, heads, head_dim), rows = batch *
  * seqlen with the token position = row % seqlen: q and k are rotated pairwise (channels 2i, 2i+1 by
  * the angle with cosine cos_table[pos][i] and sine sin_table[pos][i], fp32 tables of head_dim / 2
