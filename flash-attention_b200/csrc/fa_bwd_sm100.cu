@@ -280,7 +280,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   constexpr uint32_t idesc_dq = make_idesc(BF16, false, true, 128, D);     // dS K
   // Called by one elected lane of an issuing warp whose lanes all run the surrounding loop (see mma_ss).
   auto issue_kk = [&](uint32_t dst, uint32_t a_base, uint32_t b_base) {  // both K-major, K = D
-    const uint64_t da = make_smem_desc(a_base, 16, 1024), db = make_smem_desc(b_base, 16, 1024);
+    const uint64_t da = desc_here(make_smem_desc(a_base, 16, 1024)), db = desc_here(make_smem_desc(b_base, 16, 1024));
 #pragma unroll
     for (int ks = 0; ks < D / 16; ++ks) {
       const uint32_t off = (ks >> 2) * 16384 + (ks & 3) * 32;
@@ -289,14 +289,14 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   };
   auto issue_tt = [&](uint32_t dst, uint32_t a_base, uint32_t b_base, bool acc) {
     // A = [q][kv] read as M = kv (MN-major); B = [q][d] read as N = d (MN-major); K = q rows
-    const uint64_t da = make_smem_desc(a_base, 16384, 1024), db = make_smem_desc(b_base, 16384, 1024);
+    const uint64_t da = desc_here(make_smem_desc(a_base, 16384, 1024)), db = desc_here(make_smem_desc(b_base, 16384, 1024));
 #pragma unroll
     for (int ks = 0; ks < kBM / 16; ++ks)
       mma_ss(dst, desc_at(da, ks * 2048), desc_at(db, ks * 2048), idesc_tt, acc || ks > 0);
   };
   auto issue_dq = [&](uint32_t dst, uint32_t a_base, uint32_t b_base) {
     // A = dS [q][kv] K-major; B = K [kv][d] read as N = d (MN-major); K = kv
-    const uint64_t da = make_smem_desc(a_base, 16, 1024), db = make_smem_desc(b_base, 16384, 1024);
+    const uint64_t da = desc_here(make_smem_desc(a_base, 16, 1024)), db = desc_here(make_smem_desc(b_base, 16384, 1024));
 #pragma unroll
     for (int ks = 0; ks < kBN / 16; ++ks) {
       const uint32_t off = (ks >> 2) * 16384 + (ks & 3) * 32;
@@ -308,7 +308,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   const uint32_t tDS_ = tmem + Cfg::kTmemDS;
   auto issue_dq_t = [&](uint32_t dst, uint32_t a_tmem, uint32_t b_base) {
     // A = dS from tensor memory (16 keys = 8 columns per step); B = K [kv][d] read as N = d; K = kv
-    const uint64_t db = make_smem_desc(b_base, 16384, 1024);
+    const uint64_t db = desc_here(make_smem_desc(b_base, 16384, 1024));
 #pragma unroll
     for (int ks = 0; ks < kBN / 16; ++ks)
       mma_ts(dst, a_tmem + ks * 8, desc_at(db, ks * 2048), idesc_dq, ks > 0);

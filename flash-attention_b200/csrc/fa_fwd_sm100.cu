@@ -38,7 +38,7 @@ constexpr int kBlockM = 128;
 constexpr int kBlockN = 128;
 constexpr int kFwdThreads = 384;  // 2 softmax warpgroups + 1 (producer, MMA issuers, idle)
 
-template <int D>
+template <int D, bool DROPOUT>
 struct FwdCfg {
   static constexpr int kStages = (D == 64) ? 3 : 2;
   static constexpr int kPanels = D / 64;
@@ -49,6 +49,9 @@ struct FwdCfg {
   // S = Q K^T can be issued as soon as the softmax group has read the current S into registers.
   // At d = 128 the 512 columns are full and P overwrites the first 64 columns of its S buffer.
   static constexpr bool kSeparateP = (D == 64);
+  // d = 128 without dropout: P is handed over in two halves, so that P*V of the first 64 keys runs while the
+  // other half is exponentiated; S of the next tile waits for P*V there.
+  static constexpr bool kHalfP = !kSeparateP && !DROPOUT;
   static constexpr uint32_t kTmemP0 = kSeparateP ? 384 : kTmemS0, kTmemP1 = kSeparateP ? 448 : kTmemS1;
 };
 
@@ -57,7 +60,7 @@ constexpr int kMaxSparseTiles = 1024;  // key tiles of 128 per sequence in block
 struct FwdShared {
   uint64_t q_full[2];
   uint64_t k_full[3], k_empty[3], v_full[3], v_empty[3];
-  uint64_t s_full[2], s_free[2], p_full[2], o_full[2];
+  uint64_t s_full[2], s_free[2], p_half[2], p_full[2], o_full[2];
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -142,7 +145,7 @@ template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BLOCKSPARSE>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
               const __grid_constant__ CUtensorMap tm_v, const KernelArgs a) {
-  using Cfg = FwdCfg<D>;
+  using Cfg = FwdCfg<D, DROPOUT>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ FwdShared sh;
   // block-sparse: key tiles this CTA visits (ascending), built from the layout table
@@ -224,6 +227,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       mbar_init(smem_u32(&sh.q_full[i]), 1);
       mbar_init(smem_u32(&sh.s_full[i]), 1);
       mbar_init(smem_u32(&sh.s_free[i]), kBlockM);
+      mbar_init(smem_u32(&sh.p_half[i]), kBlockM);
       mbar_init(smem_u32(&sh.p_full[i]), kBlockM);
       mbar_init(smem_u32(&sh.o_full[i]), 1);
     }
@@ -292,8 +296,8 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       const uint64_t desc_k = make_smem_desc(smem_k, 16, 1024);
       const uint64_t desc_v = make_smem_desc(smem_v, 16384, 1024);
       auto issue_qk = [&](int g, int stage) {
-        const uint64_t qa = desc_at(desc_q, g * Cfg::kTileBytes);
-        const uint64_t ka = desc_at(desc_k, stage * Cfg::kTileBytes);
+        const uint64_t qa = desc_here(desc_at(desc_q, g * Cfg::kTileBytes));
+        const uint64_t ka = desc_here(desc_at(desc_k, stage * Cfg::kTileBytes));
         const uint32_t tS = tmem + (g == 0 ? Cfg::kTmemS0 : Cfg::kTmemS1);
         if (elect_one()) {
 #pragma unroll
@@ -304,15 +308,16 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           mma_commit(smem_u32(&sh.s_full[g]));
         }
       };
-      auto issue_pv = [&](int g, int stage, bool accumulate) {
-        const uint64_t va = desc_at(desc_v, stage * Cfg::kTileBytes);
+      // key steps [k0, k1) of 16; the last part reports the product
+      auto issue_pv = [&](int g, int stage, bool accumulate, int k0, int k1) {
+        const uint64_t va = desc_here(desc_at(desc_v, stage * Cfg::kTileBytes));
         const uint32_t tO = tmem + (g == 0 ? Cfg::kTmemO0 : Cfg::kTmemO1);
         const uint32_t tP = tmem + (g == 0 ? Cfg::kTmemP0 : Cfg::kTmemP1);
         if (elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < kBlockN / 16; ++ks)
+          for (int ks = k0; ks < k1; ++ks)
             mma_ts(tO, tP + ks * 8, desc_at(va, ks * 2048), idesc_pv, accumulate || ks > 0);
-          mma_commit(smem_u32(&sh.o_full[g]));
+          if (k1 == kBlockN / 16) mma_commit(smem_u32(&sh.o_full[g]));
         }
       };
 
@@ -360,11 +365,19 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 #pragma unroll
           for (int g = 0; g < 2; ++g) {
             if (ok && j < n_tiles[g]) {
-              ok = mbar_wait_warp(smem_u32(&sh.p_full[g]), j & 1, abort_flag);
+              constexpr int kFirst = Cfg::kHalfP ? kBlockN / 32 : 0;
+              if constexpr (Cfg::kHalfP) {
+                ok = mbar_wait_warp(smem_u32(&sh.p_half[g]), j & 1, abort_flag);
+                if (ok) {
+                  tc_fence_after();
+                  issue_pv(g, s, j > 0, 0, kFirst);
+                }
+              }
+              if (ok) ok = mbar_wait_warp(smem_u32(&sh.p_full[g]), j & 1, abort_flag);
               if (ok) {
                 FA_PROF(2 + g)
                 tc_fence_after();
-                issue_pv(g, s, j > 0);
+                issue_pv(g, s, j > 0, kFirst, kBlockN / 16);
                 FA_PROF(4)
                 if (j + 1 < n_tiles[g]) issue_qk(g, sn);
                 FA_PROF(5)
@@ -390,7 +403,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         const int s = j % Cfg::kStages;
         ok = mbar_wait_warp(smem_u32(&sh.v_full[s]), (j / Cfg::kStages) & 1, abort_flag);
         if (!ok) break;
-        const uint64_t va = desc_at(desc_v, s * Cfg::kTileBytes);
+        const uint64_t va = desc_here(desc_at(desc_v, s * Cfg::kTileBytes));
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
           if (ok && j < n_tiles[g]) {
@@ -725,29 +738,27 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       // p = exp2(s * c - m * c): packed fma, one ex2 per element, packed row sum, 16-bit pack
       uint32_t pk[64];
       uint64_t sum_a = 0ull, sum_b = 0ull;
+      auto expo_half = [&](int half) {
 #pragma unroll
-      for (int c = 0; c < 4; ++c)
+        for (int c = 2 * half; c < 2 * half + 2; ++c)
 #pragma unroll
-        for (int i = 0; i < 32; i += 4) {
-          float p0, p1, p2, p3;
-          unpack_f2(fma2(pack_f2(__uint_as_float(sr[c][i]), __uint_as_float(sr[c][i + 1])), c2, nmc2), p0, p1);
-          unpack_f2(fma2(pack_f2(__uint_as_float(sr[c][i + 2]), __uint_as_float(sr[c][i + 3])), c2, nmc2), p2, p3);
-          p0 = ex2f(p0); p1 = ex2f(p1); p2 = ex2f(p2); p3 = ex2f(p3);
-          const uint64_t p01 = pack_f2(p0, p1), p23 = pack_f2(p2, p3);
-          sum_a = add2(sum_a, p01);
-          sum_b = add2(sum_b, p23);
-          pk[c * 16 + i / 2] = pack_lowp<BF16>(p0, p1);
-          pk[c * 16 + i / 2 + 1] = pack_lowp<BF16>(p2, p3);
-        }
-      {
-        float s0, s1;
-        unpack_f2(add2(sum_a, sum_b), s0, s1);
-        l_run = l_run * alpha + (s0 + s1);
-      }
-
+          for (int i = 0; i < 32; i += 4) {
+            float p0, p1, p2, p3;
+            unpack_f2(fma2(pack_f2(__uint_as_float(sr[c][i]), __uint_as_float(sr[c][i + 1])), c2, nmc2), p0, p1);
+            unpack_f2(fma2(pack_f2(__uint_as_float(sr[c][i + 2]), __uint_as_float(sr[c][i + 3])), c2, nmc2), p2, p3);
+            p0 = ex2f(p0); p1 = ex2f(p1); p2 = ex2f(p2); p3 = ex2f(p3);
+            const uint64_t p01 = pack_f2(p0, p1), p23 = pack_f2(p2, p3);
+            sum_a = add2(sum_a, p01);
+            sum_b = add2(sum_b, p23);
+            pk[c * 16 + i / 2] = pack_lowp<BF16>(p0, p1);
+            pk[c * 16 + i / 2 + 1] = pack_lowp<BF16>(p2, p3);
+          }
+      };
+      expo_half(0);
       FA_PROF(5)
       if (row == 0) { FA_STAMP(j, g * 8 + 4) }
-      // P*V of the previous tile must have finished before O is rescaled or its P buffer reused
+      // P*V of the previous tile must have finished before O is rescaled or its P buffer reused.  (Half of the
+      // exponentials are still to come: by now it has, as a rule.)
       if (j > 0) {
         ok = mbar_wait(smem_u32(&sh.o_full[g]), (j - 1) & 1, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
@@ -757,23 +768,34 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         if (__any_sync(0xffffffffu, grow)) {
           const uint64_t alpha2 = pack_f2(alpha, alpha);
 #pragma unroll
-          for (int c = 0; c < D / 32; ++c) {
-            uint32_t orr[32];
-            tmem_ld32(tO + c * 32, orr);
+          for (int c = 0; c < D / 16; ++c) {
+            uint32_t orr[16];
+            tmem_ld16(tO + c * 16, orr);
             tmem_wait_ld();
 #pragma unroll
-            for (int i = 0; i < 32; i += 2) {
+            for (int i = 0; i < 16; i += 2) {
               float lo, hi;
               unpack_f2(mul2(pack_f2(__uint_as_float(orr[i]), __uint_as_float(orr[i + 1])), alpha2), lo, hi);
               orr[i] = __float_as_uint(lo);
               orr[i + 1] = __float_as_uint(hi);
             }
-            tmem_st32(tO + c * 32, orr);
+            tmem_st16(tO + c * 16, orr);
           }
         }
       }
-      // hand P to the tensor core through tensor memory
+      // hand P to the tensor core through tensor memory, in two halves (64 keys each)
       tmem_st32(tP, reinterpret_cast<uint32_t(&)[32]>(pk[0]));
+      if constexpr (Cfg::kHalfP) {
+        tmem_wait_st();
+        tc_fence_before();
+        mbar_arrive(smem_u32(&sh.p_half[g]));
+      }
+      expo_half(1);
+      {
+        float s0, s1;
+        unpack_f2(add2(sum_a, sum_b), s0, s1);
+        l_run = l_run * alpha + (s0 + s1);
+      }
       tmem_st32(tP + 32, reinterpret_cast<uint32_t(&)[32]>(pk[32]));
       tmem_wait_st();
       tc_fence_before();
@@ -808,7 +830,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BS>
 cudaError_t launch_one(const FwdLaunch& l, cudaStream_t stream) {
   auto kernel = fa_fwd_kernel<D, BF16, CAUSAL, DROPOUT, BS>;
-  constexpr int smem = FwdCfg<D>::kSmemBytes;
+  constexpr int smem = FwdCfg<D, DROPOUT>::kSmemBytes;
   static SmemLimitFlags smem_limit_set;  // one per template instantiation of this function
   cudaError_t e = set_smem_limit_once(kernel, smem, smem_limit_set);
   if (e != cudaSuccess) return e;

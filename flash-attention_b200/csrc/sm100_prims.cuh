@@ -233,6 +233,13 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, uint32_t lbo_
   return d;
 }
 
+// A descriptor whose value the compiler may not form ahead of the loop it is used in: an issuing warp has 56
+// registers, and the unrolled steps' descriptors of three or four operands do not fit in them.
+__device__ __forceinline__ uint64_t desc_here(uint64_t desc) {
+  asm volatile("" : "+l"(desc));
+  return desc;
+}
+
 // The descriptor `bytes` (a multiple of 16) further on: only the address field of the low word moves.
 __device__ __forceinline__ uint64_t desc_at(uint64_t desc, uint32_t bytes) {
   const uint32_t lo = static_cast<uint32_t>(desc) + (bytes >> 4);
