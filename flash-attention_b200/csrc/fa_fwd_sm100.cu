@@ -1,7 +1,9 @@
 // FlashAttention forward for sm_100a.
 //
-// One CTA owns two consecutive 128-row query tiles of one (batch, head) pair and walks the key /
-// value sequence in 128-row tiles.  Warp roles:
+// One CTA owns G = 1 or 2 consecutive 128-row query tiles of one (batch, head) pair and walks the key /
+// value sequence in 128-row tiles; launch_one says which G serves which call.  Warp roles at G = 2 (at G = 1
+// there is no softmax group 1, warps 4-7 are what warps 8-11 are here, the CTA has 256 tensor-memory
+// columns, and two CTAs share an SM):
 //   warps 0-3   softmax group 0 (query tile 0): one thread per query row; with dropout a thread
 //               holds two rows of each of the warp's two 16-row blocks and a quarter of their
 //               columns (the ownership pattern of the reference's mask generator)
@@ -36,15 +38,20 @@ namespace {
 
 constexpr int kBlockM = 128;
 constexpr int kBlockN = 128;
-constexpr int kFwdThreads = 384;  // 2 softmax warpgroups + 1 (producer, MMA issuers, idle)
 
-template <int D, bool DROPOUT>
+// G: query tiles (softmax groups) per CTA.  Two share every K / V tile, and one such CTA fills an SM.  One leaves
+// room for a second CTA on the SM, whose loads, first products and epilogue run under the tiles of the other:
+// for short sequences, where those are a third of a CTA's time (see launch_one).
+template <int D, bool DROPOUT, int G>
 struct FwdCfg {
-  static constexpr int kStages = (D == 64) ? 3 : 2;
+  static constexpr int kThreads = 128 * (G + 1);  // G softmax warpgroups + 1 (producer, MMA issuers, idle)
+  // G = 1: 80 KB (d = 64: Q, two stages) or 96 KB (d = 128: Q, one stage), so that two CTAs fit
+  static constexpr int kStages = (G == 1) ? ((D == 64) ? 2 : 1) : ((D == 64) ? 3 : 2);
   static constexpr int kPanels = D / 64;
   static constexpr int kTileBytes = kBlockM * D * 2;
-  static constexpr int kSmemBytes = (2 + 2 * kStages) * kTileBytes + 1024;
-  static constexpr uint32_t kTmemS0 = 0, kTmemS1 = 128, kTmemO0 = 256, kTmemO1 = 256 + D;
+  static constexpr int kSmemBytes = (G + 2 * kStages) * kTileBytes + 1024;
+  static constexpr uint32_t kTmemCols = 256 * G;
+  static constexpr uint32_t kTmemS0 = 0, kTmemS1 = 128, kTmemO0 = 128 * G, kTmemO1 = 128 * G + D;
   // d = 64 leaves 128 tensor-memory columns free: P gets its own columns there, so the next
   // S = Q K^T can be issued as soon as the softmax group has read the current S into registers.
   // At d = 128 the 512 columns are full and P overwrites the first 64 columns of its S buffer.
@@ -52,7 +59,9 @@ struct FwdCfg {
   // d = 128 without dropout: P is handed over in two halves, so that P*V of the first 64 keys runs while the
   // other half is exponentiated; S of the next tile waits for P*V there.
   static constexpr bool kHalfP = !kSeparateP && !DROPOUT;
-  static constexpr uint32_t kTmemP0 = kSeparateP ? 384 : kTmemS0, kTmemP1 = kSeparateP ? 448 : kTmemS1;
+  static constexpr uint32_t kTmemP0 = kSeparateP ? 192 * G : kTmemS0, kTmemP1 = kSeparateP ? 192 * G + 64 : kTmemS1;
+  // register split (per thread) of the 168 or 128 a thread is launched with
+  static constexpr int kSoftmaxRegs = (G == 1) ? 208 : 224, kOtherRegs = (G == 1) ? 48 : 56;
 };
 
 constexpr int kMaxSparseTiles = 1024;  // key tiles of 128 per sequence in block-sparse mode
@@ -141,11 +150,11 @@ __device__ __forceinline__ void store_rows(const KernelArgs& a, uint32_t tO, boo
   }
 }
 
-template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BLOCKSPARSE>
-__global__ void __launch_bounds__(kFwdThreads, 1)
+template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BLOCKSPARSE, int G>
+__global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1)
 fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
               const __grid_constant__ CUtensorMap tm_v, const KernelArgs a) {
-  using Cfg = FwdCfg<D, DROPOUT>;
+  using Cfg = FwdCfg<D, DROPOUT, G>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ FwdShared sh;
   // block-sparse: key tiles this CTA visits (ascending), built from the layout table
@@ -163,7 +172,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   const int sq = a.cu_seqlens_q[b + 1] - q_start;
   const int k_start = a.cu_seqlens_k[b];
   const int sk = a.cu_seqlens_k[b + 1] - k_start;
-  if (mp * 2 * kBlockM >= sq) return;
+  if (mp * G * kBlockM >= sq) return;
   // fail fast: once a CTA of this launch has abandoned a wait, the remaining CTAs do not start
   if (a.status && *reinterpret_cast<volatile int32_t*>(a.status) == a.launch_id) return;
 
@@ -172,15 +181,15 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     // A key tile is visited when any 16-row block of this CTA's 256 query rows has its 256-column
     // key block in the layout; rows whose block is absent are masked inside the tile.
     uint8_t* flags = reinterpret_cast<uint8_t*>(smem_raw);
-    const int rb0 = mp * (2 * kBlockM / 16);
-    const int rb1 = min(min(rb0 + 2 * kBlockM / 16, a.bs_rows16), (sq + 15) >> 4);
+    const int rb0 = mp * (G * kBlockM / 16);
+    const int rb1 = min(min(rb0 + G * kBlockM / 16, a.bs_rows16), (sq + 15) >> 4);
     n_kv_total = min(n_kv_total, kMaxSparseTiles);
-    for (int j = tid; j < n_kv_total; j += kFwdThreads) {
+    for (int j = tid; j < n_kv_total; j += Cfg::kThreads) {
       const int32_t* row = a.bs_iter + (static_cast<int64_t>(b) * a.bs_kblocks + (j >> 1)) * a.bs_rows16;
       bool any = false;
       for (int rb = rb0; rb < rb1; ++rb) any = any || (row[rb] >= 0);
       // causal: a key tile that starts behind the CTA's last query row is masked entirely
-      if (CAUSAL && j * kBlockN > mp * 2 * kBlockM + 2 * kBlockM - 1) any = false;
+      if (CAUSAL && j * kBlockN > mp * G * kBlockM + G * kBlockM - 1) any = false;
       flags[j] = any ? 1 : 0;
     }
     __syncthreads();
@@ -198,10 +207,10 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     if constexpr (BLOCKSPARSE) return tile_list[j];
     else return j;
   };
-  int m0[2], n_tiles[2];
+  int m0[G], n_tiles[G];
 #pragma unroll
-  for (int g = 0; g < 2; ++g) {
-    m0[g] = (mp * 2 + g) * kBlockM;
+  for (int g = 0; g < G; ++g) {
+    m0[g] = (mp * G + g) * kBlockM;
     const bool active = m0[g] < sq;
     int n = n_kv_total;
     if constexpr (CAUSAL && BLOCKSPARSE) {
@@ -213,12 +222,12 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     }
     n_tiles[g] = active ? n : 0;
   }
-  const int n_max = max(n_tiles[0], n_tiles[1]);
+  const int n_max = max(n_tiles[0], n_tiles[G - 1]);
 
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   const uint32_t smem_q = smem_u32(smem);
-  const uint32_t smem_k = smem_q + 2 * Cfg::kTileBytes;
+  const uint32_t smem_k = smem_q + G * Cfg::kTileBytes;
   const uint32_t smem_v = smem_k + Cfg::kStages * Cfg::kTileBytes;
 
   if (tid == 0) {
@@ -239,21 +248,21 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     }
     fence_mbar_init();
   }
-  if (warp == 8) tmem_alloc(smem_u32(&sh.tmem_base), 512);
+  if (warp == 4 * G) tmem_alloc(smem_u32(&sh.tmem_base), Cfg::kTmemCols);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sh.tmem_base;
   volatile int* abort_flag = &sh.abort_flag;
 
-  if (warp >= 8) reg_dealloc<56>();
-  if (warp == 8) {
+  if (warp >= 4 * G) reg_dealloc<Cfg::kOtherRegs>();
+  if (warp == 4 * G) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       tma_prefetch_desc(&tm_q);
       tma_prefetch_desc(&tm_k);
       tma_prefetch_desc(&tm_v);
-      for (int g = 0; g < 2; ++g) {
+      for (int g = 0; g < G; ++g) {
         if (n_tiles[g] > 0) {
           const uint32_t bar = smem_u32(&sh.q_full[g]);
           mbar_expect_tx(bar, Cfg::kTileBytes);
@@ -286,7 +295,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         }
       }
     }
-  } else if (warp == 9) {
+  } else if (warp == 4 * G + 1) {
     // ------------------------------------------------------------------ MMA issuer
     // all 32 lanes run the loop, one elected lane issues (see mma_ss)
     {
@@ -322,14 +331,14 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       };
 
       bool ok = true;
-      for (int g = 0; g < 2 && ok; ++g)
+      for (int g = 0; g < G && ok; ++g)
         if (n_tiles[g] > 0) ok = mbar_wait_warp(smem_u32(&sh.q_full[g]), 0, abort_flag);
       if (ok && n_max > 0) {
         ok = mbar_wait_warp(smem_u32(&sh.k_full[0]), 0, abort_flag);
         if (ok) {
           tc_fence_after();
 #pragma unroll
-          for (int g = 0; g < 2; ++g)
+          for (int g = 0; g < G; ++g)
             if (n_tiles[g] > 0) issue_qk(g, 0);
           if (elect_one()) mma_commit(smem_u32(&sh.k_empty[0]));
         }
@@ -348,7 +357,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         if constexpr (Cfg::kSeparateP) {
           // this warp issues only the score products; warp 10 issues P*V
 #pragma unroll
-          for (int g = 0; g < 2; ++g) {
+          for (int g = 0; g < G; ++g) {
             if (ok && j + 1 < n_tiles[g]) {
               ok = mbar_wait_warp(smem_u32(&sh.s_free[g]), j & 1, abort_flag);
               if (ok) {
@@ -363,7 +372,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           FA_PROF(5)
         } else {
 #pragma unroll
-          for (int g = 0; g < 2; ++g) {
+          for (int g = 0; g < G; ++g) {
             if (ok && j < n_tiles[g]) {
               constexpr int kFirst = Cfg::kHalfP ? kBlockN / 32 : 0;
               if constexpr (Cfg::kHalfP) {
@@ -393,7 +402,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       }
       FA_PROF_FLUSH(16, n_max)
     }
-  } else if (warp == 10) {
+  } else if (warp == 4 * G + 2) {
     // ------------------------------------------------------------------ second MMA issuer (d = 64): P*V
     if constexpr (Cfg::kSeparateP) {
       constexpr uint32_t idesc_pv = make_idesc(BF16, false, true, kBlockM, D);
@@ -405,7 +414,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         if (!ok) break;
         const uint64_t va = desc_here(desc_at(desc_v, s * Cfg::kTileBytes));
 #pragma unroll
-        for (int g = 0; g < 2; ++g) {
+        for (int g = 0; g < G; ++g) {
           if (ok && j < n_tiles[g]) {
             ok = mbar_wait_warp(smem_u32(&sh.p_full[g]), j & 1, abort_flag);
             if (ok) {
@@ -427,14 +436,14 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         if (elect_one()) mma_commit(smem_u32(&sh.v_empty[s]));
       }
     }
-  } else if (warp < 8 && DROPOUT) {
+  } else if (warp < 4 * G && DROPOUT) {
     // ------------------------------------------------------------------ softmax groups, dropout
     // Quad layout: a warp reads its 32 rows as two 16-row blocks (hh) with the 16x256b shape, so a
     // thread holds rows r8 and r8 + 8 of each block and, of every 8-column unit, two adjacent columns.
     // That is the ownership pattern of the reference's mask generator: one Philox call covers exactly
     // one thread's part of a 16 x 16 patch (QuadPhilox).  Row statistics are reduced over the four
     // lanes of a quad.  Row index ri = hh * 2 + u for row r8 + 16 * hh + 8 * u of the warp.
-    reg_alloc<224>();
+    reg_alloc<Cfg::kSoftmaxRegs>();
     const int g = warp >> 2;
     const int wq = warp & 3;
     const int r8 = lane >> 2, q4 = lane & 3;
@@ -637,9 +646,9 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       }
       store_rows<D, BF16>(a, tO, n > 0 && ok, ok, m0[g] + wq * 32 + lane, sq, q_start, b, h, m_row, l_row);
     }
-  } else if (warp < 8) {
+  } else if (warp < 4 * G) {
     // ------------------------------------------------------------------ softmax groups, no dropout
-    reg_alloc<224>();
+    reg_alloc<Cfg::kSoftmaxRegs>();
     const int g = warp >> 2;
     const int row = tid & 127;
     const int ig = m0[g] + row;  // query index within the sequence
@@ -818,8 +827,8 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 8) {
-    tmem_dealloc(tmem, 512);
+  if (warp == 4 * G) {
+    tmem_dealloc(tmem, Cfg::kTmemCols);
     if (lane == 0 && sh.abort_flag && a.status) {
       atomicExch(a.status, a.launch_id);  // stops the CTAs of this launch that have not started yet
       atomicExch(a.status + 2, 1);  // sticky: read by the host
@@ -827,16 +836,39 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   }
 }
 
+template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BS, int G>
+cudaError_t launch_groups(const FwdLaunch& l, cudaStream_t stream) {
+  auto kernel = fa_fwd_kernel<D, BF16, CAUSAL, DROPOUT, BS, G>;
+  using Cfg = FwdCfg<D, DROPOUT, G>;
+  static SmemLimitFlags smem_limit_set;  // one per template instantiation of this function
+  cudaError_t e = set_smem_limit_once(kernel, Cfg::kSmemBytes, smem_limit_set);
+  if (e != cudaSuccess) return e;
+  dim3 grid((l.max_seqlen_q + G * kBlockM - 1) / (G * kBlockM), l.args.heads, l.args.batch);
+  kernel<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(l.tm_q, l.tm_k, l.tm_v, l.args);
+  return cudaGetLastError();
+}
+
+// One query tile per CTA (two CTAs per SM) or two.  Batches of ragged sequences, 12 heads, us with two -> one:
+//   d = 64    64 x 128: 32 -> 21   64 x 512: 108 -> 86   32 x 1024: 147 -> 124   8 x 4096: 383 -> 358
+//   causal    64 x 128: 34 -> 22   64 x 512:  90 -> 80   32 x 1024: 108 -> 100   8 x 4096: 231 -> 225
+//   dropout   64 x 128: 39 -> 26   64 x 512: 162 -> 143  32 x 1024: 251 -> 229   8 x 4096: 770 -> 736
+//   d = 128   64 x 128: 42 -> 26   64 x 512: 141 -> 125  32 x 1024: 187 -> 182   8 x 4096: 498 -> 552
+// At d = 128 a CTA of one tile has a single stage of K and V, which long sequences pay for; at d = 64 the two
+// meet beyond 4096 (2 x 4 x 65536 causal training 18.98 -> 19.28 ms), where a pair's shared reads count.  A grid of
+// pairs that fills between half of the 148 SMs and all of them runs in one round either way and reads
+// K and V once per pair (16 x 8 heads, 200 queries, 1500 keys: 26 against 27 us).
+constexpr int kSms = 148;
+constexpr int kOneTileMaxD64 = 4096, kOneTileMaxD128 = 1024;
+
 template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BS>
 cudaError_t launch_one(const FwdLaunch& l, cudaStream_t stream) {
-  auto kernel = fa_fwd_kernel<D, BF16, CAUSAL, DROPOUT, BS>;
-  constexpr int smem = FwdCfg<D, DROPOUT>::kSmemBytes;
-  static SmemLimitFlags smem_limit_set;  // one per template instantiation of this function
-  cudaError_t e = set_smem_limit_once(kernel, smem, smem_limit_set);
-  if (e != cudaSuccess) return e;
-  dim3 grid((l.max_seqlen_q + 2 * kBlockM - 1) / (2 * kBlockM), l.args.heads, l.args.batch);
-  kernel<<<grid, kFwdThreads, smem, stream>>>(l.tm_q, l.tm_k, l.tm_v, l.args);
-  return cudaGetLastError();
+  if constexpr (!BS) {
+    const int64_t pairs = static_cast<int64_t>((l.max_seqlen_q + 2 * kBlockM - 1) / (2 * kBlockM)) * l.args.heads * l.args.batch;
+    const bool one_round = l.max_seqlen_q > kBlockM && pairs > kSms / 2 && pairs <= kSms;
+    if (!one_round && l.max_seqlen_q <= (D == 64 ? kOneTileMaxD64 : kOneTileMaxD128))
+      return launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 1>(l, stream);
+  }
+  return launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 2>(l, stream);
 }
 
 template <int D, bool BF16, bool CAUSAL>
