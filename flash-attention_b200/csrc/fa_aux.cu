@@ -53,7 +53,7 @@ __device__ __forceinline__ int visited_prefix(const int32_t* row, int nr, int sq
   return nr;
 }
 
-// Output rows no attention CTA writes (rows outside every sequence, and rows at or beyond the 256-row
+// Output rows no attention CTA writes (rows outside every sequence, and rows at or beyond the 128-row
 // tiles that max_seqlen_q covers) are zero in a block-sparse call (fmha_api.cpp:519 starts from
 // o = 0); zeroing the few there are replaces a pass over the whole tensor.
 struct ZeroRows {
@@ -260,7 +260,7 @@ cudaError_t launch_philox_probe(uint32_t* out, int n, unsigned long long seed, u
 cudaError_t launch_bs_table(int32_t* table, const int32_t* blockmask, const int32_t* cu_q,
                             const int32_t* cu_k, int batch, int nk, int nr, void* o, int64_t o_row_bytes,
                             int total_q, int max_seqlen_q, cudaStream_t stream) {
-  const ZeroRows z{static_cast<uint4*>(o), o_row_bytes / 16, total_q, (max_seqlen_q + 255) / 256 * 256};
+  const ZeroRows z{static_cast<uint4*>(o), o_row_bytes / 16, total_q, (max_seqlen_q + 127) / 128 * 128};
   bs_table_kernel<<<dim3(nk, batch), kTableThreads, 0, stream>>>(table, blockmask, cu_q, cu_k, nk, nr, batch, z);
   return cudaGetLastError();
 }

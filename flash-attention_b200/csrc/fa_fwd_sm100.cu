@@ -853,6 +853,7 @@ cudaError_t launch_groups(const FwdLaunch& l, cudaStream_t stream) {
 //   causal    64 x 128: 34 -> 22   64 x 512:  90 -> 80   32 x 1024: 108 -> 100   8 x 4096: 231 -> 225
 //   dropout   64 x 128: 39 -> 26   64 x 512: 162 -> 143  32 x 1024: 251 -> 229   8 x 4096: 770 -> 736
 //   d = 128   64 x 128: 42 -> 26   64 x 512: 141 -> 125  32 x 1024: 187 -> 182   8 x 4096: 498 -> 552
+//   block-sparse (16 heads, 25 %)    4 x 1024: 41 -> 38     4 x 4096: 196 -> 185
 // At d = 128 a CTA of one tile has a single stage of K and V, which long sequences pay for; at d = 64 the two
 // meet beyond 4096 (2 x 4 x 65536 causal training 18.98 -> 19.28 ms), where a pair's shared reads count.  A grid of
 // pairs that fills between half of the 148 SMs and all of them runs in one round either way and reads
@@ -862,12 +863,10 @@ constexpr int kOneTileMaxD64 = 4096, kOneTileMaxD128 = 1024;
 
 template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BS>
 cudaError_t launch_one(const FwdLaunch& l, cudaStream_t stream) {
-  if constexpr (!BS) {
-    const int64_t pairs = static_cast<int64_t>((l.max_seqlen_q + 2 * kBlockM - 1) / (2 * kBlockM)) * l.args.heads * l.args.batch;
-    const bool one_round = l.max_seqlen_q > kBlockM && pairs > kSms / 2 && pairs <= kSms;
-    if (!one_round && l.max_seqlen_q <= (D == 64 ? kOneTileMaxD64 : kOneTileMaxD128))
-      return launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 1>(l, stream);
-  }
+  const int64_t pairs = static_cast<int64_t>((l.max_seqlen_q + 2 * kBlockM - 1) / (2 * kBlockM)) * l.args.heads * l.args.batch;
+  const bool one_round = l.max_seqlen_q > kBlockM && pairs > kSms / 2 && pairs <= kSms;
+  if (!one_round && l.max_seqlen_q <= (D == 64 ? kOneTileMaxD64 : kOneTileMaxD128))
+    return launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 1>(l, stream);
   return launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 2>(l, stream);
 }
 
