@@ -500,9 +500,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       }
     } else if (warp == 14 && Cfg::kDualIssue) {
       // -------------------------------------------------------------- MMA issuer 2: dV
-      // dV and dK have a thread each: an issuing thread gets an instruction out every ~130 clk
-      // (it shares its scheduler with two compute warps), so the 16 instructions of the two products
-      // took longer to issue than to execute and the compute groups waited for the buffers.
+      // dV and dK have a warp each, so that neither waits for the other's instructions to be taken.
       bool ok = true;
       FA_PROF_DECL
       for (int t = 0; t < nm && ok; ++t) {

@@ -10,8 +10,7 @@
 //   warps 4-7   softmax group 1 (query tile 1)
 //   warp  8     TMA producer (Q once, K/V ring)
 //   warp  9     tcgen05.mma issuer (d = 128: every product; d = 64: S = Q K^T only)
-//   warp 10     d = 64: second issuer, O += P V (an issuing thread shares its scheduler with two
-//               softmax warps and gets an instruction out every 77-110 clk; two issuers keep S ahead)
+//   warp 10     d = 64: second issuer, O += P V (two issuers keep S ahead)
 //   warp 11     idle
 // Tensor memory (512 columns): S0 [0,128) S1 [128,256) fp32 scores, O0 / O1 fp32 outputs behind
 // them.  The 16-bit probabilities P feed the P*V product straight from tensor memory; at d = 128
