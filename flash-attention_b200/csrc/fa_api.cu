@@ -459,10 +459,6 @@ int run_bwd(const fa_bwd_params* p, float* accum, int stage_mask, bool bind_cont
   a.total_q = f->total_q; a.total_k = f->total_k;
   a.max_seqlen_q = f->max_seqlen_q; a.max_seqlen_k = f->max_seqlen_k;
   a.p_keep = 1.f - f->p_dropout;
-  // One contiguous block per dQ tile costs less per tile, boxes of 128-byte rows sustain more adds per second.
-  // d = 64, whole backward in us with boxes -> blocks: dropout 4 x 12 x 4096 607 -> 585, 8 x 12 x 512 60 -> 57;
-  // without dropout 16 x 8 x 200 queries 94 -> 87, 64 x 12 x 512 326 -> 311, but 4 x 12 x 4096 680 -> 728.
-  a.dq_linear = l.dpad == 64 && (l.is_dropout || f->max_seqlen_q <= 512);
   if (int rc = make_tile_map(&l.tm_q, f->q, l.is_bf16, f->total_q, f->heads, f->head_dim,
                              f->q_row_stride, f->q_head_stride, 128, bind_context)) return rc;
   if (int rc = make_tile_map(&l.tm_k, f->k, l.is_bf16, f->total_k, f->heads, f->head_dim,

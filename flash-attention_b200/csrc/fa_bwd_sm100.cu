@@ -1004,15 +1004,13 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   } else {
     // ------------------------------------------------------------------ dQ group (warps 8-11)
     // dQ tile: tensor memory -> registers -> swizzled fp32 staging in shared memory -> one TMA
-    // reduce-add per [128 rows x 32 columns] box, or one bulk reduce-add of the whole block
-    // (dq_linear), into the fp32 accumulator.  Rows past the end of
+    // reduce-add per [128 rows x 32 columns] box into the fp32 accumulator.  Rows past the end of
     // the sequence hold exact zeros (their P is zero), rows past the tensor are clipped by TMA.
     if constexpr (D == 64) reg_dealloc<72>(); else reg_dealloc<88>();
     const int row = tid - 256;
     const uint32_t lane_sel = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t tDQ = tDQ_ + lane_sel;
     const uint32_t stage_addr = smem_u32(dq_stage);
-    const bool linear = a.dq_linear;
     bool ok = true;
     bool pending = false;  // thread `row == 0`: a reduce group of this CTA may still read the staging
     uint32_t sync_phase = 0;
@@ -1126,7 +1124,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           if (ok) {
 #pragma unroll
             for (int ch = 0; ch < 8; ++ch) {
-              const uint32_t off = (linear ? row * 256 + bx * 128 : bx * 16384 + row * 128) + ((ch ^ (row & 7)) << 4);
+              const uint32_t off = bx * 16384 + row * 128 + ((ch ^ (row & 7)) << 4);
               *reinterpret_cast<uint4*>(dq_stage + off) = make_uint4(r[4 * ch], r[4 * ch + 1], r[4 * ch + 2], r[4 * ch + 3]);
             }
           }
@@ -1139,15 +1137,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         if (row == 0) {
           if (deterministic && half == 0) my_turn = ticket_wait(t);
           if (my_turn) {
-            if (linear) {
-              // without the rows past the tensor; those past the sequence add zeros
-              const int rows = min(kBM, a.total_q - (q_start + m0));
-              if (rows > 0)
-                bulk_reduce_add_f32(a.dq_accum + (static_cast<int64_t>(h) * a.total_q + q_start + m0) * 64, stage_addr, rows * 256);
-            } else {
-              tma_reduce_add_3d(&tm_dq, stage_addr, half * 64, q_start + m0, h);
-              tma_reduce_add_3d(&tm_dq, stage_addr + 16384, half * 64 + 32, q_start + m0, h);
-            }
+            tma_reduce_add_3d(&tm_dq, stage_addr, half * 64, q_start + m0, h);
+            tma_reduce_add_3d(&tm_dq, stage_addr + 16384, half * 64 + 32, q_start + m0, h);
             bulk_commit();
             pending = true;
             if (deterministic && half == D / 64 - 1) { ticket_pass(t); pending = false; }
@@ -1211,7 +1202,7 @@ __global__ void bwd_preprocess_kernel(const BwdArgs a, int dpad) {
       acc += of.x * gf.x + of.y * gf.y;
     }
     // zero this thread's share of the fp32 dQ accumulator row (dpad floats per (row, head))
-    float* zr = a.dq_accum + (a.dq_linear ? static_cast<int64_t>(h) * a.total_q + row : row * ka.heads + h) * dpad;
+    float* zr = a.dq_accum + (row * ka.heads + h) * dpad;
     for (int z = (threadIdx.x % tpr) * 4; z < dpad; z += tpr * 4)
       *reinterpret_cast<float4*>(zr + z) = make_float4(0.f, 0.f, 0.f, 0.f);
   }
@@ -1226,19 +1217,20 @@ __global__ void bwd_postprocess_kernel(const BwdArgs a, int dpad) {
   const KernelArgs& ka = a.k;
   const int d = ka.head_dim;
   const int tpr = d / 8;
-  const int b = blockIdx.z, h = blockIdx.y;
-  const int q_start = ka.cu_seqlens_q[b];
-  const int i = blockIdx.x * (blockDim.x / tpr) + threadIdx.x / tpr, c = (threadIdx.x % tpr) * 8;
-  // Rows behind the last sequence (a token buffer larger than cu_seqlens_q[batch]) belong to nobody: dq
-  // keeps what the caller put in it, as in the reference, which only ever writes rows of a sequence.
-  if (i >= ka.cu_seqlens_q[b + 1] - q_start) return;
-  const int64_t row = q_start + i;
-  if (row >= a.total_q) return;
-  const float4* src = reinterpret_cast<const float4*>(
-      a.dq_accum + (a.dq_linear ? static_cast<int64_t>(h) * a.total_q + row : row * ka.heads + h) * dpad);
-  const int swap = a.dq_linear ? (i & 7) : 0;
-  const float4 x = src[(c / 4) ^ swap];
-  const float4 y = src[(c / 4 + 1) ^ swap];
+  const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t total = static_cast<int64_t>(a.total_q) * ka.heads * tpr;
+  if (idx >= total) return;
+  const int c = static_cast<int>(idx % tpr) * 8;
+  const int64_t rh = idx / tpr;
+  const int h = static_cast<int>(rh % ka.heads);
+  const int64_t row = rh / ka.heads;
+  // Rows behind the last sequence (a token buffer larger than cu_seqlens_q[batch]) belong to nobody:
+  // the accumulator was not cleared there and dq keeps what the caller put in it, as in the
+  // reference, which only ever writes rows of a sequence.
+  if (row >= ka.cu_seqlens_q[ka.batch]) return;
+  const float* src = a.dq_accum + rh * dpad + c;
+  const float4 x = *reinterpret_cast<const float4*>(src);
+  const float4 y = *reinterpret_cast<const float4*>(src + 4);
   const float f = ka.scale * ka.rp_keep;
   uint4 out;
   out.x = pack16<BF16>(x.x * f, x.y * f);
@@ -1310,12 +1302,12 @@ cudaError_t launch_bwd(const BwdLaunch& l, cudaStream_t stream) {
   }
   // 3. postprocess
   if (stages & 4) {
-    if (a.total_q > 0) {
+    const int64_t total = static_cast<int64_t>(a.total_q) * a.k.heads * (d / 8);
+    if (total > 0) {
       const int threads = 256;
-      const int rows_per_block = threads / (d / 8);
-      dim3 grid((a.max_seqlen_q + rows_per_block - 1) / rows_per_block, a.k.heads, a.k.batch);
-      if (l.is_bf16) bwd_postprocess_kernel<true><<<grid, threads, 0, stream>>>(a, l.dpad);
-      else bwd_postprocess_kernel<false><<<grid, threads, 0, stream>>>(a, l.dpad);
+      const int blocks = static_cast<int>((total + threads - 1) / threads);
+      if (l.is_bf16) bwd_postprocess_kernel<true><<<blocks, threads, 0, stream>>>(a, l.dpad);
+      else bwd_postprocess_kernel<false><<<blocks, threads, 0, stream>>>(a, l.dpad);
       cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) return e;
     }

@@ -39,11 +39,7 @@ struct BwdArgs {
   void* dq; void* dk; void* dv;
   int64_t dq_row_stride, dq_head_stride, dk_row_stride, dk_head_stride, dv_row_stride, dv_head_stride;
   float* softmax_d;
-  // fp32 dQ accumulator: [total_q, heads, Dpad], added to through a tensor map; or (dq_linear, Dpad = 64)
-  // [heads, total_q, 64], where the 128 rows of a query tile are one 32 KB block and the 16-byte units of
-  // row i of a sequence sit at unit ^ (i % 8), as in the staging buffer.
-  float* dq_accum;
-  bool dq_linear;
+  float* dq_accum;    // fp32 [total_q, heads, Dpad]
   // Deterministic mode: one ticket per (batch, head, 128-row query tile) = number of key tiles
   // that have added their dQ tile so far; nullptr = add in arrival order.
   int32_t* dq_tickets;

@@ -112,14 +112,6 @@ __device__ __forceinline__ void tma_reduce_add_3d(const void* tmap, uint32_t src
       : "l"(reinterpret_cast<uint64_t>(tmap)), "r"(src), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
-// `bytes` of fp32 values in shared memory added element-wise into global memory (both 16-byte aligned, bytes a
-// multiple of 16).
-__device__ __forceinline__ void bulk_reduce_add_f32(float* dst, uint32_t src, uint32_t bytes) {
-  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;"
-               :
-               : "l"(__cvta_generic_to_global(dst)), "r"(src), "r"(bytes)
-               : "memory");
-}
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // all committed bulk groups of this thread have finished reading their shared-memory source
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
