@@ -16,6 +16,7 @@ import os
 import struct
 
 import torch
+import torch.autograd.forward_ad as forward_ad
 
 from . import _lib
 from ._lib import BwdParams, FwdParams, check, lib
@@ -114,8 +115,13 @@ def _status_buffer(device):
 
 def compiled_attention(x):
     """The compiled module when the differentiable functions can run through it for input `x` (its
-    device's status buffer exists afterwards), else None."""
+    device's status buffer exists afterwards), else None.
+
+    Inside a forward-mode level the Python autograd classes serve the call: they refuse an input
+    that carries a tangent, which the compiled functions do not look at."""
     if _binding is not None:
+        if forward_ad._current_level >= 0:
+            return None
         i = x.get_device()
         if i >= 0 and i not in _status_known:
             _status_buffer(x.device)

@@ -8,7 +8,8 @@ packed tensor through strided views, as the reference does (:64-68, :100-106).
 
 With the compiled binding the same functions run through one C++ autograd node instead
 (csrc/fa_torch_binding.cpp, AttnNode): a forward + backward at batch 8 x 12 heads x 128 tokens with
-dropout is bound by the host.  The classes here serve return_attn_probs and the ctypes route.
+dropout is bound by the host.  The classes here serve return_attn_probs, the ctypes route and the
+calls that flash_attn_cuda.compiled_attention() leaves to them.
 """
 import torch
 

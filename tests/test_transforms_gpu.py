@@ -1,0 +1,41 @@
+"""Calls that something other than plain eager autograd watches: forward-mode tangents, traces, function
+transforms and compiled autograd.  The functions refuse what the Python autograd classes refuse and give the
+same numbers where those run."""
+import pytest
+import torch
+
+from tests import _util as U
+
+pytestmark = pytest.mark.gpu
+
+LAYOUTS = ("qkv", "kv", "separate", "sparse")
+
+
+def _call(layout, dropout_p=0.0, seed=0):
+    """(function of the packed inputs, those inputs) of a small call."""
+    from flash_attn_b200 import flash_attn_interface as fi
+    from flash_attn_b200.flash_blocksparse_attn_interface import flash_blocksparse_attn_func
+    lens = [150, 1, 77]
+    q, k, v, _, cu, _ = U.make_varlen(lens, lens, 2, 64, torch.float16, seed=seed)
+    s = max(lens)
+    if layout == "qkv":
+        return lambda x: fi.flash_attn_unpadded_qkvpacked_func(x, cu, s, dropout_p, causal=True), [torch.stack([q, k, v], 1)]
+    if layout == "sparse":
+        block = torch.ones(16, 1, dtype=torch.int32, device="cuda")
+        return lambda x: flash_blocksparse_attn_func(x, cu, block, dropout_p, s), [torch.stack([q, k, v], 1)]
+    if layout == "kv":
+        return (lambda x, y: fi.flash_attn_unpadded_kvpacked_func(x, y, cu, cu, s, s, dropout_p),
+                [q, torch.stack([k, v], 1)])
+    return lambda x, y, z: fi.flash_attn_unpadded_func(x, y, z, cu, cu, s, s, dropout_p), [q, k, v]
+
+
+@pytest.mark.parametrize("layout", LAYOUTS)
+def test_forward_mode_tangents_are_refused(layout):
+    import torch.autograd.forward_ad as fw
+    f, x = _call(layout)
+    with fw.dual_level():
+        y = f(*x)   # no tangent: an ordinary call
+        duals = [fw.make_dual(t, torch.ones_like(t)) if i == len(x) - 1 else t for i, t in enumerate(x)]
+        with pytest.raises(NotImplementedError, match="jvp"):
+            f(*duals)
+    assert torch.equal(y, f(*x))
