@@ -23,6 +23,7 @@
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 
 #include <array>
 #include <cmath>
@@ -512,6 +513,12 @@ at::Tensor convert_blockmask(const at::Tensor& layout, bool causal) {
   return out;
 }
 
+// Whether this thread records a trace or runs inside a function transform (vmap, grad, jvp ...).
+bool recording() {
+  return torch::jit::tracer::isTracing() ||
+         c10::impl::tls_is_dispatch_key_included(at::DispatchKey::FuncTorchDynamicLayerFrontMode);
+}
+
 void set_options(bool deterministic, int64_t mask_heads_total, int64_t mask_head_offset) {
   g_deterministic = deterministic;
   g_mask_heads_total = mask_heads_total;
@@ -534,6 +541,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attn", &attn);
   m.def("attn_sparse_qkvpacked", &attn_sparse_qkvpacked);
   m.def("convert_blockmask", &convert_blockmask);
+  m.def("recording", &recording);
   m.def("set_options", &set_options);
   m.def("set_status", &set_status);
 }

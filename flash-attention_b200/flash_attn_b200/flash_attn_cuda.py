@@ -117,10 +117,13 @@ def compiled_attention(x):
     """The compiled module when the differentiable functions can run through it for input `x` (its
     device's status buffer exists afterwards), else None.
 
-    Inside a forward-mode level the Python autograd classes serve the call: they refuse an input
-    that carries a tangent, which the compiled functions do not look at."""
+    Inside a forward-mode level and a function transform the Python autograd classes serve the call:
+    they refuse an input that carries a tangent or a transform's wrapper, which the compiled
+    functions do not look at.  While a trace is recorded they do too: a class is one operation of the
+    trace, where the compiled functions would leave the allocation of their output and nothing that
+    fills it."""
     if _binding is not None:
-        if forward_ad._current_level >= 0:
+        if forward_ad._current_level >= 0 or _binding.recording():
             return None
         i = x.get_device()
         if i >= 0 and i not in _status_known:

@@ -39,3 +39,22 @@ def test_forward_mode_tangents_are_refused(layout):
         with pytest.raises(NotImplementedError, match="jvp"):
             f(*duals)
     assert torch.equal(y, f(*x))
+
+
+@pytest.mark.parametrize("layout", LAYOUTS)
+def test_a_trace_replays_on_new_inputs(layout):
+    f, x = _call(layout)
+    traced = torch.jit.trace(lambda *a: f(*a) * 2, tuple(x), check_trace=False)
+    new = _call(layout, seed=1)[1]
+    poison = [torch.full((228, 2, 64), float("nan"), dtype=torch.float16, device="cuda") for _ in range(8)]
+    del poison  # a replay that leaves its output unfilled finds these
+    assert torch.equal(traced(*new), f(*new) * 2)
+
+
+@pytest.mark.parametrize("layout", LAYOUTS)
+def test_function_transforms_are_refused(layout):
+    f, x = _call(layout)
+    with pytest.raises(RuntimeError, match="setup_context"):
+        torch.func.grad(lambda *a: f(*a).float().sum())(*x)
+    with pytest.raises(RuntimeError, match="setup_context"):
+        torch.vmap(lambda *a: f(*a))(*[t[None].expand(2, *t.shape) for t in x])
