@@ -132,6 +132,17 @@ def compiled_attention(x):
     return _binding
 
 
+def runs_now(x):
+    """True when a kernel of the library may take the place of framework operations on the CUDA tensor
+    `x`: a plain tensor with storage, and nothing that records, compiles, transforms or fakes the
+    operations (which would see neither the kernel nor what it writes)."""
+    if torch.compiler.is_compiling() or not x.is_cuda:
+        return False
+    return (type(x) in (torch.Tensor, torch.nn.Parameter) and x.layout is torch.strided
+            and not x._is_zerotensor() and torch._C._len_torch_dispatch_stack() == 0
+            and torch._C._get_tracing_state() is None and not torch._C._are_functorch_transforms_active())
+
+
 def check_device_status(device=None):
     """Synchronises and raises if any kernel on `device` reported an abandoned wait."""
     device = torch.device("cuda", torch.cuda.current_device()) if device is None else device

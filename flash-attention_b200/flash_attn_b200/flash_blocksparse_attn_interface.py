@@ -9,6 +9,18 @@ import torch
 from . import flash_attn_cuda
 
 
+# element types whose zero test the conversion kernel knows (it looks at the bits)
+_LAYOUT_DTYPES = frozenset((torch.bool, torch.uint8, torch.int8, torch.int16, torch.int32, torch.int64,
+                            torch.float16, torch.bfloat16, torch.float32, torch.float64))
+
+
+def _conversion_kernel_path(layout):
+    """Layouts the conversion kernel takes (its limits are fa_convert_blockmask's); the framework
+    operations below convert all others."""
+    return (flash_attn_cuda.runs_now(layout) and layout.dim() == 2 and layout.dtype in _LAYOUT_DTYPES
+            and 0 < layout.shape[0] < 2 ** 24 and 0 < layout.shape[1] < 2 ** 20)
+
+
 def convert_blockmask(blockmask, causal):
     """0/1 layout (rows, cols) -> int32 (cols, rows): row c lists, in ascending order, 4 * r for
     every non-zero (r, c), plus 1 when c is the first non-zero column of row r and plus 2 when it
@@ -22,7 +34,7 @@ def convert_blockmask(blockmask, causal):
     iteration index follows the visit lists alone (csrc/flash_attn/src/
     fmha_block_fprop_kernel_1xN.h:205-232 takes its loop bounds from the block mask, with no
     causal start row)."""
-    if blockmask.is_cuda and blockmask.dim() == 2 and not blockmask.is_complex():
+    if _conversion_kernel_path(blockmask):
         native = flash_attn_cuda.compiled_attention(blockmask)
         if native is not None:   # one launch instead of two dozen
             return native.convert_blockmask(blockmask, bool(causal))

@@ -58,3 +58,54 @@ def test_function_transforms_are_refused(layout):
         torch.func.grad(lambda *a: f(*a).float().sum())(*x)
     with pytest.raises(RuntimeError, match="setup_context"):
         torch.vmap(lambda *a: f(*a))(*[t[None].expand(2, *t.shape) for t in x])
+
+
+def _convert_cases():
+    from flash_attn_b200.flash_blocksparse_attn_interface import convert_blockmask
+    g = torch.Generator().manual_seed(3)
+    a, b = [(torch.rand(64, 5, generator=g) < 0.4).int().cuda() for _ in range(2)]
+    return convert_blockmask, a, b
+
+
+def test_convert_blockmask_in_a_trace():
+    convert, a, b = _convert_cases()
+    traced = torch.jit.trace(lambda m: convert(m, False), (a,), check_trace=False)
+    assert torch.equal(traced(b), convert(b, False))
+
+
+def test_convert_blockmask_in_make_fx():
+    from torch.fx.experimental.proxy_tensor import make_fx
+    convert, a, b = _convert_cases()
+    for mode in ("real", "fake"):
+        graph = make_fx(lambda m: convert(m, True), tracing_mode=mode)(a)
+        assert torch.equal(graph(b), convert(b, True)), mode
+
+
+def test_convert_blockmask_under_vmap():
+    convert, a, b = _convert_cases()
+    got = torch.vmap(lambda m: convert(m, False))(torch.stack([a, b]))
+    assert torch.equal(got, torch.stack([convert(a, False), convert(b, False)]))
+
+
+def test_convert_blockmask_on_fake_tensors():
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    convert, a, _ = _convert_cases()
+    with FakeTensorMode() as mode:
+        fake = convert(mode.from_tensor(a), False)
+    assert fake.shape == (5, 64) and fake.dtype is torch.int32
+
+
+def test_convert_blockmask_in_a_full_graph_compile():
+    convert, a, b = _convert_cases()
+    f = torch.compile(lambda m: convert(m, False), backend="eager", fullgraph=True)
+    assert torch.equal(f(a), convert(a, False)) and torch.equal(f(b), convert(b, False))
+
+
+def test_layouts_the_conversion_kernel_does_not_take():
+    """Types whose zeros are not a bit pattern of their own, and empty layouts: what the framework operations
+    accept and refuse."""
+    convert, a, _ = _convert_cases()
+    assert torch.equal(convert(a.to(torch.complex64), False), convert(a, False))
+    assert convert(a[:0], False).shape == (5, 0)
+    with pytest.raises(IndexError):
+        convert(a[:, :0], False)
