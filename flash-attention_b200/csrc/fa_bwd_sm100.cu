@@ -142,7 +142,13 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   __shared__ BwdShared sh;
 
   const int tid = threadIdx.x;
-  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // known to be the same in all lanes
+  // Known to be the same in all lanes, for the issuing warps (see mma_ss).  The compute and dQ groups take
+  // theirs anew and the epilogue works from tid: with one value kept live across all roles short
+  // calls at d = 64 lost 1-3 % to lane-0 issue, and spill loads there went from 24 to 76 bytes a thread (32
+  // with the values taken anew).  us of the whole backward, lane 0 issuing -> one value -> now: 16 x 8 heads,
+  // 200 queries, 1500 keys 79.1 -> 81.2 -> 76.4; 64 x 12 x 512 289 -> 293 -> 271; 2 x 4 x 32768 causal
+  // 3632 -> 3309 -> 3226.
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int lane = tid & 31;
   const int b = blockIdx.z;
   const int h = blockIdx.y;
@@ -540,9 +546,10 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     // ------------------------------------------------------------------ compute groups
     // group w (0 / 1) owns key columns [64 w, 64 w + 64) of the tile; one thread per query row
     if constexpr (D == 64) reg_alloc<192>(); else reg_alloc<176>();
-    const int w = warp >> 2;
+    const int cwarp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const int w = cwarp >> 2;
     const int row = tid & 127;
-    const uint32_t lane_sel = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const uint32_t lane_sel = static_cast<uint32_t>((cwarp & 3) * 32) << 16;
     const uint32_t tS = tS_ + lane_sel + w * 64;
     const uint32_t tDP = tDP_ + lane_sel + w * 64;
     const int64_t bh_sub =
@@ -568,7 +575,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       // columns of every 8-column unit, which is the ownership pattern of the reference's mask
       // generator (one Philox call = one thread's part of a 16 x 16 patch, QuadPhilox).  The packed
       // pairs go to the swizzled P~ / dS tiles with stmatrix (8 x 8 matrices = 16-byte row chunks).
-      const int wq = warp & 3, lane = tid & 31;
+      const int wq = cwarp & 3, lane = tid & 31;
       const int r8 = lane >> 2, q4 = lane & 3;
       constexpr uint32_t kHalf = 16u << 16;
       QuadPhilox<4> qp;
@@ -977,10 +984,11 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     }
     if (ok) {
       tc_fence_after();
-      const uint32_t tAcc = (w == 0 ? tDV_ : tDK_) + lane_sel;
-      const float f = (w == 0) ? rp_keep : ka.scale * rp_keep;
+      const int grp = tid >> 7;
+      const uint32_t tAcc = (grp == 0 ? tDV_ : tDK_) + (static_cast<uint32_t>(((tid >> 5) & 3) * 32) << 16);
+      const float f = (grp == 0) ? rp_keep : ka.scale * rp_keep;
       const int kr = n0 + row;
-      uint16_t* dst_row = (w == 0)
+      uint16_t* dst_row = (grp == 0)
           ? dv_base + static_cast<int64_t>(k_start + kr) * a.dv_row_stride + static_cast<int64_t>(h) * a.dv_head_stride
           : dk_base + static_cast<int64_t>(k_start + kr) * a.dk_row_stride + static_cast<int64_t>(h) * a.dk_head_stride;
 #pragma unroll
@@ -1008,7 +1016,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     // the sequence hold exact zeros (their P is zero), rows past the tensor are clipped by TMA.
     if constexpr (D == 64) reg_dealloc<72>(); else reg_dealloc<88>();
     const int row = tid - 256;
-    const uint32_t lane_sel = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const uint32_t lane_sel = static_cast<uint32_t>((__shfl_sync(0xffffffffu, tid >> 5, 0) & 3) * 32) << 16;
     const uint32_t tDQ = tDQ_ + lane_sel;
     const uint32_t stage_addr = smem_u32(dq_stage);
     bool ok = true;
