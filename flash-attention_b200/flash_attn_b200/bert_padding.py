@@ -11,6 +11,7 @@ import torch
 import torch.nn.functional as F
 
 from ._lib import check, lib
+from .flash_attn_cuda import runs_now
 
 
 def _kernel_path(values, indices):
@@ -93,7 +94,7 @@ index_put_first_axis = IndexPutFirstAxis.apply
 
 def _mask_kernel_path(mask):
     """Boolean masks only: with integer masks the lengths are the sums of the values."""
-    return (mask.is_cuda and mask.dtype is torch.bool and mask.dim() == 2 and mask.is_contiguous()
+    return (runs_now(mask) and mask.dtype is torch.bool and mask.dim() == 2 and mask.is_contiguous()
             and 0 < mask.numel() < 2 ** 31)
 
 

@@ -109,3 +109,14 @@ def test_layouts_the_conversion_kernel_does_not_take():
     assert convert(a[:0], False).shape == (5, 0)
     with pytest.raises(IndexError):
         convert(a[:, :0], False)
+
+
+def test_unpad_input_in_a_trace():
+    from flash_attn_b200 import bert_padding as bp
+    g = torch.Generator(device="cuda").manual_seed(4)
+    x = torch.randn(3, 40, 16, device="cuda", generator=g).half()
+    mask = torch.arange(40, device="cuda")[None] < torch.tensor([[40], [7], [23]], device="cuda")
+    traced = torch.jit.trace(lambda t, m: bp.unpad_input(t, m)[:3], (x, mask), check_trace=False)
+    other = mask.flip(0, 1)   # as many valid tokens, elsewhere
+    for got, want in zip(traced(x, other), bp.unpad_input(x, other)[:3]):
+        assert torch.equal(got, want)
