@@ -120,3 +120,31 @@ def test_unpad_input_in_a_trace():
     other = mask.flip(0, 1)   # as many valid tokens, elsewhere
     for got, want in zip(traced(x, other), bp.unpad_input(x, other)[:3]):
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("compiler", ["graph", "dynamo"])
+@pytest.mark.parametrize("layout,dropout_p", [("qkv", 0.0), ("qkv", 0.2), ("kv", 0.2), ("separate", 0.0), ("sparse", 0.1)])
+def test_compiled_autograd_gives_the_same_gradients(layout, dropout_p, compiler):
+    import torch._dynamo.compiled_autograd as ca
+    from flash_attn_b200 import flash_attn_cuda as fc
+    fc.options.deterministic = True
+    try:
+        for step in range(2):   # the second pass takes the graph of the first, with another mask
+            grads = []
+            for compiled in (False, True):
+                f, x = _call(layout, dropout_p, seed=step)
+                torch.cuda.manual_seed(5 + step)
+                for t in x:
+                    t.requires_grad_()
+                out = f(*x)
+                dout = torch.sin(torch.arange(out.numel(), device="cuda")).reshape(out.shape).half()
+                if compiled:
+                    with ca._enable((lambda gm: gm) if compiler == "graph" else lambda gm: torch.compile(gm, backend="eager")):
+                        out.backward(dout)
+                else:
+                    out.backward(dout)
+                grads.append([t.grad for t in x])
+            for a, b in zip(*grads):
+                assert torch.equal(a, b)
+    finally:
+        fc.options.deterministic = False
