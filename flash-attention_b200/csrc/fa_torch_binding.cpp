@@ -27,6 +27,7 @@
 #include <torch/csrc/jit/frontend/tracer.h>
 
 #include <array>
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <limits>
@@ -364,7 +365,14 @@ py::list bwd(const at::Tensor& dout, const at::Tensor& q, const at::Tensor& k, c
 // Process-wide options of the Python binding (flash_attn_cuda.options), mirrored here by its setters:
 // the backward runs on an autograd thread that does not hold the interpreter.
 std::atomic<bool> g_deterministic{false};
-std::atomic<int64_t> g_mask_heads_total{0}, g_mask_head_offset{0};
+// Head shard of the dropout mask: (total << 32 | offset) in one word, so that a backward on an autograd
+// thread never sees the total of one shard with the offset of another.
+std::atomic<uint64_t> g_mask_heads{0};
+struct MaskHeads { int64_t total, offset; };
+MaskHeads mask_heads() {
+  const uint64_t v = g_mask_heads.load();
+  return {static_cast<int32_t>(v >> 32), static_cast<int32_t>(v)};
+}
 // Per-device status buffer of the kernels (owned by the Python module, lives as long as the process).
 constexpr int kMaxDevices = 64;
 std::atomic<int64_t> g_status[kMaxDevices];
@@ -416,8 +424,9 @@ torch::autograd::variable_list attention_backward(const at::Tensor* x, int layou
   require(g.q.last_stride == 1 && g.k.last_stride == 1 && g.v.last_stride == 1,
           "dq, dk, dv must have a contiguous last dimension");
   at::Tensor softmax_d = at::empty_like(l);
+  const MaskHeads mh = mask_heads();
   const BwdCall c{k.max_q, k.max_k, k.p_dropout, k.scale, k.causal, g_deterministic.load(), 0, k.seed, k.offset,
-                  g_mask_heads_total.load(), g_mask_head_offset.load(), status_of(o.device())};
+                  mh.total, mh.offset, status_of(o.device())};
   run_bwd(s, v.q, v.k, v.v, dout, o, l, g.q, g.k, g.v, static_cast<float*>(softmax_d.data_ptr()), cq, ck,
           bm.defined() ? &bm : nullptr, c);
   return result;
@@ -511,8 +520,8 @@ at::Tensor attention(const at::Tensor* x, int layout, const at::Tensor& cu_q, co
     c10::NoGradGuard no_grad;
     at::AutoDispatchBelowADInplaceOrView below;
     const Operands v = cut(x, layout);
-    const FwdCall c{max_q, max_k, p_dropout, scale, false, causal, false,
-                    g_mask_heads_total.load(), g_mask_head_offset.load(), status_of(x[0].device())};
+    const MaskHeads mh = mask_heads();
+    const FwdCall c{max_q, max_k, p_dropout, scale, false, causal, false, mh.total, mh.offset, status_of(x[0].device())};
     r = run_fwd(v.q, v.k, v.v, x[0].options(), cu_q, cu_k, blockmask, c, c10::nullopt);
   }
   if (needs_grad) {
@@ -581,8 +590,9 @@ bool recording() {
 
 void set_options(bool deterministic, int64_t mask_heads_total, int64_t mask_head_offset) {
   g_deterministic = deterministic;
-  g_mask_heads_total = mask_heads_total;
-  g_mask_head_offset = mask_head_offset;
+  // (the kernels take 32-bit values; a call refuses an offset its total does not cover)
+  const auto word = [](int64_t v) { return static_cast<uint32_t>(std::min<int64_t>(std::max<int64_t>(v, -1), INT32_MAX)); };
+  g_mask_heads = (static_cast<uint64_t>(word(mask_heads_total)) << 32) | word(mask_head_offset);
 }
 
 void set_status(int64_t device_index, int64_t ptr) {

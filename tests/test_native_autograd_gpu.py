@@ -67,3 +67,34 @@ def test_backward_twice_is_refused():
     out.backward(dout)
     with pytest.raises(RuntimeError, match="second time"):
         out.backward(dout)
+
+
+def test_head_shard_changes_as_one_value():
+    """Backward passes on the autograd thread while another thread enters and leaves head_shard: every pass sees one
+    shard or the other, never the total of one with the offset of the other (which the call would refuse)."""
+    import sys
+    import threading
+    from flash_attn_b200 import flash_attn_cuda as fc
+    from flash_attn_b200.flash_attn_interface import flash_attn_unpadded_qkvpacked_func
+    q, k, v, dout, cu, _ = U.make_varlen([16], [16], 2, 64, torch.float16, seed=1)
+    qkv = torch.stack([q, k, v], dim=1).requires_grad_()
+    stop = threading.Event()
+
+    def toggle():
+        while not stop.is_set():
+            fc.options.mask_heads = (8, 6)
+            fc.options.mask_heads = (2, 0)
+
+    out = flash_attn_unpadded_qkvpacked_func(qkv, cu, 16, 0.1)
+    thread = threading.Thread(target=toggle)
+    interval = sys.getswitchinterval()
+    sys.setswitchinterval(1e-6)   # the two threads take turns on the interpreter
+    thread.start()
+    try:
+        for _ in range(10000):
+            torch.autograd.grad(out, qkv, dout, retain_graph=True)
+    finally:
+        stop.set()
+        thread.join()
+        sys.setswitchinterval(interval)
+        fc.options.mask_heads = None
