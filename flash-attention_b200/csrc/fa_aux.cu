@@ -1,4 +1,5 @@
 // Small helper kernels: dropout-mask dump (test hook), block-sparse iteration table.
+#include <algorithm>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <curand_kernel.h>
@@ -55,31 +56,40 @@ __device__ __forceinline__ int visited_prefix(const int32_t* row, int nr, int sq
 
 // Output rows no attention CTA writes (rows outside every sequence, and rows at or beyond the 128-row
 // tiles that max_seqlen_q covers) are zero in a block-sparse call (fmha_api.cpp:519 starts from
-// o = 0); zeroing the few there are replaces a pass over the whole tensor.
+// o = 0); zeroing the few there are replaces a pass over the whole tensor.  A token buffer of fixed size
+// may leave most of its rows unused: CTAs of their own share the rows in front of and behind the sequences, one
+// per 32 KB of o up to four per SM (those that find nothing to do read two integers).  12 x 64 heads,
+// 4 x 512 tokens, 100 000 unused rows, us of the whole call: 64 with the full pass, 2462 with one CTA, 42 so.
 struct ZeroRows {
   uint4* o;          // nullptr: nothing to zero
   int64_t row_vecs;  // 16-byte units per (contiguous) row
   int32_t total_q, max_q_tiles;  // rows per sequence that the attention grid covers
 };
+constexpr int kZeroCtaBytes = 32768, kZeroMaxCtas = 4 * 148;
 
-__device__ __forceinline__ void zero_rows(const ZeroRows& z, int64_t first, int64_t last) {
-  for (int64_t i = first * z.row_vecs + threadIdx.x; i < last * z.row_vecs; i += blockDim.x)
+__device__ __forceinline__ void zero_rows(const ZeroRows& z, int64_t first, int64_t last, int part, int parts) {
+  for (int64_t i = first * z.row_vecs + static_cast<int64_t>(part) * blockDim.x + threadIdx.x; i < last * z.row_vecs;
+       i += static_cast<int64_t>(parts) * blockDim.x)
     z.o[i] = make_uint4(0, 0, 0, 0);
 }
 
+// CTAs [0, nk * batch): key block bid % nk of batch entry bid / nk; the CTAs behind them zero rows.
 __global__ void __launch_bounds__(kTableThreads)
 bs_table_kernel(int32_t* table, const int32_t* blockmask, const int32_t* cu_q, const int32_t* cu_k, int nk, int nr,
                 int batch, ZeroRows z) {
   __shared__ int sum[kTableThreads / 32];
-  const int kb = blockIdx.x, b = blockIdx.y;
+  const int b = blockIdx.x / nk, kb = blockIdx.x - b * nk;
+  if (b >= batch) {
+    const int part = blockIdx.x - nk * batch, parts = gridDim.x - nk * batch;
+    zero_rows(z, 0, min(cu_q[0], z.total_q), part, parts);
+    zero_rows(z, max(cu_q[batch], 0), z.total_q, part, parts);
+    return;
+  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sq = cu_q[b + 1] - cu_q[b];
   const int sk = cu_k[b + 1] - cu_k[b];
-  if (z.o != nullptr && kb == 0) {
-    if (b == 0) zero_rows(z, 0, min(cu_q[0], z.total_q));
-    zero_rows(z, static_cast<int64_t>(cu_q[b]) + min(sq, z.max_q_tiles), min(cu_q[b + 1], z.total_q));
-    if (b == batch - 1) zero_rows(z, max(cu_q[batch], 0), z.total_q);
-  }
+  if (z.o != nullptr)
+    zero_rows(z, static_cast<int64_t>(cu_q[b]) + min(sq, z.max_q_tiles), min(cu_q[b + 1], z.total_q), kb, nk);
   int32_t* trow = table + (static_cast<int64_t>(b) * nk + kb) * nr;
   for (int i = threadIdx.x; i < nr; i += kTableThreads) trow[i] = -1;
   if (kb * 256 >= sk) return;
@@ -261,7 +271,10 @@ cudaError_t launch_bs_table(int32_t* table, const int32_t* blockmask, const int3
                             const int32_t* cu_k, int batch, int nk, int nr, void* o, int64_t o_row_bytes,
                             int total_q, int max_seqlen_q, cudaStream_t stream) {
   const ZeroRows z{static_cast<uint4*>(o), o_row_bytes / 16, total_q, (max_seqlen_q + 127) / 128 * 128};
-  bs_table_kernel<<<dim3(nk, batch), kTableThreads, 0, stream>>>(table, blockmask, cu_q, cu_k, nk, nr, batch, z);
+  int64_t zero_ctas = 0;
+  if (o != nullptr) zero_ctas = std::min<int64_t>(o_row_bytes * total_q / kZeroCtaBytes + 1, kZeroMaxCtas);
+  bs_table_kernel<<<static_cast<unsigned>(nk * batch + zero_ctas), kTableThreads, 0, stream>>>(table, blockmask, cu_q, cu_k,
+                                                                                               nk, nr, batch, z);
   return cudaGetLastError();
 }
 

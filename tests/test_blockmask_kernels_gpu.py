@@ -41,3 +41,39 @@ def test_rows_outside_the_sequences_are_zero(lens):
     want = fc.fwd_block(q, k, v, cu, cu, conv, s, s, 0.0, 0.125, False, False, None)[0]
     assert torch.equal(out[7:7 + sum(lens)], want)
     assert not out[:7].any() and not out[7 + sum(lens):].any()
+
+
+def _poisoned(shape, call):
+    """call()[0] in memory that held NaN: every free block of its size is filled first."""
+    garbage = [torch.full(shape, float("nan"), device="cuda", dtype=torch.float16) for _ in range(64)]
+    nbytes = garbage[0].numel() * 2
+    ranges = [(g.data_ptr(), g.data_ptr() + nbytes) for g in garbage]
+    del garbage
+    out = call()[0]
+    assert any(lo <= out.data_ptr() < hi for lo, hi in ranges), "the allocator handed out other memory"
+    return out
+
+
+@pytest.mark.parametrize("front,behind", [(0, 0), (1, 0), (0, 1), (2999, 4001), (20000, 3)])
+def test_unused_rows_of_a_token_buffer_are_zero(front, behind):
+    from flash_attn_b200 import flash_attn_cuda as fc
+    lens = [300, 0, 77]
+    n = sum(lens)
+    conv = torch.full((2, 32), -1, dtype=torch.int32, device="cuda")
+    conv[:, :19] = 4 * torch.arange(19, device="cuda")   # every block of the longest sequence
+    q, k, v, _, cu, _ = U.make_varlen(lens, lens, 2, 64, torch.float16, seed=6)
+    pad = [torch.nn.functional.pad(t, (0, 0, 0, 0, front, behind), value=3.0) for t in (q, k, v)]
+    out = _poisoned(pad[0].shape, lambda: fc.fwd_block(*pad, cu + front, cu + front, conv, 300, 300, 0.0, 0.125, False, False, None))
+    want = fc.fwd_block(q, k, v, cu, cu, conv, 300, 300, 0.0, 0.125, False, False, None)[0]
+    assert torch.equal(out[front:front + n], want) and want.any()
+    assert not out[:front].any() and not out[front + n:].any()
+
+
+def test_rows_beyond_the_covered_tiles_are_zero():
+    """A sequence longer than the 128 rows max_seqlen_q announces."""
+    from flash_attn_b200 import flash_attn_cuda as fc
+    q, k, v, _, cu_q, cu_k = U.make_varlen([300, 13], [128, 13], 2, 64, torch.float16, seed=7)
+    conv = (4 * torch.arange(16, dtype=torch.int32, device="cuda"))[None].contiguous()
+    out = _poisoned(q.shape, lambda: fc.fwd_block(q, k, v, cu_q, cu_k, conv, 128, 128, 0.0, 0.125, False, False, None))
+    assert not out[128:300].any()
+    assert torch.isfinite(out).all() and out[:128].any() and out[300:].any()
