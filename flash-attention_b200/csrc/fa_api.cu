@@ -171,8 +171,8 @@ void fill_dropout(const fa_fwd_params* p, fa::KernelArgs* a) {
 }
 
 // Block-sparse: check the scratch, build the block-visit table on the stream, point the kernel
-// arguments at it.  `forward`: also zero the rows of o that no attention CTA writes.
-int setup_blocksparse(const fa_fwd_params* p, fa::KernelArgs* a, bool forward, cudaStream_t stream) {
+// arguments at it.  `zero_unused`: also zero the rows of o that no attention CTA writes.
+int setup_blocksparse(const fa_fwd_params* p, fa::KernelArgs* a, bool zero_unused, cudaStream_t stream) {
   const int nk = p->blockmask_rows;
   const int nr = p->blockmask_cols;
   FA_REQUIRE(nk >= round_up(p->max_seqlen_k, 256) / 256, "blockmask has too few key-block rows");
@@ -187,7 +187,7 @@ int setup_blocksparse(const fa_fwd_params* p, fa::KernelArgs* a, bool forward, c
   int32_t* table = static_cast<int32_t*>(p->bs_workspace);
   // a caller with its own row stride keeps what lies between its rows
   const int64_t row = static_cast<int64_t>(p->heads) * p->head_dim;
-  const bool zero = forward && p->o_head_stride == p->head_dim && p->o_row_stride == row;
+  const bool zero = zero_unused && p->o_head_stride == p->head_dim && p->o_row_stride == row;
   FA_CUDA(fa::launch_bs_table(table, p->blockmask, p->cu_seqlens_q, p->cu_seqlens_k, p->batch, nk, nr,
                               zero ? p->o : nullptr, row * 2, p->total_q, p->max_seqlen_q, stream));
   a->bs_iter = table;
@@ -333,7 +333,7 @@ uint64_t fa_philox_increment(int32_t head_dim, int32_t max_seqlen_q, int32_t max
   return steps * mmas_n * 8 * loop_steps;
 }
 
-int fa_fwd(const fa_fwd_params* p, void* cuda_stream) {
+static int run_fwd(const fa_fwd_params* p, bool zero_unused, void* cuda_stream) {
   if (int rc = validate_common(p)) return rc;
   FA_REQUIRE(p->o && p->softmax_lse, "o and softmax_lse must be non-null");
   FA_REQUIRE((reinterpret_cast<uintptr_t>(p->o) & 15) == 0, "o must be 16-byte aligned");
@@ -346,7 +346,7 @@ int fa_fwd(const fa_fwd_params* p, void* cuda_stream) {
   std::memset(&l, 0, sizeof(l));
   fill_args(p, &l.args);
   if (p->blockmask)
-    if (int rc = setup_blocksparse(p, &l.args, true, static_cast<cudaStream_t>(cuda_stream))) return rc;
+    if (int rc = setup_blocksparse(p, &l.args, zero_unused, static_cast<cudaStream_t>(cuda_stream))) return rc;
   l.dpad = p->head_dim <= 64 ? 64 : 128;
   l.is_bf16 = p->is_bf16 != 0;
   l.is_causal = p->is_causal != 0;
@@ -374,6 +374,12 @@ int fa_fwd(const fa_fwd_params* p, void* cuda_stream) {
                               p->k_row_stride, p->k_head_stride, l.args, p->max_seqlen_q, p->max_seqlen_k,
                               l.is_bf16, l.is_causal, l.is_dropout, static_cast<cudaStream_t>(cuda_stream)));
   return FA_OK;
+}
+
+int fa_fwd(const fa_fwd_params* p, void* cuda_stream) { return run_fwd(p, false, cuda_stream); }
+
+int fa_fwd_ex(const fa_fwd_params* p, int32_t zero_unused_rows, void* cuda_stream) {
+  return run_fwd(p, zero_unused_rows != 0, cuda_stream);
 }
 
 int fa_debug_dropout_mask(uint8_t* mask_out, int32_t batch_idx, int32_t head_idx,

@@ -241,7 +241,7 @@ FwdResult run_fwd(const View& q, const View& k, const View& v, const at::TensorO
     p.s_cols = sk_r;
   }
   if (sparse) bs_ws = attach_blockmask(p, *blockmask, s.batch);
-  check_rc(fa_fwd(&p, at::cuda::getCurrentCUDAStream().stream()));
+  check_rc(fa_fwd_ex(&p, sparse ? 1 : 0, at::cuda::getCurrentCUDAStream().stream()));
   return r;
 }
 

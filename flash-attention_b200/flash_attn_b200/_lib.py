@@ -18,6 +18,7 @@ FA_STATIC_SCRATCH_BYTES = 8 << 20
 
 EXPORTED_SYMBOLS = (
     "fa_fwd",
+    "fa_fwd_ex",
     "fa_bwd",
     "fa_bwd_static_scratch",
     "fa_bwd_workspace_bytes",
@@ -114,6 +115,8 @@ def _load():
     lib = ctypes.CDLL(LIB_PATH)
     lib.fa_fwd.argtypes = [ctypes.POINTER(FwdParams), ctypes.c_void_p]
     lib.fa_fwd.restype = ctypes.c_int
+    lib.fa_fwd_ex.argtypes = [ctypes.POINTER(FwdParams), ctypes.c_int32, ctypes.c_void_p]
+    lib.fa_fwd_ex.restype = ctypes.c_int
     lib.fa_bwd.argtypes = [ctypes.POINTER(BwdParams), ctypes.c_void_p]
     lib.fa_bwd.restype = ctypes.c_int
     lib.fa_bwd_static_scratch.argtypes = [ctypes.POINTER(BwdParams), ctypes.c_void_p]

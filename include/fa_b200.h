@@ -114,9 +114,12 @@ typedef struct fa_bwd_params {
 } fa_bwd_params;
 
 /* mha_fwd (csrc/flash_attn/fmha_api.cpp:173-299) and, with blockmask != NULL, mha_fwd_block
- * (:451-573).  Writes o and softmax_lse.  A block-sparse call with a contiguous o also zeroes the rows
- * of o that lie outside the sequences (the reference starts from o = 0, :519). */
+ * (:451-573).  Writes the rows of o and softmax_lse that belong to the sequences and no others. */
 int fa_fwd(const fa_fwd_params* params, void* cuda_stream);
+
+/* fa_fwd; with zero_unused_rows != 0 a block-sparse call with a contiguous o also zeroes the rows of o
+ * that lie outside the sequences, in the same launches (mha_fwd_block starts from o = 0, :519). */
+int fa_fwd_ex(const fa_fwd_params* params, int32_t zero_unused_rows, void* cuda_stream);
 
 /* mha_bwd (csrc/flash_attn/fmha_api.cpp:302-449) and, with blockmask != NULL, mha_bwd_block
  * (:575-718).  Writes dq, dk, dv and softmax_d. */

@@ -77,3 +77,36 @@ def test_rows_beyond_the_covered_tiles_are_zero():
     out = _poisoned(q.shape, lambda: fc.fwd_block(q, k, v, cu_q, cu_k, conv, 128, 128, 0.0, 0.125, False, False, None))
     assert not out[128:300].any()
     assert torch.isfinite(out).all() and out[:128].any() and out[300:].any()
+
+
+@pytest.mark.parametrize("zero_unused,strided", [(0, False), (1, False), (1, True)])
+def test_c_entry_points_and_rows_outside_the_sequences(zero_unused, strided):
+    """fa_fwd writes the rows of the sequences and no others; fa_fwd_ex zeroes the others on request, unless o has a
+    row stride of its own."""
+    import ctypes
+    from flash_attn_b200 import flash_attn_cuda as fc
+    from flash_attn_b200._lib import check, lib
+    lens, front, behind, heads, d = [200, 57], 5, 9, 2, 64
+    n = sum(lens)
+    conv = (4 * torch.arange(16, dtype=torch.int32, device="cuda"))[None].contiguous()
+    q, k, v, _, cu, _ = U.make_varlen(lens, lens, heads, d, torch.float16, seed=8)
+    want = fc.fwd_block(q, k, v, cu, cu, conv, 200, 200, 0.0, 0.125, False, False, None)[0]
+    pad = [torch.nn.functional.pad(t, (0, 0, 0, 0, front, behind), value=3.0) for t in (q, k, v)]
+    total = n + front + behind
+    wide = torch.full((total, heads + (1 if strided else 0), d), 7.0, dtype=torch.float16, device="cuda")
+    o = wide[:, :heads]
+    lse = torch.empty(2, heads, 208, device="cuda")
+    shifted = cu + front
+    p = fc._make_fwd((2, total, total, heads, d), *pad, o, lse, shifted, shifted, 200, 200, 0.0, 0.125, False, 0, 0)
+    ws = fc._bs_workspace(q.device, 2, conv)
+    p.blockmask, (p.blockmask_rows, p.blockmask_cols) = conv.data_ptr(), conv.shape
+    p.bs_workspace, p.bs_workspace_bytes = ws.data_ptr(), ws.numel()
+    if zero_unused:
+        check(lib.fa_fwd_ex(ctypes.byref(p), 1, fc._raw_stream()))
+    else:
+        check(lib.fa_fwd(ctypes.byref(p), fc._raw_stream()))
+    assert torch.equal(o[front:front + n], want)
+    outside = torch.cat([wide[:front], wide[front + n:]])
+    assert (outside == (0.0 if zero_unused and not strided else 7.0)).all()
+    if strided:
+        assert (wide[:, heads] == 7.0).all()
