@@ -853,20 +853,51 @@ cudaError_t launch_groups(const FwdLaunch& l, cudaStream_t stream) {
 //   dropout   64 x 128: 39 -> 26   64 x 512: 162 -> 143  32 x 1024: 251 -> 229   8 x 4096: 770 -> 736
 //   d = 128   64 x 128: 42 -> 26   64 x 512: 141 -> 125  32 x 1024: 187 -> 182   8 x 4096: 498 -> 552
 //   block-sparse (16 heads, 25 %)    4 x 1024: 41 -> 38     4 x 4096: 196 -> 185
-// At d = 128 a CTA of one tile has a single stage of K and V, which long sequences pay for; at d = 64 the two
-// meet beyond 4096 (2 x 4 x 65536 causal training 18.98 -> 19.28 ms), where a pair's shared reads count.  A grid of
-// pairs that fills between half of the 148 SMs and all of them runs in one round either way and reads
-// K and V once per pair (16 x 8 heads, 200 queries, 1500 keys: 26 against 27 us).
+// What one tile gains lies at the two ends of a CTA's walk over the keys.  What it loses is a share per key tile:
+// two CTAs each read the K and V that a pair reads once, and at d = 128 a single stage holds them.  So the
+// rule looks at the keys.  Time with one tile / with two, 16 x 16 heads, not causal:
+//   keys              256   512  1024  2048  4096  8192 16384
+//   d = 64   128 q   0.72  0.77  0.77  0.80  0.80  0.82  0.84      (a pair's second tile would be empty)
+//            256 q   0.96  0.97  1.01  0.99  1.03  1.06  1.08
+//           1024 q   0.90  0.87  0.93  0.97  1.00  1.03  1.01
+//           4096 q   0.87  0.82  0.90  0.93  0.96  1.07  1.05
+//   d = 128  128 q   0.75  0.76  0.88  0.89  0.91  0.92  0.90
+//            256 q   0.98  1.03  1.08  1.14  1.15  1.15  1.17
+//           1024 q   0.92  0.96  1.04  1.10  1.13  1.14  1.04
+// Causal, queries = keys, 12 heads: d = 64 0.97 at 1024, 0.99 at 4096, 1.01 at 8192; d = 128 0.99 at 768, 1.00 at
+// 1024, 1.02 at 1536, 1.07 at 2048, 1.21 at 8192.
+// The last round of single tiles is worth more when it has at most one CTA per SM, which is then 1.4 times as fast
+// (1.2 at d = 128).  A grid of only that round spreads over twice the SMs: 16 heads, 512 queries, 4096 keys, d = 128
+// 58 -> 54 us; 16 heads, 1024 queries, 8192 keys, d = 64 97 -> 70.  Behind up to five full rounds it still decides at
+// d = 64: 256 heads, 512 queries, 8192 keys 409 -> 373 us, 48 heads, 4096 queries 580 -> 554 (256 heads, 256 queries,
+// whose last round is full: 213 -> 225).
+// Up to 128 queries both grids have as many CTAs; with long keys at d = 128 one alone on its SM then wants the
+// second stage (16 queries, 4096 keys, one -> two: 96 (batch, head) pairs 69 -> 52 us, 144 pairs 80 -> 58).  From 149
+// on two share an SM: 192 pairs 85 us, 128 with two.
+// A grid of pairs that fills between half of the SMs and all of them runs in one round either way and reads K and
+// V once per pair: 80-140 pairs of 200-1024 queries, one / two 0.94-1.23 with sequences of one length, and
+// 0.73-1.22 ragged (least for 80 pairs of which most second tiles are empty).
 constexpr int kSms = 148;
-constexpr int kOneTileMaxD64 = 4096, kOneTileMaxD128 = 1024;
+constexpr int kOneTileMaxD64 = 4096, kOneTileMaxD128 = 1024;  // queries and keys
+
+template <int D, bool CAUSAL>
+bool one_tile_per_cta(const FwdLaunch& l) {
+  const int64_t heads = static_cast<int64_t>(l.args.heads) * l.args.batch;
+  const int64_t tiles = (l.max_seqlen_q + kBlockM - 1) / kBlockM * heads;
+  const int64_t pairs = (l.max_seqlen_q + 2 * kBlockM - 1) / (2 * kBlockM) * heads;
+  constexpr int kMax = D == 64 ? kOneTileMaxD64 : kOneTileMaxD128;
+  const int keys = CAUSAL ? min(l.max_seqlen_k, l.max_seqlen_q) : l.max_seqlen_k;
+  if (l.max_seqlen_q <= kBlockM) return D == 64 || keys <= kMax || pairs > kSms;
+  if (pairs > kSms / 2 && pairs <= kSms) return false;
+  const int64_t rounds = tiles / (2 * kSms), last = tiles % (2 * kSms);
+  const bool short_end = last > 0 && last <= kSms && rounds <= (D == 64 ? 5 : 0);
+  return l.max_seqlen_q <= kMax && (keys <= kMax || short_end);
+}
 
 template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BS>
 cudaError_t launch_one(const FwdLaunch& l, cudaStream_t stream) {
-  const int64_t pairs = static_cast<int64_t>((l.max_seqlen_q + 2 * kBlockM - 1) / (2 * kBlockM)) * l.args.heads * l.args.batch;
-  const bool one_round = l.max_seqlen_q > kBlockM && pairs > kSms / 2 && pairs <= kSms;
-  if (!one_round && l.max_seqlen_q <= (D == 64 ? kOneTileMaxD64 : kOneTileMaxD128))
-    return launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 1>(l, stream);
-  return launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 2>(l, stream);
+  return one_tile_per_cta<D, CAUSAL>(l) ? launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 1>(l, stream)
+                                        : launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 2>(l, stream);
 }
 
 template <int D, bool BF16, bool CAUSAL>

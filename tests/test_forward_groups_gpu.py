@@ -51,3 +51,66 @@ def test_dropout_agrees_between_the_two(d):
         torch.cuda.manual_seed(3)
         outs.append(fc.fwd(q, k, v, c, c, n, n, 0.25, 0.1, False, False, False, None)[0])
     assert torch.equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("d,limit", [(64, 4096), (128, 1024)])
+@pytest.mark.parametrize("queries,batch", [(100, 160), (256, 80), (300, 40), (256, 10)])
+def test_both_sides_of_the_key_limit_agree(d, limit, queries, batch):
+    """The same sequences announced with the longest key sequence at the limit of one tile per CTA and just above it
+    (the same tiles in the same order: the same bits).  Two query lengths, 160-1280 and 20-80 CTAs."""
+    from flash_attn_b200 import flash_attn_cuda as fc
+    heads, keys = 2, 390
+    q, k, v, _, _, _ = U.make_varlen([queries * batch], [keys * batch], heads, d, torch.bfloat16, seed=d)
+    cu_q = torch.arange(0, queries * batch + 1, queries, dtype=torch.int32, device="cuda")
+    cu_k = torch.arange(0, keys * batch + 1, keys, dtype=torch.int32, device="cuda")
+    runs = [fc.fwd(q, k, v, cu_q, cu_k, queries, longest, 0.0, 0.1, False, False, False, None) for longest in (limit, limit + 1)]
+    fc.check_device_status()
+    assert torch.equal(runs[0][0], runs[1][0])
+    assert torch.equal(runs[0][1][:, :, :queries], runs[1][1][:, :, :queries])
+
+
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("p", [0.0, 0.2])
+def test_block_sparse_with_pairs_of_tiles(causal, p):
+    """Block-sparse calls in a grid of 75..148 pairs (two tiles per CTA) and in a smaller one (one tile): ragged
+    lengths, so that second tiles are empty or short."""
+    from flash_attn_b200 import flash_attn_cuda as fc
+    from flash_attn_b200.flash_blocksparse_attn_interface import convert_blockmask
+    lens, heads = [600, 100, 130, 512, 1, 257], 10
+    torch.manual_seed(2)
+    layout = ((torch.rand(3, 3) < 0.5) | torch.eye(3, dtype=torch.bool)).repeat_interleave(16, dim=0)
+    layout[5], layout[20] = 0, 0   # 16-row blocks without any key block
+    conv = convert_blockmask(layout.int().cuda(), causal)
+    q, k, v, _, cu, _ = U.make_varlen(lens, lens, heads, 64, torch.float16, seed=9)
+
+    def run(q, k, v, cu):
+        gen = torch.Generator(device="cuda").manual_seed(4)
+        return fc.fwd_block(q, k, v, cu, cu, conv, 600, 600, p, 0.125, causal, False, gen)
+
+    two, lse_two = run(q, k, v, cu)          # 3 x 6 x 10 pairs: one tile; the first three sequences 90: pairs
+    part, lse_part = run(q[:830], k[:830], v[:830], cu[:4].contiguous())
+    fc.check_device_status()
+    assert torch.equal(two[:830], part)
+    for b in range(3):
+        assert torch.equal(lse_two[b, :, :lens[b]], lse_part[b, :, :lens[b]])
+
+
+def test_block_sparse_above_the_one_tile_limit():
+    """4500 tokens, two heads: two tiles per CTA, against the oracle on sampled rows."""
+    from flash_attn_b200 import flash_attn_cuda as fc
+    from flash_attn_b200.flash_blocksparse_attn_interface import convert_blockmask
+    n, heads, d = 4500, 2, 64
+    blocks = (n + 255) // 256
+    torch.manual_seed(3)
+    layout = ((torch.rand(blocks, blocks) < 0.25) | torch.eye(blocks, dtype=torch.bool)).repeat_interleave(16, dim=0)
+    q, k, v, _, cu, _ = U.make_varlen([n], [n], heads, d, torch.float16, seed=10)
+    out = fc.fwd_block(q, k, v, cu, cu, convert_blockmask(layout.int().cuda(), False), n, n, 0.0, 0.125, False, False, None)[0]
+    fc.check_device_status()
+    rows = torch.cat([torch.arange(0, 40), torch.arange(1000, 1030), torch.arange(n - 300, n)]).cuda()
+    allowed = layout.cuda()[rows // 16].repeat_interleave(256, dim=1)[:, :n]
+    refs = []
+    for dtype in (torch.float32, torch.float16):   # the probabilities rounded to 16 bits in the second
+        s = torch.einsum("qhd,khd->hqk", q[rows].float(), k.float()) * 0.125
+        pr = torch.softmax(s.masked_fill(~allowed[None], float("-inf")), dim=-1).to(dtype).float()
+        refs.append(torch.einsum("hqk,khd->qhd", pr, v.float()).to(dtype))
+    U.assert_within_2x("pairs of tiles, block-sparse", out[rows], *refs)
