@@ -359,10 +359,10 @@ static int run_fwd(const fa_fwd_params* p, bool zero_unused, void* cuda_stream) 
                              p->k_row_stride, p->k_head_stride, 128)) return rc;
   if (int rc = make_tile_map(&l.tm_v, p->v, l.is_bf16, p->total_k, p->heads, p->head_dim,
                              p->v_row_stride, p->v_head_stride, 128)) return rc;
-  // A few query rows per sequence: the decoding kernel, bound by the reads of K and V.  Dropout and
-  // block-sparse calls keep the tile kernel (their mask is tied to its tiles), and so do causal ones,
-  // which see no more keys than they have query rows.
-  if (p->max_seqlen_q <= fa::kDecodeMaxRows && !l.is_dropout && !l.is_causal && !p->blockmask) {
+  // A few query rows per sequence: the decoding kernel where it is the faster one.  Dropout and block-sparse
+  // calls keep the tile kernel (their mask is tied to its tiles), and so do causal ones, which see no more
+  // keys than they have query rows.
+  if (fa::decode_serves(l)) {
     l.decode = fa::DecodeArgs{p->q, p->k, p->v, p->q_row_stride, p->q_head_stride, p->k_row_stride, p->k_head_stride,
                               p->v_row_stride, p->v_head_stride, p->total_q, p->total_k};
     FA_CUDA(fa::launch_decode(l, static_cast<cudaStream_t>(cuda_stream)));

@@ -1,9 +1,9 @@
 // Forward for a handful of query rows per sequence (a decoding step against cached keys and values).
 //
-// Bound by the HBM: every key and value is read once and used for at most kMaxRows rows, 2 to 8 FLOP a
-// byte.  The tile kernel (fa_fwd_sm100.cu) works on 256 query rows per CTA: with one row it multiplies
-// and exponentiates 255 rows of padding, holds one CTA per SM, and has batch x heads CTAs whatever the
-// length of the sequences.  Here
+// Bound by the HBM with one row: every key and value is read once and used for at most kDecodeMaxRows rows, 2
+// to 8 FLOP a byte.  The tile kernel (fa_fwd_sm100.cu) works on 128 query rows: with one row it multiplies
+// and exponentiates 127 rows of padding and has batch x heads CTAs whatever the length of the
+// sequences.  Here
 //   * the keys of a (batch, head) are split over the CTAs of a cluster (grid.x = cluster size = 1, 2,
 //     4 or 8), whose partial results meet in distributed shared memory: one launch, no workspace;
 //   * a warp reads whole rows of K and V with 16-byte loads (D / 8 lanes per row), kLoads rows of each
@@ -267,6 +267,46 @@ cudaError_t launch_d(const FwdLaunch& l, int splits, cudaStream_t stream) {
 }
 
 }  // namespace
+
+// Where this kernel is the faster one (the tile kernel takes the other calls).  It reads K and V at the rate of the
+// memory with any grid.  The tile kernel comes near that rate when the (batch, head) pairs fill a round of it,
+// 112 to 148 pairs with one CTA per SM or 223 to 296 with two, and the sequences are long enough for its prologue and
+// short enough for the memory's rate not to have been reached here (1024 keys to 64 * head_dim, or twice that with
+// more rows; 2048 at d = 16).  Four rows take up to four times the arithmetic of one per byte, which bounds the kernel at d = 64 and 128 once the
+// grid fills the chip.  us here / in the tile kernel, every sequence of `keys` keys, bf16:
+//                pairs  keys  64        256       1024       4096       8192
+//   1 row   d = 32    144   3.8/6.3   4.1/7.2    15/13      31/38      47/71
+//           d = 64     64   3.9/6.0   4.3/6.7   6.9/13      17/37      32/71
+//                     144   4.0/6.4   4.4/7.4    16/14      46/40      71/72
+//                     192   4.2/7.4   5.2/8.8    19/18      44/58     75/107
+//                     288   4.4/7.7   5.7/9.2    29/19      67/59    114/109
+//                    1024    11/19     17/23     49/59    165/195    325/385
+//           d = 128   144   3.9/7.2   5.9/8.2    23/17      70/54    117/100
+//                     192   4.3/8.2   7.7/10     27/25      74/85    134/157
+//                    1024    16/26     32/39     84/97    311/351    620/693
+//   4 rows  d = 32    144   4.4/6.4   5.0/7.1    18/13      43/38      64/71
+//                    1024    14/19     18/22     41/55    127/181    240/350
+//           d = 64     64   4.2/5.8   5.9/6.5    10/13      28/37      47/70
+//                     144   4.8/6.9   6.2/7.4    23/14      66/40     105/72
+//                    1024    15/19     26/23     72/59    250/204    501/401
+//           d = 128    64   4.9/6.6   8.8/7.4    16/16      53/52      90/97
+//                     144   5.0/6.8   9.6/7.7    40/17     122/54    210/100
+//                    1024    23/26     53/38    149/98    543/359   1078/710
+static bool decode_is_faster(int head_dim, int rows, int64_t pairs, int keys) {
+  constexpr int kSms = 148;
+  if (rows == 1 || head_dim <= 32) {
+    const bool full_round = (pairs > kSms * 3 / 4 && pairs <= kSms) || (pairs > kSms * 3 / 2 && pairs <= 2 * kSms);
+    const int longest = max(2048, (rows == 1 ? 64 : 128) * head_dim);
+    return !(full_round && keys >= 1024 && keys <= longest);
+  }
+  if (pairs <= kSms / 2) return head_dim == 64 || keys <= 64 || keys >= 512;
+  return keys <= (head_dim == 64 ? 256 : 64);
+}
+
+bool decode_serves(const FwdLaunch& l) {
+  return l.max_seqlen_q <= kDecodeMaxRows && !l.is_dropout && !l.is_causal && l.args.bs_iter == nullptr &&
+         decode_is_faster(l.args.head_dim, l.max_seqlen_q, static_cast<int64_t>(l.args.batch) * l.args.heads, l.max_seqlen_k);
+}
 
 // Key ranges per (batch, head): doubled while there are fewer CTAs than four per SM (two are resident;
 // ragged sequences want a second round to even out) and a CTA keeps at least 256 keys.

@@ -76,6 +76,7 @@ struct BwdLaunch {
 };
 
 cudaError_t launch_fwd(const FwdLaunch& l, cudaStream_t stream);
+bool decode_serves(const FwdLaunch& l);  // whether launch_decode takes the call (l.decode apart)
 cudaError_t launch_decode(const FwdLaunch& l, cudaStream_t stream);
 cudaError_t launch_bwd(const BwdLaunch& l, cudaStream_t stream);
 cudaError_t launch_sdmask(void* s_out, int64_t s_rows, int64_t s_cols, const void* q, const void* k,

@@ -83,3 +83,17 @@ def test_infinite_and_nan_scores():
         out, lse = fc.fwd(q, k, v, cu_q, cu_k, longest, 300, 0.0, 0.125, False, False, False, None)
         assert torch.isnan(out[0]).all() and torch.isnan(out[1]).all() and torch.isfinite(out[2]).all()
         assert torch.isneginf(lse[0, 0, 0]) and torch.isneginf(lse[1, 0, 0]) and torch.isfinite(lse[2, 0, 0])
+
+
+# announced key counts on the two sides of the rule that chooses the kernel: (rows, pairs, d) and the first count
+@pytest.mark.parametrize("rows,batch,heads,d,edge", [(1, 30, 4, 64, 1024), (1, 64, 4, 128, 8193), (3, 30, 4, 32, 4097), (2, 8, 4, 128, 512),
+                                                     (4, 8, 4, 128, 65), (2, 20, 4, 64, 257), (4, 20, 4, 128, 65)])
+def test_both_kernels_at_the_edges_of_the_rule(rows, batch, heads, d, edge):
+    """The same sequences through both (tolerance as above)."""
+    from flash_attn_b200 import flash_attn_cuda as fc
+    keys = [1 + (37 * i) % min(edge - 1, 700) for i in range(batch)]
+    q, k, v, _, cu_q, cu_k = U.make_varlen([rows] * batch, keys, heads, d, torch.float16, seed=rows + d)
+    runs = [fc.fwd(q, k, v, cu_q, cu_k, rows, longest, 0.0, 0.125, False, False, False, None) for longest in (edge - 1, edge)]
+    fc.check_device_status()
+    assert U.max_err(runs[0][0], runs[1][0]) <= 2 ** -10 * v.float().abs().max().item()
+    assert U.max_err(runs[0][1][:, :, :rows], runs[1][1][:, :, :rows]) < 2e-4
