@@ -92,10 +92,17 @@ class IndexPutFirstAxis(torch.autograd.Function):
 index_put_first_axis = IndexPutFirstAxis.apply
 
 
+# A CTA of the list kernels walks one sequence and sums the lengths of all sequences before it, so their time
+# grows with the longest sequence and with the square of the batch.  us of unpad_input, kernels / framework
+# operations: 64 x 512 92 / 168, 1 x 16384 104 / 166, 16384 x 64 116 / 152; 1 x 65536 173 / 149, 65536 x 16
+# 396 / 213, 1 x 1048576 1432 / 138, 1048576 x 1 93787 / 700.
+_MASK_KERNEL_MAX = 16384
+
+
 def _mask_kernel_path(mask):
     """Boolean masks only: with integer masks the lengths are the sums of the values."""
     return (runs_now(mask) and mask.dtype is torch.bool and mask.dim() == 2 and mask.is_contiguous()
-            and 0 < mask.numel() < 2 ** 31)
+            and 0 < mask.shape[0] <= _MASK_KERNEL_MAX and 0 < mask.shape[1] <= _MASK_KERNEL_MAX)
 
 
 def _mask_lists(mask):

@@ -70,3 +70,14 @@ def test_rotary_pass(heads, d, dtype):
     for i, want in enumerate((q, k)):
         bound = ulp * x[:, :, i].abs().max().item() * 2
         assert (got[:, :, i].double() - want).abs().max().item() <= bound
+
+
+@pytest.mark.parametrize("batch,seqlen,kernels", [(16384, 2, True), (16385, 2, False), (2, 16384, True), (2, 16385, False)])
+def test_masks_at_the_limit_of_the_list_kernels(batch, seqlen, kernels):
+    """Longer sequences and larger batches, which the kernels are slow at, keep the framework route."""
+    from flash_attn_b200 import bert_padding as bp
+    mask = torch.rand(batch, seqlen, device="cuda") < 0.5
+    assert bp._mask_kernel_path(mask) is kernels
+    x = torch.randn(batch, seqlen, 8, device="cuda").half()
+    for a, b in zip(bp.unpad_input(x, mask), bp.unpad_input(x, mask.int())):
+        assert torch.equal(a, b) if torch.is_tensor(a) else a == b
