@@ -81,3 +81,17 @@ def test_masks_at_the_limit_of_the_list_kernels(batch, seqlen, kernels):
     x = torch.randn(batch, seqlen, 8, device="cuda").half()
     for a, b in zip(bp.unpad_input(x, mask), bp.unpad_input(x, mask.int())):
         assert torch.equal(a, b) if torch.is_tensor(a) else a == b
+
+
+@pytest.mark.parametrize("units", [1023, 1024, 1025, 2048, 5000])
+@pytest.mark.parametrize("rows", [1, 9])
+def test_long_rows_move_in_pieces(units, rows):
+    from flash_attn_b200 import bert_padding as bp
+    g = torch.Generator(device="cuda").manual_seed(units)
+    x = torch.randn(rows + 3, units * 8, device="cuda", generator=g).half()
+    idx = torch.randperm(rows + 3, device="cuda", generator=g)[:rows]
+    got = bp.gather_rows(x, idx)
+    assert torch.equal(got, x[idx])
+    want = torch.zeros_like(x)
+    want[idx] = got
+    assert torch.equal(bp.scatter_rows(got, idx, rows + 3), want)
