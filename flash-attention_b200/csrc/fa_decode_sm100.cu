@@ -272,8 +272,9 @@ cudaError_t launch_d(const FwdLaunch& l, int splits, cudaStream_t stream) {
 // memory with any grid.  The tile kernel comes near that rate when the (batch, head) pairs fill a round of it,
 // 112 to 148 pairs with one CTA per SM or 223 to 296 with two, and the sequences are long enough for its prologue and
 // short enough for the memory's rate not to have been reached here (1024 keys to 64 * head_dim, or twice that with
-// more rows; 2048 at d = 16).  Four rows take up to four times the arithmetic of one per byte, which bounds the kernel at d = 64 and 128 once the
-// grid fills the chip.  us here / in the tile kernel, every sequence of `keys` keys, bf16:
+// more rows; 2048 at d = 16).  Four rows take up to four times the arithmetic of one per byte, which bounds the
+// kernel at d = 64 and 128 once the grid fills the chip.  us here / in the tile kernel, every sequence of
+// `keys` keys, bf16:
 //                pairs  keys  64        256       1024       4096       8192
 //   1 row   d = 32    144   3.8/6.3   4.1/7.2    15/13      31/38      47/71
 //           d = 64     64   3.9/6.0   4.3/6.7   6.9/13      17/37      32/71

@@ -177,7 +177,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 
   int n_kv_total = (sk + kBlockN - 1) / kBlockN;
   if constexpr (BLOCKSPARSE) {
-    // A key tile is visited when any 16-row block of this CTA's 256 query rows has its 256-column
+    // A key tile is visited when any 16-row block of this CTA's 128 * G query rows has its 256-column
     // key block in the layout; rows whose block is absent are masked inside the tile.
     uint8_t* flags = reinterpret_cast<uint8_t*>(smem_raw);
     const int rb0 = mp * (G * kBlockM / 16);
@@ -662,13 +662,6 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     bool ok = true;
     const uint64_t c2 = pack_f2(a.scale_log2, a.scale_log2);
 
-#ifdef FA_FWD_OFFSET
-    // experiment: start query tile 1 half a tile period behind query tile 0
-    if (g == 1) {
-      const long long t_start = clock64();
-      while (clock64() - t_start < FA_FWD_OFFSET) {}
-    }
-#endif
     FA_PROF_DECL
     for (int j = 0; j < n && ok; ++j) {
       const int col0 = kv_tile(j) * kBlockN;
@@ -867,7 +860,7 @@ cudaError_t launch_groups(const FwdLaunch& l, cudaStream_t stream) {
 // Causal, queries = keys, 12 heads: d = 64 0.97 at 1024, 0.99 at 4096, 1.01 at 8192; d = 128 0.99 at 768, 1.00 at
 // 1024, 1.02 at 1536, 1.07 at 2048, 1.21 at 8192.
 // The last round of single tiles is worth more when it has at most one CTA per SM, which is then 1.4 times as fast
-// (1.2 at d = 128).  A grid of only that round spreads over twice the SMs: 16 heads, 512 queries, 4096 keys, d = 128
+// (1.2 at d = 128).  A grid of only that round spreads over twice the SMs: 32 heads, 512 queries, 4096 keys, d = 128
 // 58 -> 54 us; 16 heads, 1024 queries, 8192 keys, d = 64 97 -> 70.  Behind up to five full rounds it still decides at
 // d = 64: 256 heads, 512 queries, 8192 keys 409 -> 373 us, 48 heads, 4096 queries 580 -> 554 (256 heads, 256 queries,
 // whose last round is full: 213 -> 225).

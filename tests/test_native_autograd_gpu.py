@@ -98,3 +98,64 @@ def test_head_shard_changes_as_one_value():
         thread.join()
         sys.setswitchinterval(interval)
         fc.options.mask_heads = None
+
+
+def _qkv(seed, n=50):
+    q, k, v, dout, cu, _ = U.make_varlen([n], [n], 2, 64, torch.float16, seed=seed)
+    return torch.stack([q, k, v], dim=1), dout, cu
+
+
+def test_retained_graph_gives_the_same_gradient_twice():
+    from flash_attn_b200.flash_attn_interface import flash_attn_unpadded_qkvpacked_func
+    qkv, dout, cu = _qkv(43)
+    qkv.requires_grad_()
+    out = flash_attn_unpadded_qkvpacked_func(qkv, cu, 50, 0.2)
+    a = torch.autograd.grad(out, qkv, dout, retain_graph=True)[0]
+    b = torch.autograd.grad(out, qkv, dout)[0]
+    assert torch.equal(a, b)   # one key tile: a single writer of dq
+
+
+def test_a_saved_input_or_output_changed_in_place_is_refused():
+    from flash_attn_b200.flash_attn_interface import flash_attn_unpadded_qkvpacked_func
+    qkv, dout, cu = _qkv(44)
+    leaf = qkv.clone().requires_grad_()
+    x = leaf * 1
+    out = flash_attn_unpadded_qkvpacked_func(x, cu, 50, 0.0)
+    x.add_(1)
+    with pytest.raises(RuntimeError, match="inplace"):
+        out.backward(dout)
+    out = flash_attn_unpadded_qkvpacked_func(leaf, cu, 50, 0.0)
+    out.add_(1)
+    with pytest.raises(RuntimeError, match="inplace"):
+        out.backward(dout)
+
+
+def test_saved_tensor_hooks_see_and_replace_what_is_saved():
+    from flash_attn_b200.flash_attn_interface import flash_attn_unpadded_qkvpacked_func
+    qkv, dout, cu = _qkv(45)
+    grads = []
+    for hooks in (False, True):
+        x = qkv.clone().requires_grad_()
+        torch.cuda.manual_seed(3)
+        with torch.autograd.graph.save_on_cpu() if hooks else torch.enable_grad():
+            out = flash_attn_unpadded_qkvpacked_func(x, cu, 50, 0.2)
+        grads.append(torch.autograd.grad(out, x, dout)[0])
+    assert torch.equal(*grads)
+
+
+def test_packed_inputs_of_other_orders_and_strides():
+    """Packed tensors that are not contiguous: heads before the three parts in memory, rows with a gap, an expanded
+    gradient."""
+    from flash_attn_b200.flash_attn_interface import flash_attn_unpadded_qkvpacked_func
+    qkv, dout, cu = _qkv(46)
+    want_x = qkv.clone().requires_grad_()
+    want = flash_attn_unpadded_qkvpacked_func(want_x, cu, 50, 0.0, causal=True)
+    want_g = torch.autograd.grad(want, want_x, dout[:1].expand_as(dout))[0]
+    wide = torch.zeros(50, 4, 3, 64, dtype=torch.float16, device="cuda")
+    wide[:, :3, :2] = qkv
+    for x in (qkv.transpose(1, 2).contiguous().transpose(1, 2), wide[:, :3, :2]):
+        x = x.detach().requires_grad_()
+        assert not x.is_contiguous()
+        out = flash_attn_unpadded_qkvpacked_func(x, cu, 50, 0.0, causal=True)
+        assert torch.equal(out, want)
+        assert torch.equal(torch.autograd.grad(out, x, dout[:1].expand_as(dout))[0], want_g)
