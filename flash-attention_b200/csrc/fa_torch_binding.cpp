@@ -508,9 +508,24 @@ struct AttnNode : public torch::autograd::Node {
   }
 };
 
-at::Tensor attention(const at::Tensor* x, int layout, const at::Tensor& cu_q, const at::Tensor& cu_k, int64_t max_q,
-                     int64_t max_k, double p_dropout, c10::optional<double> softmax_scale, bool causal,
-                     const at::Tensor* blockmask) {
+// Calls that the Python autograd classes serve.  While a trace is recorded a class is one operation of it, where
+// the functions below would leave the allocation of their output and nothing that fills it.  Inputs that
+// carry a forward-mode tangent or the wrapper of a function transform (vmap, grad, jvp ...) the classes
+// refuse; the functions below do not look at them.
+bool left_to_the_classes(const at::Tensor* x, int layout) {
+  if (torch::jit::tracer::isTracing() ||
+      c10::impl::tls_is_dispatch_key_included(at::DispatchKey::FuncTorchDynamicLayerFrontMode))
+    return true;
+  for (int i = 0; i < layout; ++i)
+    if (x[i]._fw_grad(/*level=*/0).defined()) return true;
+  return false;
+}
+
+// nullopt (None in Python): the classes serve the call
+c10::optional<at::Tensor> attention(const at::Tensor* x, int layout, const at::Tensor& cu_q, const at::Tensor& cu_k,
+                                    int64_t max_q, int64_t max_k, double p_dropout, c10::optional<double> softmax_scale,
+                                    bool causal, const at::Tensor* blockmask) {
+  if (left_to_the_classes(x, layout)) return c10::nullopt;
   const double scale = softmax_scale.has_value() ? *softmax_scale : 1.0 / std::sqrt(static_cast<double>(x[0].size(-1)));
   bool needs_grad = false;
   if (c10::GradMode::is_enabled())
@@ -544,26 +559,27 @@ at::Tensor attention(const at::Tensor* x, int layout, const at::Tensor& cu_q, co
   return r.o;
 }
 
-at::Tensor attn_qkvpacked(const at::Tensor& qkv, const at::Tensor& cu, int64_t max_s, double p_dropout,
-                          c10::optional<double> scale, bool causal) {
+c10::optional<at::Tensor> attn_qkvpacked(const at::Tensor& qkv, const at::Tensor& cu, int64_t max_s, double p_dropout,
+                                         c10::optional<double> scale, bool causal) {
   return attention(&qkv, kQkvPacked, cu, cu, max_s, max_s, p_dropout, scale, causal, nullptr);
 }
 
-at::Tensor attn_kvpacked(const at::Tensor& q, const at::Tensor& kv, const at::Tensor& cu_q, const at::Tensor& cu_k,
-                         int64_t max_q, int64_t max_k, double p_dropout, c10::optional<double> scale, bool causal) {
+c10::optional<at::Tensor> attn_kvpacked(const at::Tensor& q, const at::Tensor& kv, const at::Tensor& cu_q,
+                                        const at::Tensor& cu_k, int64_t max_q, int64_t max_k, double p_dropout,
+                                        c10::optional<double> scale, bool causal) {
   const at::Tensor x[2] = {q, kv};
   return attention(x, kKvPacked, cu_q, cu_k, max_q, max_k, p_dropout, scale, causal, nullptr);
 }
 
-at::Tensor attn(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& cu_q,
-                const at::Tensor& cu_k, int64_t max_q, int64_t max_k, double p_dropout, c10::optional<double> scale,
-                bool causal) {
+c10::optional<at::Tensor> attn(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& cu_q,
+                               const at::Tensor& cu_k, int64_t max_q, int64_t max_k, double p_dropout,
+                               c10::optional<double> scale, bool causal) {
   const at::Tensor x[3] = {q, k, v};
   return attention(x, kSeparate, cu_q, cu_k, max_q, max_k, p_dropout, scale, causal, nullptr);
 }
 
-at::Tensor attn_sparse_qkvpacked(const at::Tensor& qkv, const at::Tensor& cu, const at::Tensor& blockmask,
-                                 double p_dropout, int64_t max_s, c10::optional<double> scale, bool causal) {
+c10::optional<at::Tensor> attn_sparse_qkvpacked(const at::Tensor& qkv, const at::Tensor& cu, const at::Tensor& blockmask,
+                                                double p_dropout, int64_t max_s, c10::optional<double> scale, bool causal) {
   require(qkv.dim() == 4 && qkv.size(1) == 3, "qkv must be (total, 3, heads, head_dim)");
   return attention(&qkv, kQkvPacked, cu, cu, max_s, max_s, p_dropout, scale, causal, &blockmask);
 }
@@ -580,12 +596,6 @@ at::Tensor convert_blockmask(const at::Tensor& layout, bool causal) {
                                 causal ? 1 : 0, static_cast<int32_t*>(out.data_ptr()),
                                 at::cuda::getCurrentCUDAStream().stream()));
   return out;
-}
-
-// Whether this thread records a trace or runs inside a function transform (vmap, grad, jvp ...).
-bool recording() {
-  return torch::jit::tracer::isTracing() ||
-         c10::impl::tls_is_dispatch_key_included(at::DispatchKey::FuncTorchDynamicLayerFrontMode);
 }
 
 void set_options(bool deterministic, int64_t mask_heads_total, int64_t mask_head_offset) {
@@ -611,7 +621,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attn", &attn);
   m.def("attn_sparse_qkvpacked", &attn_sparse_qkvpacked);
   m.def("convert_blockmask", &convert_blockmask);
-  m.def("recording", &recording);
   m.def("set_options", &set_options);
   m.def("set_status", &set_status);
 }

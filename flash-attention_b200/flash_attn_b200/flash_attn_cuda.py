@@ -16,7 +16,6 @@ import os
 import struct
 
 import torch
-import torch.autograd.forward_ad as forward_ad
 
 from . import _lib
 from ._lib import BwdParams, FwdParams, check, lib
@@ -115,16 +114,10 @@ def _status_buffer(device):
 
 def compiled_attention(x):
     """The compiled module when the differentiable functions can run through it for input `x` (its
-    device's status buffer exists afterwards), else None.
-
-    Inside a forward-mode level and a function transform the Python autograd classes serve the call:
-    they refuse an input that carries a tangent or a transform's wrapper, which the compiled
-    functions do not look at.  While a trace is recorded they do too: a class is one operation of the
-    trace, where the compiled functions would leave the allocation of their output and nothing that
-    fills it."""
+    device's status buffer exists afterwards), else None.  Its attn* functions return None for calls
+    that they leave to the Python autograd classes (traces, function transforms, forward-mode
+    tangents)."""
     if _binding is not None:
-        if forward_ad._current_level >= 0 or _binding.recording():
-            return None
         i = x.get_device()
         if i >= 0 and i not in _status_known:
             _status_buffer(x.device)

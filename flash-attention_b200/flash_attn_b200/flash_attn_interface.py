@@ -9,7 +9,7 @@ packed tensor through strided views, as the reference does (:64-68, :100-106).
 With the compiled binding the same functions run through one C++ autograd node instead
 (csrc/fa_torch_binding.cpp, AttnNode): a forward + backward at batch 8 x 12 heads x 128 tokens with
 dropout is bound by the host.  The classes here serve return_attn_probs, the ctypes route and the
-calls that flash_attn_cuda.compiled_attention() leaves to them.
+calls that the compiled functions leave to them (flash_attn_cuda.compiled_attention).
 """
 import torch
 
@@ -179,8 +179,9 @@ def flash_attn_unpadded_qkvpacked_func(qkv, cu_seqlens, max_seqlen, dropout_p, s
     """
     native = flash_attn_cuda.compiled_attention(qkv)
     if native is not None and not return_attn_probs:
-        return native.attn_qkvpacked(qkv, cu_seqlens, int(max_seqlen), float(dropout_p),
-                                     softmax_scale, bool(causal))
+        out = native.attn_qkvpacked(qkv, cu_seqlens, int(max_seqlen), float(dropout_p), softmax_scale, bool(causal))
+        if out is not None:
+            return out
     return FlashAttnQKVPackedFunc.apply(qkv, cu_seqlens, max_seqlen, dropout_p, softmax_scale,
                                         causal, return_attn_probs)
 
@@ -194,8 +195,10 @@ def flash_attn_unpadded_kvpacked_func(q, kv, cu_seqlens_q, cu_seqlens_k, max_seq
     j <= i (both counted from the start of their sequence)."""
     native = flash_attn_cuda.compiled_attention(q)
     if native is not None and not return_attn_probs:
-        return native.attn_kvpacked(q, kv, cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q), int(max_seqlen_k),
-                                    float(dropout_p), softmax_scale, bool(causal))
+        out = native.attn_kvpacked(q, kv, cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q), int(max_seqlen_k),
+                                   float(dropout_p), softmax_scale, bool(causal))
+        if out is not None:
+            return out
     return FlashAttnKVPackedFunc.apply(q, kv, cu_seqlens_q, cu_seqlens_k, max_seqlen_q,
                                        max_seqlen_k, dropout_p, softmax_scale, causal,
                                        return_attn_probs)
@@ -207,8 +210,10 @@ def flash_attn_unpadded_func(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, 
     Arguments and returns as in flash_attn_unpadded_kvpacked_func."""
     native = flash_attn_cuda.compiled_attention(q)
     if native is not None and not return_attn_probs:
-        return native.attn(q, k, v, cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q), int(max_seqlen_k),
-                           float(dropout_p), softmax_scale, bool(causal))
+        out = native.attn(q, k, v, cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q), int(max_seqlen_k),
+                          float(dropout_p), softmax_scale, bool(causal))
+        if out is not None:
+            return out
     return FlashAttnFunc.apply(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k,
                                dropout_p, softmax_scale, causal, return_attn_probs)
 

@@ -129,13 +129,13 @@ def flash_blocksparse_attn_func(qkv, cu_seqlens, blockmask, dropout_p, max_s, so
     """Block-sparse variable-length self-attention.  qkv (total, 3, heads, d) fp16, blockmask a 0/1
     layout of shape (ceil(max_s / 256) * 16, ceil(max_s / 256)) (or an already converted mask with
     convert_mask=False).  dropout_p should be 0.0 for evaluation."""
-    native = flash_attn_cuda.compiled_attention(qkv)
-    if native is not None and not return_attn_probs:
-        if convert_mask:
-            blockmask = convert_blockmask(blockmask, causal=causal)
-        return native.attn_sparse_qkvpacked(qkv, cu_seqlens, blockmask, float(dropout_p), int(max_s),
-                                            softmax_scale, bool(causal))
-    func = FlashBlocksparseAttnFunWithS if return_attn_probs else FlashBlocksparseAttnFun
     if convert_mask:
         blockmask = convert_blockmask(blockmask, causal=causal)
+    native = flash_attn_cuda.compiled_attention(qkv)
+    if native is not None and not return_attn_probs:
+        out = native.attn_sparse_qkvpacked(qkv, cu_seqlens, blockmask, float(dropout_p), int(max_s),
+                                           softmax_scale, bool(causal))
+        if out is not None:
+            return out
+    func = FlashBlocksparseAttnFunWithS if return_attn_probs else FlashBlocksparseAttnFun
     return func.apply(qkv, cu_seqlens, blockmask, dropout_p, max_s, softmax_scale, causal)
