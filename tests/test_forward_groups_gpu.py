@@ -53,11 +53,12 @@ def test_dropout_agrees_between_the_two(d):
     assert torch.equal(outs[0], outs[1])
 
 
-@pytest.mark.parametrize("d,limit", [(64, 4096), (128, 1024)])
-@pytest.mark.parametrize("queries,batch", [(100, 160), (256, 80), (300, 40), (256, 10)])
+@pytest.mark.parametrize("d,limit,queries,batch", [(64, 4096, 300, 40), (64, 4096, 256, 140), (128, 1024, 100, 40),
+                                                   (128, 1024, 256, 80), (128, 1024, 300, 40)])
 def test_both_sides_of_the_key_limit_agree(d, limit, queries, batch):
     """The same sequences announced with the longest key sequence at the limit of one tile per CTA and just above it
-    (the same tiles in the same order: the same bits).  Two query lengths, 160-1280 and 20-80 CTAs."""
+    (the same tiles in the same order: the same bits).  The grids have 80 pairs of up to 128 queries or 160-280 pairs
+    whose last round is not a short one, so that the key limit alone decides."""
     from flash_attn_b200 import flash_attn_cuda as fc
     heads, keys = 2, 390
     q, k, v, _, _, _ = U.make_varlen([queries * batch], [keys * batch], heads, d, torch.bfloat16, seed=d)
@@ -87,12 +88,12 @@ def test_block_sparse_with_pairs_of_tiles(causal, p):
         gen = torch.Generator(device="cuda").manual_seed(4)
         return fc.fwd_block(q, k, v, cu, cu, conv, 600, 600, p, 0.125, causal, False, gen)
 
-    two, lse_two = run(q, k, v, cu)          # 3 x 6 x 10 pairs: one tile; the first three sequences 90: pairs
+    one, lse_one = run(q, k, v, cu)          # 3 x 6 x 10 pairs: one tile; the first three sequences 90: pairs
     part, lse_part = run(q[:830], k[:830], v[:830], cu[:4].contiguous())
     fc.check_device_status()
-    assert torch.equal(two[:830], part)
+    assert torch.equal(one[:830], part)
     for b in range(3):
-        assert torch.equal(lse_two[b, :, :lens[b]], lse_part[b, :, :lens[b]])
+        assert torch.equal(lse_one[b, :, :lens[b]], lse_part[b, :, :lens[b]])
 
 
 def test_block_sparse_above_the_one_tile_limit():
