@@ -35,6 +35,7 @@
 // tensor-memory columns it shares with dP.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <type_traits>
 #include "fa_kernels.h"
 #include "fa_math.cuh"
 #include "sm100_prims.cuh"
@@ -616,85 +617,93 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         const int32_t bs_it[2] = {bs_nx[0], bs_nx[1]};
         if (t + 1 < nm) fetch_stats(t + 1);
 
-        // keep words of the thread's 2 x 4 patches (they do not depend on the scores: drawn before
-        // the wait).  kw[hh * 4 + grp][2 * u + half]: row u, columns 16 grp + 8 half + 2 q4 (+1 high)
-        uint32_t kw[8][4];
+        // (rows whose 16-row block is not in the layout are masked too)
+        const bool need_mask = (n0 + kBN > sk) || (CAUSAL && (n0 + kBN - 1 > m0)) ||
+                               (BLOCKSPARSE && (bs_it[0] < 0 || bs_it[1] < 0));
+        // One 16-row block of the warp after the other: 32 scores, 32 dP values and 16 keep words a thread.
+        // Whether a tile needs masks is decided once per block, outside the unrolled loops.
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
-          int64_t it_tile;
-          if constexpr (BLOCKSPARSE) it_tile = bs_it[hh];
-          else it_tile = fa_iter_index(CAUSAL, n0 >> ka.drop.n_shift, (m0 + wq * 32 + hh * 16) >> 4, L16, ka.drop.n_shift);
-          qp.set_tile(ka.drop, it_tile, n0);
+          // keep words of the block's four calls (they do not depend on the scores).  kw[grp][2 * u + half]:
+          // row u, columns 16 grp + 8 half + 2 q4 (+1 in the high 16 bits)
+          uint32_t kw[4][4];
+          auto draw = [&]() {
+            int64_t it_tile;
+            if constexpr (BLOCKSPARSE) it_tile = bs_it[hh];
+            else it_tile = fa_iter_index(CAUSAL, n0 >> ka.drop.n_shift, (m0 + wq * 32 + hh * 16) >> 4, L16, ka.drop.n_shift);
+            qp.set_tile(ka.drop, it_tile, n0);
 #pragma unroll
-          for (int g4 = 0; g4 < 4; ++g4) qp.start(g4, kw[hh * 4 + g4]);
-        }
+            for (int g4 = 0; g4 < 4; ++g4) qp.start(g4, kw[g4]);
 #pragma unroll
-        for (int r = 2; r < 7; ++r)
+            for (int r = 2; r < 7; ++r)
 #pragma unroll
-          for (int k8 = 0; k8 < 8; ++k8) QuadPhilox<4>::round(ka.drop, kw[k8], r);
-
-        const bool need_mask = (n0 + kBN > sk) || (CAUSAL && (n0 + kBN - 1 > m0));
-        FA_PROF(1)
-        if (w == 0 && row == 0) { FA_STAMP(t, 0) }
-        ok = mbar_wait(smem_u32(&sh.sdp_full), t & 1, abort_flag);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        FA_PROF(2)
-        if (w == 0 && row == 0) { FA_STAMP(t, 1) }
-        tc_fence_after();
-        // everything goes to registers at once, so that the next tile's S and dP products can overwrite
-        // tensor memory while this tile is still being processed
-        uint32_t sr[2][32], dr[2][32];  // [hh][4 * unit + 2 * u + c]
-        tmem_ld_quad32(tS, sr[0]);
-        tmem_ld_quad32(tS + kHalf, sr[1]);
-        tmem_ld_quad32(tDP, dr[0]);
-        tmem_ld_quad32(tDP + kHalf, dr[1]);
-        tmem_wait_ld();
-        tc_fence_before();
-        mbar_arrive(smem_u32(&sh.sdp_consumed));
-        if (w == 0 && row == 0) { FA_STAMP(t, 2) }
-
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-          uint32_t pp[16], pds[16];  // [2 * unit + u]: the stmatrix register order
-          const bool blk_in_layout = !BLOCKSPARSE || bs_it[hh] >= 0;
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int ri = hh * 2 + u;
-            const int ig = row0 + hh * 16 + u * 8;
-            const uint64_t nlse2 = pack_f2(-lse2[ri], -lse2[ri]);
-            const uint64_t nd2 = pack_f2(-d_i[ri], -d_i[ri]);
-#pragma unroll
-            for (int unit = 0; unit < 8; ++unit) {
-              const int i = 4 * unit + 2 * u;
-              float p0, p1;
-              unpack_f2(fma2(pack_f2(__uint_as_float(sr[hh][i]), __uint_as_float(sr[hh][i + 1])), c2, nlse2), p0, p1);
-              p0 = ex2f(p0);
-              p1 = ex2f(p1);
-              if (need_mask) {
-                const int col = cbase + unit * 8 + 2 * q4;
-                bool v0 = col < sk, v1 = col + 1 < sk;
-                if (CAUSAL) { v0 = v0 && (col <= ig); v1 = v1 && (col + 1 <= ig); }
-                if (!v0) p0 = 0.f;
-                if (!v1) p1 = 0.f;
-              }
-              if (BLOCKSPARSE && !blk_in_layout) { p0 = 0.f; p1 = 0.f; }
-              const uint32_t word = kw[hh * 4 + (unit >> 1)][2 * u + (unit & 1)];
-              const uint64_t p01 = pack_f2(p0, p1);
-              const uint64_t k01 = mul2(p01, pack_f2(fa_keep_factor_lo(word, thr_term), fa_keep_factor_hi(word, thr_term)));
-              float k0, k1, s0, s1;
-              unpack_f2(k01, k0, k1);
-              // dS = P~ * dP - P * D  (P~ = P where kept, 0 where dropped)
-              unpack_f2(fma2(k01, pack_f2(__uint_as_float(dr[hh][i]), __uint_as_float(dr[hh][i + 1])), mul2(p01, nd2)), s0, s1);
-              pp[2 * unit + u] = pack_lowp<BF16>(k0, k1);
-              pds[2 * unit + u] = pack_lowp<BF16>(s0, s1);
-            }
+              for (int g4 = 0; g4 < 4; ++g4) QuadPhilox<4>::round(ka.drop, kw[g4], r);
+          };
+          uint32_t sr[32], dr[32];  // [4 * unit + 2 * u + c]
+          if (hh == 0) {
+            draw();
+            FA_PROF(1)
+            if (w == 0 && row == 0) { FA_STAMP(t, 0) }
+            ok = mbar_wait(smem_u32(&sh.sdp_full), t & 1, abort_flag);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            FA_PROF(2)
+            if (w == 0 && row == 0) { FA_STAMP(t, 1) }
+            tc_fence_after();
           }
+          tmem_ld_quad32(tS + hh * kHalf, sr);
+          tmem_ld_quad32(tDP + hh * kHalf, dr);
+          if (hh == 1) draw();
+          tmem_wait_ld();
+          if (hh == 1) {
+            tc_fence_before();
+            mbar_arrive(smem_u32(&sh.sdp_consumed));
+            if (w == 0 && row == 0) { FA_STAMP(t, 2) }
+          }
+
+          uint32_t pp[16], pds[16];  // [2 * unit + u]: the stmatrix register order
+          auto block_math = [&](auto masked) {
+            constexpr bool kMasked = decltype(masked)::value;
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              const int ri = hh * 2 + u;
+              const int ig = row0 + hh * 16 + u * 8;
+              const uint64_t nlse2 = pack_f2(-lse2[ri], -lse2[ri]);
+              const uint64_t nd2 = pack_f2(-d_i[ri], -d_i[ri]);
+#pragma unroll
+              for (int unit = 0; unit < 8; ++unit) {
+                const int i = 4 * unit + 2 * u;
+                float p0, p1;
+                unpack_f2(fma2(pack_f2(__uint_as_float(sr[i]), __uint_as_float(sr[i + 1])), c2, nlse2), p0, p1);
+                p0 = ex2f(p0);
+                p1 = ex2f(p1);
+                if constexpr (kMasked) {
+                  const int col = cbase + unit * 8 + 2 * q4;
+                  bool v0 = col < sk, v1 = col + 1 < sk;
+                  if (CAUSAL) { v0 = v0 && (col <= ig); v1 = v1 && (col + 1 <= ig); }
+                  if (BLOCKSPARSE && bs_it[hh] < 0) { v0 = false; v1 = false; }
+                  if (!v0) p0 = 0.f;
+                  if (!v1) p1 = 0.f;
+                }
+                const uint32_t word = kw[unit >> 1][2 * u + (unit & 1)];
+                const uint64_t p01 = pack_f2(p0, p1);
+                const uint64_t k01 = mul2(p01, pack_f2(fa_keep_factor_lo(word, thr_term), fa_keep_factor_hi(word, thr_term)));
+                float k0, k1, s0, s1;
+                unpack_f2(k01, k0, k1);
+                // dS = P~ * dP - P * D  (P~ = P where kept, 0 where dropped)
+                unpack_f2(fma2(k01, pack_f2(__uint_as_float(dr[i]), __uint_as_float(dr[i + 1])), mul2(p01, nd2)), s0, s1);
+                pp[2 * unit + u] = pack_lowp<BF16>(k0, k1);
+                pds[2 * unit + u] = pack_lowp<BF16>(s0, s1);
+              }
+            }
+          };
+          if (need_mask) block_math(std::true_type{}); else block_math(std::false_type{});
           // the previous tile's products must have finished reading the P~ / dS buffers
           if (hh == 0) { FA_PROF(3) }
           if (hh == 0 && t > 0) {
             ok = mbar_wait(smem_u32(&sh.pds_free), (t - 1) & 1, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
           }
           if (hh == 0) { FA_PROF(4) }
           if (hh == 0 && w == 0 && row == 0) { FA_STAMP(t, 3) }
@@ -769,7 +778,9 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         for (int g4 = 0; g4 < 4; ++g4) lp.finish(st[2 * g4], st[2 * g4 + 1], wd + g4 * 8);
       }
 
-      const bool need_mask = (n0 + kBN > sk) || (CAUSAL && (n0 + kBN - 1 > m0));
+      // one decision for the warp: its threads' rows may lie in two 16-row blocks of the layout
+      const bool need_mask = (n0 + kBN > sk) || (CAUSAL && (n0 + kBN - 1 > m0)) ||
+                             (BLOCKSPARSE && __any_sync(0xffffffffu, !row_in_layout));
       if constexpr (Cfg::kTwoPhase) {
         // ---- phase one: P from S.  P~ goes to shared memory (dV can start), P stays in registers.
         FA_PROF(1)
@@ -781,6 +792,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         if (w == 0 && row == 0) { FA_STAMP(t, 1) }
         tc_fence_after();
         uint32_t pf[2][32];
+        auto phase_one = [&](auto masked) {
+        constexpr bool kMasked = decltype(masked)::value;
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           uint32_t sr[32];
@@ -798,14 +811,14 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             unpack_f2(fma2(pack_f2(__uint_as_float(sr[i]), __uint_as_float(sr[i + 1])), c2, nlse2), p0, p1);
             p0 = ex2f(p0);
             p1 = ex2f(p1);
-            if (need_mask) {
+            if (kMasked && need_mask) {
               const int col = cbase + c * 32 + i;
               bool v0 = col < sk, v1 = col + 1 < sk;
               if (CAUSAL) { v0 = v0 && (col <= ig); v1 = v1 && (col + 1 <= ig); }
+              if (BLOCKSPARSE && !row_in_layout) { v0 = false; v1 = false; }
               if (!v0) p0 = 0.f;
               if (!v1) p1 = 0.f;
             }
-            if (BLOCKSPARSE && !row_in_layout) { p0 = 0.f; p1 = 0.f; }
             pf[c][i] = __float_as_uint(p0);
             pf[c][i + 1] = __float_as_uint(p1);
             float k0 = p0, k1 = p1;
@@ -829,6 +842,9 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                 make_uint4(pp[4 * ch4], pp[4 * ch4 + 1], pp[4 * ch4 + 2], pp[4 * ch4 + 3]);
           }
         }
+        };
+        // (one copy where two cost more: with dropout and no causal mask, 4 x 12 x 2048, 397 against 410 us)
+        if ((DROPOUT && !CAUSAL) || need_mask) phase_one(std::true_type{}); else phase_one(std::false_type{});
         if (!ok) break;
         fence_async_smem();
         mbar_arrive(smem_u32(&sh.p_ready));
@@ -900,6 +916,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         mbar_arrive(smem_u32(&sh.sdp_consumed));
         if (w == 0 && row == 0) { FA_STAMP(t, 2) }
       }
+      auto tile_math = [&](auto masked) {
+      constexpr bool kMasked = decltype(masked)::value;
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         uint32_t(&sr)[32] = sr_all[kEarly ? c : 0];
@@ -916,14 +934,14 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           unpack_f2(fma2(pack_f2(__uint_as_float(sr[i]), __uint_as_float(sr[i + 1])), c2, nlse2), p0, p1);
           p0 = ex2f(p0);
           p1 = ex2f(p1);
-          if (need_mask) {
+          if constexpr (kMasked) {
             const int col = cbase + c * 32 + i;
             bool v0 = col < sk, v1 = col + 1 < sk;
             if (CAUSAL) { v0 = v0 && (col <= ig); v1 = v1 && (col + 1 <= ig); }
+            if (BLOCKSPARSE && !row_in_layout) { v0 = false; v1 = false; }
             if (!v0) p0 = 0.f;
             if (!v1) p1 = 0.f;
           }
-          if (BLOCKSPARSE && !row_in_layout) { p0 = 0.f; p1 = 0.f; }
           float k0 = p0, k1 = p1;
           uint64_t k01 = pack_f2(p0, p1);
           if constexpr (DROPOUT) {
@@ -959,6 +977,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         // second copy of dS for the dQ product (32 keys = 16 packed columns of this half)
         if constexpr (kDsInTmem) tmem_st16(tDS_ + lane_sel + w * 32 + c * 16, pds);
       }
+      };
+      if (need_mask) tile_math(std::true_type{}); else tile_math(std::false_type{});
       }
       if (!ok) break;
       FA_PROF(6)
