@@ -1,25 +1,26 @@
 // FlashAttention forward for sm_100a.
 //
 // One CTA owns G = 1 or 2 consecutive 128-row query tiles of one (batch, head) pair and walks the key /
-// value sequence in 128-row tiles; launch_one says which G serves which call.  Warp roles at G = 2 (at G = 1
-// there is no softmax group 1, warps 4-7 are what warps 8-11 are here, the CTA has 256 tensor-memory
-// columns, and two CTAs share an SM):
-//   warps 0-3   softmax group 0 (query tile 0): one thread per query row; with dropout a thread
-//               holds two rows of each of the warp's two 16-row blocks and a quarter of their
-//               columns (the ownership pattern of the reference's mask generator)
-//   warps 4-7   softmax group 1 (query tile 1)
-//   warp  8     TMA producer (Q once, K/V ring)
-//   warp  9     tcgen05.mma issuer (d = 128: every product; d = 64: S = Q K^T only)
-//   warp 10     d = 64: second issuer, O += P V (two issuers keep S ahead)
-//   warp 11     idle
-// Tensor memory (512 columns): S0 [0,128) S1 [128,256) fp32 scores, O0 / O1 fp32 outputs behind
-// them.  The 16-bit probabilities P feed the P*V product straight from tensor memory; at d = 128
-// they overwrite the first 64 columns of their S buffer, at d = 64 they have columns of their own,
-// so the next score product can start as soon as the group has read its scores into registers.
-// The softmax groups are the bottleneck at every head size: their run time follows the sum of their
-// instruction costs (exponentials on the special-function unit, the dropout generator on the wide
-// integer multiplies, packed fp32 arithmetic), about 12 clk per score element and scheduler without
-// dropout and 25 with, against 4 (d = 64) or 8 (d = 128) clk of tensor-core time.
+// value sequence in 128-row tiles; one_tile_per_cta says which G serves which call.  With G = 1 two CTAs share an
+// SM.  Warp roles: G softmax groups, then four warps:
+//   first    TMA producer (Q once, K/V ring)
+//   second   tcgen05.mma issuer (d = 128: every product; d = 64: S = Q K^T only)
+//   third    d = 64: second issuer, O += P V (two issuers keep S ahead)
+//   fourth   idle
+// Tensor memory per query tile: 128 columns of fp32 scores S, D of fp32 output O, and at d = 64 64 of the 16-bit
+// probabilities P, which feed the P*V product straight from tensor memory.  At d = 128 P overwrites the first 64
+// columns of S; at d = 64 the next score product starts as soon as the group has read its scores.
+//
+// Softmax groups.  Quads (d = 64 beyond short sequences, and every call with dropout): eight warps per query tile, a warp owns 16 rows and
+// a thread two of them with a quarter of their columns.  That is four softmax warps per scheduler; their work (per score
+// element 8 clk of the exponential unit, about 5 instructions, 12 with dropout) overlaps where two warps
+// per scheduler, each with a serial chain of waits, maxima and exponentials, fell into step and left the units idle
+// for half of the time.  us, the four-warp groups before -> now: 8 x 12 x 4096 (d = 64) 526 -> 484, with dropout
+// (ragged) 783 -> 616, 2 x 4 x 16384 causal 423 -> 383 (one tile per CTA at any length).  ncu, 8 x 12 x 2048 with
+// dropout: issue slots busy 48 -> 63 %, 516 000 -> 404 000 clk.
+// Rows (d = 128 without dropout, and short sequences): four warps per query tile, one thread per row.  At d = 128 the score product waits for P V
+// of its own tile, two groups take turns on the tensor cores, and quads, whose group needs longer for a tile
+// of its own, measured 8 % slower (4 x 12 x 8192 causal: 717 against 770 us).
 //
 // Numerics follow the reference forward (csrc/flash_attn/src/fmha_fprop_kernel_1xN.h:365-638):
 // scores in fp32, p = exp2(scale*log2e*(s - max)), row sum of the un-dropped p, P rounded to the
@@ -41,9 +42,14 @@ constexpr int kBlockN = 128;
 // G: query tiles (softmax groups) per CTA.  Two share every K / V tile, and one such CTA fills an SM.  One leaves
 // room for a second CTA on the SM, whose loads, first products and epilogue run under the tiles of the other:
 // for short sequences, where those are a third of a CTA's time (see launch_one).
-template <int D, bool DROPOUT, int G>
+template <int D, bool DROPOUT, int G, bool ROWS>
 struct FwdCfg {
-  static constexpr int kThreads = 128 * (G + 1);  // G softmax warpgroups + 1 (producer, MMA issuers, idle)
+  // Softmax layout.  Rows: a warpgroup per query tile, one thread per row.  Quads: eight warps per query tile, 16
+  // rows each (see the softmax code for both).
+  static constexpr bool kRows = ROWS;
+  static constexpr int kGroupWarps = kRows ? 4 : 8;
+  static constexpr int kSoftmaxWarps = G * kGroupWarps;
+  static constexpr int kThreads = 32 * kSoftmaxWarps + 128;  // + 1 warpgroup (producer, MMA issuers, idle)
   // G = 1: 80 KB (d = 64: Q, two stages) or 96 KB (d = 128: Q, one stage), so that two CTAs fit
   static constexpr int kStages = (G == 1) ? ((D == 64) ? 2 : 1) : ((D == 64) ? 3 : 2);
   static constexpr int kPanels = D / 64;
@@ -57,10 +63,12 @@ struct FwdCfg {
   static constexpr bool kSeparateP = (D == 64);
   // d = 128 without dropout: P is handed over in two halves, so that P*V of the first 64 keys runs while the
   // other half is exponentiated; S of the next tile waits for P*V there.
-  static constexpr bool kHalfP = !kSeparateP && !DROPOUT;
+  static constexpr bool kHalfP = kRows && !kSeparateP;
   static constexpr uint32_t kTmemP0 = kSeparateP ? 192 * G : kTmemS0, kTmemP1 = kSeparateP ? 192 * G + 64 : kTmemS1;
-  // register split (per thread) of the 168 or 128 a thread is launched with
-  static constexpr int kSoftmaxRegs = (G == 1) ? 208 : 224, kOtherRegs = (G == 1) ? 48 : 56;
+  // register split (per thread) of the 128 or 168 (rows), 80 or 96 (quads) a thread is launched with
+  static constexpr int kSoftmaxRegs = kRows ? ((G == 1) ? 208 : 224) : ((G == 1) ? 96 : 104);
+  static constexpr int kOtherRegs = kRows ? ((G == 1) ? 48 : 56) : ((G == 1) ? 48 : 64);
+  static constexpr uint32_t kArrivals = kRows ? 128 : 8;  // of a softmax group: every thread, or one lane per warp
 };
 
 constexpr int kMaxSparseTiles = 1024;  // key tiles of 128 per sequence in block-sparse mode
@@ -69,27 +77,10 @@ struct FwdShared {
   uint64_t q_full[2];
   uint64_t k_full[3], k_empty[3], v_full[3], v_empty[3];
   uint64_t s_full[2], s_free[2], p_half[2], p_full[2], o_full[2];
+  float2 row_stats[2][kBlockM];  // (max, sum) of every query row, for the epilogue
   uint32_t tmem_base;
   int abort_flag;
 };
-
-// Optional cycle accounting (build with -DFA_PROFILE): thread 0 of softmax group 0 and the MMA
-// thread of CTA (0,0,0) accumulate the cycles they spend in each phase into status[8..].
-#ifdef FA_PROFILE
-#define FA_PROF_DECL long long prof_t = clock64(); long long prof_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-#define FA_PROF(slot) { const long long now_ = clock64(); prof_acc[slot] += now_ - prof_t; prof_t = now_; }
-#define FA_PROF_FLUSH(base, n) if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && a.status) { \
-    for (int i_ = 0; i_ < 8; ++i_) a.status[(base) + i_] = static_cast<int32_t>(prof_acc[i_] / ((n) > 0 ? (n) : 1)); }
-// time stamps (low 32 bits of the SM clock) of the events of kv steps 5, 6 of CTA (0,0,0): slot =
-// 64 + (step - 5) * 24 + idx, for a timeline across the roles
-#define FA_STAMP(step, idx) if ((step) >= 5 && (step) <= 6 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && a.status) { \
-    a.status[64 + ((step) - 5) * 24 + (idx)] = static_cast<int32_t>(clock64()); }
-#else
-#define FA_PROF_DECL
-#define FA_PROF(slot)
-#define FA_PROF_FLUSH(base, n)
-#define FA_STAMP(step, idx)
-#endif
 
 template <int N>
 __device__ __forceinline__ void reg_alloc() {
@@ -111,31 +102,33 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   }
 }
 
-// Epilogue of one query row (thread = row, 32x32b shape): O = acc / (sum * p_keep) in the 16-bit
-// type, LSE = max * scale + ln(sum); a row without any valid key gets zeros and -inf.
-template <int D, bool BF16>
-__device__ __forceinline__ void store_rows(const KernelArgs& a, uint32_t tO, bool have_acc, bool ok, int ig,
-                                           int sq, int q_start, int b, int h, float m_run, float l_run) {
+// Epilogue of one query row (thread = row, 32x32b shape), NC 32-column groups from c0 on: O = acc / (sum * p_keep) in the
+// 16-bit type; the thread of the first group also writes LSE = max * scale + ln(sum).  A row without any valid key
+// gets zeros and -inf.
+template <bool BF16, int NC>
+__device__ __forceinline__ void store_row(const KernelArgs& a, uint32_t tO, int c0, bool have_acc, bool ok, int ig,
+                                          int sq, int q_start, int b, int h, float m_run, float l_run) {
   const bool bad_sum = (l_run == 0.f) || (l_run != l_run);
   const float inv = bad_sum ? 1.f : (1.f / l_run) * a.rp_keep;
-  const bool store_row = ok && (ig < sq);
+  const bool store = ok && (ig < sq);
   uint16_t* orow = reinterpret_cast<uint16_t*>(a.o) + static_cast<int64_t>(q_start + ig) * a.o_row_stride +
                    static_cast<int64_t>(h) * a.o_head_stride;
 #pragma unroll
-  for (int c = 0; c < D / 32; ++c) {
+  for (int i = 0; i < NC; ++i) {
+    const int c = c0 + i;
     uint32_t orr[32];
     if (have_acc) {
       tmem_ld32(tO + c * 32, orr);
       tmem_wait_ld();
     } else {
 #pragma unroll
-      for (int i = 0; i < 32; ++i) orr[i] = 0u;
+      for (int k = 0; k < 32; ++k) orr[k] = 0u;
     }
-    if (store_row && c * 32 < a.head_dim) {
+    if (store && c * 32 < a.head_dim) {
       uint32_t pko[16];
 #pragma unroll
-      for (int i = 0; i < 16; ++i)
-        pko[i] = pack_lowp<BF16>(__uint_as_float(orr[2 * i]) * inv, __uint_as_float(orr[2 * i + 1]) * inv);
+      for (int k = 0; k < 16; ++k)
+        pko[k] = pack_lowp<BF16>(__uint_as_float(orr[2 * k]) * inv, __uint_as_float(orr[2 * k + 1]) * inv);
       uint4* dst = reinterpret_cast<uint4*>(orow + c * 32);
       const int nvec = min(4, (a.head_dim - c * 32) / 8);
 #pragma unroll
@@ -143,17 +136,17 @@ __device__ __forceinline__ void store_rows(const KernelArgs& a, uint32_t tO, boo
         if (v < nvec) dst[v] = make_uint4(pko[4 * v], pko[4 * v + 1], pko[4 * v + 2], pko[4 * v + 3]);
     }
   }
-  if (store_row) {
+  if (store && c0 == 0) {
     const float lse = bad_sum ? -INFINITY : (m_run * a.scale + __logf(l_run));
     a.lse[(static_cast<int64_t>(b) * a.heads + h) * a.lse_stride + ig] = lse;
   }
 }
 
-template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BLOCKSPARSE, int G>
-__global__ void __launch_bounds__(128 * (G + 1), G == 1 ? 2 : 1)
+template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BLOCKSPARSE, int G, bool ROWS>
+__global__ void __launch_bounds__(FwdCfg<D, DROPOUT, G, ROWS>::kThreads, G == 1 ? 2 : 1)
 fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
               const __grid_constant__ CUtensorMap tm_v, const KernelArgs a) {
-  using Cfg = FwdCfg<D, DROPOUT, G>;
+  using Cfg = FwdCfg<D, DROPOUT, G, ROWS>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ FwdShared sh;
   // block-sparse: key tiles this CTA visits (ascending), built from the layout table
@@ -234,9 +227,9 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&sh.q_full[i]), 1);
       mbar_init(smem_u32(&sh.s_full[i]), 1);
-      mbar_init(smem_u32(&sh.s_free[i]), kBlockM);
-      mbar_init(smem_u32(&sh.p_half[i]), kBlockM);
-      mbar_init(smem_u32(&sh.p_full[i]), kBlockM);
+      mbar_init(smem_u32(&sh.s_free[i]), Cfg::kArrivals);
+      mbar_init(smem_u32(&sh.p_half[i]), Cfg::kArrivals);
+      mbar_init(smem_u32(&sh.p_full[i]), Cfg::kArrivals);
       mbar_init(smem_u32(&sh.o_full[i]), 1);
     }
     for (int i = 0; i < 3; ++i) {
@@ -247,15 +240,15 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     }
     fence_mbar_init();
   }
-  if (warp == 4 * G) tmem_alloc(smem_u32(&sh.tmem_base), Cfg::kTmemCols);
+  if (warp == Cfg::kSoftmaxWarps) tmem_alloc(smem_u32(&sh.tmem_base), Cfg::kTmemCols);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sh.tmem_base;
   volatile int* abort_flag = &sh.abort_flag;
 
-  if (warp >= 4 * G) reg_dealloc<Cfg::kOtherRegs>();
-  if (warp == 4 * G) {
+  if (warp >= Cfg::kSoftmaxWarps) reg_dealloc<Cfg::kOtherRegs>();
+  if (warp == Cfg::kSoftmaxWarps) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       tma_prefetch_desc(&tm_q);
@@ -294,7 +287,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         }
       }
     }
-  } else if (warp == 4 * G + 1) {
+  } else if (warp == Cfg::kSoftmaxWarps + 1) {
     // ------------------------------------------------------------------ MMA issuer
     // all 32 lanes run the loop, one elected lane issues (see mma_ss)
     {
@@ -342,17 +335,14 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           if (elect_one()) mma_commit(smem_u32(&sh.k_empty[0]));
         }
       }
-      FA_PROF_DECL
       for (int j = 0; j < n_max && ok; ++j) {
         const int s = j % Cfg::kStages;
         const int sn = (j + 1) % Cfg::kStages;
         const bool has_next = j + 1 < n_max;
-        FA_PROF(0)
         if (!Cfg::kSeparateP) ok = mbar_wait_warp(smem_u32(&sh.v_full[s]), (j / Cfg::kStages) & 1, abort_flag);
         if (ok && has_next)
           ok = mbar_wait_warp(smem_u32(&sh.k_full[sn]), ((j + 1) / Cfg::kStages) & 1, abort_flag);
         if (!ok) break;
-        FA_PROF(1)
         if constexpr (Cfg::kSeparateP) {
           // this warp issues only the score products; warp 10 issues P*V
 #pragma unroll
@@ -361,14 +351,11 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
               ok = mbar_wait_warp(smem_u32(&sh.s_free[g]), j & 1, abort_flag);
               if (ok) {
                 tc_fence_after();
-                FA_STAMP(j, 16 + g * 2)
                 issue_qk(g, sn);
-                FA_STAMP(j, 17 + g * 2)
               }
             }
           }
           if (!ok) break;
-          FA_PROF(5)
         } else {
 #pragma unroll
           for (int g = 0; g < G; ++g) {
@@ -383,12 +370,9 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
               }
               if (ok) ok = mbar_wait_warp(smem_u32(&sh.p_full[g]), j & 1, abort_flag);
               if (ok) {
-                FA_PROF(2 + g)
                 tc_fence_after();
                 issue_pv(g, s, j > 0, kFirst, kBlockN / 16);
-                FA_PROF(4)
                 if (j + 1 < n_tiles[g]) issue_qk(g, sn);
-                FA_PROF(5)
               }
             }
           }
@@ -399,9 +383,8 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           if (has_next) mma_commit(smem_u32(&sh.k_empty[sn]));
         }
       }
-      FA_PROF_FLUSH(16, n_max)
     }
-  } else if (warp == 4 * G + 2) {
+  } else if (warp == Cfg::kSoftmaxWarps + 2) {
     // ------------------------------------------------------------------ second MMA issuer (d = 64): P*V
     if constexpr (Cfg::kSeparateP) {
       constexpr uint32_t idesc_pv = make_idesc(BF16, false, true, kBlockM, D);
@@ -418,7 +401,6 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             ok = mbar_wait_warp(smem_u32(&sh.p_full[g]), j & 1, abort_flag);
             if (ok) {
               tc_fence_after();
-              FA_STAMP(j, 20 + g * 2)
               const uint32_t tO = tmem + (g == 0 ? Cfg::kTmemO0 : Cfg::kTmemO1);
               const uint32_t tP = tmem + (g == 0 ? Cfg::kTmemP0 : Cfg::kTmemP1);
               if (elect_one()) {
@@ -427,7 +409,6 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                   mma_ts(tO, tP + ks * 8, desc_at(va, ks * 2048), idesc_pv, j > 0 || ks > 0);
                 mma_commit(smem_u32(&sh.o_full[g]));
               }
-              FA_STAMP(j, 21 + g * 2)
             }
           }
         }
@@ -435,218 +416,8 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         if (elect_one()) mma_commit(smem_u32(&sh.v_empty[s]));
       }
     }
-  } else if (warp < 4 * G && DROPOUT) {
-    // ------------------------------------------------------------------ softmax groups, dropout
-    // Quad layout: a warp reads its 32 rows as two 16-row blocks (hh) with the 16x256b shape, so a
-    // thread holds rows r8 and r8 + 8 of each block and, of every 8-column unit, two adjacent columns.
-    // That is the ownership pattern of the reference's mask generator: one Philox call covers exactly
-    // one thread's part of a 16 x 16 patch (QuadPhilox).  Row statistics are reduced over the four
-    // lanes of a quad.  Row index ri = hh * 2 + u for row r8 + 16 * hh + 8 * u of the warp.
-    reg_alloc<Cfg::kSoftmaxRegs>();
-    const int g = warp >> 2;
-    const int wq = warp & 3;
-    const int r8 = lane >> 2, q4 = lane & 3;
-    const int row_base = m0[g] + wq * 32 + r8;  // + 16 * hh + 8 * u: query index within the sequence
-    const uint32_t lane_sel = static_cast<uint32_t>(wq * 32) << 16;
-    constexpr uint32_t kHalf = 16u << 16;  // second 16-row block of the warp
-    const uint32_t tS = tmem + (g == 0 ? Cfg::kTmemS0 : Cfg::kTmemS1) + lane_sel;
-    const uint32_t tO = tmem + (g == 0 ? Cfg::kTmemO0 : Cfg::kTmemO1) + lane_sel;
-    const uint32_t tP = tmem + (g == 0 ? Cfg::kTmemP0 : Cfg::kTmemP1) + lane_sel;
-    const int n = n_tiles[g];
-    const bool active = m0[g] < sq;
-
-    float m_run[4], l_run[4];  // l_run: this thread's share of the row sum (its 32 columns per tile)
-#pragma unroll
-    for (int ri = 0; ri < 4; ++ri) { m_run[ri] = -INFINITY; l_run[ri] = 0.f; }
-    bool ok = true;
-    const uint64_t c2 = pack_f2(a.scale_log2, a.scale_log2);
-
-    const int64_t bh_sub =
-        (static_cast<int64_t>(b) * a.drop.heads_total + a.drop.head_offset + h) * 256;
-    const int L16 = (sq + 15) >> 4;
-    const int i16_base = (m0[g] + wq * 32) >> 4;  // 16-row block index of hh = 0
-    QuadPhilox<8> qp;
-    qp.init(a.drop, bh_sub, lane);
-    const float thr_term = fa_keep_thr_term(a.drop.threshold);
-
-    for (int j = 0; j < n && ok; ++j) {
-      const int col0 = kv_tile(j) * kBlockN;
-      int32_t bs_it[2] = {0, 0};
-      if constexpr (BLOCKSPARSE) {
-        const int kb = col0 >> 8;
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh)
-          bs_it[hh] = (i16_base + hh) < a.bs_rows16
-                          ? a.bs_iter[(static_cast<int64_t>(b) * a.bs_kblocks + kb) * a.bs_rows16 + i16_base + hh]
-                          : -1;
-      }
-      bool need_mask = (col0 + kBlockN > sk);
-      if (CAUSAL) need_mask = need_mask || (col0 + kBlockN - 1 > m0[g]);
-      float alpha[4];
-      bool grow_any = false;
-      // pk[hh][2 * unit + u]: the 16x128b register of (row u, packed column pair 4 * unit + q4)
-      uint32_t pk[2][32];
-      // The two 16-row blocks of the warp one after the other (their rows are independent), which
-      // keeps the live registers at one block of keep words, scores and packed probabilities.
-#pragma unroll
-      for (int hh = 0; hh < 2; ++hh) {
-        // Keep words of the block: 8 calls (one per 16-column group), rounds interleaved so that their
-        // multiply chains overlap.  kw[grp][2 * u + half]: row u, columns 16 grp + 8 half + 2 q4 (+1 in
-        // the high 16 bits).  One iteration index per tile: a 128-column tile lies inside one key block.
-        uint32_t kw[8][4];
-        {
-          int64_t it_index;
-          if constexpr (BLOCKSPARSE) it_index = bs_it[hh];
-          else it_index = fa_iter_index(CAUSAL, col0 >> a.drop.n_shift, i16_base + hh, L16, a.drop.n_shift);
-          qp.set_tile(a.drop, it_index, col0);
-#pragma unroll
-          for (int grp = 0; grp < 8; ++grp) qp.start(grp, kw[grp]);
-#pragma unroll
-          for (int r = 2; r < 7; ++r)
-#pragma unroll
-            for (int k = 0; k < 8; ++k) QuadPhilox<8>::round(a.drop, kw[k], r);
-        }
-        if (hh == 0) {
-          ok = mbar_wait(smem_u32(&sh.s_full[g]), j & 1, abort_flag);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-          tc_fence_after();
-        }
-        // sr[4 * unit + 2 * u + c]: row u of the block, column 8 * unit + 2 * q4 + c of the tile
-        uint32_t sr[64];
-        tmem_ld_quad64(tS + hh * kHalf, sr);
-        tmem_wait_ld();
-        if constexpr (Cfg::kSeparateP) {
-          if (hh == 1) {
-            tc_fence_before();
-            mbar_arrive(smem_u32(&sh.s_free[g]));
-          }
-        }
-        if (need_mask) {
-#pragma unroll
-          for (int i = 0; i < 64; ++i) {
-            const int col = col0 + (i >> 2) * 8 + 2 * q4 + (i & 1);
-            const int ig = row_base + hh * 16 + ((i >> 1) & 1) * 8;
-            bool valid = col < sk;
-            if (CAUSAL) valid = valid && (col <= ig);
-            if (!valid) sr[i] = __float_as_uint(-INFINITY);
-          }
-        }
-        if constexpr (BLOCKSPARSE) {
-          // a 16-row block that is not in the layout for this 256-column key block sees -inf
-          if (bs_it[hh] < 0) {
-#pragma unroll
-            for (int i = 0; i < 64; ++i) sr[i] = __float_as_uint(-INFINITY);
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int ri = hh * 2 + u;
-          // row maximum: 32 own columns, then the quad
-          float mxa = -INFINITY, mxb = -INFINITY;
-#pragma unroll
-          for (int unit = 0; unit < 16; unit += 2) {
-            mxa = max3(mxa, __uint_as_float(sr[4 * unit + 2 * u]), __uint_as_float(sr[4 * unit + 2 * u + 1]));
-            mxb = max3(mxb, __uint_as_float(sr[4 * unit + 4 + 2 * u]), __uint_as_float(sr[4 * unit + 5 + 2 * u]));
-          }
-          float mx = fmaxf(mxa, mxb);
-          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-          const float m_new = fmaxf(m_run[ri], mx);
-          // The running max is only raised when it would grow by more than 2^8 in the exponent:
-          // until then the stale max keeps every p below 256 and saves rescaling O.
-          const bool grow = (m_new - m_run[ri]) * a.scale_log2 > 8.f;
-          const float m_next = grow ? m_new : m_run[ri];
-          alpha[ri] = (!grow || m_run[ri] == -INFINITY) ? (grow ? 0.f : 1.f)
-                                                        : ex2f((m_run[ri] - m_new) * a.scale_log2);
-          m_run[ri] = m_next;
-          const float mc = (m_next == -INFINITY) ? 0.f : m_next * a.scale_log2;
-          grow_any = grow_any || grow;
-
-          // p = exp2(s * c - m * c): packed fma, one ex2 per element, packed row sum; the row sum
-          // takes the un-dropped p, P*V takes p times the keep factor (1 or 0), rounded to 16 bits
-          const uint64_t nmc2 = pack_f2(-mc, -mc);
-          uint64_t sum_a = 0ull, sum_b = 0ull;
-#pragma unroll
-          for (int unit = 0; unit < 16; unit += 2) {
-            float p0, p1, p2, p3;
-            unpack_f2(fma2(pack_f2(__uint_as_float(sr[4 * unit + 2 * u]), __uint_as_float(sr[4 * unit + 2 * u + 1])), c2, nmc2), p0, p1);
-            unpack_f2(fma2(pack_f2(__uint_as_float(sr[4 * unit + 4 + 2 * u]), __uint_as_float(sr[4 * unit + 5 + 2 * u])), c2, nmc2), p2, p3);
-            p0 = ex2f(p0); p1 = ex2f(p1); p2 = ex2f(p2); p3 = ex2f(p3);
-            const uint64_t p01 = pack_f2(p0, p1), p23 = pack_f2(p2, p3);
-            sum_a = add2(sum_a, p01);
-            sum_b = add2(sum_b, p23);
-            const uint32_t w01 = kw[unit / 2][2 * u], w23 = kw[unit / 2][2 * u + 1];
-            unpack_f2(mul2(p01, pack_f2(fa_keep_factor_lo(w01, thr_term), fa_keep_factor_hi(w01, thr_term))), p0, p1);
-            unpack_f2(mul2(p23, pack_f2(fa_keep_factor_lo(w23, thr_term), fa_keep_factor_hi(w23, thr_term))), p2, p3);
-            pk[hh][2 * unit + u] = pack_lowp<BF16>(p0, p1);
-            pk[hh][2 * unit + 2 + u] = pack_lowp<BF16>(p2, p3);
-          }
-          float s0, s1;
-          unpack_f2(add2(sum_a, sum_b), s0, s1);
-          l_run[ri] = l_run[ri] * alpha[ri] + (s0 + s1);
-        }
-      }
-      if (!ok) break;
-
-      // P*V of the previous tile must have finished before O is rescaled or its P buffer reused
-      if (j > 0) {
-        ok = mbar_wait(smem_u32(&sh.o_full[g]), (j - 1) & 1, abort_flag);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        tc_fence_after();
-        if (__any_sync(0xffffffffu, grow_any)) {
-#pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {
-            const uint64_t al0 = pack_f2(alpha[hh * 2], alpha[hh * 2]);
-            const uint64_t al1 = pack_f2(alpha[hh * 2 + 1], alpha[hh * 2 + 1]);
-#pragma unroll
-            for (int c = 0; c < D / 64; ++c) {
-              uint32_t orr[32];
-              tmem_ld_quad32(tO + hh * kHalf + c * 64, orr);
-              tmem_wait_ld();
-#pragma unroll
-              for (int i = 0; i < 32; i += 2) {
-                float lo, hi;
-                unpack_f2(mul2(pack_f2(__uint_as_float(orr[i]), __uint_as_float(orr[i + 1])), (i & 2) ? al1 : al0), lo, hi);
-                orr[i] = __float_as_uint(lo);
-                orr[i + 1] = __float_as_uint(hi);
-              }
-              tmem_st_quad32(tO + hh * kHalf + c * 64, orr);
-            }
-          }
-        }
-      }
-      // hand P to the tensor core through tensor memory
-      tmem_st_pair32(tP, pk[0]);
-      tmem_st_pair32(tP + kHalf, pk[1]);
-      tmem_wait_st();
-      tc_fence_before();
-      mbar_arrive(smem_u32(&sh.p_full[g]));
-    }
-
-    // ---------------- epilogue: O = acc / (sum * p_keep), LSE, one thread per query row again
-    if (active) {
-      if (n > 0 && ok) {
-        ok = mbar_wait(smem_u32(&sh.o_full[g]), (n - 1) & 1, abort_flag);
-        ok = __all_sync(0xffffffffu, ok);
-        tc_fence_after();
-      }
-      // row lane (0..31 of the warp) = 16 * hh + 8 * u + r8: its statistics sit in the quad r8 under ri = lane / 8
-      float m_row = -INFINITY, l_row = 0.f;
-#pragma unroll
-      for (int ri = 0; ri < 4; ++ri) {
-        float l = l_run[ri];
-        l += __shfl_xor_sync(0xffffffffu, l, 1);
-        l += __shfl_xor_sync(0xffffffffu, l, 2);
-        const float l_src = __shfl_sync(0xffffffffu, l, (lane & 7) * 4);
-        const float m_src = __shfl_sync(0xffffffffu, m_run[ri], (lane & 7) * 4);
-        if ((lane >> 3) == ri) { l_row = l_src; m_row = m_src; }
-      }
-      store_rows<D, BF16>(a, tO, n > 0 && ok, ok, m0[g] + wq * 32 + lane, sq, q_start, b, h, m_row, l_row);
-    }
-  } else if (warp < 4 * G) {
-    // ------------------------------------------------------------------ softmax groups, no dropout
+  } else if (Cfg::kRows && warp < Cfg::kSoftmaxWarps) {
+    // ------------------------------------------------------------------ softmax groups, one thread per query row
     reg_alloc<Cfg::kSoftmaxRegs>();
     const int g = warp >> 2;
     const int row = tid & 127;
@@ -662,23 +433,16 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     bool ok = true;
     const uint64_t c2 = pack_f2(a.scale_log2, a.scale_log2);
 
-    FA_PROF_DECL
     for (int j = 0; j < n && ok; ++j) {
       const int col0 = kv_tile(j) * kBlockN;
       int32_t bs_it = 0;
-      if constexpr (BLOCKSPARSE) {
-        const int kb = col0 >> 8;
+      if constexpr (BLOCKSPARSE)
         bs_it = (ig >> 4) < a.bs_rows16
-                    ? a.bs_iter[(static_cast<int64_t>(b) * a.bs_kblocks + kb) * a.bs_rows16 + (ig >> 4)]
+                    ? a.bs_iter[(static_cast<int64_t>(b) * a.bs_kblocks + (col0 >> 8)) * a.bs_rows16 + (ig >> 4)]
                     : -1;
-      }
-      FA_PROF(0)
-      if (row == 0) { FA_STAMP(j, g * 8 + 0) }
       ok = mbar_wait(smem_u32(&sh.s_full[g]), j & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
-      FA_PROF(1)
-      if (row == 0) { FA_STAMP(j, g * 8 + 1) }
       tc_fence_after();
       uint32_t sr[4][32];
 #pragma unroll
@@ -688,8 +452,6 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         tc_fence_before();
         mbar_arrive(smem_u32(&sh.s_free[g]));
       }
-      FA_PROF(2)
-      if (row == 0) { FA_STAMP(j, g * 8 + 2) }
 
       bool need_mask = (col0 + kBlockN > sk);
       if (CAUSAL) need_mask = need_mask || (col0 + kBlockN - 1 > m0[g]);
@@ -723,8 +485,6 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           mxb = max3(mxb, __uint_as_float(sr[c][i + 2]), __uint_as_float(sr[c][i + 3]));
         }
       const float m_new = max3(m_run, mxa, mxb);
-      FA_PROF(3)
-      if (row == 0) { FA_STAMP(j, g * 8 + 3) }
 
       // The running max is only raised when it would grow by more than 2^8 in the exponent:
       // until then the stale max keeps every p below 256 and saves rescaling O.
@@ -732,7 +492,6 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       const float m_next = grow ? m_new : m_run;
       const float alpha = (!grow || m_run == -INFINITY) ? (grow ? 0.f : 1.f) : ex2f((m_run - m_new) * a.scale_log2);
       m_run = m_next;
-      FA_PROF(4)
       const float mc = (m_next == -INFINITY) ? 0.f : m_next * a.scale_log2;
       const uint64_t nmc2 = pack_f2(-mc, -mc);
 
@@ -756,15 +515,12 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           }
       };
       expo_half(0);
-      FA_PROF(5)
-      if (row == 0) { FA_STAMP(j, g * 8 + 4) }
       // P*V of the previous tile must have finished before O is rescaled or its P buffer reused.  (Half of the
       // exponentials are still to come: by now it has, as a rule.)
       if (j > 0) {
         ok = mbar_wait(smem_u32(&sh.o_full[g]), (j - 1) & 1, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
-        if (row == 0) { FA_STAMP(j, g * 8 + 5) }
         tc_fence_after();
         if (__any_sync(0xffffffffu, grow)) {
           const uint64_t alpha2 = pack_f2(alpha, alpha);
@@ -801,10 +557,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       tmem_wait_st();
       tc_fence_before();
       mbar_arrive(smem_u32(&sh.p_full[g]));
-      FA_PROF(7)
-      if (row == 0) { FA_STAMP(j, g * 8 + 6) }
     }
-    if (g == 0 && row == 0) { FA_PROF_FLUSH(8, n) }
 
     // ---------------- epilogue: O = acc / (sum * p_keep), LSE
     if (active) {
@@ -813,13 +566,230 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
       }
-      store_rows<D, BF16>(a, tO, n > 0 && ok, ok, ig, sq, q_start, b, h, m_run, l_run);
+      store_row<BF16, D / 32>(a, tO, 0, n > 0 && ok, ok, ig, sq, q_start, b, h, m_run, l_run);
+    }
+  } else if (warp < Cfg::kSoftmaxWarps) {
+    // ------------------------------------------------------------------ softmax warps
+    // A warp owns 16 query rows.  It reads their scores with the 16x256b shape, in which a thread holds rows r8 and
+    // r8 + 8 and, of every 8-column unit, two adjacent columns: the ownership pattern of the reference's mask
+    // generator (one Philox call covers exactly one thread's part of a 16 x 16 patch, QuadPhilox).
+    reg_alloc<Cfg::kSoftmaxRegs>();
+    const int g = (G == 1) ? 0 : warp >> 3;
+    const int hh = (warp >> 2) & 1, wq = warp & 3;
+    const int r8 = lane >> 2, q4 = lane & 3;
+    const int m_first = m0[G == 1 ? 0 : g];
+    const int row0 = m_first + wq * 32 + hh * 16;  // of the warp; query index within the sequence
+    const uint32_t lane_sel = static_cast<uint32_t>(wq * 32 + hh * 16) << 16;
+    const uint32_t tS = tmem + (g == 0 ? Cfg::kTmemS0 : Cfg::kTmemS1) + lane_sel;
+    const uint32_t tO = tmem + (g == 0 ? Cfg::kTmemO0 : Cfg::kTmemO1) + lane_sel;
+    const uint32_t tP = tmem + (g == 0 ? Cfg::kTmemP0 : Cfg::kTmemP1) + lane_sel;
+    const int n = n_tiles[G == 1 ? 0 : g];
+    const bool active = m_first < sq;
+
+    // rows r8 (u = 0) and r8 + 8 (u = 1); l_run: this thread's share of the row sum (its 32 columns per tile)
+    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
+    bool ok = true;
+    const uint64_t c2 = pack_f2(a.scale_log2, a.scale_log2);
+
+    const int64_t bh_sub =
+        (static_cast<int64_t>(b) * a.drop.heads_total + a.drop.head_offset + h) * 256;
+    const int L16 = (sq + 15) >> 4;
+    const int i16 = row0 >> 4;
+    QuadPhilox<8> qp;
+    float thr_term = 0.f;
+    if constexpr (DROPOUT) {
+      qp.init(a.drop, bh_sub, lane);
+      thr_term = fa_keep_thr_term(a.drop.threshold);
+    }
+    auto arrive_warp = [&](uint64_t& bar) {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&bar));
+    };
+
+    for (int j = 0; j < n && ok; ++j) {
+      const int col0 = kv_tile(j) * kBlockN;
+      int32_t bs_it = 0;
+      if constexpr (BLOCKSPARSE)
+        bs_it = i16 < a.bs_rows16
+                    ? a.bs_iter[(static_cast<int64_t>(b) * a.bs_kblocks + (col0 >> 8)) * a.bs_rows16 + i16]
+                    : -1;
+      const bool need_mask = (col0 + kBlockN > sk) || (CAUSAL && (col0 + kBlockN - 1 > m_first)) ||
+                             (BLOCKSPARSE && bs_it < 0);
+      // -inf for columns without a key, keys behind the diagonal and 16-row blocks that are not in the layout; s[]
+      // holds the units from unit0 on, s[4 * unit + 2 * u + c] = (row r8 + 8 u, column 8 unit + 2 q4 + c)
+      auto mask = [&](auto& s, int unit0) {
+        constexpr int kValues = sizeof(s) / 4;
+#pragma unroll
+        for (int i = 0; i < kValues; ++i) {
+          const int col = col0 + (unit0 + (i >> 2)) * 8 + 2 * q4 + (i & 1);
+          bool valid = col < sk;
+          if (CAUSAL) valid = valid && (col <= row0 + r8 + ((i >> 1) & 1) * 8);
+          if (BLOCKSPARSE) valid = valid && bs_it >= 0;
+          if (!valid) s[i] = __float_as_uint(-INFINITY);
+        }
+      };
+      ok = mbar_wait_warp(smem_u32(&sh.s_full[g]), j & 1, abort_flag);
+      if (!ok) break;
+      tc_fence_after();
+      uint32_t sr[64];
+      tmem_ld_quad32(tS, reinterpret_cast<uint32_t(&)[32]>(sr[0]));
+      tmem_ld_quad32(tS + 64, reinterpret_cast<uint32_t(&)[32]>(sr[32]));
+      tmem_wait_ld();
+      if constexpr (Cfg::kSeparateP && !DROPOUT) arrive_warp(sh.s_free[g]);
+      if (need_mask) mask(sr, 0);
+
+      // Row maxima.  The running max is only raised when it would grow by more than 2^8 in the exponent: until then
+      // the stale max keeps every p below 256 and saves rescaling O.  Whether any row of the warp grows
+      // shows without putting the quads' columns together.
+      float mx[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        float mxa = -INFINITY, mxb = -INFINITY;
+#pragma unroll
+        for (int unit = 0; unit < 16; unit += 2) {
+          mxa = max3(mxa, __uint_as_float(sr[4 * unit + 2 * u]), __uint_as_float(sr[4 * unit + 2 * u + 1]));
+          mxb = max3(mxb, __uint_as_float(sr[4 * unit + 4 + 2 * u]), __uint_as_float(sr[4 * unit + 5 + 2 * u]));
+        }
+        mx[u] = max3(m_run[u], mxa, mxb);
+      }
+      const bool grows = (mx[0] - m_run[0]) * a.scale_log2 > 8.f || (mx[1] - m_run[1]) * a.scale_log2 > 8.f;
+      if (__any_sync(0xffffffffu, grows)) {
+        float alpha[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          float m_new = fmaxf(mx[u], __shfl_xor_sync(0xffffffffu, mx[u], 1));
+          m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, 2));
+          const bool grow = (m_new - m_run[u]) * a.scale_log2 > 8.f;
+          alpha[u] = (!grow || m_run[u] == -INFINITY) ? (grow ? 0.f : 1.f)
+                                                      : ex2f((m_run[u] - m_new) * a.scale_log2);
+          if (grow) m_run[u] = m_new;
+          l_run[u] *= alpha[u];
+        }
+        if (j > 0) {
+          // P*V of the previous tile must have finished before O is rescaled
+          ok = mbar_wait_warp(smem_u32(&sh.o_full[g]), (j - 1) & 1, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          const uint64_t al[2] = {pack_f2(alpha[0], alpha[0]), pack_f2(alpha[1], alpha[1])};
+#pragma unroll 1
+          for (int c = 0; c < D; c += 32) {
+            uint32_t orr[16];
+            tmem_ld_quad16(tO + c, orr);
+            tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) {
+              float lo, hi;
+              unpack_f2(mul2(pack_f2(__uint_as_float(orr[i]), __uint_as_float(orr[i + 1])), al[(i >> 1) & 1]), lo, hi);
+              orr[i] = __float_as_uint(lo);
+              orr[i + 1] = __float_as_uint(hi);
+            }
+            tmem_st_quad16(tO + c, orr);
+          }
+          tmem_wait_st();
+        }
+      }
+      uint64_t nmc2[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const float mc = (m_run[u] == -INFINITY) ? 0.f : m_run[u] * a.scale_log2;
+        nmc2[u] = pack_f2(-mc, -mc);
+      }
+
+      // p = exp2(s * c - m * c): packed fma, one ex2 per element, packed row sum, 16-bit pack.  The row sum takes the
+      // un-dropped p, P*V takes p times the keep factor (1 or 0).  64 columns after the other; s[] holds those of `half`.
+      uint64_t sum_a[2] = {0ull, 0ull}, sum_b[2] = {0ull, 0ull};
+      if constexpr (DROPOUT) {
+        int64_t it_index;
+        if constexpr (BLOCKSPARSE) it_index = bs_it;
+        else it_index = fa_iter_index(CAUSAL, col0 >> a.drop.n_shift, i16, L16, a.drop.n_shift);
+        qp.set_tile(a.drop, it_index, col0);
+      }
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        uint32_t kw[DROPOUT ? 4 : 1][4];
+        uint32_t sh_[DROPOUT ? 32 : 1];
+        if constexpr (DROPOUT) {
+          // The scores are read again (the first pass was for the maxima): 32 instead of 64 of them live beside the
+          // keep words of the half's four calls, kw[grp][2 * u + v] = row u, columns 16 grp + 8 v + 2 q4 (+1 high).
+          tmem_ld_quad32(tS + half * 64, sh_);
+#pragma unroll
+          for (int grp = 0; grp < 4; ++grp) qp.start(half * 4 + grp, kw[grp]);
+#pragma unroll
+          for (int r = 2; r < 7; ++r)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) QuadPhilox<8>::round(a.drop, kw[k], r);
+          tmem_wait_ld();
+          if (Cfg::kSeparateP && half == 1) arrive_warp(sh.s_free[g]);
+          if (need_mask) mask(sh_, half * 8);
+        }
+        const uint32_t* s = DROPOUT ? sh_ : sr + half * 32;
+        uint32_t pk[16];  // [2 * unit + u]: the 16x128b register of (row u, packed column pair 4 * unit + q4)
+#pragma unroll
+        for (int unit = 0; unit < 8; unit += 2) {
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            float p0, p1, p2, p3;
+            unpack_f2(fma2(pack_f2(__uint_as_float(s[4 * unit + 2 * u]), __uint_as_float(s[4 * unit + 2 * u + 1])), c2, nmc2[u]), p0, p1);
+            unpack_f2(fma2(pack_f2(__uint_as_float(s[4 * unit + 4 + 2 * u]), __uint_as_float(s[4 * unit + 5 + 2 * u])), c2, nmc2[u]), p2, p3);
+            p0 = ex2f(p0); p1 = ex2f(p1); p2 = ex2f(p2); p3 = ex2f(p3);
+            const uint64_t p01 = pack_f2(p0, p1), p23 = pack_f2(p2, p3);
+            sum_a[u] = add2(sum_a[u], p01);
+            sum_b[u] = add2(sum_b[u], p23);
+            if constexpr (DROPOUT) {
+              const uint32_t w01 = kw[unit / 2][2 * u], w23 = kw[unit / 2][2 * u + 1];
+              unpack_f2(mul2(p01, pack_f2(fa_keep_factor_lo(w01, thr_term), fa_keep_factor_hi(w01, thr_term))), p0, p1);
+              unpack_f2(mul2(p23, pack_f2(fa_keep_factor_lo(w23, thr_term), fa_keep_factor_hi(w23, thr_term))), p2, p3);
+            }
+            pk[2 * unit + u] = pack_lowp<BF16>(p0, p1);
+            pk[2 * unit + 2 + u] = pack_lowp<BF16>(p2, p3);
+          }
+        }
+        if (half == 0 && j > 0) {
+          // P*V of the previous tile must have finished before its P buffer is reused
+          ok = mbar_wait_warp(smem_u32(&sh.o_full[g]), (j - 1) & 1, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+        }
+        // hand P to the tensor core through tensor memory
+        tmem_st_pair16(tP + half * 32, pk);
+      }
+      if (ok) {
+        tmem_wait_st();
+        arrive_warp(sh.p_full[g]);
+      }
+      if (!ok) break;
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        float s0, s1;
+        unpack_f2(add2(sum_a[u], sum_b[u]), s0, s1);
+        l_run[u] += s0 + s1;
+      }
+    }
+
+    // ---------------- epilogue: O = acc / (sum * p_keep), LSE.  One thread per query row (32 rows per warp, half of the
+    // columns): the statistics of a row pass through shared memory.
+    if (active) {
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        float l = l_run[u];
+        l += __shfl_xor_sync(0xffffffffu, l, 1);
+        l += __shfl_xor_sync(0xffffffffu, l, 2);
+        if (q4 == 0) sh.row_stats[g][wq * 32 + hh * 16 + u * 8 + r8] = make_float2(m_run[u], l);
+      }
+      named_barrier_sync(1 + g, 32 * Cfg::kGroupWarps);  // every warp of the group comes here, also after an abandoned wait
+      if (n > 0 && ok) {
+        ok = mbar_wait_warp(smem_u32(&sh.o_full[g]), (n - 1) & 1, abort_flag);
+        tc_fence_after();
+      }
+      const float2 st = sh.row_stats[g][wq * 32 + lane];
+      store_row<BF16, D / 64>(a, tO - (static_cast<uint32_t>(hh * 16) << 16), hh * (D / 64), n > 0 && ok, ok, m_first + wq * 32 + lane, sq, q_start, b, h, st.x, st.y);
     }
   }
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 4 * G) {
+  if (warp == Cfg::kSoftmaxWarps) {
     tmem_dealloc(tmem, Cfg::kTmemCols);
     if (lane == 0 && sh.abort_flag && a.status) {
       atomicExch(a.status, a.launch_id);  // stops the CTAs of this launch that have not started yet
@@ -828,10 +798,10 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   }
 }
 
-template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BS, int G>
+template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BS, int G, bool ROWS>
 cudaError_t launch_groups(const FwdLaunch& l, cudaStream_t stream) {
-  auto kernel = fa_fwd_kernel<D, BF16, CAUSAL, DROPOUT, BS, G>;
-  using Cfg = FwdCfg<D, DROPOUT, G>;
+  auto kernel = fa_fwd_kernel<D, BF16, CAUSAL, DROPOUT, BS, G, ROWS>;
+  using Cfg = FwdCfg<D, DROPOUT, G, ROWS>;
   static SmemLimitFlags smem_limit_set;  // one per template instantiation of this function
   cudaError_t e = set_smem_limit_once(kernel, Cfg::kSmemBytes, smem_limit_set);
   if (e != cudaSuccess) return e;
@@ -840,57 +810,61 @@ cudaError_t launch_groups(const FwdLaunch& l, cudaStream_t stream) {
   return cudaGetLastError();
 }
 
-// One query tile per CTA (two CTAs per SM) or two.  Batches of ragged sequences, 12 heads, us with two -> one:
-//   d = 64    64 x 128: 32 -> 21   64 x 512: 108 -> 86   32 x 1024: 147 -> 124   8 x 4096: 383 -> 358
-//   causal    64 x 128: 34 -> 22   64 x 512:  90 -> 80   32 x 1024: 108 -> 100   8 x 4096: 231 -> 225
-//   dropout   64 x 128: 39 -> 26   64 x 512: 162 -> 143  32 x 1024: 251 -> 229   8 x 4096: 770 -> 736
-//   d = 128   64 x 128: 42 -> 26   64 x 512: 141 -> 125  32 x 1024: 187 -> 182   8 x 4096: 498 -> 552
-//   block-sparse (16 heads, 25 %)    4 x 1024: 41 -> 38     4 x 4096: 196 -> 185
-// What one tile gains lies at the two ends of a CTA's walk over the keys.  What it loses is a share per key tile:
-// two CTAs each read the K and V that a pair reads once, and at d = 128 a single stage holds them.  So the
-// rule looks at the keys.  Time with one tile / with two, 16 x 16 heads, not causal:
-//   keys              256   512  1024  2048  4096  8192 16384
-//   d = 64   128 q   0.72  0.77  0.77  0.80  0.80  0.82  0.84      (a pair's second tile would be empty)
-//            256 q   0.96  0.97  1.01  0.99  1.03  1.06  1.08
-//           1024 q   0.90  0.87  0.93  0.97  1.00  1.03  1.01
-//           4096 q   0.87  0.82  0.90  0.93  0.96  1.07  1.05
-//   d = 128  128 q   0.75  0.76  0.88  0.89  0.91  0.92  0.90
-//            256 q   0.98  1.03  1.08  1.14  1.15  1.15  1.17
-//           1024 q   0.92  0.96  1.04  1.10  1.13  1.14  1.04
-// Causal, queries = keys, 12 heads: d = 64 0.97 at 1024, 0.99 at 4096, 1.01 at 8192; d = 128 0.99 at 768, 1.00 at
-// 1024, 1.02 at 1536, 1.07 at 2048, 1.21 at 8192.
-// The last round of single tiles is worth more when it has at most one CTA per SM, which is then 1.4 times as fast
-// (1.2 at d = 128).  A grid of only that round spreads over twice the SMs: 32 heads, 512 queries, 4096 keys, d = 128
-// 58 -> 54 us; 16 heads, 1024 queries, 8192 keys, d = 64 97 -> 70.  Behind up to five full rounds it still decides at
-// d = 64: 256 heads, 512 queries, 8192 keys 409 -> 373 us, 48 heads, 4096 queries 580 -> 554 (256 heads, 256 queries,
-// whose last round is full: 213 -> 225).
-// Up to 128 queries both grids have as many CTAs; with long keys at d = 128 one alone on its SM then wants the
-// second stage (16 queries, 4096 keys, one -> two: 96 (batch, head) pairs 69 -> 52 us, 144 pairs 80 -> 58).  From 149
-// on two share an SM: 192 pairs 85 us, 128 with two.
+// One query tile per CTA (two CTAs per SM) or two.  What one tile gains lies at the two ends of a CTA's walk over the
+// keys, which run under the tiles of the SM's other CTA.  What it loses is a share per key tile: two CTAs each read the K
+// and V that a pair reads once, and at d = 128 a single stage holds them.
+// Time with one tile / with two, 16 x 16 heads, not causal:
+//                        quads d = 64   dropout d = 64   rows d = 128   dropout d = 128
+//   128 queries, 512 keys     0.74           0.79            0.76            0.79
+//   256, 512                  0.95           0.97            1.00            1.02
+//   256, 4096                 1.02           1.04            1.12            1.19
+//   1024, 1024                0.91           0.93            0.98            0.96
+//   1024, 8192                1.02           1.02            1.14            1.13
+//   4096, 4096 (4 x 16)       0.96           0.99            1.13            1.10
+// so d = 64 takes single tiles at every length (causal calls too: 0.95-0.98), and d = 128 up to 1024 keys without
+// dropout (causal calls count the keys up to the longest query).
+// A grid of single tiles that fits one per SM spreads over twice the SMs: 16 heads, 1024 queries, 8192 keys 0.72 (d = 64),
+// 0.92 (d = 128), 0.63 and 0.78 with dropout.
 // A grid of pairs that fills between half of the SMs and all of them runs in one round either way and reads K and
-// V once per pair: 80-140 pairs of 200-1024 queries, one / two 0.94-1.23 with sequences of one length, and
-// 0.73-1.22 ragged (least for 80 pairs of which most second tiles are empty).
+// V once per pair: 80-140 pairs of 200-4000 queries 1.02-1.13, with dropout 0.99-1.15.
+// Up to 128 queries both grids have as many CTAs; with long keys at d = 128 one alone on its SM then wants the second
+// stage (16 queries, 4096 keys, one -> two: 96 (batch, head) pairs 69 -> 52 us, 144 pairs 80 -> 58).  From 149 on two
+// share an SM: 192 pairs 85 us, 128 with two.
 constexpr int kSms = 148;
-constexpr int kOneTileMaxD64 = 4096, kOneTileMaxD128 = 1024;  // queries and keys
+constexpr int kOneTileMaxD128 = 1024;  // queries and keys
 
-template <int D, bool CAUSAL>
+template <int D, bool CAUSAL, bool DROPOUT>
 bool one_tile_per_cta(const FwdLaunch& l) {
   const int64_t heads = static_cast<int64_t>(l.args.heads) * l.args.batch;
   const int64_t tiles = (l.max_seqlen_q + kBlockM - 1) / kBlockM * heads;
   const int64_t pairs = (l.max_seqlen_q + 2 * kBlockM - 1) / (2 * kBlockM) * heads;
-  constexpr int kMax = D == 64 ? kOneTileMaxD64 : kOneTileMaxD128;
   const int keys = CAUSAL ? min(l.max_seqlen_k, l.max_seqlen_q) : l.max_seqlen_k;
-  if (l.max_seqlen_q <= kBlockM) return D == 64 || keys <= kMax || pairs > kSms;
-  if (pairs > kSms / 2 && pairs <= kSms) return false;
-  const int64_t rounds = tiles / (2 * kSms), last = tiles % (2 * kSms);
-  const bool short_end = last > 0 && last <= kSms && rounds <= (D == 64 ? 5 : 0);
-  return l.max_seqlen_q <= kMax && (keys <= kMax || short_end);
+  const bool one_round = pairs > kSms / 2 && pairs <= kSms;
+  if (l.max_seqlen_q <= kBlockM) return D == 64 || DROPOUT || keys <= kOneTileMaxD128 || pairs > kSms;
+  if (one_round) return false;
+  if (D == 64) return true;
+  if (tiles <= kSms) return l.max_seqlen_q <= kOneTileMaxD128;
+  return !DROPOUT && l.max_seqlen_q <= kOneTileMaxD128 && keys <= kOneTileMaxD128;
 }
+
+// Rows for d = 128 without dropout, and for d = 64 without dropout up to 512 keys: there the ends of a CTA's
+// walk are most of it, and twelve warps take longer through them than eight (quads / rows: 12 heads of 128 queries and
+// keys 5.9 / 5.7 us, 16 x 16 heads, 128 queries, 512 keys 12.5 / 11.8, 1024 keys and queries 0.98).
+constexpr int kRowsMaxD64 = 512;  // keys
 
 template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BS>
 cudaError_t launch_one(const FwdLaunch& l, cudaStream_t stream) {
-  return one_tile_per_cta<D, CAUSAL>(l) ? launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 1>(l, stream)
-                                        : launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 2>(l, stream);
+  const bool one_tile = one_tile_per_cta<D, CAUSAL, DROPOUT>(l);
+  if constexpr (!DROPOUT) {
+    if (D == 128 || l.max_seqlen_k <= kRowsMaxD64)
+      return one_tile ? launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 1, true>(l, stream)
+                      : launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 2, true>(l, stream);
+  }
+  if constexpr (D == 64 || DROPOUT) {
+    return one_tile ? launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 1, false>(l, stream)
+                    : launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 2, false>(l, stream);
+  }
+  return cudaErrorInvalidValue;
 }
 
 template <int D, bool BF16, bool CAUSAL>
