@@ -151,10 +151,9 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   // 3632 -> 3309 -> 3226.
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int lane = tid & 31;
-  const int b = blockIdx.z;
-  const int h = blockIdx.y;
-  const int nt = blockIdx.x;  // key tile
   const KernelArgs& ka = a.k;
+  int b = blockIdx.z, h = blockIdx.y, nt = blockIdx.x;  // nt: key tile
+  if constexpr (CAUSAL) causal_block(ka, nt, h, b);
 
   const int q_start = ka.cu_seqlens_q[b];
   const int sq = ka.cu_seqlens_q[b + 1] - q_start;
@@ -1281,7 +1280,12 @@ cudaError_t launch_main(const BwdLaunch& l, cudaStream_t stream) {
   cudaError_t e = set_smem_limit_once(kernel, smem, smem_limit_set);
   if (e != cudaSuccess) return e;
   dim3 grid((l.args.max_seqlen_k + kBN - 1) / kBN, l.args.k.heads, l.args.k.batch);
-  kernel<<<grid, kBwdThreads, smem, stream>>>(l.tm_q, l.tm_k, l.tm_v, l.tm_do, l.tm_dq, l.args);
+  BwdArgs args = l.args;
+  if constexpr (CAUSAL) {
+    set_causal_grid(&args.k, grid.x, int64_t(8) * D * args.max_seqlen_q);  // Q, dO and the fp32 dQ
+    grid = dim3(grid.x * grid.y * grid.z, 1, 1);
+  }
+  kernel<<<grid, kBwdThreads, smem, stream>>>(l.tm_q, l.tm_k, l.tm_v, l.tm_do, l.tm_dq, args);
   return cudaGetLastError();
 }
 

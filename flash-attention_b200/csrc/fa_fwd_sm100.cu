@@ -157,9 +157,12 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // known to be the same in all lanes
   const int lane = tid & 31;
 
-  const int b = blockIdx.z;
-  const int h = blockIdx.y;
-  const int mp = CAUSAL ? (gridDim.x - 1 - blockIdx.x) : blockIdx.x;  // heavy tiles first
+  int b = blockIdx.z, h = blockIdx.y, mp = blockIdx.x;
+  if constexpr (CAUSAL) {
+    int rank;
+    causal_block(a, rank, h, b);
+    mp = a.grid_tiles - 1 - rank;
+  }
   const int q_start = a.cu_seqlens_q[b];
   const int sq = a.cu_seqlens_q[b + 1] - q_start;
   const int k_start = a.cu_seqlens_k[b];
@@ -806,7 +809,12 @@ cudaError_t launch_groups(const FwdLaunch& l, cudaStream_t stream) {
   cudaError_t e = set_smem_limit_once(kernel, Cfg::kSmemBytes, smem_limit_set);
   if (e != cudaSuccess) return e;
   dim3 grid((l.max_seqlen_q + G * kBlockM - 1) / (G * kBlockM), l.args.heads, l.args.batch);
-  kernel<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(l.tm_q, l.tm_k, l.tm_v, l.args);
+  KernelArgs args = l.args;
+  if constexpr (CAUSAL) {
+    set_causal_grid(&args, grid.x, int64_t(4) * D * l.max_seqlen_k);  // K and V
+    grid = dim3(grid.x * grid.y * grid.z, 1, 1);
+  }
+  kernel<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(l.tm_q, l.tm_k, l.tm_v, args);
   return cudaGetLastError();
 }
 

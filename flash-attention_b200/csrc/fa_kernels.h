@@ -28,7 +28,44 @@ struct KernelArgs {
   DropoutParams drop;
   int32_t* status;
   int32_t launch_id;  // non-zero serial number of this call: what an aborting CTA leaves in status[0]
+  int32_t grid_tiles, grid_heads, grid_first;  // causal grids (see set_causal_grid)
 };
+
+// Block order of the causal grids, whose tiles differ in work by their number of keys (forward) or queries
+// (backward).  The (batch, head) pairs come in sections of equal size whose streamed operands fit the L2 together (the
+// first section takes what the division leaves over); within a section the heaviest tiles of all its pairs come first, so
+// that the last blocks to start are short ones.  With the tiles of one pair after the other, the last pair's heavy tiles
+// ran on while most SMs were done.  Kernel clk, pair by pair -> sections: 2 x 4 x 16384 (d = 64) forward 684 000 ->
+// 576 000, backward 1 356 000 -> 1 323 000; 4 x 32 x 3000 (d = 128) 585 000 -> 575 000 and 1 857 000 -> 1 820 000;
+// 16 x 12 x 1000 backward 471 000 -> 450 000.
+constexpr int64_t kSectionBytes = 32 << 20;
+inline void set_causal_grid(KernelArgs* a, int tiles, int64_t bytes_per_pair) {
+  const int64_t pairs = static_cast<int64_t>(a->heads) * a->batch;
+  const int64_t most = kSectionBytes > bytes_per_pair ? kSectionBytes / bytes_per_pair : 1;
+  const int64_t sections = (pairs + most - 1) / most;
+  a->grid_tiles = tiles;
+  a->grid_heads = static_cast<int32_t>((pairs + sections - 1) / sections);
+  a->grid_first = static_cast<int32_t>(pairs - (sections - 1) * a->grid_heads);
+}
+#ifdef __CUDACC__
+// rank: 0 for the heaviest tile of a pair
+__device__ __forceinline__ void causal_block(const KernelArgs& a, int& rank, int& h, int& b) {
+  const uint32_t tiles = a.grid_tiles, heads = a.heads;
+  uint32_t n = a.grid_first, pair = 0, rest = blockIdx.x;
+  if (rest >= n * tiles) {
+    pair = n;
+    rest -= n * tiles;
+    n = a.grid_heads;
+    const uint32_t section = rest / (n * tiles);
+    pair += section * n;
+    rest -= section * n * tiles;
+  }
+  rank = rest / n;
+  pair += rest - rank * n;
+  b = pair / heads;
+  h = pair - b * heads;
+}
+#endif
 
 struct BwdArgs {
   KernelArgs k;
