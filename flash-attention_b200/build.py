@@ -43,7 +43,6 @@ def _digest(paths):
             h.update(p.encode())
             h.update(f.read())
     h.update(" ".join(NVCC_FLAGS).encode())
-    h.update(os.environ.get("FA_PROFILE", "").encode())
     h.update(os.environ.get("FA_DEFS", "").encode())
     return h.hexdigest()
 
@@ -61,8 +60,7 @@ def build(force=False, verbose=False):
         return LIB_PATH
 
     nvcc = _nvcc()
-    extra = ["-DFA_PROFILE"] if os.environ.get("FA_PROFILE") else []
-    extra += os.environ.get("FA_DEFS", "").split()  # extra -D switches of kernel variants
+    extra = os.environ.get("FA_DEFS", "").split()  # extra -D switches of kernel variants
 
     def compile_one(src):
         obj = os.path.join(OBJ_DIR, os.path.basename(src).replace(".cu", ".o"))

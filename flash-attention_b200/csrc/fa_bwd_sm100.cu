@@ -17,14 +17,16 @@
 // (:333), dropped entries contribute -P*D (:402-418), dQ and dK scaled by scale/p_keep (:583,
 // :628), dV by 1/p_keep (:613-619), P~ and dS rounded to the 16-bit type before their products.
 //
-// Warp roles in bwd_main (512 threads):
-//   warps 0-3   compute group 0: key columns 0-63 of the tile, S, dP -> P~, dS (one thread per
-//               query row; at d = 64 with dropout the 16x256b quad layout, in which one Philox call
-//               is private to a thread, and stmatrix stores); dV epilogue
-//   warps 4-7   compute group 1: key columns 64-127; dK epilogue
-//   warps 8-11  dQ group: tensor memory -> global reductions
-//   warp 12     TMA producer     warp 13  MMA issuer (S, dP, dQ; everything at d = 128)
-//   warp 14, 15 second and third MMA issuer (dV | dK) at d = 64
+// Warp roles in bwd_main:
+//   compute     eight warps (sixteen at d = 64 with dropout): S, dP -> P~, dS.  Eight: warps 0-3 take key columns 0-63
+//               of the tile, warps 4-7 the others, one thread per query row.  Sixteen: a 16-row block and one half of
+//               the columns each, in the 16x256b quad layout in which one Philox call is private to a thread, with
+//               stmatrix stores; four warps per scheduler cover each other's generator chains and waits.  Main kernel,
+//               us, eight -> sixteen: 8 x 12 x 4096 ragged 1037 -> 944, causal 8 x 12 x 2048 255 -> 245,
+//               8 x 16 x 1000 (d = 32) 110 -> 104, 32 x 12 x 200 50.8 -> 49.9.
+//   then four   dQ group: tensor memory -> global reductions
+//   last four   TMA producer, MMA issuer (S, dP, dQ; everything at d = 128), second and third issuer (dV | dK) at d = 64
+// The compute warps write dV and dK at the end.
 //
 // Schedules.  d = 64: Q and dO travel together through a three-stage ring; S and dP of tile t + 1
 // are issued as soon as the compute groups have read tile t into registers.  d = 128: shared
@@ -46,11 +48,10 @@ namespace {
 
 constexpr int kBM = 128;  // query rows per tile
 constexpr int kBN = 128;  // key rows per tile
-constexpr int kBwdThreads = 512;
 constexpr int kMaxSparseTiles = 1024;  // query tiles of 128 per sequence in block-sparse mode
 
 // BS: block-sparse variant (its tile list takes shared memory that the third Q / dO stage would need)
-template <int D, bool BS = false>
+template <int D, bool BS = false, bool DROPOUT = false>
 struct BwdCfg {
   // d = 128 runs a different schedule: shared memory holds a single stage of Q and of dO, each
   // with its own barriers, and the compute groups work in two phases (P~ from S, then dS from dP)
@@ -61,6 +62,17 @@ struct BwdCfg {
   // tile start late and the compute groups wait; the third stage lets the load run a whole tile
   // ahead.
   static constexpr int kQStages = (D == 64) ? (BS ? 2 : 3) : 1;
+  // Compute warps.  d = 64 with dropout: sixteen of one 16-row block and one half of the keys each (quad layout), four
+  // per scheduler, which cover each other's waits and generator chains; else eight, a thread per row and half.
+  static constexpr bool kQuad = DROPOUT && !kTwoPhase;
+  static constexpr int kComputeWarps = kQuad ? 16 : 8;
+  static constexpr int kThreads = 32 * kComputeWarps + 256;  // + the dQ group, + producer and issuers
+  // register split (per thread) of the 128 (80 with sixteen compute warps) a thread is launched with
+  static constexpr int kComputeRegs = kQuad ? 96 : kTwoPhase ? 176 : 192;
+  static constexpr int kDqRegs = kQuad ? 56 : kTwoPhase ? 88 : 72;
+  static constexpr int kOtherRegs = kQuad ? 40 : kTwoPhase ? 72 : 56;
+  // arrivals of the compute warps at a barrier: every thread, or one lane per warp
+  static constexpr uint32_t kComputeArrivals = kQuad ? 16 : 256;
   static constexpr bool kAliasDq = kTwoPhase;     // dQ shares tensor-memory columns with dP
   static constexpr bool kDualIssue = !kTwoPhase;  // second MMA-issuing warp for dV, dK
   static constexpr int kTileBytes = 128 * D * 2;
@@ -105,23 +117,6 @@ __device__ __forceinline__ uint32_t pack16(float lo, float hi) {
   }
 }
 
-// Optional cycle accounting (build with -DFA_PROFILE): one thread of each role of CTA (0,0,0)
-// accumulates the cycles it spends per phase into status[8..].
-#ifdef FA_PROFILE
-#define FA_PROF_DECL long long prof_t = clock64(); long long prof_acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-// time stamps (low 32 bits of the SM clock) of one tile's events, for a timeline across the roles
-#define FA_STAMP(tile, idx) if ((tile) >= 5 && (tile) <= 7 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && ka.status) { \
-    ka.status[64 + ((tile) - 5) * 20 + (idx)] = static_cast<int32_t>(clock64()); }
-#define FA_PROF(slot) { const long long now_ = clock64(); prof_acc[slot] += now_ - prof_t; prof_t = now_; }
-#define FA_PROF_FLUSH(base, n) if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && ka.status) { \
-    for (int i_ = 0; i_ < 8; ++i_) ka.status[(base) + i_] = static_cast<int32_t>(prof_acc[i_] / ((n) > 0 ? (n) : 1)); }
-#else
-#define FA_PROF_DECL
-#define FA_STAMP(tile, idx)
-#define FA_PROF(slot)
-#define FA_PROF_FLUSH(base, n)
-#endif
-
 template <int N>
 __device__ __forceinline__ void reg_alloc() {
   asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
@@ -133,11 +128,12 @@ __device__ __forceinline__ void reg_dealloc() {
 
 // ------------------------------------------------------------------------------------------------
 template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BLOCKSPARSE>
-__global__ void __launch_bounds__(kBwdThreads, 1)
+__global__ void __launch_bounds__(BwdCfg<D, BLOCKSPARSE, DROPOUT>::kThreads, 1)
 fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
               const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
               const __grid_constant__ CUtensorMap tm_dq, const BwdArgs a) {
-  using Cfg = BwdCfg<D, BLOCKSPARSE>;
+  using Cfg = BwdCfg<D, BLOCKSPARSE, DROPOUT>;
+  constexpr int kDqWarp = Cfg::kComputeWarps, kProducer = kDqWarp + 4;  // first warp of the dQ group, of the last four
   constexpr bool kDsInTmem = Cfg::kDsInTmemCapable && !DROPOUT;
   extern __shared__ uint8_t smem_raw[];
   __shared__ BwdShared sh;
@@ -178,7 +174,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     const int rb_end = min(ka.bs_rows16, (sq + 15) >> 4);
     const int mt = min(m_tiles, kMaxSparseTiles);
     uint16_t* order_all = reinterpret_cast<uint16_t*>(smem_raw + kMaxSparseTiles);
-    for (int m = threadIdx.x; m < mt; m += kBwdThreads) {
+    for (int m = threadIdx.x; m < mt; m += Cfg::kThreads) {
       bool any = false;
       for (int rb = m * (kBM / 16); rb < min((m + 1) * (kBM / 16), rb_end); ++rb) any = any || (brow[rb] >= 0);
       if (CAUSAL && m < m_begin) any = false;  // query tiles entirely before this key tile see none of it
@@ -225,7 +221,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 
   if (nm <= 0) {
     // no query row sees these keys: their gradients are zero
-    for (int idx = tid; idx < kBN * (ka.head_dim / 8); idx += kBwdThreads) {
+    for (int idx = tid; idx < kBN * (ka.head_dim / 8); idx += Cfg::kThreads) {
       const int r = idx / (ka.head_dim / 8), c = (idx % (ka.head_dim / 8)) * 8;
       if (n0 + r < sk) {
         const int64_t row = k_start + n0 + r;
@@ -260,18 +256,18 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     mbar_init(smem_u32(&sh.do_full), 1);
     mbar_init(smem_u32(&sh.do_empty), 1);
     mbar_init(smem_u32(&sh.sdp_full), 1);
-    mbar_init(smem_u32(&sh.sdp_consumed), 2 * kBM);
-    mbar_init(smem_u32(&sh.pds_ready), 2 * kBM);
+    mbar_init(smem_u32(&sh.sdp_consumed), Cfg::kComputeArrivals);
+    mbar_init(smem_u32(&sh.pds_ready), Cfg::kComputeArrivals);
     mbar_init(smem_u32(&sh.pds_free), Cfg::kDualIssue ? 3 : 1);  // d = 64: dQ, dV and dK each commit
     mbar_init(smem_u32(&sh.dq_full), 1);
     mbar_init(smem_u32(&sh.dq_consumed), kBM);
     mbar_init(smem_u32(&sh.dq_group), kBM);
     mbar_init(smem_u32(&sh.s_full), 1);
-    mbar_init(smem_u32(&sh.p_ready), 2 * kBM);
+    mbar_init(smem_u32(&sh.p_ready), Cfg::kComputeArrivals);
     mbar_init(smem_u32(&sh.ds_free), 1);
     fence_mbar_init();
   }
-  if (warp == 12) tmem_alloc(smem_u32(&sh.tmem_base), 512);
+  if (warp == kProducer) tmem_alloc(smem_u32(&sh.tmem_base), 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -320,10 +316,9 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       mma_ts(dst, a_tmem + ks * 8, desc_at(db, ks * 2048), idesc_dq, ks > 0);
   };
 
-  if (warp >= 12) {
-    // register split (per thread): d = 64: 192 compute / 72 dQ / 56 here; d = 128: 176 / 88 / 72
-    if constexpr (D == 64) reg_dealloc<56>(); else reg_dealloc<72>();
-    if (warp == 12 && lane == 0) {
+  if (warp >= kProducer) {
+    reg_dealloc<Cfg::kOtherRegs>();
+    if (warp == kProducer && lane == 0) {
       // -------------------------------------------------------------- TMA producer
       tma_prefetch_desc(&tm_q);
       tma_prefetch_desc(&tm_k);
@@ -344,7 +339,6 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         if (!Cfg::kTwoPhase && t >= Cfg::kQStages)
           ok = mbar_wait(smem_u32(&sh.q_empty[s]), ((t / Cfg::kQStages) & 1) ^ 1, abort_flag);
         if (!ok) break;
-        if (!Cfg::kTwoPhase) { FA_STAMP(t - 1, 16) }
         const int row = q_start + q_tile(t) * kBM;
         if constexpr (Cfg::kTwoPhase) {
           // dO(t) follows dV(t - 1), Q(t) follows dK(t - 1): the order in which they finish
@@ -355,7 +349,6 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           for (int p = 0; p < D / 64; ++p) tma_load_3d(smem_do + p * 16384, &tm_do, bar_do, p * 64, row, h);
           if (t >= 1) ok = mbar_wait(smem_u32(&sh.q_empty[0]), (t & 1) ^ 1, abort_flag);
           if (!ok) break;
-          FA_STAMP(t - 1, 16)
           const uint32_t bar = smem_u32(&sh.q_full[0]);
           mbar_expect_tx(bar, Cfg::kTileBytes);
           for (int p = 0; p < D / 64; ++p) tma_load_3d(smem_q + p * 16384, &tm_q, bar, p * 64, row, h);
@@ -368,7 +361,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           }
         }
       }
-    } else if (warp == 13) {
+    } else if (warp == kProducer + 1) {
       // -------------------------------------------------------------- MMA issuer 1
       bool ok = mbar_wait_warp(smem_u32(&sh.kv_full), 0, abort_flag);
       if (ok) ok = mbar_wait_warp(smem_u32(&sh.q_full[0]), 0, abort_flag);
@@ -394,24 +387,18 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             mma_commit(smem_u32(&sh.sdp_full));
           }
         }
-        FA_PROF_DECL
         for (int t = 0; t < nm && ok; ++t) {
           const bool has_next = t + 1 < nm;
-          FA_PROF(0)
           ok = mbar_wait_warp(smem_u32(&sh.p_ready), t & 1, abort_flag);
           if (!ok) break;
-          FA_PROF(1)
           tc_fence_after();
           if (elect_one()) {
             issue_tt(tDV_, smem_p, smem_do, t > 0);
             mma_commit(smem_u32(&sh.pds_free));
             mma_commit(smem_u32(&sh.do_empty));
           }
-          FA_STAMP(t, 11)
           ok = mbar_wait_warp(smem_u32(&sh.pds_ready), t & 1, abort_flag);
           if (!ok) break;
-          FA_PROF(2)
-          FA_STAMP(t, 9)
           tc_fence_after();
           if (elect_one()) {
             issue_tt(tDK_, smem_ds, smem_q, t > 0);
@@ -420,12 +407,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             mma_commit(smem_u32(&sh.dq_full));
             mma_commit(smem_u32(&sh.ds_free));
           }
-          FA_STAMP(t, 10)
-          FA_PROF(3)
           if (has_next) {
-            FA_STAMP(t, 5)
             ok = mbar_wait_warp(smem_u32(&sh.q_full[0]), (t + 1) & 1, abort_flag);
-            FA_STAMP(t, 6)
             if (ok) ok = mbar_wait_warp(smem_u32(&sh.sdp_consumed), t & 1, abort_flag);
             if (!ok) break;
             tc_fence_after();
@@ -433,22 +416,16 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
               issue_kk(tS_, smem_q, smem_k);
               mma_commit(smem_u32(&sh.s_full));
             }
-            FA_STAMP(t, 12)
-            FA_PROF(4)
             ok = mbar_wait_warp(smem_u32(&sh.do_full), (t + 1) & 1, abort_flag);
             if (ok) ok = mbar_wait_warp(smem_u32(&sh.dq_consumed), t & 1, abort_flag);
             if (!ok) break;
-            FA_STAMP(t, 7)
             tc_fence_after();
             if (elect_one()) {
               issue_kk(tDP_, smem_do, smem_v);
               mma_commit(smem_u32(&sh.sdp_full));
             }
-            FA_STAMP(t, 8)
-            FA_PROF(5)
           }
         }
-        FA_PROF_FLUSH(16, nm)
       } else {
         // d = 64: S, dP and dQ (dV, dK go through issuer 2)
         if (ok) {
@@ -459,74 +436,53 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             mma_commit(smem_u32(&sh.sdp_full));
           }
         }
-        FA_PROF_DECL
         for (int t = 0; t < nm && ok; ++t) {
           const bool has_next = t + 1 < nm;
           const int sn = (t + 1) % Cfg::kQStages;
-          FA_PROF(0)
           if (has_next) {
-            FA_STAMP(t, 5)
             ok = mbar_wait_warp(smem_u32(&sh.q_full[sn]), ((t + 1) / Cfg::kQStages) & 1, abort_flag);
-            FA_STAMP(t, 6)
             if (ok) ok = mbar_wait_warp(smem_u32(&sh.sdp_consumed), t & 1, abort_flag);
-            FA_STAMP(t, 7)
             if (!ok) break;
-            FA_PROF(1)
             tc_fence_after();
             if (elect_one()) {
               issue_kk(tS_, smem_q + sn * Cfg::kTileBytes, smem_k);
               issue_kk(tDP_, smem_do + sn * Cfg::kTileBytes, smem_v);
               mma_commit(smem_u32(&sh.sdp_full));
             }
-            FA_PROF(2)
-            FA_STAMP(t, 8)
           }
           ok = mbar_wait_warp(smem_u32(&sh.pds_ready), t & 1, abort_flag);
           if (!ok) break;
-          FA_PROF(3)
-          FA_STAMP(t, 9)
           tc_fence_after();
           if (t > 0) {
             ok = mbar_wait_warp(smem_u32(&sh.dq_consumed), (t - 1) & 1, abort_flag);
             if (!ok) break;
             tc_fence_after();
           }
-          FA_PROF(4)
           // its tile is read out of tensor memory while dV / dK are still running
           if (elect_one()) {
             if constexpr (kDsInTmem) issue_dq_t(tDQ_, tDS_, smem_k);
             else issue_dq(tDQ_, smem_ds, smem_k);
             mma_commit(smem_u32(&sh.dq_full));
-            FA_STAMP(t, 10)
             mma_commit(smem_u32(&sh.pds_free));
           }
-          FA_PROF(5)
         }
-        FA_PROF_FLUSH(16, nm)
       }
-    } else if (warp == 14 && Cfg::kDualIssue) {
+    } else if (warp == kProducer + 2 && Cfg::kDualIssue) {
       // -------------------------------------------------------------- MMA issuer 2: dV
       // dV and dK have a warp each, so that neither waits for the other's instructions to be taken.
       bool ok = true;
-      FA_PROF_DECL
       for (int t = 0; t < nm && ok; ++t) {
         const int s = t % Cfg::kQStages;
-        FA_PROF(0)
         ok = mbar_wait_warp(smem_u32(&sh.pds_ready), t & 1, abort_flag);
         if (!ok) break;
-        FA_PROF(1)
-        FA_STAMP(t, 11)
         tc_fence_after();
         if (elect_one()) {
           issue_tt(tDV_, smem_p, smem_do + s * Cfg::kTileBytes, t > 0);
-          FA_STAMP(t, 12)
           mma_commit(smem_u32(&sh.pds_free));
           mma_commit(smem_u32(&sh.q_empty[s]));
         }
-        FA_PROF(2)
       }
-      FA_PROF_FLUSH(24, nm)
-    } else if (warp == 15 && Cfg::kDualIssue) {
+    } else if (warp == kProducer + 3 && Cfg::kDualIssue) {
       // -------------------------------------------------------------- MMA issuer 3: dK
       bool ok = true;
       for (int t = 0; t < nm && ok; ++t) {
@@ -536,18 +492,17 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         tc_fence_after();
         if (elect_one()) {
           issue_tt(tDK_, smem_ds, smem_q + s * Cfg::kTileBytes, t > 0);
-          FA_STAMP(t, 13)
           mma_commit(smem_u32(&sh.pds_free));
           mma_commit(smem_u32(&sh.q_empty[s]));
         }
       }
     }
-  } else if (warp < 8) {
+  } else if (warp < kDqWarp) {
     // ------------------------------------------------------------------ compute groups
     // group w (0 / 1) owns key columns [64 w, 64 w + 64) of the tile; one thread per query row
-    if constexpr (D == 64) reg_alloc<192>(); else reg_alloc<176>();
+    reg_alloc<Cfg::kComputeRegs>();
     const int cwarp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-    const int w = cwarp >> 2;
+    const int w = (cwarp >> 2) & 1;
     const int row = tid & 127;
     const uint32_t lane_sel = static_cast<uint32_t>((cwarp & 3) * 32) << 16;
     const uint32_t tS = tS_ + lane_sel + w * 64;
@@ -567,130 +522,113 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     }
     const int cbase = n0 + w * 64;  // first key column of this thread
     bool ok = true;
-    FA_PROF_DECL
-    constexpr bool kQuad = DROPOUT && !Cfg::kTwoPhase;
-    if constexpr (kQuad) {
-      // ---- d = 64 with dropout: quad layout.  A warp reads its 32 query rows as two 16-row blocks
-      // (hh) with the 16x256b shape: a thread holds rows r8 and r8 + 8 of a block and two adjacent
-      // columns of every 8-column unit, which is the ownership pattern of the reference's mask
+    if constexpr (Cfg::kQuad) {
+      // ---- d = 64 with dropout: quad layout.  A warp owns a 16-row block (hh) of its 32 lanes and one half of
+      // the keys, and reads both products with the 16x256b shape: a thread holds rows r8 and r8 + 8 and
+      // two adjacent columns of every 8-column unit, which is the ownership pattern of the reference's mask
       // generator (one Philox call = one thread's part of a 16 x 16 patch, QuadPhilox).  The packed
       // pairs go to the swizzled P~ / dS tiles with stmatrix (8 x 8 matrices = 16-byte row chunks).
-      const int wq = cwarp & 3, lane = tid & 31;
+      const int wq = cwarp & 3, hh = cwarp >> 3, lane = tid & 31;
       const int r8 = lane >> 2, q4 = lane & 3;
-      constexpr uint32_t kHalf = 16u << 16;
+      const uint32_t tSq = tS + (static_cast<uint32_t>(hh * 16) << 16), tDPq = tDP + (static_cast<uint32_t>(hh * 16) << 16);
       QuadPhilox<4> qp;
       qp.init(ka.drop, bh_sub, lane, w * 4);
       // stmatrix row address of this lane: matrix k = lane / 8 is (row half k & 1, unit k >> 1)
-      const int st_row = wq * 32 + ((lane >> 3) & 1) * 8 + (lane & 7);   // + 16 * hh
-      const int st_unit = lane >> 4;                                     // + first unit of the quadruple
-      // per-row statistics (ri = hh * 2 + u) of the first tile; those of tile t + 1 are fetched while
-      // tile t is processed
-      float lse_nx[4], d_nx[4];
-      int32_t bs_nx[2] = {0, 0};
+      const int st_row = wq * 32 + hh * 16 + ((lane >> 3) & 1) * 8 + (lane & 7);
+      const uint32_t st_off = w * 16384 + st_row * 128;
+      const int st_unit = (lane >> 4) ^ (st_row & 7);  // unit 0 or 1 of a pair, swizzled (pairs start at even units)
+      auto arrive_warp = [&](uint64_t& bar) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&bar));
+      };
+      // statistics of rows r8 and r8 + 8 of the first tile; those of tile t + 1 are fetched while tile t is processed
+      float lse_nx[2], d_nx[2];
+      int32_t bs_nx = 0;
       auto fetch_stats = [&](int t) {
+        const int i0 = q_tile(t) * kBM + wq * 32 + hh * 16;
 #pragma unroll
-        for (int ri = 0; ri < 4; ++ri) {
-          const int ig_n = q_tile(t) * kBM + wq * 32 + (ri >> 1) * 16 + (ri & 1) * 8 + r8;
+        for (int u = 0; u < 2; ++u) {
+          const int ig_n = i0 + u * 8 + r8;
           const bool valid = ig_n < sq;
-          lse_nx[ri] = valid ? lse_row[ig_n] : INFINITY;
-          d_nx[ri] = valid ? d_row[ig_n] : 0.f;
+          lse_nx[u] = valid ? lse_row[ig_n] : INFINITY;
+          d_nx[u] = valid ? d_row[ig_n] : 0.f;
         }
-        if constexpr (BLOCKSPARSE) {
-#pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {
-            const int i16 = (q_tile(t) * kBM + wq * 32 + hh * 16) >> 4;
-            bs_nx[hh] = i16 < ka.bs_rows16
-                            ? ka.bs_iter[(static_cast<int64_t>(b) * ka.bs_kblocks + (n0 >> 8)) * ka.bs_rows16 + i16]
-                            : -1;
-          }
-        }
+        if constexpr (BLOCKSPARSE)
+          bs_nx = (i0 >> 4) < ka.bs_rows16
+                      ? ka.bs_iter[(static_cast<int64_t>(b) * ka.bs_kblocks + (n0 >> 8)) * ka.bs_rows16 + (i0 >> 4)]
+                      : -1;
       };
       fetch_stats(0);
       for (int t = 0; t < nm && ok; ++t) {
-        FA_PROF(0)
         const int m0 = q_tile(t) * kBM;
-        const int row0 = m0 + wq * 32 + r8;  // + 16 * hh + 8 * u
-        float lse2[4], d_i[4];
+        const int row0 = m0 + wq * 32 + hh * 16 + r8;  // + 8 * u
+        uint64_t nlse2[2], nd2[2];
 #pragma unroll
-        for (int ri = 0; ri < 4; ++ri) { lse2[ri] = lse_nx[ri] * 1.4426950408889634f; d_i[ri] = d_nx[ri]; }
-        const int32_t bs_it[2] = {bs_nx[0], bs_nx[1]};
+        for (int u = 0; u < 2; ++u) {
+          const float l2 = lse_nx[u] * 1.4426950408889634f;
+          nlse2[u] = pack_f2(-l2, -l2);
+          nd2[u] = pack_f2(-d_nx[u], -d_nx[u]);
+        }
+        const int32_t bs_it = bs_nx;
         if (t + 1 < nm) fetch_stats(t + 1);
+        // (a block that is not in the layout is masked too)
+        const bool need_mask = (n0 + kBN > sk) || (CAUSAL && (n0 + kBN - 1 > m0)) || (BLOCKSPARSE && bs_it < 0);
 
-        // (rows whose 16-row block is not in the layout are masked too)
-        const bool need_mask = (n0 + kBN > sk) || (CAUSAL && (n0 + kBN - 1 > m0)) ||
-                               (BLOCKSPARSE && (bs_it[0] < 0 || bs_it[1] < 0));
-        // One 16-row block of the warp after the other: 32 scores, 32 dP values and 16 keep words a thread.
-        // Whether a tile needs masks is decided once per block, outside the unrolled loops.
+        // keep words of the thread's four patches (they do not depend on the scores: drawn before the wait).
+        // kw[grp][2 * u + half]: row u, columns 16 grp + 8 half + 2 q4 (+1 in the high 16 bits)
+        uint32_t kw[4][4];
+        {
+          int64_t it_tile;
+          if constexpr (BLOCKSPARSE) it_tile = bs_it;
+          else it_tile = fa_iter_index(CAUSAL, n0 >> ka.drop.n_shift, (m0 + wq * 32 + hh * 16) >> 4, L16, ka.drop.n_shift);
+          qp.set_tile(ka.drop, it_tile, n0);
 #pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-          // keep words of the block's four calls (they do not depend on the scores).  kw[grp][2 * u + half]:
-          // row u, columns 16 grp + 8 half + 2 q4 (+1 in the high 16 bits)
-          uint32_t kw[4][4];
-          auto draw = [&]() {
-            int64_t it_tile;
-            if constexpr (BLOCKSPARSE) it_tile = bs_it[hh];
-            else it_tile = fa_iter_index(CAUSAL, n0 >> ka.drop.n_shift, (m0 + wq * 32 + hh * 16) >> 4, L16, ka.drop.n_shift);
-            qp.set_tile(ka.drop, it_tile, n0);
+          for (int g4 = 0; g4 < 4; ++g4) qp.start(g4, kw[g4]);
 #pragma unroll
-            for (int g4 = 0; g4 < 4; ++g4) qp.start(g4, kw[g4]);
+          for (int r = 2; r < 7; ++r)
 #pragma unroll
-            for (int r = 2; r < 7; ++r)
+            for (int g4 = 0; g4 < 4; ++g4) QuadPhilox<4>::round(ka.drop, kw[g4], r);
+        }
+        ok = mbar_wait_warp(smem_u32(&sh.sdp_full), t & 1, abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        // 32 columns after the other: 16 scores, 16 dP values a thread
 #pragma unroll
-              for (int g4 = 0; g4 < 4; ++g4) QuadPhilox<4>::round(ka.drop, kw[g4], r);
-          };
-          uint32_t sr[32], dr[32];  // [4 * unit + 2 * u + c]
-          if (hh == 0) {
-            draw();
-            FA_PROF(1)
-            if (w == 0 && row == 0) { FA_STAMP(t, 0) }
-            ok = mbar_wait(smem_u32(&sh.sdp_full), t & 1, abort_flag);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
-            FA_PROF(2)
-            if (w == 0 && row == 0) { FA_STAMP(t, 1) }
-            tc_fence_after();
-          }
-          tmem_ld_quad32(tS + hh * kHalf, sr);
-          tmem_ld_quad32(tDP + hh * kHalf, dr);
-          if (hh == 1) draw();
+        for (int c = 0; c < 2; ++c) {
+          uint32_t sr[16], dr[16];  // [4 * unit + 2 * u + column]
+          tmem_ld_quad16(tSq + c * 32, sr);
+          tmem_ld_quad16(tDPq + c * 32, dr);
           tmem_wait_ld();
-          if (hh == 1) {
+          if (c == 1) {
             tc_fence_before();
-            mbar_arrive(smem_u32(&sh.sdp_consumed));
-            if (w == 0 && row == 0) { FA_STAMP(t, 2) }
+            arrive_warp(sh.sdp_consumed);
           }
-
-          uint32_t pp[16], pds[16];  // [2 * unit + u]: the stmatrix register order
+          uint32_t pp[8], pds[8];  // [2 * unit + u]: the stmatrix register order
           auto block_math = [&](auto masked) {
-            constexpr bool kMasked = decltype(masked)::value;
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              const int ri = hh * 2 + u;
-              const int ig = row0 + hh * 16 + u * 8;
-              const uint64_t nlse2 = pack_f2(-lse2[ri], -lse2[ri]);
-              const uint64_t nd2 = pack_f2(-d_i[ri], -d_i[ri]);
+            for (int unit = 0; unit < 4; ++unit) {
 #pragma unroll
-              for (int unit = 0; unit < 8; ++unit) {
+              for (int u = 0; u < 2; ++u) {
                 const int i = 4 * unit + 2 * u;
                 float p0, p1;
-                unpack_f2(fma2(pack_f2(__uint_as_float(sr[i]), __uint_as_float(sr[i + 1])), c2, nlse2), p0, p1);
+                unpack_f2(fma2(pack_f2(__uint_as_float(sr[i]), __uint_as_float(sr[i + 1])), c2, nlse2[u]), p0, p1);
                 p0 = ex2f(p0);
                 p1 = ex2f(p1);
-                if constexpr (kMasked) {
-                  const int col = cbase + unit * 8 + 2 * q4;
+                if constexpr (decltype(masked)::value) {
+                  const int col = cbase + c * 32 + unit * 8 + 2 * q4, ig = row0 + u * 8;
                   bool v0 = col < sk, v1 = col + 1 < sk;
                   if (CAUSAL) { v0 = v0 && (col <= ig); v1 = v1 && (col + 1 <= ig); }
-                  if (BLOCKSPARSE && bs_it[hh] < 0) { v0 = false; v1 = false; }
+                  if (BLOCKSPARSE && bs_it < 0) { v0 = false; v1 = false; }
                   if (!v0) p0 = 0.f;
                   if (!v1) p1 = 0.f;
                 }
-                const uint32_t word = kw[unit >> 1][2 * u + (unit & 1)];
+                const uint32_t word = kw[2 * c + (unit >> 1)][2 * u + (unit & 1)];
                 const uint64_t p01 = pack_f2(p0, p1);
                 const uint64_t k01 = mul2(p01, pack_f2(fa_keep_factor_lo(word, thr_term), fa_keep_factor_hi(word, thr_term)));
                 float k0, k1, s0, s1;
                 unpack_f2(k01, k0, k1);
                 // dS = P~ * dP - P * D  (P~ = P where kept, 0 where dropped)
-                unpack_f2(fma2(k01, pack_f2(__uint_as_float(dr[i]), __uint_as_float(dr[i + 1])), mul2(p01, nd2)), s0, s1);
+                unpack_f2(fma2(k01, pack_f2(__uint_as_float(dr[i]), __uint_as_float(dr[i + 1])), mul2(p01, nd2[u])), s0, s1);
                 pp[2 * unit + u] = pack_lowp<BF16>(k0, k1);
                 pds[2 * unit + u] = pack_lowp<BF16>(s0, s1);
               }
@@ -698,31 +636,22 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           };
           if (need_mask) block_math(std::true_type{}); else block_math(std::false_type{});
           // the previous tile's products must have finished reading the P~ / dS buffers
-          if (hh == 0) { FA_PROF(3) }
-          if (hh == 0 && t > 0) {
-            ok = mbar_wait(smem_u32(&sh.pds_free), (t - 1) & 1, abort_flag);
-            ok = __all_sync(0xffffffffu, ok);
+          if (c == 0 && t > 0) {
+            ok = mbar_wait_warp(smem_u32(&sh.pds_free), (t - 1) & 1, abort_flag);
             if (!ok) break;
           }
-          if (hh == 0) { FA_PROF(4) }
-          if (hh == 0 && w == 0 && row == 0) { FA_STAMP(t, 3) }
           // four 8 x 8 matrices per instruction: (u = 0, 1) x (units a, a + 1) of the 64-column panel w
-          const int srow = st_row + hh * 16;
 #pragma unroll
-          for (int a2 = 0; a2 < 8; a2 += 2) {
-            const uint32_t off = w * 16384 + srow * 128 + (((a2 + st_unit) ^ (srow & 7)) << 4);
-            stmatrix_x4(smem_u32(p_ptr + off), pp[2 * a2], pp[2 * a2 + 1], pp[2 * a2 + 2], pp[2 * a2 + 3]);
-            stmatrix_x4(smem_u32(ds_ptr + off), pds[2 * a2], pds[2 * a2 + 1], pds[2 * a2 + 2], pds[2 * a2 + 3]);
+          for (int a2 = 0; a2 < 4; a2 += 2) {
+            const uint32_t off = st_off + (((c * 4 + a2) ^ st_unit) << 4);
+            stmatrix_x4(smem_u32(p_ptr) + off, pp[2 * a2], pp[2 * a2 + 1], pp[2 * a2 + 2], pp[2 * a2 + 3]);
+            stmatrix_x4(smem_u32(ds_ptr) + off, pds[2 * a2], pds[2 * a2 + 1], pds[2 * a2 + 2], pds[2 * a2 + 3]);
           }
         }
         if (!ok) break;
-        FA_PROF(5)
         fence_async_smem();
-        mbar_arrive(smem_u32(&sh.pds_ready));
-        FA_PROF(7)
-        if (w == 0 && row == 0) { FA_STAMP(t, 4) }
+        arrive_warp(sh.pds_ready);
       }
-      if (w == 0 && row == 0) { FA_PROF_FLUSH(8, nm) }
     } else {
 
     // per-row statistics of the first tile; those of tile t + 1 are fetched while tile t is processed
@@ -742,7 +671,6 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     fetch_row_stats(0);
 
     for (int t = 0; t < nm && ok; ++t) {
-      FA_PROF(0)
       const int m0 = q_tile(t) * kBM;
       const int ig = m0 + row;
       const float lse2 = lse_next * 1.4426950408889634f;
@@ -782,13 +710,9 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                              (BLOCKSPARSE && __any_sync(0xffffffffu, !row_in_layout));
       if constexpr (Cfg::kTwoPhase) {
         // ---- phase one: P from S.  P~ goes to shared memory (dV can start), P stays in registers.
-        FA_PROF(1)
-        if (w == 0 && row == 0) { FA_STAMP(t, 0) }
         ok = mbar_wait(smem_u32(&sh.s_full), t & 1, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
-        FA_PROF(2)
-        if (w == 0 && row == 0) { FA_STAMP(t, 1) }
         tc_fence_after();
         uint32_t pf[2][32];
         auto phase_one = [&](auto masked) {
@@ -801,7 +725,6 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           if (c == 1) {
             tc_fence_before();
             mbar_arrive(smem_u32(&sh.sdp_consumed));
-            if (w == 0 && row == 0) { FA_STAMP(t, 2) }
           }
           uint32_t pp[16];
 #pragma unroll
@@ -847,15 +770,11 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         if (!ok) break;
         fence_async_smem();
         mbar_arrive(smem_u32(&sh.p_ready));
-        FA_PROF(3)
-        if (w == 0 && row == 0) { FA_STAMP(t, 3) }
 
         // ---- phase two: dS = P~ * dP - P * D from dP
         ok = mbar_wait(smem_u32(&sh.sdp_full), t & 1, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
-        FA_PROF(4)
-        if (w == 0 && row == 0) { FA_STAMP(t, 13) }
         tc_fence_after();
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
@@ -890,13 +809,9 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         }
         tc_fence_before();  // the dP columns are about to be overwritten by dQ
       } else {
-      FA_PROF(1)
-      if (w == 0 && row == 0) { FA_STAMP(t, 0) }
       ok = mbar_wait(smem_u32(&sh.sdp_full), t & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
-      FA_PROF(2)
-      if (w == 0 && row == 0) { FA_STAMP(t, 1) }
       tc_fence_after();
 
       // This thread's 64 scores and 64 dP values go to registers at once, so that the next tile's
@@ -913,7 +828,6 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         tmem_wait_ld();
         tc_fence_before();
         mbar_arrive(smem_u32(&sh.sdp_consumed));
-        if (w == 0 && row == 0) { FA_STAMP(t, 2) }
       }
       auto tile_math = [&](auto masked) {
       constexpr bool kMasked = decltype(masked)::value;
@@ -956,13 +870,10 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           pds[i >> 1] = pack_lowp<BF16>(s0, s1);
         }
         // the previous tile's products must have finished reading the P~ / dS buffers
-        if (c == 0) { FA_PROF(3) }
         if (c == 0 && t > 0) {
           ok = mbar_wait(smem_u32(&sh.pds_free), (t - 1) & 1, abort_flag);
           ok = __all_sync(0xffffffffu, ok);
         }
-        if (c == 0) { FA_PROF(4) }
-        if (c == 0 && w == 0 && row == 0) { FA_STAMP(t, 3) }
         // 32 16-bit values = 4 chunks of 16 bytes of this row in the 64-column panel w
 #pragma unroll
         for (int ch4 = 0; ch4 < 4; ++ch4) {
@@ -980,17 +891,13 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       if (need_mask) tile_math(std::true_type{}); else tile_math(std::false_type{});
       }
       if (!ok) break;
-      FA_PROF(6)
       if constexpr (kDsInTmem) {
         tmem_wait_st();
         tc_fence_before();
       }
       fence_async_smem();
       mbar_arrive(smem_u32(&sh.pds_ready));
-      FA_PROF(7)
-      if (w == 0 && row == 0) { FA_STAMP(t, 4) }
     }
-    if (w == 0 && row == 0) { FA_PROF_FLUSH(8, nm) }
     }  // row-per-thread layout
 
     // ---------------- epilogue: group 0 writes dV = acc / p_keep, group 1 writes dK = acc * scale / p_keep
@@ -1006,7 +913,10 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       // From tid (see `warp`), except where that spills more: d = 128 with dropout and no causal mask, 132
       // against 48 bytes of loads a thread (2 x 12 x 4096: 780 us from tid, 770 so).
       constexpr bool kFromTid = !(D == 128 && DROPOUT && !CAUSAL);
-      const int grp = kFromTid ? tid >> 7 : w;
+      const int grp = kFromTid ? (tid >> 7) & 1 : w;
+      // sixteen warps: warps 8-15 take the second half of the columns
+      const int part = Cfg::kQuad ? tid >> 8 : 0;
+      constexpr int kChunks = Cfg::kQuad ? D / 64 : D / 32;
       const uint32_t tAcc = (grp == 0 ? tDV_ : tDK_) +
                             (kFromTid ? static_cast<uint32_t>(((tid >> 5) & 3) * 32) << 16 : lane_sel);
       const float f = (grp == 0) ? rp_keep : ka.scale * rp_keep;
@@ -1015,15 +925,16 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           ? dv_base + static_cast<int64_t>(k_start + kr) * a.dv_row_stride + static_cast<int64_t>(h) * a.dv_head_stride
           : dk_base + static_cast<int64_t>(k_start + kr) * a.dk_row_stride + static_cast<int64_t>(h) * a.dk_head_stride;
 #pragma unroll
-      for (int c = 0; c < D / 32; ++c) {
+      for (int i = 0; i < kChunks; ++i) {
+        const int c = part * kChunks + i;
         uint32_t r[32];
         tmem_ld32(tAcc + c * 32, r);
         tmem_wait_ld();
         if (kr < sk && c * 32 < ka.head_dim) {
           uint32_t pk[16];
 #pragma unroll
-          for (int i = 0; i < 16; ++i)
-            pk[i] = pack_lowp<BF16>(__uint_as_float(r[2 * i]) * f, __uint_as_float(r[2 * i + 1]) * f);
+          for (int k = 0; k < 16; ++k)
+            pk[k] = pack_lowp<BF16>(__uint_as_float(r[2 * k]) * f, __uint_as_float(r[2 * k + 1]) * f);
           uint4* dst = reinterpret_cast<uint4*>(dst_row + c * 32);
           const int nvec = min(4, (ka.head_dim - c * 32) / 8);
 #pragma unroll
@@ -1037,8 +948,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     // dQ tile: tensor memory -> registers -> swizzled fp32 staging in shared memory -> one TMA
     // reduce-add per [128 rows x 32 columns] box into the fp32 accumulator.  Rows past the end of
     // the sequence hold exact zeros (their P is zero), rows past the tensor are clipped by TMA.
-    if constexpr (D == 64) reg_dealloc<72>(); else reg_dealloc<88>();
-    const int row = tid - 256;
+    reg_dealloc<Cfg::kDqRegs>();
+    const int row = tid - 32 * kDqWarp;
     const uint32_t lane_sel = static_cast<uint32_t>((__shfl_sync(0xffffffffu, tid >> 5, 0) & 3) * 32) << 16;
     const uint32_t tDQ = tDQ_ + lane_sel;
     const uint32_t stage_addr = smem_u32(dq_stage);
@@ -1081,15 +992,11 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       int32_t* tk = ticket_row + q_tile(t);
       asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(tk) : "memory");
     };
-    FA_PROF_DECL
     for (int t = 0; t < nm && ok; ++t) {
       const int m0 = q_tile(t) * kBM;
-      FA_PROF(0)
       ok = mbar_wait(smem_u32(&sh.dq_full), t & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
-      FA_PROF(1)
-      if (row == 0) { FA_STAMP(t, 14) }
       tc_fence_after();
       if constexpr (Cfg::kAliasDq) {
         // dQ shares its columns with the next dP, so the columns are released as early as possible:
@@ -1177,16 +1084,13 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         }
       }
       }
-      FA_PROF(2)
-      if (row == 0) { FA_STAMP(t, 15) }
     }
     if (row == 0 && pending) bulk_wait_all();
-    if (row == 0) { FA_PROF_FLUSH(32, nm) }
   }
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 12) {
+  if (warp == kProducer) {
     tmem_dealloc(tmem, 512);
     if (lane == 0 && sh.abort_flag && ka.status) {
       atomicExch(ka.status, ka.launch_id);  // stops the CTAs of this launch that have not started yet
@@ -1275,7 +1179,8 @@ __global__ void bwd_postprocess_kernel(const BwdArgs a, int dpad) {
 template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BS>
 cudaError_t launch_main(const BwdLaunch& l, cudaStream_t stream) {
   auto kernel = fa_bwd_kernel<D, BF16, CAUSAL, DROPOUT, BS>;
-  constexpr int smem = BwdCfg<D, BS>::kSmemBytes;
+  using Cfg = BwdCfg<D, BS, DROPOUT>;
+  constexpr int smem = Cfg::kSmemBytes;
   static SmemLimitFlags smem_limit_set;  // one per template instantiation of this function
   cudaError_t e = set_smem_limit_once(kernel, smem, smem_limit_set);
   if (e != cudaSuccess) return e;
@@ -1285,7 +1190,7 @@ cudaError_t launch_main(const BwdLaunch& l, cudaStream_t stream) {
     set_causal_grid(&args.k, grid.x, int64_t(8) * D * args.max_seqlen_q);  // Q, dO and the fp32 dQ
     grid = dim3(grid.x * grid.y * grid.z, 1, 1);
   }
-  kernel<<<grid, kBwdThreads, smem, stream>>>(l.tm_q, l.tm_k, l.tm_v, l.tm_do, l.tm_dq, args);
+  kernel<<<grid, Cfg::kThreads, smem, stream>>>(l.tm_q, l.tm_k, l.tm_v, l.tm_do, l.tm_dq, args);
   return cudaGetLastError();
 }
 
