@@ -48,6 +48,7 @@ namespace {
 
 constexpr int kBM = 128;  // query rows per tile
 constexpr int kBN = 128;  // key rows per tile
+constexpr int kSms = 148;
 constexpr int kMaxSparseTiles = 1024;  // query tiles of 128 per sequence in block-sparse mode
 
 // BS: block-sparse variant (its tile list takes shared memory that the third Q / dO stage would need)
@@ -68,9 +69,9 @@ struct BwdCfg {
   static constexpr int kComputeWarps = kQuad ? 16 : 8;
   static constexpr int kThreads = 32 * kComputeWarps + 256;  // + the dQ group, + producer and issuers
   // register split (per thread) of the 128 (80 with sixteen compute warps) a thread is launched with
-  static constexpr int kComputeRegs = kQuad ? 96 : kTwoPhase ? 176 : 192;
-  static constexpr int kDqRegs = kQuad ? 56 : kTwoPhase ? 88 : 72;
-  static constexpr int kOtherRegs = kQuad ? 40 : kTwoPhase ? 72 : 56;
+  static constexpr int kComputeRegs = kQuad ? 96 : kTwoPhase ? 168 : 184;
+  static constexpr int kDqRegs = kQuad ? 64 : kTwoPhase ? 104 : 88;
+  static constexpr int kOtherRegs = kQuad ? 32 : kTwoPhase ? 72 : 56;
   // arrivals of the compute warps at a barrier: every thread, or one lane per warp
   static constexpr uint32_t kComputeArrivals = kQuad ? 16 : 256;
   static constexpr bool kAliasDq = kTwoPhase;     // dQ shares tensor-memory columns with dP
@@ -91,8 +92,18 @@ struct BwdCfg {
   static constexpr uint32_t kTmemDS = 256 + 3 * D;
 };
 
+// What a block works on: key tile n0 / 128 of one (batch, head) pair.  nm: query tiles to walk, -1 behind the last block
+struct BlockInfo {
+  int q_start, sq, k_start, sk, n0, h, b, nm;
+};
+
 struct BwdShared {
-  uint64_t kv_full;
+  uint64_t k_full, v_full, k_empty, v_empty;  // the key tile's operands, once per key tile
+  uint64_t acc_free;                          // dV and dK read out, once per key tile
+  uint64_t next_full;                         // the answer to a request for another block is in `next`
+  uint64_t blk_full[2], blk_done[2];          // the block after is in `blk`; every role has finished the one there
+  alignas(16) uint4 next;
+  alignas(16) BlockInfo blk[2];               // block k in entry k % 2
   uint64_t q_full[3], q_empty[3];
   uint64_t do_full, do_empty;  // dO ring of the two-phase schedule (one stage)
   // d = 64: S and dP together / P~ and dS together.  Two-phase schedule: sdp_full = dP landed,
@@ -148,27 +159,49 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int lane = tid & 31;
   const KernelArgs& ka = a.k;
-  int b = blockIdx.z, h = blockIdx.y, nt = blockIdx.x;  // nt: key tile
-  if constexpr (CAUSAL) causal_block(ka, nt, h, b);
-
-  const int q_start = ka.cu_seqlens_q[b];
-  const int sq = ka.cu_seqlens_q[b + 1] - q_start;
-  const int k_start = ka.cu_seqlens_k[b];
-  const int sk = ka.cu_seqlens_k[b + 1] - k_start;
-  const int n0 = nt * kBN;
-  if (n0 >= sk) return;
+  // One CTA per SM takes over one block of the grid after the other (cluster launch control, in the order of the grid):
+  // the next key tile's operands load and its first products run while dV, dK and the last dQ tiles of the one before
+  // leave, instead of after its CTA's end and the start of another, which cost about two query tiles per
+  // key tile.  Every role walks the same blocks; c counts the key tiles with work, g the query tiles walked so far,
+  // which give the phases of the barriers.  Main kernel, us, a CTA per block -> now: 16 x 8 heads, 200 queries, 1500
+  // keys 72.5 -> 52.5; 64 x 12 x 512 227 -> 170; 16 x 12 x 1000 causal (d = 128) 249 -> 205; 8 x 12 x 512 with dropout
+  // 41.6 -> 36.9; 2 x 4 x 16384 causal 711 -> 689; 4 x 12 x 8192 causal (d = 128) 2199 -> 2131.
+  constexpr bool kTakeOver = !BLOCKSPARSE;
+  auto decode = [&](uint32_t block) -> BlockInfo {
+    BlockInfo x;
+    int nt;
+    if constexpr (CAUSAL) {
+      causal_block(ka, block, nt, x.h, x.b);
+    } else if (kTakeOver && a.take_over) {
+      const uint32_t pair = block / ka.grid_tiles;
+      nt = block - pair * ka.grid_tiles;
+      x.b = pair / ka.heads;
+      x.h = pair - x.b * ka.heads;
+    } else {
+      nt = blockIdx.x; x.h = blockIdx.y; x.b = blockIdx.z;
+    }
+    x.q_start = ka.cu_seqlens_q[x.b];
+    x.sq = ka.cu_seqlens_q[x.b + 1] - x.q_start;
+    x.k_start = ka.cu_seqlens_k[x.b];
+    x.sk = ka.cu_seqlens_k[x.b + 1] - x.k_start;
+    x.n0 = nt * kBN;
+    const int m_tiles = (x.sq + kBM - 1) / kBM;
+    x.nm = x.n0 < x.sk ? m_tiles - (CAUSAL ? min(m_tiles, x.n0 / kBM) : 0) : 0;
+    return x;
+  };
+  BlockInfo first = decode(blockIdx.x);
+  if (!kTakeOver && first.n0 >= first.sk) return;
   // fail fast: once a CTA of this launch has abandoned a wait, the remaining CTAs do not start
   if (ka.status && *reinterpret_cast<volatile int32_t*>(ka.status) == ka.launch_id) return;
 
-  const int m_tiles = (sq + kBM - 1) / kBM;
-  const int m_begin = CAUSAL ? min(m_tiles, n0 / kBM) : 0;
-  int nm = m_tiles - m_begin;
   // block-sparse: query tiles that have at least one 16-row block in this key block's list
   __shared__ uint16_t qtile_list[BLOCKSPARSE ? kMaxSparseTiles : 1];
   // deterministic mode: how many key tiles before this one add into the same query tile
   __shared__ uint16_t qtile_order[BLOCKSPARSE ? kMaxSparseTiles : 1];
   __shared__ int qtile_count;
   if constexpr (BLOCKSPARSE) {
+    const int b = first.b, sq = first.sq, n0 = first.n0, nt = n0 / kBN;
+    const int m_tiles = (sq + kBM - 1) / kBM, m_begin = CAUSAL ? min(m_tiles, n0 / kBM) : 0;
     uint8_t* flags = reinterpret_cast<uint8_t*>(smem_raw);
     const int32_t* brow = ka.bs_iter + (static_cast<int64_t>(b) * ka.bs_kblocks + (n0 >> 8)) * ka.bs_rows16;
     const int rb_end = min(ka.bs_rows16, (sq + 15) >> 4);
@@ -202,7 +235,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       qtile_count = n;
     }
     __syncthreads();
-    nm = qtile_count;
+    first.nm = qtile_count;
     __syncthreads();
   }
   // Deterministic mode: the key tiles of one (batch, head) add into a query tile in ascending
@@ -211,28 +244,28 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   // would idle until tile n - 1 arrives at its first query tile).
   const bool deterministic = a.dq_tickets != nullptr;
   const bool walk_down = CAUSAL && !BLOCKSPARSE && deterministic;
-  auto q_tile = [&](int t) -> int {
+  auto q_tile = [&](const BlockInfo& x, int t) -> int {
     if constexpr (BLOCKSPARSE) return qtile_list[t];
-    else return walk_down ? (m_tiles - 1 - t) : (m_begin + t);
+    const int m_tiles = (x.sq + kBM - 1) / kBM;
+    return walk_down ? m_tiles - 1 - t : m_tiles - x.nm + t;  // causal: from the tile of the first key on
   };
 
   uint16_t* dk_base = reinterpret_cast<uint16_t*>(a.dk);
   uint16_t* dv_base = reinterpret_cast<uint16_t*>(a.dv);
 
-  if (nm <= 0) {
-    // no query row sees these keys: their gradients are zero
-    for (int idx = tid; idx < kBN * (ka.head_dim / 8); idx += Cfg::kThreads) {
+  // no query row sees these keys: their gradients are zero (`threads` threads from thread 0 on)
+  auto zero_tile = [&](const BlockInfo& x, int threads) {
+    for (int idx = tid; idx < kBN * (ka.head_dim / 8); idx += threads) {
       const int r = idx / (ka.head_dim / 8), c = (idx % (ka.head_dim / 8)) * 8;
-      if (n0 + r < sk) {
-        const int64_t row = k_start + n0 + r;
-        *reinterpret_cast<uint4*>(dk_base + row * a.dk_row_stride + h * a.dk_head_stride + c) =
+      if (x.n0 + r < x.sk) {
+        const int64_t row = x.k_start + x.n0 + r;
+        *reinterpret_cast<uint4*>(dk_base + row * a.dk_row_stride + x.h * a.dk_head_stride + c) =
             make_uint4(0, 0, 0, 0);
-        *reinterpret_cast<uint4*>(dv_base + row * a.dv_row_stride + h * a.dv_head_stride + c) =
+        *reinterpret_cast<uint4*>(dv_base + row * a.dv_row_stride + x.h * a.dv_head_stride + c) =
             make_uint4(0, 0, 0, 0);
       }
     }
-    return;
-  }
+  };
 
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -248,7 +281,17 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 
   if (tid == 0) {
     sh.abort_flag = 0;
-    mbar_init(smem_u32(&sh.kv_full), 1);
+    mbar_init(smem_u32(&sh.k_full), 1);
+    mbar_init(smem_u32(&sh.v_full), 1);
+    mbar_init(smem_u32(&sh.k_empty), 1);
+    mbar_init(smem_u32(&sh.v_empty), 1);
+    mbar_init(smem_u32(&sh.acc_free), Cfg::kComputeWarps);
+    mbar_init(smem_u32(&sh.next_full), 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_u32(&sh.blk_full[i]), 1);
+      mbar_init(smem_u32(&sh.blk_done[i]), Cfg::kComputeWarps + 4 + (Cfg::kDualIssue ? 3 : 1));  // all but the producer
+    }
+    sh.blk[0] = first;
     for (int i = 0; i < 3; ++i) {
       mbar_init(smem_u32(&sh.q_full[i]), 1);
       mbar_init(smem_u32(&sh.q_empty[i]), Cfg::kDualIssue ? 2 : 1);  // d = 64: dV (reads dO) and dK (reads Q)
@@ -316,6 +359,17 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       mma_ts(dst, a_tmem + ks * 8, desc_at(db, ks * 2048), idesc_dq, ks > 0);
   };
 
+  // (not in the deterministic mode, whose blocks wait for blocks of smaller index: those start first only as the
+  // hardware launches them; and not where every block has an SM at once)
+  const bool take_over = kTakeOver && a.take_over && !deterministic;
+  // A warp has finished block k: waits for the next one, if any (or until a wait is abandoned).
+  auto next_block = [&](uint32_t k) -> bool {
+    if (!take_over) return false;
+    __syncwarp();
+    if (elect_one()) mbar_arrive(smem_u32(&sh.blk_done[k & 1]));
+    return mbar_wait_warp(smem_u32(&sh.blk_full[(k + 1) & 1]), (k >> 1) & 1, abort_flag) && sh.blk[(k + 1) & 1].nm >= 0;
+  };
+
   if (warp >= kProducer) {
     reg_dealloc<Cfg::kOtherRegs>();
     if (warp == kProducer && lane == 0) {
@@ -325,46 +379,88 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       tma_prefetch_desc(&tm_v);
       tma_prefetch_desc(&tm_do);
       tma_prefetch_desc(&tm_dq);
-      {
-        const uint32_t bar = smem_u32(&sh.kv_full);
-        mbar_expect_tx(bar, 2 * Cfg::kTileBytes);
-        for (int p = 0; p < D / 64; ++p) {
-          tma_load_3d(smem_k + p * 16384, &tm_k, bar, p * 64, k_start + n0, h);
-          tma_load_3d(smem_v + p * 16384, &tm_v, bar, p * 64, k_start + n0, h);
-        }
-      }
       bool ok = true;
-      for (int t = 0; t < nm && ok; ++t) {
-        const int s = t % Cfg::kQStages;
-        if (!Cfg::kTwoPhase && t >= Cfg::kQStages)
-          ok = mbar_wait(smem_u32(&sh.q_empty[s]), ((t / Cfg::kQStages) & 1) ^ 1, abort_flag);
-        if (!ok) break;
-        const int row = q_start + q_tile(t) * kBM;
-        if constexpr (Cfg::kTwoPhase) {
-          // dO(t) follows dV(t - 1), Q(t) follows dK(t - 1): the order in which they finish
-          if (t >= 1) ok = mbar_wait(smem_u32(&sh.do_empty), (t & 1) ^ 1, abort_flag);
-          if (!ok) break;
-          const uint32_t bar_do = smem_u32(&sh.do_full);
-          mbar_expect_tx(bar_do, Cfg::kTileBytes);
-          for (int p = 0; p < D / 64; ++p) tma_load_3d(smem_do + p * 16384, &tm_do, bar_do, p * 64, row, h);
-          if (t >= 1) ok = mbar_wait(smem_u32(&sh.q_empty[0]), (t & 1) ^ 1, abort_flag);
-          if (!ok) break;
-          const uint32_t bar = smem_u32(&sh.q_full[0]);
-          mbar_expect_tx(bar, Cfg::kTileBytes);
-          for (int p = 0; p < D / 64; ++p) tma_load_3d(smem_q + p * 16384, &tm_q, bar, p * 64, row, h);
-        } else {
-          const uint32_t bar = smem_u32(&sh.q_full[s]);
-          mbar_expect_tx(bar, 2 * Cfg::kTileBytes);
-          for (int p = 0; p < D / 64; ++p) {
-            tma_load_3d(smem_q + s * Cfg::kTileBytes + p * 16384, &tm_q, bar, p * 64, row, h);
-            tma_load_3d(smem_do + s * Cfg::kTileBytes + p * 16384, &tm_do, bar, p * 64, row, h);
+      int c = 0, g0 = 0;
+      BlockInfo x = sh.blk[0];
+      for (uint32_t k = 0; ok; ++k) {
+        const int nm = x.nm, h = x.h;
+        // asked for when the last query tile is under way: a block taken earlier would wait here while other SMs run dry
+        auto take_next = [&]() {
+          if (!take_over) return;
+          mbar_expect_tx(smem_u32(&sh.next_full), 16);
+          clc_try_cancel(smem_u32(&sh.next), smem_u32(&sh.next_full));
+        };
+        if (nm <= 0) take_next();
+        for (int t = 0; t < nm && ok; ++t) {
+          const int g = g0 + t;
+          const int s = g % Cfg::kQStages;
+          const int row = x.q_start + q_tile(x, t) * kBM;
+          auto load_k = [&]() {
+            if (c > 0) ok = mbar_wait(smem_u32(&sh.k_empty), (c & 1) ^ 1, abort_flag);
+            if (!ok) return;
+            mbar_expect_tx(smem_u32(&sh.k_full), Cfg::kTileBytes);
+            for (int p = 0; p < D / 64; ++p)
+              tma_load_3d(smem_k + p * 16384, &tm_k, smem_u32(&sh.k_full), p * 64, x.k_start + x.n0, h);
+          };
+          if (t == 0 && c == 0) load_k();
+          if (t == 0) {
+            // V is free after the last dP of the key tile before, K after its last dQ
+            if (c > 0) ok = mbar_wait(smem_u32(&sh.v_empty), (c & 1) ^ 1, abort_flag);
+            if (!ok) break;
+            mbar_expect_tx(smem_u32(&sh.v_full), Cfg::kTileBytes);
+            for (int p = 0; p < D / 64; ++p)
+              tma_load_3d(smem_v + p * 16384, &tm_v, smem_u32(&sh.v_full), p * 64, x.k_start + x.n0, h);
           }
+          if constexpr (Cfg::kTwoPhase) {
+            // dO(g) follows dV(g - 1), Q(g) follows dK(g - 1): the order in which they finish
+            if (g >= 1) ok = mbar_wait(smem_u32(&sh.do_empty), (g & 1) ^ 1, abort_flag);
+            if (!ok) break;
+            const uint32_t bar_do = smem_u32(&sh.do_full);
+            mbar_expect_tx(bar_do, Cfg::kTileBytes);
+            for (int p = 0; p < D / 64; ++p) tma_load_3d(smem_do + p * 16384, &tm_do, bar_do, p * 64, row, h);
+            if (g >= 1) ok = mbar_wait(smem_u32(&sh.q_empty[0]), (g & 1) ^ 1, abort_flag);
+            if (!ok) break;
+            const uint32_t bar = smem_u32(&sh.q_full[0]);
+            mbar_expect_tx(bar, Cfg::kTileBytes);
+            for (int p = 0; p < D / 64; ++p) tma_load_3d(smem_q + p * 16384, &tm_q, bar, p * 64, row, h);
+          } else {
+            if (g >= Cfg::kQStages) ok = mbar_wait(smem_u32(&sh.q_empty[s]), ((g / Cfg::kQStages) & 1) ^ 1, abort_flag);
+            if (!ok) break;
+            const uint32_t bar = smem_u32(&sh.q_full[s]);
+            mbar_expect_tx(bar, 2 * Cfg::kTileBytes);
+            for (int p = 0; p < D / 64; ++p) {
+              tma_load_3d(smem_q + s * Cfg::kTileBytes + p * 16384, &tm_q, bar, p * 64, row, h);
+              tma_load_3d(smem_do + s * Cfg::kTileBytes + p * 16384, &tm_do, bar, p * 64, row, h);
+            }
+          }
+          if (t == 0 && c > 0) load_k();
+          if (ok && t + 1 == nm) take_next();
         }
+        if (!ok || !take_over) break;
+        if (nm > 0) { ++c; g0 += nm; }
+        ok = mbar_wait(smem_u32(&sh.next_full), k & 1, abort_flag);
+        if (!ok) break;
+        uint32_t block;
+        const bool more = clc_answer(smem_u32(&sh.next), block);
+        fence_async_smem();
+        if (more) x = decode(block);
+        else x.nm = -1;
+        // its place is free once every role has finished block k - 1
+        if (k >= 1) ok = mbar_wait(smem_u32(&sh.blk_done[(k + 1) & 1]), ((k - 1) >> 1) & 1, abort_flag);
+        if (!ok) break;
+        sh.blk[(k + 1) & 1] = x;
+        mbar_arrive(smem_u32(&sh.blk_full[(k + 1) & 1]));
+        if (!more) break;
       }
     } else if (warp == kProducer + 1) {
       // -------------------------------------------------------------- MMA issuer 1
-      bool ok = mbar_wait_warp(smem_u32(&sh.kv_full), 0, abort_flag);
-      if (ok) ok = mbar_wait_warp(smem_u32(&sh.q_full[0]), 0, abort_flag);
+      bool ok = true;
+      int c = 0, g0 = 0;
+      uint32_t k = 0;
+      do {
+      const int nm = __shfl_sync(0xffffffffu, sh.blk[k & 1].nm, 0);
+      if (nm <= 0) continue;
+      ok = mbar_wait_warp(smem_u32(&sh.k_full), c & 1, abort_flag);
       if constexpr (Cfg::kTwoPhase) {
         // d = 128: every product, issued by this thread in the order
         //   dV(t) | dK(t), dQ(t) | S(t+1) | dP(t+1)
@@ -372,24 +468,38 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         // refill while phase two is still running.  dK, dQ follow dS; dK releases Q.  S(t+1) is
         // issued when Q has landed, dP(t+1) when dO has landed and the dQ group has read dQ(t)
         // out of the columns it shares with dP.
-        if (ok) {
+        auto scores = [&](int g) {
+          ok = mbar_wait_warp(smem_u32(&sh.q_full[0]), g & 1, abort_flag);
+          if (ok && g > 0) ok = mbar_wait_warp(smem_u32(&sh.sdp_consumed), (g & 1) ^ 1, abort_flag);
+          if (!ok) return;
           tc_fence_after();
           if (elect_one()) {
             issue_kk(tS_, smem_q, smem_k);
             mma_commit(smem_u32(&sh.s_full));
           }
-          ok = mbar_wait_warp(smem_u32(&sh.do_full), 0, abort_flag);
-        }
-        if (ok) {
+        };
+        auto grad_p = [&](int g, bool last) {
+          ok = mbar_wait_warp(smem_u32(&sh.do_full), g & 1, abort_flag);
+          if (ok && g > 0) ok = mbar_wait_warp(smem_u32(&sh.dq_consumed), (g & 1) ^ 1, abort_flag);
+          if (!ok) return;
           tc_fence_after();
           if (elect_one()) {
             issue_kk(tDP_, smem_do, smem_v);
             mma_commit(smem_u32(&sh.sdp_full));
+            if (last) mma_commit(smem_u32(&sh.v_empty));
           }
-        }
+        };
+        if (ok) scores(g0);
+        if (ok) ok = mbar_wait_warp(smem_u32(&sh.v_full), c & 1, abort_flag);
+        if (ok) grad_p(g0, nm == 1);
         for (int t = 0; t < nm && ok; ++t) {
+          const int g = g0 + t;
           const bool has_next = t + 1 < nm;
-          ok = mbar_wait_warp(smem_u32(&sh.p_ready), t & 1, abort_flag);
+          if (t == 0 && c > 0) {
+            ok = mbar_wait_warp(smem_u32(&sh.acc_free), (c & 1) ^ 1, abort_flag);
+            if (!ok) break;
+          }
+          ok = mbar_wait_warp(smem_u32(&sh.p_ready), g & 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
           if (elect_one()) {
@@ -397,7 +507,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             mma_commit(smem_u32(&sh.pds_free));
             mma_commit(smem_u32(&sh.do_empty));
           }
-          ok = mbar_wait_warp(smem_u32(&sh.pds_ready), t & 1, abort_flag);
+          ok = mbar_wait_warp(smem_u32(&sh.pds_ready), g & 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
           if (elect_one()) {
@@ -406,96 +516,95 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             issue_dq(tDQ_, smem_ds, smem_k);
             mma_commit(smem_u32(&sh.dq_full));
             mma_commit(smem_u32(&sh.ds_free));
+            if (!has_next) mma_commit(smem_u32(&sh.k_empty));
           }
           if (has_next) {
-            ok = mbar_wait_warp(smem_u32(&sh.q_full[0]), (t + 1) & 1, abort_flag);
-            if (ok) ok = mbar_wait_warp(smem_u32(&sh.sdp_consumed), t & 1, abort_flag);
-            if (!ok) break;
-            tc_fence_after();
-            if (elect_one()) {
-              issue_kk(tS_, smem_q, smem_k);
-              mma_commit(smem_u32(&sh.s_full));
-            }
-            ok = mbar_wait_warp(smem_u32(&sh.do_full), (t + 1) & 1, abort_flag);
-            if (ok) ok = mbar_wait_warp(smem_u32(&sh.dq_consumed), t & 1, abort_flag);
-            if (!ok) break;
-            tc_fence_after();
-            if (elect_one()) {
-              issue_kk(tDP_, smem_do, smem_v);
-              mma_commit(smem_u32(&sh.sdp_full));
-            }
+            scores(g + 1);
+            if (ok) grad_p(g + 1, t + 2 == nm);
           }
         }
       } else {
         // d = 64: S, dP and dQ (dV, dK go through issuer 2)
-        if (ok) {
+        auto scores = [&](int g, bool last) {
+          const int s = g % Cfg::kQStages;
+          ok = mbar_wait_warp(smem_u32(&sh.q_full[s]), (g / Cfg::kQStages) & 1, abort_flag);
+          if (ok && g > 0) ok = mbar_wait_warp(smem_u32(&sh.sdp_consumed), (g & 1) ^ 1, abort_flag);
+          if (!ok) return;
           tc_fence_after();
           if (elect_one()) {
-            issue_kk(tS_, smem_q, smem_k);
-            issue_kk(tDP_, smem_do, smem_v);
+            issue_kk(tS_, smem_q + s * Cfg::kTileBytes, smem_k);
+            issue_kk(tDP_, smem_do + s * Cfg::kTileBytes, smem_v);
             mma_commit(smem_u32(&sh.sdp_full));
+            if (last) mma_commit(smem_u32(&sh.v_empty));
           }
-        }
+        };
+        if (ok) ok = mbar_wait_warp(smem_u32(&sh.v_full), c & 1, abort_flag);
+        if (ok) scores(g0, nm == 1);
         for (int t = 0; t < nm && ok; ++t) {
-          const bool has_next = t + 1 < nm;
-          const int sn = (t + 1) % Cfg::kQStages;
-          if (has_next) {
-            ok = mbar_wait_warp(smem_u32(&sh.q_full[sn]), ((t + 1) / Cfg::kQStages) & 1, abort_flag);
-            if (ok) ok = mbar_wait_warp(smem_u32(&sh.sdp_consumed), t & 1, abort_flag);
-            if (!ok) break;
-            tc_fence_after();
-            if (elect_one()) {
-              issue_kk(tS_, smem_q + sn * Cfg::kTileBytes, smem_k);
-              issue_kk(tDP_, smem_do + sn * Cfg::kTileBytes, smem_v);
-              mma_commit(smem_u32(&sh.sdp_full));
-            }
-          }
-          ok = mbar_wait_warp(smem_u32(&sh.pds_ready), t & 1, abort_flag);
+          const int g = g0 + t;
+          if (t + 1 < nm) scores(g + 1, t + 2 == nm);
+          if (ok) ok = mbar_wait_warp(smem_u32(&sh.pds_ready), g & 1, abort_flag);
+          if (ok && g > 0) ok = mbar_wait_warp(smem_u32(&sh.dq_consumed), (g & 1) ^ 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
-          if (t > 0) {
-            ok = mbar_wait_warp(smem_u32(&sh.dq_consumed), (t - 1) & 1, abort_flag);
-            if (!ok) break;
-            tc_fence_after();
-          }
           // its tile is read out of tensor memory while dV / dK are still running
           if (elect_one()) {
             if constexpr (kDsInTmem) issue_dq_t(tDQ_, tDS_, smem_k);
             else issue_dq(tDQ_, smem_ds, smem_k);
             mma_commit(smem_u32(&sh.dq_full));
             mma_commit(smem_u32(&sh.pds_free));
+            if (t + 1 == nm) mma_commit(smem_u32(&sh.k_empty));
           }
         }
       }
+      ++c;
+      g0 += nm;
+      } while (ok && next_block(k++));
     } else if (warp == kProducer + 2 && Cfg::kDualIssue) {
       // -------------------------------------------------------------- MMA issuer 2: dV
       // dV and dK have a warp each, so that neither waits for the other's instructions to be taken.
       bool ok = true;
-      for (int t = 0; t < nm && ok; ++t) {
-        const int s = t % Cfg::kQStages;
-        ok = mbar_wait_warp(smem_u32(&sh.pds_ready), t & 1, abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-        if (elect_one()) {
-          issue_tt(tDV_, smem_p, smem_do + s * Cfg::kTileBytes, t > 0);
-          mma_commit(smem_u32(&sh.pds_free));
-          mma_commit(smem_u32(&sh.q_empty[s]));
+      int c = 0, g = 0;
+      uint32_t k = 0;
+      do {
+        const int nm = __shfl_sync(0xffffffffu, sh.blk[k & 1].nm, 0);
+        if (nm <= 0) continue;
+        if (c > 0) ok = mbar_wait_warp(smem_u32(&sh.acc_free), (c & 1) ^ 1, abort_flag);
+        for (int t = 0; t < nm && ok; ++t, ++g) {
+          const int s = g % Cfg::kQStages;
+          ok = mbar_wait_warp(smem_u32(&sh.pds_ready), g & 1, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          if (elect_one()) {
+            issue_tt(tDV_, smem_p, smem_do + s * Cfg::kTileBytes, t > 0);
+            mma_commit(smem_u32(&sh.pds_free));
+            mma_commit(smem_u32(&sh.q_empty[s]));
+          }
         }
-      }
+        ++c;
+      } while (ok && next_block(k++));
     } else if (warp == kProducer + 3 && Cfg::kDualIssue) {
       // -------------------------------------------------------------- MMA issuer 3: dK
       bool ok = true;
-      for (int t = 0; t < nm && ok; ++t) {
-        const int s = t % Cfg::kQStages;
-        ok = mbar_wait_warp(smem_u32(&sh.pds_ready), t & 1, abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-        if (elect_one()) {
-          issue_tt(tDK_, smem_ds, smem_q + s * Cfg::kTileBytes, t > 0);
-          mma_commit(smem_u32(&sh.pds_free));
-          mma_commit(smem_u32(&sh.q_empty[s]));
+      int c = 0, g = 0;
+      uint32_t k = 0;
+      do {
+        const int nm = __shfl_sync(0xffffffffu, sh.blk[k & 1].nm, 0);
+        if (nm <= 0) continue;
+        if (c > 0) ok = mbar_wait_warp(smem_u32(&sh.acc_free), (c & 1) ^ 1, abort_flag);
+        for (int t = 0; t < nm && ok; ++t, ++g) {
+          const int s = g % Cfg::kQStages;
+          ok = mbar_wait_warp(smem_u32(&sh.pds_ready), g & 1, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          if (elect_one()) {
+            issue_tt(tDK_, smem_ds, smem_q + s * Cfg::kTileBytes, t > 0);
+            mma_commit(smem_u32(&sh.pds_free));
+            mma_commit(smem_u32(&sh.q_empty[s]));
+          }
         }
-      }
+        ++c;
+      } while (ok && next_block(k++));
     }
   } else if (warp < kDqWarp) {
     // ------------------------------------------------------------------ compute groups
@@ -507,11 +616,22 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     const uint32_t lane_sel = static_cast<uint32_t>((cwarp & 3) * 32) << 16;
     const uint32_t tS = tS_ + lane_sel + w * 64;
     const uint32_t tDP = tDP_ + lane_sel + w * 64;
+    bool ok = true;
+    int g0 = 0;
+    uint32_t k = 0;
+    do {
+    // with eight compute warps read where it is used, to hold few registers across the tiles (with sixteen, which have
+    // them, 8 x 12 x 4096 takes 973 us so and 924 from registers)
+    using Block = std::conditional_t<Cfg::kQuad, const BlockInfo, const BlockInfo&>;
+    Block x = sh.blk[k & 1];
+    const int nm = x.nm;
+    if (nm <= 0) {
+      zero_tile(x, 32 * Cfg::kComputeWarps);
+      continue;
+    }
     const int64_t bh_sub =
-        (static_cast<int64_t>(b) * ka.drop.heads_total + ka.drop.head_offset + h) * 256;
-    const int L16 = (sq + 15) >> 4;
-    const float* lse_row = ka.lse + (static_cast<int64_t>(b) * ka.heads + h) * ka.lse_stride;
-    const float* d_row = a.softmax_d + (static_cast<int64_t>(b) * ka.heads + h) * ka.lse_stride;
+        (static_cast<int64_t>(x.b) * ka.drop.heads_total + ka.drop.head_offset + x.h) * 256;
+    const int64_t stats = (static_cast<int64_t>(x.b) * ka.heads + x.h) * ka.lse_stride;  // row of LSE and D
     const uint64_t c2 = pack_f2(ka.scale_log2, ka.scale_log2);
     // dropout: per-lane generator state (lanes l and l ^ 8 share every Philox call)
     LanePhilox lp;
@@ -520,8 +640,6 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       lp.init(ka.drop, bh_sub, row);
       thr_term = fa_keep_thr_term(ka.drop.threshold);
     }
-    const int cbase = n0 + w * 64;  // first key column of this thread
-    bool ok = true;
     if constexpr (Cfg::kQuad) {
       // ---- d = 64 with dropout: quad layout.  A warp owns a 16-row block (hh) of its 32 lanes and one half of
       // the keys, and reads both products with the 16x256b shape: a thread holds rows r8 and r8 + 8 and
@@ -545,22 +663,25 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       float lse_nx[2], d_nx[2];
       int32_t bs_nx = 0;
       auto fetch_stats = [&](int t) {
-        const int i0 = q_tile(t) * kBM + wq * 32 + hh * 16;
+        const int i0 = q_tile(x, t) * kBM + wq * 32 + hh * 16;
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           const int ig_n = i0 + u * 8 + r8;
-          const bool valid = ig_n < sq;
-          lse_nx[u] = valid ? lse_row[ig_n] : INFINITY;
-          d_nx[u] = valid ? d_row[ig_n] : 0.f;
+          const bool valid = ig_n < x.sq;
+          lse_nx[u] = valid ? ka.lse[stats + ig_n] : INFINITY;
+          d_nx[u] = valid ? a.softmax_d[stats + ig_n] : 0.f;
         }
         if constexpr (BLOCKSPARSE)
           bs_nx = (i0 >> 4) < ka.bs_rows16
-                      ? ka.bs_iter[(static_cast<int64_t>(b) * ka.bs_kblocks + (n0 >> 8)) * ka.bs_rows16 + (i0 >> 4)]
+                      ? ka.bs_iter[(static_cast<int64_t>(x.b) * ka.bs_kblocks + (x.n0 >> 8)) * ka.bs_rows16 + (i0 >> 4)]
                       : -1;
       };
       fetch_stats(0);
       for (int t = 0; t < nm && ok; ++t) {
-        const int m0 = q_tile(t) * kBM;
+        const int g = g0 + t;
+        const int n0 = x.n0, sk = x.sk, L16 = (x.sq + 15) >> 4;
+        const int cbase = n0 + w * 64;  // first key column of this thread
+        const int m0 = q_tile(x, t) * kBM;
         const int row0 = m0 + wq * 32 + hh * 16 + r8;  // + 8 * u
         uint64_t nlse2[2], nd2[2];
 #pragma unroll
@@ -589,7 +710,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 #pragma unroll
             for (int g4 = 0; g4 < 4; ++g4) QuadPhilox<4>::round(ka.drop, kw[g4], r);
         }
-        ok = mbar_wait_warp(smem_u32(&sh.sdp_full), t & 1, abort_flag);
+        ok = mbar_wait_warp(smem_u32(&sh.sdp_full), g & 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
         // 32 columns after the other: 16 scores, 16 dP values a thread
@@ -636,8 +757,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           };
           if (need_mask) block_math(std::true_type{}); else block_math(std::false_type{});
           // the previous tile's products must have finished reading the P~ / dS buffers
-          if (c == 0 && t > 0) {
-            ok = mbar_wait_warp(smem_u32(&sh.pds_free), (t - 1) & 1, abort_flag);
+          if (c == 0 && g > 0) {
+            ok = mbar_wait_warp(smem_u32(&sh.pds_free), (g & 1) ^ 1, abort_flag);
             if (!ok) break;
           }
           // four 8 x 8 matrices per instruction: (u = 0, 1) x (units a, a + 1) of the 64-column panel w
@@ -658,20 +779,23 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     float lse_next = INFINITY, d_next = 0.f;
     int32_t bs_next = 0;
     auto fetch_row_stats = [&](int t) {
-      const int ig_n = q_tile(t) * kBM + row;
-      const bool valid = ig_n < sq;
-      lse_next = valid ? lse_row[ig_n] : INFINITY;  // scaled at its first use, one tile later
-      d_next = valid ? d_row[ig_n] : 0.f;
+      const int ig_n = q_tile(x, t) * kBM + row;
+      const bool valid = ig_n < x.sq;
+      lse_next = valid ? ka.lse[stats + ig_n] : INFINITY;  // scaled at its first use, one tile later
+      d_next = valid ? a.softmax_d[stats + ig_n] : 0.f;
       if constexpr (BLOCKSPARSE) {
         bs_next = (ig_n >> 4) < ka.bs_rows16
-                      ? ka.bs_iter[(static_cast<int64_t>(b) * ka.bs_kblocks + (n0 >> 8)) * ka.bs_rows16 + (ig_n >> 4)]
+                      ? ka.bs_iter[(static_cast<int64_t>(x.b) * ka.bs_kblocks + (x.n0 >> 8)) * ka.bs_rows16 + (ig_n >> 4)]
                       : -1;
       }
     };
     fetch_row_stats(0);
 
     for (int t = 0; t < nm && ok; ++t) {
-      const int m0 = q_tile(t) * kBM;
+      const int g = g0 + t;
+      const int n0 = x.n0, sk = x.sk, L16 = (x.sq + 15) >> 4;
+      const int cbase = n0 + w * 64;  // first key column of this thread
+      const int m0 = q_tile(x, t) * kBM;
       const int ig = m0 + row;
       const float lse2 = lse_next * 1.4426950408889634f;
       const float d_i = d_next;
@@ -710,7 +834,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                              (BLOCKSPARSE && __any_sync(0xffffffffu, !row_in_layout));
       if constexpr (Cfg::kTwoPhase) {
         // ---- phase one: P from S.  P~ goes to shared memory (dV can start), P stays in registers.
-        ok = mbar_wait(smem_u32(&sh.s_full), t & 1, abort_flag);
+        ok = mbar_wait(smem_u32(&sh.s_full), g & 1, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
@@ -752,8 +876,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             pp[i >> 1] = pack_lowp<BF16>(k0, k1);
           }
           // dV of the previous tile must have finished reading the P~ buffer
-          if (c == 0 && t > 0) {
-            ok = mbar_wait(smem_u32(&sh.pds_free), (t - 1) & 1, abort_flag);
+          if (c == 0 && g > 0) {
+            ok = mbar_wait(smem_u32(&sh.pds_free), (g & 1) ^ 1, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
           }
 #pragma unroll
@@ -772,7 +896,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         mbar_arrive(smem_u32(&sh.p_ready));
 
         // ---- phase two: dS = P~ * dP - P * D from dP
-        ok = mbar_wait(smem_u32(&sh.sdp_full), t & 1, abort_flag);
+        ok = mbar_wait(smem_u32(&sh.sdp_full), g & 1, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
@@ -795,8 +919,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             pds[i >> 1] = pack_lowp<BF16>(s0, s1);
           }
           // dK, dQ of the previous tile must have finished reading the dS buffer
-          if (c == 0 && t > 0) {
-            ok = mbar_wait(smem_u32(&sh.ds_free), (t - 1) & 1, abort_flag);
+          if (c == 0 && g > 0) {
+            ok = mbar_wait(smem_u32(&sh.ds_free), (g & 1) ^ 1, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
           }
 #pragma unroll
@@ -809,7 +933,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         }
         tc_fence_before();  // the dP columns are about to be overwritten by dQ
       } else {
-      ok = mbar_wait(smem_u32(&sh.sdp_full), t & 1, abort_flag);
+      ok = mbar_wait(smem_u32(&sh.sdp_full), g & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
@@ -870,8 +994,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           pds[i >> 1] = pack_lowp<BF16>(s0, s1);
         }
         // the previous tile's products must have finished reading the P~ / dS buffers
-        if (c == 0 && t > 0) {
-          ok = mbar_wait(smem_u32(&sh.pds_free), (t - 1) & 1, abort_flag);
+        if (c == 0 && g > 0) {
+          ok = mbar_wait(smem_u32(&sh.pds_free), (g & 1) ^ 1, abort_flag);
           ok = __all_sync(0xffffffffu, ok);
         }
         // 32 16-bit values = 4 chunks of 16 bytes of this row in the 64-column panel w
@@ -902,9 +1026,9 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 
     // ---------------- epilogue: group 0 writes dV = acc / p_keep, group 1 writes dK = acc * scale / p_keep
     if (ok) {
-      ok = mbar_wait(smem_u32(&sh.pds_free), (nm - 1) & 1, abort_flag);
+      ok = mbar_wait(smem_u32(&sh.pds_free), (g0 + nm - 1) & 1, abort_flag);
       if constexpr (Cfg::kTwoPhase) {
-        if (ok) ok = mbar_wait(smem_u32(&sh.ds_free), (nm - 1) & 1, abort_flag);
+        if (ok) ok = mbar_wait(smem_u32(&sh.ds_free), (g0 + nm - 1) & 1, abort_flag);
       }
       ok = __all_sync(0xffffffffu, ok);
     }
@@ -920,17 +1044,18 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       const uint32_t tAcc = (grp == 0 ? tDV_ : tDK_) +
                             (kFromTid ? static_cast<uint32_t>(((tid >> 5) & 3) * 32) << 16 : lane_sel);
       const float f = (grp == 0) ? rp_keep : ka.scale * rp_keep;
-      const int kr = n0 + row;
+      const BlockInfo e = sh.blk[k & 1];
+      const int kr = e.n0 + row;
       uint16_t* dst_row = (grp == 0)
-          ? dv_base + static_cast<int64_t>(k_start + kr) * a.dv_row_stride + static_cast<int64_t>(h) * a.dv_head_stride
-          : dk_base + static_cast<int64_t>(k_start + kr) * a.dk_row_stride + static_cast<int64_t>(h) * a.dk_head_stride;
+          ? dv_base + static_cast<int64_t>(e.k_start + kr) * a.dv_row_stride + static_cast<int64_t>(e.h) * a.dv_head_stride
+          : dk_base + static_cast<int64_t>(e.k_start + kr) * a.dk_row_stride + static_cast<int64_t>(e.h) * a.dk_head_stride;
 #pragma unroll
       for (int i = 0; i < kChunks; ++i) {
         const int c = part * kChunks + i;
         uint32_t r[32];
         tmem_ld32(tAcc + c * 32, r);
         tmem_wait_ld();
-        if (kr < sk && c * 32 < ka.head_dim) {
+        if (kr < e.sk && c * 32 < ka.head_dim) {
           uint32_t pk[16];
 #pragma unroll
           for (int k = 0; k < 16; ++k)
@@ -943,8 +1068,13 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         }
       }
     }
+    tc_fence_before();
+    __syncwarp();
+    if (elect_one()) mbar_arrive(smem_u32(&sh.acc_free));
+    g0 += nm;
+    } while (ok && next_block(k++));
   } else {
-    // ------------------------------------------------------------------ dQ group (warps 8-11)
+    // ------------------------------------------------------------------ dQ group
     // dQ tile: tensor memory -> registers -> swizzled fp32 staging in shared memory -> one TMA
     // reduce-add per [128 rows x 32 columns] box into the fp32 accumulator.  Rows past the end of
     // the sequence hold exact zeros (their P is zero), rows past the tensor are clipped by TMA.
@@ -964,13 +1094,14 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     };
     // Deterministic mode (thread `row == 0` only): wait until the key tiles before this one have
     // added their share of the query tile, add, wait for the adds to complete and pass the turn on.
-    int32_t* ticket_row = deterministic
-        ? a.dq_tickets + (static_cast<int64_t>(b) * ka.heads + h) * a.ticket_stride : nullptr;
-    auto ticket_wait = [&](int t) -> bool {
+    auto ticket = [&](const BlockInfo& x, int t) -> int32_t* {
+      return a.dq_tickets + (static_cast<int64_t>(x.b) * ka.heads + x.h) * a.ticket_stride + q_tile(x, t);
+    };
+    auto ticket_wait = [&](const BlockInfo& x, int t) -> bool {
       int32_t want;
       if constexpr (BLOCKSPARSE) want = qtile_order[t];
-      else want = nt;
-      const volatile int32_t* tk = ticket_row + q_tile(t);
+      else want = x.n0 / kBN;
+      const volatile int32_t* tk = ticket(x, t);
       if (*abort_flag) return false;
       const long long t0 = clock64();
       while (true) {
@@ -985,16 +1116,20 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       return true;
     };
     bool my_turn = true;
-    auto ticket_pass = [&](int t) {
+    auto ticket_pass = [&](const BlockInfo& x, int t) {
       bulk_wait_all();
       asm volatile("fence.proxy.async.global;" ::: "memory");
       __threadfence();
-      int32_t* tk = ticket_row + q_tile(t);
+      int32_t* tk = ticket(x, t);
       asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(tk) : "memory");
     };
-    for (int t = 0; t < nm && ok; ++t) {
-      const int m0 = q_tile(t) * kBM;
-      ok = mbar_wait(smem_u32(&sh.dq_full), t & 1, abort_flag);
+    int g = 0;
+    uint32_t k = 0;
+    do {
+    const BlockInfo& x = sh.blk[k & 1];  // read where it is used: the group has few registers
+    const int nm = x.nm;
+    for (int t = 0; t < nm && ok; ++t, ++g) {
+      ok = mbar_wait(smem_u32(&sh.dq_full), g & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
@@ -1030,13 +1165,13 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           if (row == 0) {
             // on expiry the abort flag is set, this tile's add is skipped and every role leaves
             // at its next wait
-            if (deterministic && half == 0) my_turn = ticket_wait(t);
+            if (deterministic && half == 0) my_turn = ticket_wait(x, t);
             if (my_turn) {
-              tma_reduce_add_3d(&tm_dq, stage_addr, half * 64, q_start + m0, h);
-              tma_reduce_add_3d(&tm_dq, stage_addr + 16384, half * 64 + 32, q_start + m0, h);
+              tma_reduce_add_3d(&tm_dq, stage_addr, half * 64, x.q_start + q_tile(x, t) * kBM, x.h);
+              tma_reduce_add_3d(&tm_dq, stage_addr + 16384, half * 64 + 32, x.q_start + q_tile(x, t) * kBM, x.h);
               bulk_commit();
               pending = true;
-              if (deterministic && half == D / 64 - 1) { ticket_pass(t); pending = false; }
+              if (deterministic && half == D / 64 - 1) { ticket_pass(x, t); pending = false; }
             }
           }
         }
@@ -1073,18 +1208,19 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         if (row == 0) {
-          if (deterministic && half == 0) my_turn = ticket_wait(t);
+          if (deterministic && half == 0) my_turn = ticket_wait(x, t);
           if (my_turn) {
-            tma_reduce_add_3d(&tm_dq, stage_addr, half * 64, q_start + m0, h);
-            tma_reduce_add_3d(&tm_dq, stage_addr + 16384, half * 64 + 32, q_start + m0, h);
+            tma_reduce_add_3d(&tm_dq, stage_addr, half * 64, x.q_start + q_tile(x, t) * kBM, x.h);
+            tma_reduce_add_3d(&tm_dq, stage_addr + 16384, half * 64 + 32, x.q_start + q_tile(x, t) * kBM, x.h);
             bulk_commit();
             pending = true;
-            if (deterministic && half == D / 64 - 1) { ticket_pass(t); pending = false; }
+            if (deterministic && half == D / 64 - 1) { ticket_pass(x, t); pending = false; }
           }
         }
       }
       }
     }
+    } while (ok && next_block(k++));
     if (row == 0 && pending) bulk_wait_all();
   }
 
@@ -1186,10 +1322,10 @@ cudaError_t launch_main(const BwdLaunch& l, cudaStream_t stream) {
   if (e != cudaSuccess) return e;
   dim3 grid((l.args.max_seqlen_k + kBN - 1) / kBN, l.args.k.heads, l.args.k.batch);
   BwdArgs args = l.args;
-  if constexpr (CAUSAL) {
-    set_causal_grid(&args.k, grid.x, int64_t(8) * D * args.max_seqlen_q);  // Q, dO and the fp32 dQ
-    grid = dim3(grid.x * grid.y * grid.z, 1, 1);
-  }
+  args.k.grid_tiles = grid.x;
+  args.take_over = int64_t(grid.x) * grid.y * grid.z > kSms;
+  if constexpr (CAUSAL) set_causal_grid(&args.k, grid.x, int64_t(8) * D * args.max_seqlen_q);  // Q, dO and the fp32 dQ
+  if (CAUSAL || (!BS && args.take_over)) grid = dim3(grid.x * grid.y * grid.z, 1, 1);
   kernel<<<grid, Cfg::kThreads, smem, stream>>>(l.tm_q, l.tm_k, l.tm_v, l.tm_do, l.tm_dq, args);
   return cudaGetLastError();
 }

@@ -160,7 +160,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   int b = blockIdx.z, h = blockIdx.y, mp = blockIdx.x;
   if constexpr (CAUSAL) {
     int rank;
-    causal_block(a, rank, h, b);
+    causal_block(a, blockIdx.x, rank, h, b);
     mp = a.grid_tiles - 1 - rank;
   }
   const int q_start = a.cu_seqlens_q[b];

@@ -48,10 +48,10 @@ inline void set_causal_grid(KernelArgs* a, int tiles, int64_t bytes_per_pair) {
   a->grid_first = static_cast<int32_t>(pairs - (sections - 1) * a->grid_heads);
 }
 #ifdef __CUDACC__
-// rank: 0 for the heaviest tile of a pair
-__device__ __forceinline__ void causal_block(const KernelArgs& a, int& rank, int& h, int& b) {
+// Place of a block of such a grid; rank: 0 for the heaviest tile of a pair
+__device__ __forceinline__ void causal_block(const KernelArgs& a, uint32_t block, int& rank, int& h, int& b) {
   const uint32_t tiles = a.grid_tiles, heads = a.heads;
-  uint32_t n = a.grid_first, pair = 0, rest = blockIdx.x;
+  uint32_t n = a.grid_first, pair = 0, rest = block;
   if (rest >= n * tiles) {
     pair = n;
     rest -= n * tiles;
@@ -80,6 +80,7 @@ struct BwdArgs {
   // Deterministic mode: one ticket per (batch, head, 128-row query tile) = number of key tiles
   // that have added their dQ tile so far; nullptr = add in arrival order.
   int32_t* dq_tickets;
+  bool take_over;  // the grid has more blocks than SMs: a CTA goes on with blocks that have not started
   int32_t ticket_stride;  // tickets per (batch, head): ceil(max_seqlen_q / 128)
   int32_t total_q, total_k, max_seqlen_q, max_seqlen_k;
   float p_keep;

@@ -128,6 +128,37 @@ __device__ __forceinline__ void fence_async_smem() {
 }
 
 // ---------------------------------------------------------------------------------------------
+// taking over the work of blocks that have not started (cluster launch control)
+// ---------------------------------------------------------------------------------------------
+// Asks for a block of the grid that has not been launched; the 16-byte answer arrives at `response` and counts 16
+// transaction bytes on `bar`.  Not to be asked again once an answer was negative.
+__device__ __forceinline__ void clc_try_cancel(uint32_t response, uint32_t bar) {
+  asm volatile(
+      "clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(response),
+      "r"(bar)
+      : "memory");
+}
+// Whether the answer names a block, and its blockIdx.x (one-dimensional grids).
+__device__ __forceinline__ bool clc_answer(uint32_t response, uint32_t& block) {
+  uint32_t ok, x;
+  asm volatile(
+      "{\n\t"
+      ".reg .b128 h;\n\t"
+      ".reg .pred p;\n\t"
+      "ld.shared.b128 h, [%2];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+      "selp.u32 %1, 1, 0, p;\n\t"
+      "mov.u32 %0, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%0, _, _, _}, h;\n\t"
+      "}\n"
+      : "=r"(x), "=r"(ok)
+      : "r"(response)
+      : "memory");
+  block = x;
+  return ok != 0;
+}
+
+// ---------------------------------------------------------------------------------------------
 // tensor memory
 // ---------------------------------------------------------------------------------------------
 // One full warp calls these.

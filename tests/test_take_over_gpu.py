@@ -1,0 +1,67 @@
+"""GPU tests of the backward's grids with more blocks than SMs, whose CTAs go on with blocks that have not started: the same
+tiles in the same order as in grids where every block has a CTA of its own, so dK and dV have the same bits.  dQ is summed in
+arrival order (at most three fp32 terms here), so it may round differently: one unit of the 16-bit type."""
+import math
+
+import pytest
+import torch
+
+from tests import _util as U
+
+pytestmark = pytest.mark.gpu
+
+# tiles without keys, without queries, with one row, at the edges of 128; causal: key tiles that no query sees
+LENS_Q = [128, 0, 1, 300, 129, 64, 384, 127, 256, 17] * 4
+LENS_K = [128, 40, 129, 300, 0, 257, 100, 384, 1, 130] * 4
+
+
+def _assert_dq(dq, ref):
+    eps = 2.0 ** -7 if dq.dtype == torch.bfloat16 else 2.0 ** -10
+    torch.testing.assert_close(dq.float(), ref.float(), rtol=eps, atol=1e-5 * ref.float().abs().max().item())
+
+
+@pytest.mark.parametrize("d,dtype", [(32, torch.float16), (64, torch.bfloat16), (128, torch.bfloat16)])
+@pytest.mark.parametrize("causal", [False, True])
+def test_one_launch_and_one_per_sequence_agree(d, dtype, causal):
+    from flash_attn_b200 import flash_attn_cuda as fc
+    heads, scale = 6, 1.0 / math.sqrt(d)   # 40 x 6 x 3 blocks against 6 x 3
+    q, k, v, dout, cu_q, cu_k = U.make_varlen(LENS_Q, LENS_K, heads, d, dtype, seed=d)
+    out, lse = fc.fwd(q, k, v, cu_q, cu_k, 384, 384, 0.0, scale, False, causal, False, None)
+
+    def run(cq, ck, stats):
+        grads = [torch.full_like(t, float("nan")) for t in (q, k, v)]
+        fc.bwd(dout, q, k, v, out, stats, *grads, cq, ck, 384, 384, 0.0, scale, False, causal, None)
+        fc.check_device_status()
+        return grads
+
+    dq, dk, dv = run(cu_q, cu_k, lse)
+    for b in range(len(LENS_Q)):
+        one = run(cu_q[b:b + 2].contiguous(), cu_k[b:b + 2].contiguous(), lse[b:b + 1].contiguous())
+        rq, rk = slice(int(cu_q[b]), int(cu_q[b + 1])), slice(int(cu_k[b]), int(cu_k[b + 1]))
+        assert torch.equal(dk[rk], one[1][rk]) and torch.equal(dv[rk], one[2][rk])
+        if rq.stop > rq.start:
+            _assert_dq(dq[rq], one[0][rq])
+
+
+@pytest.mark.parametrize("d", [64, 128])
+def test_dropout_agrees_with_the_deterministic_mode(d):
+    """(which launches a CTA for every block)"""
+    from flash_attn_b200 import flash_attn_cuda as fc
+    heads, scale = 6, 1.0 / math.sqrt(d)
+    q, k, v, dout, cu_q, cu_k = U.make_varlen(LENS_Q, LENS_K, heads, d, torch.float16, seed=d)
+    out, lse, *philox = fc.fwd(q, k, v, cu_q, cu_k, 384, 384, 0.2, scale, False, False, False, None, return_philox=True)
+
+    def run():
+        grads = [torch.full_like(t, float("nan")) for t in (q, k, v)]
+        fc.bwd(dout, q, k, v, out, lse, *grads, cu_q, cu_k, 384, 384, 0.2, scale, False, False, None, philox=tuple(philox))
+        fc.check_device_status()
+        return grads
+
+    dq, dk, dv = run()
+    fc.options.deterministic = True
+    try:
+        one = run()
+    finally:
+        fc.options.deterministic = False
+    assert torch.equal(dk, one[1]) and torch.equal(dv, one[2])
+    _assert_dq(dq, one[0])
