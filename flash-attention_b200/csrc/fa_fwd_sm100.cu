@@ -91,17 +91,6 @@ __device__ __forceinline__ void reg_dealloc() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
-template <bool BF16>
-__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-  if constexpr (BF16) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&v);
-  } else {
-    __half2 v = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&v);
-  }
-}
-
 // Epilogue of one query row (thread = row, 32x32b shape), NC 32-column groups from c0 on: O = acc / (sum * p_keep) in the
 // 16-bit type; the thread of the first group also writes LSE = max * scale + ln(sum).  A row without any valid key
 // gets zeros and -inf.
