@@ -382,13 +382,16 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       bool ok = true;
       int c = 0, g0 = 0;
       BlockInfo x = sh.blk[0];
-      for (uint32_t k = 0; ok; ++k) {
+      bool asked = false;  // an answer is on its way into shared memory
+      uint32_t k = 0;
+      for (; ok; ++k) {
         const int nm = x.nm, h = x.h;
         // asked for when the last query tile is under way: a block taken earlier would wait here while other SMs run dry
         auto take_next = [&]() {
           if (!take_over) return;
           mbar_expect_tx(smem_u32(&sh.next_full), 16);
           clc_try_cancel(smem_u32(&sh.next), smem_u32(&sh.next_full));
+          asked = true;
         };
         if (nm <= 0) take_next();
         for (int t = 0; t < nm && ok; ++t) {
@@ -440,6 +443,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         if (nm > 0) { ++c; g0 += nm; }
         ok = mbar_wait(smem_u32(&sh.next_full), k & 1, abort_flag);
         if (!ok) break;
+        asked = false;
         uint32_t block;
         const bool more = clc_answer(smem_u32(&sh.next), block);
         fence_async_smem();
@@ -452,6 +456,9 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         mbar_arrive(smem_u32(&sh.blk_full[(k + 1) & 1]));
         if (!more) break;
       }
+      // after an abandoned wait: the CTA's shared memory may not go before the answer has arrived (bounded too)
+      for (const long long t0 = clock64(); asked && clock64() - t0 < WAIT_LIMIT_CYCLES;)
+        asked = !mbar_try_wait(smem_u32(&sh.next_full), k & 1);
     } else if (warp == kProducer + 1) {
       // -------------------------------------------------------------- MMA issuer 1
       bool ok = true;
