@@ -1057,32 +1057,37 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       const uint32_t tAcc = (grp == 0 ? tDV_ : tDK_) + (static_cast<uint32_t>(((tid >> 5) & 3) * 32) << 16);
       const float f = (grp == 0) ? rp_keep : ka.scale * rp_keep;
       const BlockInfo e = sh.blk[k & 1];
-      const int kr = e.n0 + row;
-      uint16_t* dst_row = (grp == 0)
-          ? dv_base + static_cast<int64_t>(e.k_start + kr) * a.dv_row_stride + static_cast<int64_t>(e.h) * a.dv_head_stride
-          : dk_base + static_cast<int64_t>(e.k_start + kr) * a.dk_row_stride + static_cast<int64_t>(e.h) * a.dk_head_stride;
+      const int r0 = e.n0 + ((tid >> 5) & 3) * 32;  // first key row of the warp
+      const int64_t stride = grp == 0 ? a.dv_row_stride : a.dk_row_stride;
+      uint16_t* dst = (grp == 0 ? dv_base : dk_base) + static_cast<int64_t>(e.k_start + r0) * stride +
+                      static_cast<int64_t>(e.h) * (grp == 0 ? a.dv_head_stride : a.dk_head_stride) + part * (kChunks * 32);
+      // Out through the rows of the P~ and dS tiles that this warp alone writes (see stage_offset): other warps may be in the
+      // next block already.
+      constexpr int CH = Cfg::kQuad ? 4 : 8;
+      const uint32_t piece = grp * 16384 + ((tid >> 5) & 3) * 4096 + part * 2048;
 #pragma unroll
       for (int i = 0; i < kChunks; ++i) {
-        const int c = part * kChunks + i;
         uint32_t r[32];
-        tmem_ld32(tAcc + c * 32, r);
+        tmem_ld32(tAcc + (part * kChunks + i) * 32, r);
         tmem_wait_ld();
-        if (kr < e.sk && c * 32 < ka.head_dim) {
-          uint32_t pk[16];
 #pragma unroll
-          for (int k = 0; k < 16; ++k)
-            pk[k] = pack_lowp<BF16>(__uint_as_float(r[2 * k]) * f, __uint_as_float(r[2 * k + 1]) * f);
-          uint4* dst = reinterpret_cast<uint4*>(dst_row + c * 32);
-          const int nvec = min(4, (ka.head_dim - c * 32) / 8);
+        for (int v = 0; v < 4; ++v) {
+          uint32_t pk[4];
 #pragma unroll
-          for (int v = 0; v < 4; ++v)
-            if (v < nvec) dst[v] = make_uint4(pk[4 * v], pk[4 * v + 1], pk[4 * v + 2], pk[4 * v + 3]);
+          for (int k = 0; k < 4; ++k)
+            pk[k] = pack_lowp<BF16>(__uint_as_float(r[8 * v + 2 * k]) * f, __uint_as_float(r[8 * v + 2 * k + 1]) * f);
+          *reinterpret_cast<uint4*>((i / 2 == 0 ? p_ptr : ds_ptr) + piece + stage_offset<CH>(tid & 31, (i & 1) * 4 + v)) =
+              make_uint4(pk[0], pk[1], pk[2], pk[3]);
         }
       }
+      tc_fence_before();
+      __syncwarp();
+      if (elect_one()) mbar_arrive(smem_u32(&sh.acc_free));
+#pragma unroll
+      for (int p = 0; p < (kChunks + 1) / 2; ++p)
+        stage_copy_out<CH>((p == 0 ? p_ptr : ds_ptr) + piece, dst + p * 64, stride, e.sk - r0,
+                           ka.head_dim / 8 - part * 4 - p * 8, tid & 31);
     }
-    tc_fence_before();
-    __syncwarp();
-    if (elect_one()) mbar_arrive(smem_u32(&sh.acc_free));
     g0 += nm;
     } while (ok && next_block(k++));
   } else {

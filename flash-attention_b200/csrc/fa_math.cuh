@@ -54,4 +54,28 @@ __device__ __forceinline__ uint32_t pack_lowp(float lo, float hi) {
   return r;
 }
 
+// A tile of 32 rows whose threads hold one row each leaves through shared memory: stored straight from the registers, every
+// 16-byte store of a warp touches 32 rows, one L1 tag cycle each.  The rows are put in a warp's own piece of shared memory
+// (32 rows of CH 16-byte chunks, swizzled so that neither side has bank conflicts) and read back CH lanes to a row.  dK and dV
+// of a block of 128 keys: 4096 (d = 128) and 2048 (d = 64) tag cycles -> 512 and 256, which counts where a block has few query
+// tiles.  Whole backward, us, before -> now: 64 x 12 x 512 (d = 64) 305 -> 278, 16 x 12 x 1024 230 -> 218, 8 x 12 x 4096 1185
+// -> 1135, with dropout 1343 -> 1330; 16 x 12 x 1000 causal (d = 128) 287 -> 271.
+template <int CH>
+__device__ __forceinline__ uint32_t stage_offset(int row, int chunk) {
+  static_assert(CH == 4 || CH == 8, "64 or 128 bytes a row");
+  return row * (CH * 16) + ((chunk ^ (CH == 8 ? row & 7 : (row >> 1) & 3)) << 4);
+}
+// Rows below `rows` and chunks below `chunks` of a warp's piece to global memory; `dst`: row 0, chunk 0.
+template <int CH>
+__device__ __forceinline__ void stage_copy_out(const uint8_t* piece, uint16_t* dst, int64_t row_stride, int rows, int chunks,
+                                               int lane) {
+  const int r0 = lane / CH, c = lane % CH;
+#pragma unroll 4
+  for (int i = 0; i < CH; ++i) {
+    const int r = i * (32 / CH) + r0;
+    if (r < rows && c < chunks)
+      *reinterpret_cast<uint4*>(dst + r * row_stride + c * 8) = *reinterpret_cast<const uint4*>(piece + stage_offset<CH>(r, c));
+  }
+}
+
 }  // namespace fa
