@@ -92,43 +92,46 @@ __device__ __forceinline__ void reg_dealloc() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
-// Epilogue of one query row (thread = row, 32x32b shape), NC 32-column groups from c0 on: O = acc / (sum * p_keep) in the
-// 16-bit type; the thread of the first group also writes LSE = max * scale + ln(sum).  A row without any valid key
-// gets zeros and -inf.
+// Epilogue of 32 query rows (a warp, thread = row, 32x32b shape), NC 32-column groups from c0 on: O = acc / (sum * p_keep)
+// in the 16-bit type; the warp of the first group also writes LSE = max * scale + ln(sum).  A row without any valid key
+// gets zeros and -inf.  `piece`: the warp's NC * 2048 bytes of shared memory, for the way out (see stage_offset).
+// ig: first query row of the warp.
 template <bool BF16, int NC>
-__device__ __forceinline__ void store_row(const KernelArgs& a, uint32_t tO, int c0, bool have_acc, bool ok, int ig,
-                                          int sq, int q_start, int b, int h, float m_run, float l_run) {
+__device__ __forceinline__ void store_rows(const KernelArgs& a, uint32_t tO, int c0, bool have_acc, bool ok, int ig, int lane,
+                                           int sq, int q_start, int b, int h, float m_run, float l_run, uint8_t* piece) {
+  constexpr int CH = NC == 1 ? 4 : 8;  // 16-byte chunks of a row in one panel of the piece
   const bool bad_sum = (l_run == 0.f) || (l_run != l_run);
   const float inv = bad_sum ? 1.f : (1.f / l_run) * a.rp_keep;
-  const bool store = ok && (ig < sq);
-  uint16_t* orow = reinterpret_cast<uint16_t*>(a.o) + static_cast<int64_t>(q_start + ig) * a.o_row_stride +
-                   static_cast<int64_t>(h) * a.o_head_stride;
 #pragma unroll
   for (int i = 0; i < NC; ++i) {
-    const int c = c0 + i;
     uint32_t orr[32];
     if (have_acc) {
-      tmem_ld32(tO + c * 32, orr);
+      tmem_ld32(tO + (c0 + i) * 32, orr);
       tmem_wait_ld();
     } else {
 #pragma unroll
       for (int k = 0; k < 32; ++k) orr[k] = 0u;
     }
-    if (store && c * 32 < a.head_dim) {
-      uint32_t pko[16];
+    uint8_t* panel = piece + (i / 2) * 4096;
 #pragma unroll
-      for (int k = 0; k < 16; ++k)
-        pko[k] = pack_lowp<BF16>(__uint_as_float(orr[2 * k]) * inv, __uint_as_float(orr[2 * k + 1]) * inv);
-      uint4* dst = reinterpret_cast<uint4*>(orow + c * 32);
-      const int nvec = min(4, (a.head_dim - c * 32) / 8);
+    for (int v = 0; v < 4; ++v) {
+      uint32_t w[4];
 #pragma unroll
-      for (int v = 0; v < 4; ++v)
-        if (v < nvec) dst[v] = make_uint4(pko[4 * v], pko[4 * v + 1], pko[4 * v + 2], pko[4 * v + 3]);
+      for (int k = 0; k < 4; ++k)
+        w[k] = pack_lowp<BF16>(__uint_as_float(orr[8 * v + 2 * k]) * inv, __uint_as_float(orr[8 * v + 2 * k + 1]) * inv);
+      *reinterpret_cast<uint4*>(panel + stage_offset<CH>(lane, (i & 1) * 4 + v)) = make_uint4(w[0], w[1], w[2], w[3]);
     }
   }
-  if (store && c0 == 0) {
+  __syncwarp();
+  if (!ok) return;
+  uint16_t* orow = reinterpret_cast<uint16_t*>(a.o) + static_cast<int64_t>(q_start + ig) * a.o_row_stride +
+                   static_cast<int64_t>(h) * a.o_head_stride + c0 * 32;
+#pragma unroll
+  for (int p = 0; p < (NC + 1) / 2; ++p)
+    stage_copy_out<CH>(piece + p * 4096, orow + p * 64, a.o_row_stride, sq - ig, a.head_dim / 8 - c0 * 4 - p * 8, lane);
+  if (ig + lane < sq && c0 == 0) {
     const float lse = bad_sum ? -INFINITY : (m_run * a.scale + __logf(l_run));
-    a.lse[(static_cast<int64_t>(b) * a.heads + h) * a.lse_stride + ig] = lse;
+    a.lse[(static_cast<int64_t>(b) * a.heads + h) * a.lse_stride + ig + lane] = lse;
   }
 }
 
@@ -215,8 +218,19 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   const uint32_t smem_q = smem_u32(smem);
   const uint32_t smem_k = smem_q + G * Cfg::kTileBytes;
   const uint32_t smem_v = smem_k + Cfg::kStages * Cfg::kTileBytes;
+  // the 128 rows from `row` on of one operand (one thread)
+  auto load_tile = [&](uint32_t dst, const CUtensorMap* map, uint64_t& bar, int row) {
+    mbar_expect_tx(smem_u32(&bar), Cfg::kTileBytes);
+    for (int p = 0; p < Cfg::kPanels; ++p) tma_load_3d(dst + p * 16384, map, smem_u32(&bar), p * 64, row, h);
+  };
 
-  if (tid == 0) {
+  // The producer sets up the barriers and asks for Q and the first K and V at once, ahead of everything else a CTA does: behind
+  // the tensor memory, the register split and the barrier of the CTA the first load left 3100 clk after the start of a CTA and
+  // the first scores came at 5600 (16 x 12 x 1000 causal, d = 128, 51 000 clk for eight key tiles).  With K waited for where it
+  // is used (issuer) and the rows stored through shared memory (store_rows, 3500 clk before), us, before -> now: 16 x 12 x 1000
+  // causal (d = 128) 97 -> 83; d = 64: 64 x 12 x 512 100 -> 95, 16 x 12 x 1024 87 -> 80, 8 x 12 x 4096 479 -> 465, 2 x 4 x 16384
+  // causal 310 -> 307.
+  if (tid == 32 * Cfg::kSoftmaxWarps) {
     sh.abort_flag = 0;
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&sh.q_full[i]), 1);
@@ -234,8 +248,15 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       mbar_init(smem_u32(&sh.v_empty[i]), 1);
     }
     fence_mbar_init();
+    fence_async_smem();
+    if (n_max > 0) {
+      for (int g = 0; g < G; ++g)
+        if (n_tiles[g] > 0) load_tile(smem_q + g * Cfg::kTileBytes, &tm_q, sh.q_full[g], q_start + m0[g]);
+      load_tile(smem_k, &tm_k, sh.k_full[0], k_start + kv_tile(0) * kBlockN);
+      load_tile(smem_v, &tm_v, sh.v_full[0], k_start + kv_tile(0) * kBlockN);
+    }
   }
-  if (warp == Cfg::kSoftmaxWarps) tmem_alloc(smem_u32(&sh.tmem_base), Cfg::kTmemCols);
+  if (warp == Cfg::kSoftmaxWarps + 1) tmem_alloc(smem_u32(&sh.tmem_base), Cfg::kTmemCols);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -246,43 +267,19 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   if (warp == Cfg::kSoftmaxWarps) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      tma_prefetch_desc(&tm_q);
-      tma_prefetch_desc(&tm_k);
-      tma_prefetch_desc(&tm_v);
-      for (int g = 0; g < G; ++g) {
-        if (n_tiles[g] > 0) {
-          const uint32_t bar = smem_u32(&sh.q_full[g]);
-          mbar_expect_tx(bar, Cfg::kTileBytes);
-          for (int p = 0; p < Cfg::kPanels; ++p)
-            tma_load_3d(smem_q + g * Cfg::kTileBytes + p * 16384, &tm_q, bar, p * 64,
-                        q_start + m0[g], h);
-        }
-      }
       bool ok = true;
-      int loads_k = 0, loads_v = 0;
-      for (int j = 0; j < n_max && ok; ++j) {
+      int loads_k = min(n_max, 1), loads_v = loads_k;  // so far
+      for (int j = 1; j < n_max && ok; ++j) {
         const int s = j % Cfg::kStages;
         const uint32_t ph = ((j / Cfg::kStages) & 1) ^ 1;
         if (j >= Cfg::kStages) ok = mbar_wait(smem_u32(&sh.k_empty[s]), ph, abort_flag);
         if (!ok) break;
-        {
-          const uint32_t bar = smem_u32(&sh.k_full[s]);
-          mbar_expect_tx(bar, Cfg::kTileBytes);
-          for (int p = 0; p < Cfg::kPanels; ++p)
-            tma_load_3d(smem_k + s * Cfg::kTileBytes + p * 16384, &tm_k, bar, p * 64,
-                        k_start + kv_tile(j) * kBlockN, h);
-          loads_k = j + 1;
-        }
+        load_tile(smem_k + s * Cfg::kTileBytes, &tm_k, sh.k_full[s], k_start + kv_tile(j) * kBlockN);
+        loads_k = j + 1;
         if (j >= Cfg::kStages) ok = mbar_wait(smem_u32(&sh.v_empty[s]), ph, abort_flag);
         if (!ok) break;
-        {
-          const uint32_t bar = smem_u32(&sh.v_full[s]);
-          mbar_expect_tx(bar, Cfg::kTileBytes);
-          for (int p = 0; p < Cfg::kPanels; ++p)
-            tma_load_3d(smem_v + s * Cfg::kTileBytes + p * 16384, &tm_v, bar, p * 64,
-                        k_start + kv_tile(j) * kBlockN, h);
-          loads_v = j + 1;
-        }
+        load_tile(smem_v + s * Cfg::kTileBytes, &tm_v, sh.v_full[s], k_start + kv_tile(j) * kBlockN);
+        loads_v = j + 1;
       }
       for (int g = 0; g < G; ++g)
         if (n_tiles[g] > 0) mbar_drain(smem_u32(&sh.q_full[g]), 0);
@@ -341,12 +338,11 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         const int s = j % Cfg::kStages;
         const int sn = (j + 1) % Cfg::kStages;
         const bool has_next = j + 1 < n_max;
-        if (!Cfg::kSeparateP) ok = mbar_wait_warp(smem_u32(&sh.v_full[s]), (j / Cfg::kStages) & 1, abort_flag);
-        if (ok && has_next)
-          ok = mbar_wait_warp(smem_u32(&sh.k_full[sn]), ((j + 1) / Cfg::kStages) & 1, abort_flag);
-        if (!ok) break;
+        auto wait_k = [&]() { ok = mbar_wait_warp(smem_u32(&sh.k_full[sn]), ((j + 1) / Cfg::kStages) & 1, abort_flag); };
         if constexpr (Cfg::kSeparateP) {
           // this warp issues only the score products; the next one issues P*V
+          if (has_next) wait_k();
+          if (!ok) break;
 #pragma unroll
           for (int g = 0; g < G; ++g) {
             if (ok && j + 1 < n_tiles[g]) {
@@ -359,6 +355,10 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           }
           if (!ok) break;
         } else {
+          ok = mbar_wait_warp(smem_u32(&sh.v_full[s]), (j / Cfg::kStages) & 1, abort_flag);
+          // K of the next tile is waited for behind P V of this one, which does not need it (its load takes about 2000 clk where
+          // two CTAs with a stage each share an SM)
+          bool k_here = false;
 #pragma unroll
           for (int g = 0; g < G; ++g) {
             if (ok && j < n_tiles[g]) {
@@ -374,7 +374,11 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
               if (ok) {
                 tc_fence_after();
                 issue_pv(g, s, j > 0, kFirst, kBlockN / 16);
-                if (j + 1 < n_tiles[g]) issue_qk(g, sn);
+                if (j + 1 < n_tiles[g]) {
+                  if (!k_here) wait_k();
+                  k_here = true;
+                  if (ok) issue_qk(g, sn);
+                }
               }
             }
           }
@@ -570,7 +574,9 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
       }
-      store_row<BF16, D / 32>(a, tO, 0, n > 0 && ok, ok, ig, sq, q_start, b, h, m_run, l_run);
+      // every product that reads this group's Q has finished: its tile takes the output
+      store_rows<BF16, D / 32>(a, tO, 0, n > 0 && ok, ok, m0[g] + (warp & 3) * 32, lane, sq, q_start, b, h, m_run, l_run,
+                               smem + g * Cfg::kTileBytes + (warp & 3) * (D * 64));
     }
   } else if (warp < Cfg::kSoftmaxWarps) {
     // ------------------------------------------------------------------ softmax warps
@@ -787,13 +793,15 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         tc_fence_after();
       }
       const float2 st = sh.row_stats[g][wq * 32 + lane];
-      store_row<BF16, D / 64>(a, tO - (static_cast<uint32_t>(hh * 16) << 16), hh * (D / 64), n > 0 && ok, ok, m_first + wq * 32 + lane, sq, q_start, b, h, st.x, st.y);
+      store_rows<BF16, D / 64>(a, tO - (static_cast<uint32_t>(hh * 16) << 16), hh * (D / 64), n > 0 && ok, ok,
+                               m_first + wq * 32, lane, sq, q_start, b, h, st.x, st.y,
+                               smem + g * Cfg::kTileBytes + (wq * 2 + hh) * (D * 32));
     }
   }
 
   tc_fence_before();
   __syncthreads();
-  if (warp == Cfg::kSoftmaxWarps) {
+  if (warp == Cfg::kSoftmaxWarps + 1) {
     tmem_dealloc(tmem, Cfg::kTmemCols);
     if (lane == 0 && sh.abort_flag && a.status) {
       atomicExch(a.status, a.launch_id);  // stops the CTAs of this launch that have not started yet
