@@ -191,6 +191,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     x.nm = x.n0 < x.sk ? m_tiles - (CAUSAL ? min(m_tiles, x.n0 / kBM) : 0) : 0;
     return x;
   };
+  const int32_t failed = ka.status ? *reinterpret_cast<volatile int32_t*>(ka.status) : 0;  // on its way beside the lengths
   BlockInfo first = decode(blockIdx.x);
   // (not in the deterministic mode, whose blocks wait for blocks of smaller index: those start first only as the
   // hardware launches them; and not where every block has an SM at once)
@@ -204,7 +205,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   auto launch_failed = [&]() -> bool {
     return ka.status && *reinterpret_cast<volatile int32_t*>(ka.status) == ka.launch_id;
   };
-  if (launch_failed()) return;
+  if (failed == ka.launch_id) return;
 
   // block-sparse: query tiles that have at least one 16-row block in this key block's list
   __shared__ uint16_t qtile_list[BLOCKSPARSE ? kMaxSparseTiles : 1];

@@ -151,19 +151,40 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // known to be the same in all lanes
   const int lane = tid & 31;
 
+  // Fail fast: once a CTA of this launch has abandoned a wait, the remaining CTAs do not start.  (Read beside cu_seqlens and
+  // looked at behind them: one after the other they were 600 clk each of a CTA's 14 000, 64 x 12 x 512, d = 64.)
+  const int32_t failed = a.status ? *reinterpret_cast<volatile int32_t*>(a.status) : 0;
   int b = blockIdx.z, h = blockIdx.y, mp = CAUSAL ? gridDim.x - 1 - blockIdx.x : blockIdx.x;  // heavy tiles first
   if constexpr (ORDERED) tail_block(a, blockIdx.x, mp, h, b);
   const int q_start = a.cu_seqlens_q[b];
   const int sq = a.cu_seqlens_q[b + 1] - q_start;
   const int k_start = a.cu_seqlens_k[b];
   const int sk = a.cu_seqlens_k[b + 1] - k_start;
+  if (tid == 32 * Cfg::kSoftmaxWarps) {  // while the lengths are on their way
+    sh.abort_flag = 0;
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_u32(&sh.q_full[i]), 1);
+      mbar_init(smem_u32(&sh.s_full[i]), 1);
+      mbar_init(smem_u32(&sh.s_free[i]), Cfg::kArrivals);
+      mbar_init(smem_u32(&sh.p_half[i]), Cfg::kArrivals);
+      mbar_init(smem_u32(&sh.p_full[i]), Cfg::kArrivals);
+      mbar_init(smem_u32(&sh.o_full[i]), 1);
+      mbar_init(smem_u32(&sh.drained[i]), 1);
+    }
+    for (int i = 0; i < 3; ++i) {
+      mbar_init(smem_u32(&sh.k_full[i]), 1);
+      mbar_init(smem_u32(&sh.k_empty[i]), 1);
+      mbar_init(smem_u32(&sh.v_full[i]), 1);
+      mbar_init(smem_u32(&sh.v_empty[i]), 1);
+    }
+    fence_mbar_init();
+    fence_async_smem();
+  }
   if constexpr (ORDERED) {
     mp = (sq + G * kBlockM - 1) / (G * kBlockM) - 1 - mp;  // of the sequence's own tiles; empty blocks last
     if (mp < 0) return;
   }
-  if (mp * G * kBlockM >= sq) return;
-  // fail fast: once a CTA of this launch has abandoned a wait, the remaining CTAs do not start
-  if (a.status && *reinterpret_cast<volatile int32_t*>(a.status) == a.launch_id) return;
+  if (mp * G * kBlockM >= sq || failed == a.launch_id) return;
 
   int n_kv_total = (sk + kBlockN - 1) / kBlockN;
   if constexpr (BLOCKSPARSE) {
@@ -224,37 +245,17 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     for (int p = 0; p < Cfg::kPanels; ++p) tma_load_3d(dst + p * 16384, map, smem_u32(&bar), p * 64, row, h);
   };
 
-  // The producer sets up the barriers and asks for Q and the first K and V at once, ahead of everything else a CTA does: behind
+  // The producer asks for Q and the first K and V at once, ahead of everything else a CTA does: behind
   // the tensor memory, the register split and the barrier of the CTA the first load left 3100 clk after the start of a CTA and
   // the first scores came at 5600 (16 x 12 x 1000 causal, d = 128, 51 000 clk for eight key tiles).  With K waited for where it
   // is used (issuer) and the rows stored through shared memory (store_rows, 3500 clk before), us, before -> now: 16 x 12 x 1000
   // causal (d = 128) 97 -> 83; d = 64: 64 x 12 x 512 100 -> 95, 16 x 12 x 1024 87 -> 80, 8 x 12 x 4096 479 -> 465, 2 x 4 x 16384
   // causal 310 -> 307.
-  if (tid == 32 * Cfg::kSoftmaxWarps) {
-    sh.abort_flag = 0;
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(smem_u32(&sh.q_full[i]), 1);
-      mbar_init(smem_u32(&sh.s_full[i]), 1);
-      mbar_init(smem_u32(&sh.s_free[i]), Cfg::kArrivals);
-      mbar_init(smem_u32(&sh.p_half[i]), Cfg::kArrivals);
-      mbar_init(smem_u32(&sh.p_full[i]), Cfg::kArrivals);
-      mbar_init(smem_u32(&sh.o_full[i]), 1);
-      mbar_init(smem_u32(&sh.drained[i]), 1);
-    }
-    for (int i = 0; i < 3; ++i) {
-      mbar_init(smem_u32(&sh.k_full[i]), 1);
-      mbar_init(smem_u32(&sh.k_empty[i]), 1);
-      mbar_init(smem_u32(&sh.v_full[i]), 1);
-      mbar_init(smem_u32(&sh.v_empty[i]), 1);
-    }
-    fence_mbar_init();
-    fence_async_smem();
-    if (n_max > 0) {
-      for (int g = 0; g < G; ++g)
-        if (n_tiles[g] > 0) load_tile(smem_q + g * Cfg::kTileBytes, &tm_q, sh.q_full[g], q_start + m0[g]);
-      load_tile(smem_k, &tm_k, sh.k_full[0], k_start + kv_tile(0) * kBlockN);
-      load_tile(smem_v, &tm_v, sh.v_full[0], k_start + kv_tile(0) * kBlockN);
-    }
+  if (tid == 32 * Cfg::kSoftmaxWarps && n_max > 0) {
+    for (int g = 0; g < G; ++g)
+      if (n_tiles[g] > 0) load_tile(smem_q + g * Cfg::kTileBytes, &tm_q, sh.q_full[g], q_start + m0[g]);
+    load_tile(smem_k, &tm_k, sh.k_full[0], k_start + kv_tile(0) * kBlockN);
+    load_tile(smem_v, &tm_v, sh.v_full[0], k_start + kv_tile(0) * kBlockN);
   }
   if (warp == Cfg::kSoftmaxWarps + 1) tmem_alloc(smem_u32(&sh.tmem_base), Cfg::kTmemCols);
   tc_fence_before();
