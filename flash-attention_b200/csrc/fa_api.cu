@@ -257,6 +257,14 @@ int fa_mask_index(const uint8_t* mask, int32_t batch, int32_t seqlen, int32_t* c
   return FA_OK;
 }
 
+int fa_mask_bounds(const uint8_t* mask, int32_t batch, int32_t seqlen, int32_t* bounds, int32_t* summary, void* cuda_stream) {
+  FA_REQUIRE(batch > 0 && seqlen > 0, "sizes must be positive");
+  FA_REQUIRE(static_cast<int64_t>(batch) * seqlen <= 0x7fffffffLL, "mask too large");
+  FA_REQUIRE(mask && bounds && summary, "null pointer");
+  FA_CUDA(fa::launch_mask_bounds(mask, batch, seqlen, bounds, summary, static_cast<cudaStream_t>(cuda_stream)));
+  return FA_OK;
+}
+
 int fa_rotary_qkv(const void* qkv, void* out, const float* cos_table, const float* sin_table,
                   int64_t rows, int32_t seqlen, int32_t heads, int32_t head_dim, int32_t is_bf16,
                   int32_t conjugate, void* cuda_stream) {
@@ -333,7 +341,8 @@ uint64_t fa_philox_increment(int32_t head_dim, int32_t max_seqlen_q, int32_t max
   return steps * mmas_n * 8 * loop_steps;
 }
 
-static int run_fwd(const fa_fwd_params* p, bool zero_unused, void* cuda_stream) {
+// `bounds`: a padded batch (fa_fwd_padded), else null
+static int run_fwd(const fa_fwd_params* p, bool zero_unused, const int32_t* bounds, void* cuda_stream) {
   if (int rc = validate_common(p)) return rc;
   FA_REQUIRE(p->o && p->softmax_lse, "o and softmax_lse must be non-null");
   FA_REQUIRE((reinterpret_cast<uintptr_t>(p->o) & 15) == 0, "o must be 16-byte aligned");
@@ -360,6 +369,12 @@ static int run_fwd(const fa_fwd_params* p, bool zero_unused, void* cuda_stream) 
                              p->k_row_stride, p->k_head_stride, 128)) return rc;
   if (int rc = make_tile_map(&l.tm_v, p->v, l.is_bf16, p->total_k, p->heads, p->head_dim,
                              p->v_row_stride, p->v_head_stride, 128)) return rc;
+  if (bounds) {
+    l.args.cu_seqlens_q = l.args.cu_seqlens_k = bounds;
+    l.args.pad_rows = p->max_seqlen_q;
+    FA_CUDA(fa::launch_fwd_padded(l, static_cast<cudaStream_t>(cuda_stream)));
+    return FA_OK;
+  }
   // A few query rows per sequence: the decoding kernel where it is the faster one.  Dropout and block-sparse
   // calls keep the tile kernel (their mask is tied to its tiles), and so do causal ones, which see no more
   // keys than they have query rows.
@@ -377,10 +392,22 @@ static int run_fwd(const fa_fwd_params* p, bool zero_unused, void* cuda_stream) 
   return FA_OK;
 }
 
-int fa_fwd(const fa_fwd_params* p, void* cuda_stream) { return run_fwd(p, false, cuda_stream); }
+int fa_fwd(const fa_fwd_params* p, void* cuda_stream) { return run_fwd(p, false, nullptr, cuda_stream); }
 
 int fa_fwd_ex(const fa_fwd_params* p, int32_t zero_unused_rows, void* cuda_stream) {
-  return run_fwd(p, zero_unused_rows != 0, cuda_stream);
+  return run_fwd(p, zero_unused_rows != 0, nullptr, cuda_stream);
+}
+
+int fa_fwd_padded(const fa_fwd_params* p, const int32_t* bounds, void* cuda_stream) {
+  FA_REQUIRE(p != nullptr && bounds != nullptr, "params and bounds must be non-null");
+  FA_REQUIRE(!p->is_bf16 && p->p_dropout == 0.f && !p->blockmask && !p->s_dmask,
+             "padded batches: fp16, no dropout, no block mask, no s_dmask");
+  FA_REQUIRE(p->max_seqlen_q == p->max_seqlen_k && p->total_q == p->total_k &&
+                 static_cast<int64_t>(p->batch) * p->max_seqlen_q == p->total_q,
+             "padded batches: batch x max_seqlen rows of q, k and v");
+  fa_fwd_params padded = *p;
+  padded.cu_seqlens_q = padded.cu_seqlens_k = bounds;
+  return run_fwd(&padded, false, bounds, cuda_stream);
 }
 
 int fa_debug_dropout_mask(uint8_t* mask_out, int32_t batch_idx, int32_t head_idx,

@@ -135,8 +135,34 @@ __device__ __forceinline__ void store_rows(const KernelArgs& a, uint32_t tO, int
   }
 }
 
-// ORDERED: causal grids with the order of set_tail_grid
-template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BLOCKSPARSE, int G, bool ROWS, bool ORDERED>
+// Padded batches.  A V tile that reaches behind its sequence's last token holds whatever the padding holds, and its
+// probabilities there are zero: the rows are cleared, so that an infinity or a NaN in the padding stays out of the sum.
+// One warp, behind the tile's load and ahead of the product.
+template <int PANELS>
+__device__ __forceinline__ void clear_v_rows(uint8_t* tile, int first, int lane) {
+#pragma unroll
+  for (int p = 0; p < PANELS; ++p)
+    for (int i = first * 8 + lane; i < kBlockN * 8; i += 32)
+      *reinterpret_cast<uint4*>(tile + p * 16384 + i * 16) = make_uint4(0, 0, 0, 0);
+  fence_async_smem();
+  __syncwarp();
+}
+
+// Rows [r0, r1) of sequence b's padded rows that hold no token (`first`, `len`: its run) get zeros, by `threads` threads.
+__device__ __forceinline__ void zero_padding(const KernelArgs& a, int b, int h, int r0, int r1, int first, int len, int thread,
+                                             int threads) {
+  const int chunks = a.head_dim / 8;
+  uint16_t* o = reinterpret_cast<uint16_t*>(a.o) + static_cast<int64_t>(b) * a.pad_rows * a.o_row_stride +
+                static_cast<int64_t>(h) * a.o_head_stride;
+  for (int i = r0 * chunks + thread; i < min(r1, a.pad_rows) * chunks; i += threads) {
+    const int r = i / chunks;
+    if (r < first || r >= first + len)
+      *reinterpret_cast<uint4*>(o + r * a.o_row_stride + (i - r * chunks) * 8) = make_uint4(0, 0, 0, 0);
+  }
+}
+
+// ORDERED: causal grids with the order of set_tail_grid.  PADDED: see KernelArgs::pad_rows
+template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BLOCKSPARSE, int G, bool ROWS, bool ORDERED, bool PADDED>
 __global__ void __launch_bounds__(FwdCfg<D, G, ROWS>::kThreads, G == 1 ? 2 : 1)
 fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
               const __grid_constant__ CUtensorMap tm_v, const KernelArgs a) {
@@ -156,10 +182,10 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   const int32_t failed = a.status ? *reinterpret_cast<volatile int32_t*>(a.status) : 0;
   int b = blockIdx.z, h = blockIdx.y, mp = CAUSAL ? gridDim.x - 1 - blockIdx.x : blockIdx.x;  // heavy tiles first
   if constexpr (ORDERED) tail_block(a, blockIdx.x, mp, h, b);
-  const int q_start = a.cu_seqlens_q[b];
-  const int sq = a.cu_seqlens_q[b + 1] - q_start;
-  const int k_start = a.cu_seqlens_k[b];
-  const int sk = a.cu_seqlens_k[b + 1] - k_start;
+  const int q_start = a.cu_seqlens_q[PADDED ? 2 * b : b];
+  const int sq = a.cu_seqlens_q[PADDED ? 2 * b + 1 : b + 1] - q_start;
+  const int k_start = PADDED ? q_start : a.cu_seqlens_k[b];
+  const int sk = PADDED ? sq : a.cu_seqlens_k[b + 1] - k_start;
   if (tid == 32 * Cfg::kSoftmaxWarps) {  // while the lengths are on their way
     sh.abort_flag = 0;
     for (int i = 0; i < 2; ++i) {
@@ -183,6 +209,11 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   if constexpr (ORDERED) {
     mp = (sq + G * kBlockM - 1) / (G * kBlockM) - 1 - mp;  // of the sequence's own tiles; empty blocks last
     if (mp < 0) return;
+  }
+  if constexpr (PADDED) {
+    if (q_start < 0) return;
+    if (mp * G * kBlockM >= sq)
+      zero_padding(a, b, h, mp * G * kBlockM, (mp + 1) * G * kBlockM, q_start - b * a.pad_rows, sq, tid, Cfg::kThreads);
   }
   if (mp * G * kBlockM >= sq || failed == a.launch_id) return;
 
@@ -357,6 +388,8 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           if (!ok) break;
         } else {
           ok = mbar_wait_warp(smem_u32(&sh.v_full[s]), (j / Cfg::kStages) & 1, abort_flag);
+          if (PADDED && ok && (j + 1) * kBlockN > sk)
+            clear_v_rows<Cfg::kPanels>(smem + (smem_v - smem_q) + s * Cfg::kTileBytes, sk - j * kBlockN, lane);
           // K of the next tile is waited for behind P V of this one, which does not need it (its load takes about 2000 clk where
           // two CTAs with a stage each share an SM)
           bool k_here = false;
@@ -402,6 +435,8 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         const int s = j % Cfg::kStages;
         ok = mbar_wait_warp(smem_u32(&sh.v_full[s]), (j / Cfg::kStages) & 1, abort_flag);
         if (!ok) break;
+        if (PADDED && (j + 1) * kBlockN > sk)
+          clear_v_rows<Cfg::kPanels>(smem + (smem_v - smem_q) + s * Cfg::kTileBytes, sk - j * kBlockN, lane);
         const uint64_t va = desc_here(desc_at(desc_v, s * Cfg::kTileBytes));
 #pragma unroll
         for (int g = 0; g < G; ++g) {
@@ -425,6 +460,8 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       }
       mma_drain(smem_u32(&sh.drained[1]));
     }
+  } else if (PADDED && warp == Cfg::kSoftmaxWarps + 3) {
+    zero_padding(a, b, h, mp * G * kBlockM, (mp + 1) * G * kBlockM, q_start - b * a.pad_rows, sq, lane, 32);
   } else if (Cfg::kRows && warp < Cfg::kSoftmaxWarps) {
     // ------------------------------------------------------------------ softmax groups, one thread per query row
     reg_alloc<Cfg::kSoftmaxRegs>();
@@ -828,12 +865,12 @@ bool tail_order(const FwdLaunch& l, int tiles) {
          static_cast<int64_t>(tiles) * l.args.heads * l.args.batch > (G == 1 ? 2 : 1) * kSms;
 }
 
-template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BS, int G, bool ROWS, bool ORDERED = false>
+template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BS, int G, bool ROWS, bool ORDERED = false, bool PADDED = false>
 cudaError_t launch_groups(const FwdLaunch& l, cudaStream_t stream) {
   dim3 grid((l.max_seqlen_q + G * kBlockM - 1) / (G * kBlockM), l.args.heads, l.args.batch);
-  if constexpr (CAUSAL && !ORDERED)
+  if constexpr (CAUSAL && !ORDERED && !PADDED)
     if (tail_order<G>(l, grid.x)) return launch_groups<D, BF16, CAUSAL, DROPOUT, BS, G, ROWS, true>(l, stream);
-  auto kernel = fa_fwd_kernel<D, BF16, CAUSAL, DROPOUT, BS, G, ROWS, ORDERED>;
+  auto kernel = fa_fwd_kernel<D, BF16, CAUSAL, DROPOUT, BS, G, ROWS, ORDERED, PADDED>;
   using Cfg = FwdCfg<D, G, ROWS>;
   static SmemLimitFlags smem_limit_set;  // one per template instantiation of this function
   cudaError_t e = set_smem_limit_once(kernel, Cfg::kSmemBytes, smem_limit_set);
@@ -891,17 +928,17 @@ bool one_tile_per_cta(const FwdLaunch& l) {
 // keys 5.9 / 5.7 us, 16 x 16 heads, 128 queries, 512 keys 12.5 / 11.8, 1024 keys and queries 0.98).
 constexpr int kRowsMaxD64 = 512;  // keys
 
-template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BS>
+template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BS, bool PADDED = false>
 cudaError_t launch_one(const FwdLaunch& l, cudaStream_t stream) {
   const bool one_tile = one_tile_per_cta<D, CAUSAL, DROPOUT>(l);
   if constexpr (!DROPOUT) {
     if (D == 128 || l.max_seqlen_k <= kRowsMaxD64)
-      return one_tile ? launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 1, true>(l, stream)
-                      : launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 2, true>(l, stream);
+      return one_tile ? launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 1, true, false, PADDED>(l, stream)
+                      : launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 2, true, false, PADDED>(l, stream);
   }
   if constexpr (D == 64 || DROPOUT) {
-    return one_tile ? launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 1, false>(l, stream)
-                    : launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 2, false>(l, stream);
+    return one_tile ? launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 1, false, false, PADDED>(l, stream)
+                    : launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 2, false, false, PADDED>(l, stream);
   }
   return cudaErrorInvalidValue;
 }
@@ -932,6 +969,15 @@ cudaError_t launch_fwd(const FwdLaunch& l, cudaStream_t stream) {
                         : launch_one<64, false, false, false, true>(l, stream);
   }
   return l.dpad == 64 ? launch_d<64>(l, stream) : launch_d<128>(l, stream);
+}
+
+cudaError_t launch_fwd_padded(const FwdLaunch& l, cudaStream_t stream) {
+  if (l.is_bf16 || l.is_dropout || l.args.bs_iter != nullptr) return cudaErrorInvalidValue;
+  if (l.dpad == 64)
+    return l.is_causal ? launch_one<64, false, true, false, false, true>(l, stream)
+                       : launch_one<64, false, false, false, false, true>(l, stream);
+  return l.is_causal ? launch_one<128, false, true, false, false, true>(l, stream)
+                     : launch_one<128, false, false, false, false, true>(l, stream);
 }
 
 }  // namespace fa

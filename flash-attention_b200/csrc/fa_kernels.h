@@ -48,6 +48,9 @@ struct KernelArgs {
   int32_t grid_tiles, grid_heads, grid_first;  // the backward's causal grids (see set_causal_grid)
   FastDiv tail_tiles, tail_pairs, tail_heads;  // the forward's (see set_tail_grid)
   int32_t tail_first;
+  // Padded batches (fa_fwd_padded): every sequence has pad_rows rows, and the tokens of sequence b, one run of them, lie in rows
+  // [cu_seqlens[2 b], cu_seqlens[2 b + 1]); a negative start: the launch has nothing to do.  0: packed tokens.
+  int32_t pad_rows;
 };
 
 // Whether the blocks of a grid of (tiles, heads, batch) can be counted along its x dimension.  Beyond 2^31 - 1 blocks a
@@ -175,6 +178,7 @@ struct BwdLaunch {
 };
 
 cudaError_t launch_fwd(const FwdLaunch& l, cudaStream_t stream);
+cudaError_t launch_fwd_padded(const FwdLaunch& l, cudaStream_t stream);
 bool decode_serves(const FwdLaunch& l);  // whether launch_decode takes the call (l.decode apart)
 cudaError_t launch_decode(const FwdLaunch& l, cudaStream_t stream);
 cudaError_t launch_bwd(const BwdLaunch& l, cudaStream_t stream);
@@ -201,6 +205,8 @@ cudaError_t launch_scatter_rows(const void* src, const int64_t* indices, void* d
 
 cudaError_t launch_mask_index(const uint8_t* mask, int batch, int seqlen, int32_t* counts, int32_t* cu_seqlens,
                               int64_t* indices, int32_t* summary, cudaStream_t stream);
+cudaError_t launch_mask_bounds(const uint8_t* mask, int batch, int seqlen, int32_t* bounds, int32_t* summary,
+                               cudaStream_t stream);
 
 cudaError_t launch_rotary_qkv(const void* qkv, void* out, const float* cos_t, const float* sin_t,
                               int64_t rows, int seqlen, int heads, int d, bool bf16, bool conj,

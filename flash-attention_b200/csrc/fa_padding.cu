@@ -184,7 +184,72 @@ mask_index_kernel(const uint8_t* __restrict__ mask, int batch, int seqlen, const
   }
 }
 
+// Where the valid tokens of every sequence of a padded batch lie, where they are one run each: bounds[2 b], bounds[2 b + 1] =
+// first and last-but-one row of the flattened batch; -1, -1 in all of them where a sequence has holes.  summary = (1 if all are
+// runs, longest, tokens).  Latency bound: one CTA, a warp per sequence, the whole answer in one launch.
+constexpr int kBoundsThreads = 1024;
+__global__ void __launch_bounds__(kBoundsThreads)
+mask_bounds_kernel(const uint8_t* __restrict__ mask, int batch, int seqlen, bool words, int32_t* __restrict__ bounds,
+                   volatile int32_t* summary) {
+  __shared__ int longest, total;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  if (threadIdx.x == 0) longest = total = 0;
+  __syncthreads();
+  bool holes = false;
+  for (int b = warp; b < batch; b += kBoundsThreads / 32) {
+    const uint8_t* row = mask + static_cast<int64_t>(b) * seqlen;
+    int n = 0, first = seqlen, end = 0;
+    if (words) {  // rows of whole, aligned 32-bit words
+      const uint32_t* w = reinterpret_cast<const uint32_t*>(row);
+#pragma unroll 4
+      for (int i = lane; i < seqlen / 4; i += 32) {
+        const uint32_t set = __vcmpne4(w[i], 0u);  // 0xff for every valid token
+        if (set != 0) {
+          n += __popc(set) / 8;
+          first = min(first, 4 * i + (__ffs(set) - 1) / 8);
+          end = max(end, 4 * i + (31 - __clz(set)) / 8 + 1);
+        }
+      }
+    } else {
+#pragma unroll 4
+      for (int i = lane; i < seqlen; i += 32)
+        if (row[i] != 0) {
+          ++n;
+          first = min(first, i);
+          end = max(end, i + 1);
+        }
+    }
+    n = __reduce_add_sync(0xffffffffu, n);
+    first = __reduce_min_sync(0xffffffffu, first);
+    end = __reduce_max_sync(0xffffffffu, end);
+    if (n == 0) first = end = 0;
+    holes = holes || n != end - first;
+    if (lane == 0) {
+      atomicMax(&longest, n);
+      atomicAdd(&total, n);
+      bounds[2 * b] = b * seqlen + first;
+      bounds[2 * b + 1] = b * seqlen + end;
+    }
+  }
+  holes = __syncthreads_or(holes);
+  if (holes)
+    for (int i = threadIdx.x; i < 2 * batch; i += kBoundsThreads) bounds[i] = -1;
+  if (threadIdx.x == 0) {
+    summary[0] = holes ? 0 : 1;
+    summary[1] = longest;
+    summary[2] = total;
+    __threadfence_system();
+  }
+}
+
 }  // namespace
+
+cudaError_t launch_mask_bounds(const uint8_t* mask, int batch, int seqlen, int32_t* bounds, int32_t* summary,
+                               cudaStream_t stream) {
+  const bool words = seqlen % 4 == 0 && (reinterpret_cast<uintptr_t>(mask) & 3) == 0;
+  mask_bounds_kernel<<<1, kBoundsThreads, 0, stream>>>(mask, batch, seqlen, words, bounds, summary);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_gather_rows(const void* src, const int64_t* indices, void* dst, int64_t n_rows,
                                int64_t src_rows, int64_t row_bytes, cudaStream_t stream) {

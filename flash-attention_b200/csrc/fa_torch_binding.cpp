@@ -17,6 +17,7 @@
 #include <torch/extension.h>
 
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
 #include <ATen/cuda/CUDAGeneratorImpl.h>
 #include <c10/cuda/CUDAGuard.h>
 
@@ -578,6 +579,82 @@ c10::optional<at::Tensor> attn(const at::Tensor& q, const at::Tensor& k, const a
   return attention(x, kSeparate, cu_q, cu_k, max_q, max_k, p_dropout, scale, causal, nullptr);
 }
 
+// Attention on a padded batch, qkv (batch, seqlen, 3, heads, d), mask (batch, seqlen) bool, without gradient and dropout:
+// what unpad_input, attn_qkvpacked and pad_input give, in one pass over the batch as it stands.  nullopt: a call that is
+// left to those functions.  Where the tokens of a sequence lie is found on the device and the attention is launched behind it;
+// the host meanwhile waits for the answer whether they form one run each.  If not, the launch has done nothing and the
+// batch is packed (attn_with_holes).  us, those functions -> here: 64 x 512 tokens, 12 x 64 heads, lengths U[256, 512] 199 -> 93,
+// with holes 193 -> 181; 16 x 128 tokens (bound by the host) 108 -> 21; 8 x 1024 tokens, 12 x 128 heads 132 -> 53.
+constexpr int64_t kPaddedMaxTokens = 1 << 20;  // of the one CTA that reads the mask
+
+// rows (batch * seqlen, 3, heads, d) -> (batch * seqlen, heads, d); total, longest: of the mask, known by now
+at::Tensor attn_with_holes(const at::Tensor& rows, const at::Tensor& mask, int64_t total, int64_t longest, double scale,
+                           bool causal) {
+  const int64_t batch = mask.size(0), seqlen = mask.size(1), heads = rows.size(2), d = rows.size(3);
+  const auto stream = at::cuda::getCurrentCUDAStream().stream();
+  const at::TensorOptions ints = mask.options().dtype(at::kInt);
+  const at::Tensor lists = at::empty({2 * batch + 3}, ints);  // lengths, (total, longest), cu_seqlens
+  const at::Tensor indices = at::empty({batch * seqlen}, mask.options().dtype(at::kLong));
+  const at::Tensor cu = lists.slice(0, batch + 2);
+  int32_t* counts = static_cast<int32_t*>(lists.data_ptr());
+  const int64_t* index = static_cast<const int64_t*>(indices.data_ptr());
+  check_rc(fa_mask_index(static_cast<const uint8_t*>(mask.data_ptr()), static_cast<int32_t>(batch), static_cast<int32_t>(seqlen),
+                         counts, static_cast<int32_t*>(cu.data_ptr()), static_cast<int64_t*>(indices.data_ptr()), counts + batch,
+                         stream));
+  const at::Tensor packed = at::empty({total, 3, heads, d}, rows.options());
+  check_rc(fa_gather_rows(rows.data_ptr(), index, packed.data_ptr(), total, batch * seqlen, 6 * heads * d, stream));
+  const FwdCall c{longest, longest, 0.0, scale, false, causal, false, 0, 0, status_of(rows.device())};
+  const FwdResult r = run_fwd(view_of(packed, 0), view_of(packed, 1), view_of(packed, 2), rows.options(), cu, cu, nullptr, c,
+                              c10::nullopt);
+  const at::Tensor out = at::empty({batch * seqlen, heads, d}, rows.options());
+  const at::Tensor inverse = at::empty({batch * seqlen}, ints);
+  check_rc(fa_scatter_rows(r.o.data_ptr(), index, out.data_ptr(), total, batch * seqlen, 2 * heads * d,
+                           static_cast<int32_t*>(inverse.data_ptr()), stream));
+  return out;
+}
+
+c10::optional<at::Tensor> attn_padded_qkv(const at::Tensor& qkv, const at::Tensor& mask, c10::optional<double> softmax_scale,
+                                          bool causal) {
+  if (qkv.dim() != 5 || mask.dim() != 2 || qkv.size(2) != 3 || qkv.size(0) != mask.size(0) || qkv.size(1) != mask.size(1) ||
+      !qkv.is_cuda() || qkv.device() != mask.device() || qkv.scalar_type() != at::kHalf || mask.scalar_type() != at::kBool ||
+      !qkv.is_contiguous() || !mask.is_contiguous() || reinterpret_cast<uintptr_t>(qkv.data_ptr()) % 16 != 0 ||
+      mask.numel() == 0 || mask.numel() > kPaddedMaxTokens || left_to_the_classes(&qkv, 1) ||
+      (c10::GradMode::is_enabled() && qkv.requires_grad()))
+    return c10::nullopt;
+  const int64_t batch = qkv.size(0), seqlen = qkv.size(1), heads = qkv.size(3), d = qkv.size(4);
+  if (!(d == 16 || d == 32 || d == 64 || d == 128) || heads < 1 || heads > 65535 || batch > 65535) return c10::nullopt;
+  c10::cuda::CUDAGuard guard(qkv.device());
+  const auto stream = at::cuda::getCurrentCUDAStream();
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream.stream(), &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return c10::nullopt;
+  c10::NoGradGuard no_grad;
+  at::AutoDispatchBelowADInplaceOrView below;
+  const at::TensorOptions ints = mask.options().dtype(at::kInt);
+  const at::Tensor bounds = at::empty({2 * batch}, ints);
+  const at::Tensor summary = at::empty({3}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+  const at::Tensor rows = qkv.view({batch * seqlen, 3, heads, d});
+  at::Tensor out = at::empty({batch * seqlen, heads, d}, qkv.options());
+  const at::Tensor lse = at::empty({batch, heads, round_up(seqlen, 16)}, qkv.options().dtype(at::kFloat));
+  check_rc(fa_mask_bounds(static_cast<const uint8_t*>(mask.data_ptr()), static_cast<int32_t>(batch), static_cast<int32_t>(seqlen),
+                          static_cast<int32_t*>(bounds.data_ptr()), static_cast<int32_t*>(summary.data_ptr()), stream.stream()));
+  at::cuda::CUDAEvent answered;
+  answered.record(stream);
+  fa_fwd_params p;
+  const double scale = softmax_scale.has_value() ? *softmax_scale : 1.0 / std::sqrt(static_cast<double>(d));
+  fill_fwd(p, Dims{batch, batch * seqlen, batch * seqlen, heads, d}, view_of(rows, 0), view_of(rows, 1), view_of(rows, 2), out, lse,
+           bounds, bounds, seqlen, seqlen, 0.0, scale, causal, 0, 0, 0, 0, status_of(qkv.device()));
+  const int rc = fa_fwd_padded(&p, static_cast<const int32_t*>(bounds.data_ptr()), stream.stream());
+  {
+    // (also after an error: the kernel that writes the page-locked words has finished before they are given back)
+    py::gil_scoped_release release;
+    answered.synchronize();
+  }
+  check_rc(rc);
+  const int32_t* s = static_cast<const int32_t*>(summary.data_ptr());
+  if (s[2] == 0) return c10::nullopt;
+  return (s[0] != 0 ? out : attn_with_holes(rows, mask, s[2], s[1], scale, causal)).view({batch, seqlen, heads, d});
+}
+
 c10::optional<at::Tensor> attn_sparse_qkvpacked(const at::Tensor& qkv, const at::Tensor& cu, const at::Tensor& blockmask,
                                                 double p_dropout, int64_t max_s, c10::optional<double> scale, bool causal) {
   require(qkv.dim() == 4 && qkv.size(1) == 3, "qkv must be (total, 3, heads, head_dim)");
@@ -620,6 +697,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attn_kvpacked", &attn_kvpacked);
   m.def("attn", &attn);
   m.def("attn_sparse_qkvpacked", &attn_sparse_qkvpacked);
+  m.def("attn_padded_qkv", &attn_padded_qkv);
   m.def("convert_blockmask", &convert_blockmask);
   m.def("set_options", &set_options);
   m.def("set_status", &set_status);

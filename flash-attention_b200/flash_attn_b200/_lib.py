@@ -31,6 +31,8 @@ EXPORTED_SYMBOLS = (
     "fa_gather_rows",
     "fa_scatter_rows",
     "fa_mask_index",
+    "fa_mask_bounds",
+    "fa_fwd_padded",
     "fa_rotary_qkv",
     "fa_convert_blockmask",
     "fa_status_string",
@@ -147,6 +149,11 @@ def _load():
     lib.fa_mask_index.argtypes = [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32, ctypes.c_void_p,
                                   ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
     lib.fa_mask_index.restype = ctypes.c_int
+    lib.fa_mask_bounds.argtypes = [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32, ctypes.c_void_p, ctypes.c_void_p,
+                                   ctypes.c_void_p]
+    lib.fa_mask_bounds.restype = ctypes.c_int
+    lib.fa_fwd_padded.argtypes = [ctypes.POINTER(FwdParams), ctypes.c_void_p, ctypes.c_void_p]
+    lib.fa_fwd_padded.restype = ctypes.c_int
     lib.fa_rotary_qkv.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
                                   ctypes.c_int64, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,
                                   ctypes.c_int32, ctypes.c_int32, ctypes.c_void_p]

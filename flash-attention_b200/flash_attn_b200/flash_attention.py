@@ -3,7 +3,9 @@
 import torch
 import torch.nn as nn
 
+from . import flash_attn_cuda
 from .bert_padding import pad_input, unpad_input
+from .flash_attn_cuda import runs_now
 from .flash_attn_interface import flash_attn_unpadded_qkvpacked_func
 from .rotary import RotaryEmbedding, RotaryEmbedding2D
 
@@ -54,6 +56,12 @@ class FlashAttention(nn.Module):
             return out.reshape(batch, seqlen, heads, d), None
 
         mask = _mask_matrix(key_padding_mask)
+        # without gradient and dropout: on the batch as it stands
+        native = flash_attn_cuda.compiled_attention(qkv) if p == 0.0 and runs_now(qkv) and runs_now(mask) else None
+        if native is not None:
+            out = native.attn_padded_qkv(qkv, mask, self.softmax_scale, bool(causal))
+            if out is not None:
+                return out, None
         x_unpad, indices, cu, max_len = unpad_input(qkv.reshape(batch, seqlen, three * heads * d), mask)
         out_unpad = flash_attn_unpadded_qkvpacked_func(
             x_unpad.reshape(-1, three, heads, d), cu, max_len, p,

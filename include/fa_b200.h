@@ -208,6 +208,20 @@ int fa_scatter_rows(const void* src, const int64_t* indices, void* dst, int64_t 
 int fa_mask_index(const uint8_t* mask, int32_t batch, int32_t seqlen, int32_t* counts, int32_t* cu_seqlens,
                   int64_t* indices, int32_t* summary, void* cuda_stream);
 
+/* Where the valid tokens of every sequence lie in a padded batch, where they form one run each (padding in front, behind or on
+ * both sides): bounds[2 b] and bounds[2 b + 1] (2 * batch entries) = first row and the row behind the last, counted in the
+ * flattened batch; -1 in all entries where a sequence has holes.  summary (3 entries, device memory or page-locked host memory)
+ * = (1 if every sequence is one run, longest sequence, number of valid tokens).  mask as in fa_mask_index. */
+int fa_mask_bounds(const uint8_t* mask, int32_t batch, int32_t seqlen, int32_t* bounds, int32_t* summary,
+                   void* cuda_stream);
+
+/* Self-attention on a padded batch as it stands: q, k, v and o have batch * max_seqlen_q rows (= total_q = total_k), sequence b
+ * takes rows [b * max_seqlen_q, (b + 1) * max_seqlen_q), `bounds` (device memory, of fa_mask_bounds) says which of them hold
+ * tokens; the other rows of o become zero, and nothing that the inputs hold there has an effect.  With -1 in bounds nothing is
+ * written.  Equals unpad_input, attention and pad_input (flash_attn/flash_attention.py:52-68) in one pass over the batch.
+ * fp16, no dropout, no block mask; cu_seqlens of `p` are not read. */
+int fa_fwd_padded(const fa_fwd_params* p, const int32_t* bounds, void* cuda_stream);
+
 /* Rotary position embedding on a packed qkv tensor (rows, 3, heads, head_dim), rows = batch *
  * seqlen with the token position = row % seqlen: q and k are rotated pairwise (channels 2i, 2i+1 by
  * the angle with cosine cos_table[pos][i] and sine sin_table[pos][i], fp32 tables of head_dim / 2

@@ -1,0 +1,80 @@
+"""FlashAttention on a padded batch without gradient: the kernels run on the batch as it stands (fa_mask_bounds, fa_fwd_padded)
+where every sequence's tokens form one run, and give what unpad_input, attention and pad_input give."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _mask(kind, batch, seqlen, seed):
+    g = torch.Generator().manual_seed(seed)
+    length = torch.randint(1, seqlen + 1, (batch,), generator=g)
+    length[0] = seqlen
+    if batch > 2:
+        length[1] = 0
+    first = torch.zeros(batch, dtype=torch.long)
+    if kind == "front":
+        first = seqlen - length
+    elif kind == "both":
+        first = ((seqlen - length) * torch.rand(batch, generator=g)).long()
+    pos = torch.arange(seqlen)[None, :]
+    return ((pos >= first[:, None]) & (pos < (first + length)[:, None])).cuda()
+
+
+def _reference(qkv, mask, causal):
+    """Per sequence in 64 bits."""
+    out = torch.zeros(qkv.shape[:2] + qkv.shape[3:], dtype=torch.float64, device=qkv.device)
+    for b in range(qkv.shape[0]):
+        idx = mask[b].nonzero().flatten()
+        if idx.numel():
+            q, k, v = qkv[b, idx].double().permute(1, 2, 0, 3)
+            s = q @ k.transpose(-1, -2) * qkv.shape[-1] ** -0.5
+            if causal:
+                s = s.masked_fill(torch.ones_like(s[0], dtype=torch.bool).triu(1), float("-inf"))
+            out[b, idx] = (s.softmax(-1) @ v).transpose(0, 1)
+    return out
+
+
+@pytest.mark.parametrize("batch,seqlen,heads,d,causal,kind", [
+    (3, 1, 2, 64, False, "back"), (3, 7, 2, 16, True, "front"), (4, 127, 2, 64, False, "both"), (4, 128, 3, 128, True, "back"),
+    (4, 129, 2, 32, False, "front"), (5, 300, 2, 64, True, "both"), (4, 300, 2, 128, False, "both"), (3, 520, 2, 64, False, "both"),
+    (3, 777, 2, 64, True, "front"), (30, 520, 12, 64, False, "back"), (6, 1100, 4, 128, True, "both"), (3, 1300, 2, 128, False, "back"),
+    (12, 200, 12, 64, False, "both")])
+def test_padded_batch(batch, seqlen, heads, d, causal, kind):
+    from flash_attn_b200 import flash_attn_cuda
+    from flash_attn_b200.flash_attention import FlashAttention
+    g = torch.Generator(device="cuda").manual_seed(batch * 1000 + seqlen)
+    qkv = torch.randn(batch, seqlen, 3, heads, d, device="cuda", generator=g).half()
+    mask = _mask(kind, batch, seqlen, seqlen)
+    want = _reference(qkv, mask, causal)
+    # what lies in the padding has no effect
+    dirty = qkv.clone()
+    dirty[~mask] = torch.tensor([float("nan"), float("inf"), -float("inf"), 6e4], device="cuda").half().repeat(d // 4)
+    native = flash_attn_cuda.compiled_attention(qkv)
+    for x in (qkv, dirty):
+        got = native.attn_padded_qkv(x, mask, None, causal)
+        assert got is not None
+        assert torch.equal(got, FlashAttention()(x, key_padding_mask=mask, causal=causal)[0])
+        assert torch.all(got[~mask] == 0)
+        # P and the result are rounded to 11 bits: 2^-11 max|v| each
+        assert float((got.double() - want).abs().max()) <= 2 ** -10 * float(qkv[mask][:, 2].abs().max())
+
+
+def test_masks_with_holes_and_calls_left_to_the_packed_way():
+    from flash_attn_b200 import flash_attn_cuda
+    from flash_attn_b200.flash_attention import FlashAttention
+    qkv = torch.randn(4, 200, 3, 2, 64, device="cuda", generator=torch.Generator(device="cuda").manual_seed(0)).half()
+    mask = _mask("back", 4, 200, 5)
+    native = flash_attn_cuda.compiled_attention(qkv)
+    holes = mask.clone()
+    holes[0, 57] = False
+    for causal in (False, True):
+        got = native.attn_padded_qkv(qkv, holes, None, causal)
+        want = _reference(qkv, holes, causal)
+        assert torch.equal(got, FlashAttention()(qkv, key_padding_mask=holes, causal=causal)[0])
+        assert torch.all(got[~holes] == 0) and float((got.double() - want).abs().max()) <= 2 ** -10 * float(qkv.abs().max())
+    assert native.attn_padded_qkv(qkv, torch.zeros_like(mask), None, False) is None  # no token at all: refused by the packed way
+    assert native.attn_padded_qkv(qkv.clone().requires_grad_(), mask, None, False) is None
+    assert native.attn_padded_qkv(qkv, mask.int(), None, False) is None
+    assert native.attn_padded_qkv(qkv[:, :, :, :, :32], mask, None, False) is None  # not contiguous
+    assert native.attn_padded_qkv(qkv.bfloat16(), mask, None, False) is None
