@@ -51,14 +51,14 @@ EncodeTiledFn get_encode_tiled() {
 }
 
 // 3-D map over a [rows, heads, head_dim] tensor with arbitrary row / head strides:
-// dim0 = head_dim, dim1 = rows, dim2 = heads; box = 64 columns x box_rows rows x 1 head, stored
-// with the 128-byte swizzle.  Columns beyond head_dim and rows beyond `rows` read as zero.
+// dim0 = head_dim, dim1 = rows, dim2 = heads; box = box_columns (64 or 32) columns x box_rows rows x 1 head, stored
+// with the 128-byte (64-byte) swizzle.  Columns beyond head_dim and rows beyond `rows` read as zero.
 // `bind_context`: a thread that has only used the runtime API lazily (an autograd worker, for
 // instance) may not have the primary context bound yet and the driver call below needs it;
 // cudaFree(nullptr) binds it.  The entry point that must not touch the allocator passes false
 // (it has bound the context with cudaSetDevice already).
 int make_tile_map(CUtensorMap* tm, const void* base, bool bf16, int64_t rows, int heads, int head_dim,
-                  int64_t row_stride, int64_t head_stride, int box_rows, bool bind_context = true) {
+                  int64_t row_stride, int64_t head_stride, int box_rows, bool bind_context = true, int box_columns = 64) {
   EncodeTiledFn enc = get_encode_tiled();
   if (!enc) return fail(FA_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   static thread_local bool context_bound = false;
@@ -69,11 +69,11 @@ int make_tile_map(CUtensorMap* tm, const void* base, bool bf16, int64_t rows, in
   FA_REQUIRE((reinterpret_cast<uintptr_t>(base) & 15) == 0, "tensor base must be 16-byte aligned");
   FA_REQUIRE((row_stride * 2) % 16 == 0 && (head_stride * 2) % 16 == 0,
              "row and head strides must be multiples of 8 elements");
-  // A descriptor is a pure function of these eight values, and a training loop presents the same
+  // A descriptor is a pure function of these nine values, and a training loop presents the same
   // ones again and again (the caching allocator hands back the same blocks): a small per-thread
   // cache saves the driver call, which is a large share of the host time of a short-sequence call.
   struct Entry {
-    const void* base; int64_t rows, row_stride, head_stride; int32_t heads, head_dim, box_rows, bf16;
+    const void* base; int64_t rows, row_stride, head_stride; int32_t heads, head_dim, box_rows, box_columns, bf16;
     CUtensorMap map;
   };
   constexpr int kCacheSize = 32;
@@ -82,7 +82,8 @@ int make_tile_map(CUtensorMap* tm, const void* base, bool bf16, int64_t rows, in
   for (int i = 0; i < cache_used; ++i) {
     const Entry& e = cache[i];
     if (e.base == base && e.rows == rows && e.row_stride == row_stride && e.head_stride == head_stride &&
-        e.heads == heads && e.head_dim == head_dim && e.box_rows == box_rows && e.bf16 == (bf16 ? 1 : 0)) {
+        e.heads == heads && e.head_dim == head_dim && e.box_rows == box_rows && e.box_columns == box_columns &&
+        e.bf16 == (bf16 ? 1 : 0)) {
       *tm = e.map;
       return FA_OK;
     }
@@ -91,16 +92,16 @@ int make_tile_map(CUtensorMap* tm, const void* base, bool bf16, int64_t rows, in
                         static_cast<cuuint64_t>(heads)};
   cuuint64_t strides[2] = {static_cast<cuuint64_t>(row_stride) * 2,
                            static_cast<cuuint64_t>(head_stride) * 2};
-  cuuint32_t box[3] = {64, static_cast<cuuint32_t>(box_rows), 1};
+  cuuint32_t box[3] = {static_cast<cuuint32_t>(box_columns), static_cast<cuuint32_t>(box_rows), 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = enc(tm, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3,
                    const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   box_columns == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
     return fail(FA_ERR_CUDA, "cuTensorMapEncodeTiled failed with code " + std::to_string((int)r));
   Entry& slot = cache[cache_next];
-  slot = Entry{base, rows, row_stride, head_stride, heads, head_dim, box_rows, bf16 ? 1 : 0, *tm};
+  slot = Entry{base, rows, row_stride, head_stride, heads, head_dim, box_rows, box_columns, bf16 ? 1 : 0, *tm};
   cache_next = (cache_next + 1) % kCacheSize;
   if (cache_used < kCacheSize) ++cache_used;
   return FA_OK;
@@ -446,7 +447,7 @@ size_t fa_bwd_workspace_bytes(int32_t total_q, int32_t heads, int32_t head_dim) 
 
 namespace {
 
-// Body shared by fa_bwd and fa_bwd_static_scratch: validation, kernel arguments, the five tensor
+// Body shared by fa_bwd and fa_bwd_static_scratch: validation, kernel arguments, the tensor
 // maps and the launches.  `accum` is the fp32 dQ accumulator (already checked to be large enough).
 int run_bwd(const fa_bwd_params* p, float* accum, int stage_mask, bool bind_context, cudaStream_t stream) {
   const fa_fwd_params* f = &p->fwd;
@@ -501,6 +502,11 @@ int run_bwd(const fa_bwd_params* p, float* accum, int stage_mask, bool bind_cont
                              f->v_row_stride, f->v_head_stride, 128, bind_context)) return rc;
   if (int rc = make_tile_map(&l.tm_do, p->dout, l.is_bf16, f->total_q, f->heads, f->head_dim,
                              a.do_row_stride, a.do_head_stride, 128, bind_context)) return rc;
+  const int columns = fa::grad_box_columns(l.dpad, l.is_dropout);
+  if (int rc = make_tile_map(&l.tm_dk, a.dk, l.is_bf16, f->total_k, f->heads, f->head_dim,
+                             a.dk_row_stride, a.dk_head_stride, 32, bind_context, columns)) return rc;
+  if (int rc = make_tile_map(&l.tm_dv, a.dv, l.is_bf16, f->total_k, f->heads, f->head_dim,
+                             a.dv_row_stride, a.dv_head_stride, 32, bind_context, columns)) return rc;
   if (int rc = make_accum_map(&l.tm_dq, a.dq_accum, f->total_q, f->heads, l.dpad)) return rc;
   FA_CUDA(fa::launch_bwd(l, stream));
   return FA_OK;

@@ -75,6 +75,8 @@ struct BwdCfg {
   static constexpr int kOtherRegs = kQuad ? 32 : kTwoPhase ? 72 : 56;
   // arrivals of the compute warps at a barrier: every thread, or one lane per warp
   static constexpr uint32_t kComputeArrivals = kQuad ? 16 : 256;
+  // a warp of the epilogue holds 32 rows and these columns of dK or dV at a time
+  static constexpr int kBoxColumns = kQuad ? 32 : 64;
   static constexpr bool kAliasDq = kTwoPhase;     // dQ shares tensor-memory columns with dP
   static constexpr bool kDualIssue = !kTwoPhase;  // second MMA-issuing warp for dV, dK
   static constexpr int kTileBytes = 128 * D * 2;
@@ -177,9 +179,15 @@ template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BLOCKSPARSE>
 __global__ void __launch_bounds__(BwdCfg<D, BLOCKSPARSE, DROPOUT>::kThreads, 1)
 fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
               const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
-              const __grid_constant__ CUtensorMap tm_dq, const BwdArgs a) {
+              const __grid_constant__ CUtensorMap tm_dq, const __grid_constant__ CUtensorMap tm_dk,
+              const __grid_constant__ CUtensorMap tm_dv, const BwdArgs a) {
   using Cfg = BwdCfg<D, BLOCKSPARSE, DROPOUT>;
   constexpr int kDqWarp = Cfg::kComputeWarps, kProducer = kDqWarp + 4;  // first warp of the dQ group, of the last four
+  // dK and dV leave by TMA, except at d = 64 without dropout and causal mask: there half as many bytes are stored as at d = 128, and
+  // the first P~ of the next block would wait for them behind dQ adds and loads (16 x 12 x 1024: 198 us by the LSU, 210 by TMA).
+  // Whole backward, us, by the LSU -> now: 16 x 12 x 1000 causal (d = 128) 263 -> 255, 32 x 12 x 512 196 -> 189, 4 x 12 x 8192
+  // 2319 -> 2289; 8 x 12 x 512 with dropout (d = 64) 52.2 -> 50.2, 2 x 4 x 16384 causal 744 -> 733.
+  constexpr bool kTmaRows = Cfg::kTwoPhase || Cfg::kQuad || CAUSAL;
   constexpr bool kDsInTmem = Cfg::kDsInTmemCapable && !DROPOUT;
   extern __shared__ uint8_t smem_raw[];
   __shared__ BwdShared sh;
@@ -690,6 +698,33 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     bool ok = true;
     int g0 = 0;
     uint32_t k = 0;
+    // Row statistics of the next tile (rows r8 and r8 + 8 of the warp's block in the quad layout, else one row per thread), asked
+    // for while the tile before is worked on; those of a block's first tile before the epilogue of the block before.
+    float lse_nx[Cfg::kQuad ? 2 : 1], d_nx[Cfg::kQuad ? 2 : 1];
+    int32_t bs_nx = 0;
+    bool fetched = false;
+    auto fetch_stats = [&](const BlockInfo& x, int t) {
+      const int64_t stats = (static_cast<int64_t>(x.b) * ka.heads + x.h) * ka.lse_stride;  // row of LSE and D
+      const int i0 = q_tile(x, t) * kBM + (Cfg::kQuad ? (cwarp & 3) * 32 + (cwarp >> 3) * 16 : row);
+#pragma unroll
+      for (int u = 0; u < (Cfg::kQuad ? 2 : 1); ++u) {
+        const int i = Cfg::kQuad ? i0 + u * 8 + ((tid & 31) >> 2) : i0;
+        const bool valid = i < x.sq;
+        lse_nx[u] = valid ? ka.lse[stats + i] : INFINITY;  // scaled at its first use, one tile later
+        d_nx[u] = valid ? a.softmax_d[stats + i] : 0.f;
+      }
+      if constexpr (BLOCKSPARSE)
+        bs_nx = (i0 >> 4) < ka.bs_rows16
+                    ? ka.bs_iter[(static_cast<int64_t>(x.b) * ka.bs_kblocks + (x.n0 >> 8)) * ka.bs_rows16 + (i0 >> 4)]
+                    : -1;
+    };
+    // The warp's rows of the P~ and dS tiles are free for the first P~ of a block once the stores of the epilogue before
+    // (by lane 0) have read them.
+    auto rows_free = [&](int t) {
+      if (!kTmaRows || t > 0 || k == 0) return;
+      if ((tid & 31) == 0) bulk_wait_read();
+      __syncwarp();
+    };
     do {
     // with eight compute warps read where it is used, to hold few registers across the tiles (with sixteen, which have
     // them, 8 x 12 x 4096 with blocks taken over takes 973 us so and 924 from registers)
@@ -702,7 +737,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     }
     const int64_t bh_sub =
         (static_cast<int64_t>(x.b) * ka.drop.heads_total + ka.drop.head_offset + x.h) * 256;
-    const int64_t stats = (static_cast<int64_t>(x.b) * ka.heads + x.h) * ka.lse_stride;  // row of LSE and D
+    if (!fetched) fetch_stats(x, 0);
+    fetched = false;
     const uint64_t c2 = pack_f2(ka.scale_log2, ka.scale_log2);
     // dropout: per-lane generator state (lanes l and l ^ 8 share every Philox call)
     LanePhilox lp;
@@ -730,24 +766,6 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&bar));
       };
-      // statistics of rows r8 and r8 + 8 of the first tile; those of tile t + 1 are fetched while tile t is processed
-      float lse_nx[2], d_nx[2];
-      int32_t bs_nx = 0;
-      auto fetch_stats = [&](int t) {
-        const int i0 = q_tile(x, t) * kBM + wq * 32 + hh * 16;
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int ig_n = i0 + u * 8 + r8;
-          const bool valid = ig_n < x.sq;
-          lse_nx[u] = valid ? ka.lse[stats + ig_n] : INFINITY;
-          d_nx[u] = valid ? a.softmax_d[stats + ig_n] : 0.f;
-        }
-        if constexpr (BLOCKSPARSE)
-          bs_nx = (i0 >> 4) < ka.bs_rows16
-                      ? ka.bs_iter[(static_cast<int64_t>(x.b) * ka.bs_kblocks + (x.n0 >> 8)) * ka.bs_rows16 + (i0 >> 4)]
-                      : -1;
-      };
-      fetch_stats(0);
       for (int t = 0; t < nm && ok; ++t) {
         const int g = g0 + t;
         const int n0 = x.n0, sk = x.sk, L16 = (x.sq + 15) >> 4;
@@ -762,7 +780,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           nd2[u] = pack_f2(-d_nx[u], -d_nx[u]);
         }
         const int32_t bs_it = bs_nx;
-        if (t + 1 < nm) fetch_stats(t + 1);
+        if (t + 1 < nm) fetch_stats(x, t + 1);
         // (a block that is not in the layout is masked too)
         const bool need_mask = (n0 + kBN > sk) || (CAUSAL && (n0 + kBN - 1 > m0)) || (BLOCKSPARSE && bs_it < 0);
 
@@ -831,6 +849,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           if (c == 0 && g > 0) {
             ok = mbar_wait_warp(smem_u32(&sh.pds_free), (g & 1) ^ 1, abort_flag);
             if (!ok) break;
+            rows_free(t);
           }
           // four 8 x 8 matrices per instruction: (u = 0, 1) x (units a, a + 1) of the 64-column panel w
 #pragma unroll
@@ -846,35 +865,19 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       }
     } else {
 
-    // per-row statistics of the first tile; those of tile t + 1 are fetched while tile t is processed
-    float lse_next = INFINITY, d_next = 0.f;
-    int32_t bs_next = 0;
-    auto fetch_row_stats = [&](int t) {
-      const int ig_n = q_tile(x, t) * kBM + row;
-      const bool valid = ig_n < x.sq;
-      lse_next = valid ? ka.lse[stats + ig_n] : INFINITY;  // scaled at its first use, one tile later
-      d_next = valid ? a.softmax_d[stats + ig_n] : 0.f;
-      if constexpr (BLOCKSPARSE) {
-        bs_next = (ig_n >> 4) < ka.bs_rows16
-                      ? ka.bs_iter[(static_cast<int64_t>(x.b) * ka.bs_kblocks + (x.n0 >> 8)) * ka.bs_rows16 + (ig_n >> 4)]
-                      : -1;
-      }
-    };
-    fetch_row_stats(0);
-
     for (int t = 0; t < nm && ok; ++t) {
       const int g = g0 + t;
       const int n0 = x.n0, sk = x.sk, L16 = (x.sq + 15) >> 4;
       const int cbase = n0 + w * 64;  // first key column of this thread
       const int m0 = q_tile(x, t) * kBM;
       const int ig = m0 + row;
-      const float lse2 = lse_next * 1.4426950408889634f;
-      const float d_i = d_next;
+      const float lse2 = lse_nx[0] * 1.4426950408889634f;
+      const float d_i = d_nx[0];
       const uint64_t nlse2 = pack_f2(-lse2, -lse2);
       const uint64_t nd2 = pack_f2(-d_i, -d_i);
-      const int32_t bs_it = bs_next;
+      const int32_t bs_it = bs_nx;
       const bool row_in_layout = !BLOCKSPARSE || bs_it >= 0;
-      if (t + 1 < nm) fetch_row_stats(t + 1);
+      if (t + 1 < nm) fetch_stats(x, t + 1);
 
       // Keep words of this thread's 64 columns (wd[p] covers columns 2p, 2p + 1).  They do not depend
       // on the scores, so they are drawn before the wait for S and dP: eight independent Philox
@@ -950,6 +953,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           if (c == 0 && g > 0) {
             ok = mbar_wait(smem_u32(&sh.pds_free), (g & 1) ^ 1, abort_flag);
             ok = __all_sync(0xffffffffu, ok);
+            rows_free(t);
           }
 #pragma unroll
           for (int ch4 = 0; ch4 < 4; ++ch4) {
@@ -1047,6 +1051,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         if (c == 0 && g > 0) {
           ok = mbar_wait(smem_u32(&sh.pds_free), (g & 1) ^ 1, abort_flag);
           ok = __all_sync(0xffffffffu, ok);
+          rows_free(t);
         }
         // 32 16-bit values = 4 chunks of 16 bytes of this row in the 64-column panel w
 #pragma unroll
@@ -1075,6 +1080,11 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     }  // row-per-thread layout
 
     // ---------------- epilogue: group 0 writes dV = acc / p_keep, group 1 writes dK = acc * scale / p_keep
+    if (ok && take_over) {
+      ok = mbar_wait_warp(smem_u32(&sh.blk_full[(k + 1) & 1]), (k >> 1) & 1, abort_flag);
+      fetched = ok && sh.blk[(k + 1) & 1].nm > 0;
+      if (fetched) fetch_stats(sh.blk[(k + 1) & 1], 0);
+    }
     if (ok) {
       ok = mbar_wait(smem_u32(&sh.pds_free), (g0 + nm - 1) & 1, abort_flag);
       if constexpr (Cfg::kTwoPhase) {
@@ -1117,15 +1127,31 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         }
       }
       tc_fence_before();
+      fence_async_smem();
       __syncwarp();
-      if (elect_one()) mbar_arrive(smem_u32(&sh.acc_free));
+      if ((tid & 31) == 0) mbar_arrive(smem_u32(&sh.acc_free));
+      // Whole rows by TMA, which leaves the warp free for the next block (64 KB through the LSU took it 3500 clk at d = 128, with
+      // the first statistics of the next block behind them another 2350; a query tile takes 5500).  The warp that holds the
+      // sequence's end stores its rows itself, since those behind it are the next sequence's.
+      if (kTmaRows && r0 + 32 <= e.sk) {
+        if ((tid & 31) == 0) {
 #pragma unroll
-      for (int p = 0; p < (kChunks + 1) / 2; ++p)
-        stage_copy_out<CH>((p == 0 ? p_ptr : ds_ptr) + piece, dst + p * 64, stride, e.sk - r0,
-                           ka.head_dim / 8 - part * 4 - p * 8, tid & 31);
+          for (int p = 0; p < (kChunks + 1) / 2; ++p)
+            if (part * 32 + p * 64 < ka.head_dim)
+              tma_store_3d(grp == 0 ? &tm_dv : &tm_dk, smem_u32(p == 0 ? p_ptr : ds_ptr) + piece,
+                           part * 32 + p * 64, e.k_start + r0, e.h);
+          bulk_commit();
+        }
+      } else {
+#pragma unroll
+        for (int p = 0; p < (kChunks + 1) / 2; ++p)
+          stage_copy_out<CH>((p == 0 ? p_ptr : ds_ptr) + piece, dst + p * 64, stride, e.sk - r0,
+                             ka.head_dim / 8 - part * 4 - p * 8, tid & 31);
+      }
     }
     g0 += nm;
     } while (ok && next_block(k++));
+    if ((tid & 31) == 0) bulk_wait_all();
   } else {
     // ------------------------------------------------------------------ dQ group
     // dQ tile: tensor memory -> registers -> swizzled fp32 staging in shared memory -> one TMA
@@ -1386,7 +1412,7 @@ cudaError_t launch_main(const BwdLaunch& l, cudaStream_t stream) {
   args.take_over = !BS && linear && l.args.dq_tickets == nullptr;
   if constexpr (CAUSAL) set_causal_grid(&args.k, grid.x, int64_t(8) * D * args.max_seqlen_q);  // Q, dO and the fp32 dQ
   if (linear && (CAUSAL || args.take_over)) grid = dim3(grid.x * grid.y * grid.z, 1, 1);
-  return launch(overlap_launches(l), kernel, grid, Cfg::kThreads, smem, stream, l.tm_q, l.tm_k, l.tm_v, l.tm_do, l.tm_dq, args);
+  return launch(overlap_launches(l), kernel, grid, Cfg::kThreads, smem, stream, l.tm_q, l.tm_k, l.tm_v, l.tm_do, l.tm_dq, l.tm_dk, l.tm_dv, args);
 }
 
 template <int D, bool BF16, bool CAUSAL>

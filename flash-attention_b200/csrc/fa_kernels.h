@@ -170,6 +170,7 @@ struct FwdLaunch {
 struct BwdLaunch {
   CUtensorMap tm_q, tm_k, tm_v, tm_do;
   CUtensorMap tm_dq;  // fp32 dQ accumulator [total_q, heads, dpad], 32-column boxes
+  CUtensorMap tm_dk, tm_dv;  // outputs, boxes of 32 rows and grad_box_columns columns
   BwdArgs args;
   bool is_bf16, is_causal, is_dropout;
   int32_t dpad;  // 64 or 128
@@ -181,6 +182,8 @@ cudaError_t launch_fwd(const FwdLaunch& l, cudaStream_t stream);
 cudaError_t launch_fwd_padded(const FwdLaunch& l, cudaStream_t stream);
 bool decode_serves(const FwdLaunch& l);  // whether launch_decode takes the call (l.decode apart)
 cudaError_t launch_decode(const FwdLaunch& l, cudaStream_t stream);
+// Columns of dK and dV that a warp of the backward's epilogue stores at once (see its kBoxColumns).
+inline int grad_box_columns(int dpad, bool is_dropout) { return dpad == 64 && is_dropout ? 32 : 64; }
 cudaError_t launch_bwd(const BwdLaunch& l, cudaStream_t stream);
 cudaError_t launch_sdmask(void* s_out, int64_t s_rows, int64_t s_cols, const void* q, const void* k,
                           int64_t q_row_stride, int64_t q_head_stride, int64_t k_row_stride,
