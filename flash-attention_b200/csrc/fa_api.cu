@@ -473,7 +473,8 @@ int run_bwd(const fa_bwd_params* p, float* accum, int stage_mask, bool bind_cont
   l.is_causal = f->is_causal != 0;
   l.is_dropout = f->p_dropout > 0.f;
   l.stage_mask = stage_mask;
-  l.deterministic = p->deterministic != 0;
+  const bool single = fa::one_launch(f->max_seqlen_q, f->max_seqlen_k, static_cast<int64_t>(f->batch) * f->heads, f->blockmask != nullptr, stage_mask);
+  l.deterministic = p->deterministic != 0 && !single;  // one key tile adds to a query tile: nothing to put in order
   fa::BwdArgs& a = l.args;
   a.o_in = f->o;
   a.dout = p->dout;
@@ -485,6 +486,7 @@ int run_bwd(const fa_bwd_params* p, float* accum, int stage_mask, bool bind_cont
   a.dv_row_stride = p->dv_row_stride; a.dv_head_stride = p->dv_head_stride;
   a.softmax_d = p->softmax_d;
   a.dq_accum = accum;
+  a.one_launch = single;
   if (l.deterministic) {
     // ticket words sit behind the accumulator (fa_bwd_workspace_bytes_ex)
     const size_t off = fa_bwd_workspace_bytes(f->total_q, f->heads, f->head_dim);
@@ -507,12 +509,18 @@ int run_bwd(const fa_bwd_params* p, float* accum, int stage_mask, bool bind_cont
                              a.dk_row_stride, a.dk_head_stride, 32, bind_context, columns)) return rc;
   if (int rc = make_tile_map(&l.tm_dv, a.dv, l.is_bf16, f->total_k, f->heads, f->head_dim,
                              a.dv_row_stride, a.dv_head_stride, 32, bind_context, columns)) return rc;
-  if (int rc = make_accum_map(&l.tm_dq, a.dq_accum, f->total_q, f->heads, l.dpad)) return rc;
+  if (!single)
+    if (int rc = make_accum_map(&l.tm_dq, a.dq_accum, f->total_q, f->heads, l.dpad)) return rc;
   FA_CUDA(fa::launch_bwd(l, stream));
   return FA_OK;
 }
 
 }  // namespace
+
+int fa_bwd_needs_workspace(int32_t batch, int32_t heads, int32_t max_seqlen_q, int32_t max_seqlen_k, int32_t is_blocksparse,
+                           int32_t stage_mask) {
+  return fa::one_launch(max_seqlen_q, max_seqlen_k, static_cast<int64_t>(batch) * heads, is_blocksparse != 0, stage_mask) ? 0 : 1;
+}
 
 size_t fa_bwd_workspace_bytes_ex(int32_t total_q, int32_t heads, int32_t head_dim, int32_t batch,
                                  int32_t max_seqlen_q, int32_t deterministic) {
@@ -533,6 +541,13 @@ int fa_bwd(const fa_bwd_params* p, void* cuda_stream) {
     return fail(FA_ERR_WORKSPACE, "workspace must hold " + std::to_string(need) + " bytes");
   return run_bwd(p, static_cast<float*>(p->workspace), p->stage_mask, true,
                  static_cast<cudaStream_t>(cuda_stream));
+}
+
+int fa_bwd_one_launch(const fa_bwd_params* p, void* cuda_stream) {
+  FA_REQUIRE(p != nullptr, "params is null");
+  FA_REQUIRE(!fa_bwd_needs_workspace(p->fwd.batch, p->fwd.heads, p->fwd.max_seqlen_q, p->fwd.max_seqlen_k, p->fwd.blockmask != nullptr, p->stage_mask),
+             "fa_bwd_one_launch: this call needs a workspace (see fa_bwd_needs_workspace)");
+  return run_bwd(p, nullptr, 0, true, static_cast<cudaStream_t>(cuda_stream));
 }
 
 // ---------------------------------------------------------------------------------------------

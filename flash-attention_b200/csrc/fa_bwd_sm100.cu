@@ -116,6 +116,7 @@ struct BwdShared {
   uint64_t s_full;    // two-phase: S landed
   uint64_t p_ready;   // two-phase: P~ stored
   uint64_t ds_free;   // two-phase: dK and dQ have finished reading the dS buffer
+  uint64_t stat_ready;  // one launch: softmax_d is written
   uint64_t dq_group;  // rendezvous of the 128 threads of the dQ group (bounded, unlike bar.sync)
   uint32_t tmem_base;
   int abort_flag;
@@ -130,6 +131,26 @@ __device__ __forceinline__ uint32_t pack16(float lo, float hi) {
     __half2 v = __floats2half2_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
   }
+}
+
+// sum of the products of eight 16-bit values, in order
+template <bool BF16>
+__device__ __forceinline__ float dot8(const uint4& ov, const uint4& gv) {
+  const uint32_t ow[4] = {ov.x, ov.y, ov.z, ov.w}, gw[4] = {gv.x, gv.y, gv.z, gv.w};
+  float acc = 0.f;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    float2 of, gf;
+    if constexpr (BF16) {
+      of = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ow[k]));
+      gf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gw[k]));
+    } else {
+      of = __half22float2(*reinterpret_cast<const __half2*>(&ow[k]));
+      gf = __half22float2(*reinterpret_cast<const __half2*>(&gw[k]));
+    }
+    acc += of.x * gf.x + of.y * gf.y;
+  }
+  return acc;
 }
 
 template <int N>
@@ -151,7 +172,7 @@ __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.w
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 bool overlap_launches(const BwdLaunch& l) {
-  return l.stage_mask == 0 &&
+  return l.stage_mask == 0 && !l.args.one_launch &&
          static_cast<int64_t>((l.args.max_seqlen_k + kBN - 1) / kBN) * l.args.k.heads * l.args.k.batch > kSms;
 }
 
@@ -175,7 +196,8 @@ cudaError_t launch(bool overlap, void (*kernel)(P...), dim3 grid, int threads, i
 }
 
 // ------------------------------------------------------------------------------------------------
-template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BLOCKSPARSE>
+// ONE_LAUNCH: see one_launch()
+template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BLOCKSPARSE, bool ONE_LAUNCH>
 __global__ void __launch_bounds__(BwdCfg<D, BLOCKSPARSE, DROPOUT>::kThreads, 1)
 fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
               const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
@@ -229,7 +251,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     x.sk = ka.cu_seqlens_k[x.b + 1] - x.k_start;
     x.n0 = nt * kBN;
     const int m_tiles = (x.sq + kBM - 1) / kBM;
-    x.nm = x.n0 < x.sk ? m_tiles - (CAUSAL ? min(m_tiles, x.n0 / kBM) : 0) : 0;
+    // (a call of one launch also writes dq = 0 for a sequence without keys)
+    x.nm = x.n0 < x.sk || ONE_LAUNCH ? m_tiles - (CAUSAL ? min(m_tiles, x.n0 / kBM) : 0) : 0;
     return x;
   };
   grid_dep_launch();
@@ -241,7 +264,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   // a block behind its sequence's last key.  A CTA of its own leaves here, before it takes tensor memory and sets up its
   // barriers: 1 x 4096 and 63 x 128, 12 heads, deterministic, us, through the whole kernel -> here: 869 -> 642 (d = 64),
   // 1311 -> 1044 (d = 128)
-  if (!take_over && first.n0 >= first.sk) return;
+  if (!take_over && first.n0 >= first.sk && !ONE_LAUNCH) return;
   // fail fast: once a CTA of this launch has abandoned a wait, the blocks that have not started do not, whether a CTA of
   // their own or one that takes them over looks
   auto launch_failed = [&]() -> bool {
@@ -337,6 +360,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   if (tid == 0) {
     sh.abort_flag = 0;
     mbar_init(smem_u32(&sh.k_full), 1);
+    mbar_init(smem_u32(&sh.stat_ready), 4);
     mbar_init(smem_u32(&sh.v_full), 1);
     mbar_init(smem_u32(&sh.k_empty), 1);
     mbar_init(smem_u32(&sh.v_empty), 1);
@@ -704,6 +728,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     int32_t bs_nx = 0;
     bool fetched = false;
     auto fetch_stats = [&](const BlockInfo& x, int t) {
+      if (ONE_LAUNCH) ok = mbar_wait_warp(smem_u32(&sh.stat_ready), 0, abort_flag);
       const int64_t stats = (static_cast<int64_t>(x.b) * ka.heads + x.h) * ka.lse_stride;  // row of LSE and D
       const int i0 = q_tile(x, t) * kBM + (Cfg::kQuad ? (cwarp & 3) * 32 + (cwarp >> 3) * 16 : row);
 #pragma unroll
@@ -1203,11 +1228,67 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       int32_t* tk = ticket_row + m;
       asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(tk) : "memory");
     };
+    // One launch: softmax_d = p_keep * rowsum(dO * O), 32 rows a warp, in the order of bwd_preprocess_kernel.
+    auto write_d = [&](const BlockInfo& x) {
+      const int dlane = row & 31, tpr = ka.head_dim / 8, rows = 32 / tpr;
+      const int r0 = (row & ~31) + dlane / tpr;
+      const int64_t token = x.q_start + r0;
+      const uint16_t* o = reinterpret_cast<const uint16_t*>(a.o_in) + token * ka.o_row_stride + x.h * ka.o_head_stride + (dlane % tpr) * 8;
+      const uint16_t* dout = reinterpret_cast<const uint16_t*>(a.dout) + token * a.do_row_stride + x.h * a.do_head_stride + (dlane % tpr) * 8;
+      float* d = a.softmax_d + (static_cast<int64_t>(x.b) * ka.heads + x.h) * ka.lse_stride + r0;
+#pragma unroll 4
+      for (int i = 0; i < tpr; ++i) {
+        const bool valid = r0 + i * rows < x.sq;
+        float acc = 0.f;
+        if (valid)
+          acc = dot8<BF16>(*reinterpret_cast<const uint4*>(o + i * rows * ka.o_row_stride),
+                           *reinterpret_cast<const uint4*>(dout + i * rows * a.do_row_stride));
+        for (int off = tpr / 2; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
+        if (valid && dlane % tpr == 0) d[i * rows] = acc * a.p_keep;
+      }
+      __syncwarp();
+      if (dlane == 0) mbar_arrive(smem_u32(&sh.stat_ready));
+    };
+    // One launch: this warp's 32 rows of a dQ tile are all of dQ.
+    auto write_dq = [&](const BlockInfo& x) {
+      const int dlane = row & 31, r0 = row & ~31;
+      const float f = ka.scale * ka.rp_keep;
+      uint8_t* piece = dq_stage + (row >> 5) * 4096;
+      uint16_t* dst = reinterpret_cast<uint16_t*>(a.dq) + (x.q_start + r0) * a.dq_row_stride + x.h * a.dq_head_stride;
+#pragma unroll 1
+      for (int half = 0; half < D / 64; ++half) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t r[16];
+          tmem_ld16(tDQ + half * 64 + c * 16, r);
+          tmem_wait_ld();
+          uint32_t pk[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            pk[i] = x.sk > 0 ? pack_lowp<BF16>(__uint_as_float(r[2 * i]) * f, __uint_as_float(r[2 * i + 1]) * f) : 0;
+          *reinterpret_cast<uint4*>(piece + stage_offset<8>(dlane, 2 * c)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+          *reinterpret_cast<uint4*>(piece + stage_offset<8>(dlane, 2 * c + 1)) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+        }
+        __syncwarp();
+        stage_copy_out<8>(piece, dst + half * 64, a.dq_row_stride, x.sq - r0, ka.head_dim / 8 - half * 8, dlane);
+        __syncwarp();
+      }
+    };
     int g = 0;
     uint32_t k = 0;
     do {
     const BlockInfo& x = sh.blk[k & 1];  // read where it is used: the group has few registers
     const int nm = x.nm;
+    if constexpr (ONE_LAUNCH) {
+      if (nm <= 0) continue;
+      write_d(x);
+      ok = mbar_wait_warp(smem_u32(&sh.dq_full), 0, abort_flag);
+      if (ok) {
+        tc_fence_after();
+        write_dq(x);
+      }
+      continue;
+    }
     for (int t = 0; t < nm && ok; ++t, ++g) {
       const int m = q_tile(x, t), q_row = x.q_start + m * kBM, q_head = x.h;  // ahead of the waits
       ok = mbar_wait(smem_u32(&sh.dq_full), g & 1, abort_flag);
@@ -1343,19 +1424,7 @@ __global__ void bwd_preprocess_kernel(const BwdArgs a, int dpad) {
     // 16 x 12 x 1000 causal (d = 128) 253 -> 250, 32 x 12 x 512 185 -> 183)
     const uint4 ov = __ldcs(reinterpret_cast<const uint4*>(o));
     const uint4 gv = *reinterpret_cast<const uint4*>(g);
-    const uint32_t ow[4] = {ov.x, ov.y, ov.z, ov.w}, gw[4] = {gv.x, gv.y, gv.z, gv.w};
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      float2 of, gf;
-      if constexpr (BF16) {
-        of = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ow[k]));
-        gf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gw[k]));
-      } else {
-        of = __half22float2(*reinterpret_cast<const __half2*>(&ow[k]));
-        gf = __half22float2(*reinterpret_cast<const __half2*>(&gw[k]));
-      }
-      acc += of.x * gf.x + of.y * gf.y;
-    }
+    acc = dot8<BF16>(ov, gv);
     // zero this thread's share of the fp32 dQ accumulator row (dpad floats per (row, head))
     float* zr = a.dq_accum + (row * ka.heads + h) * dpad;
     for (int z = (threadIdx.x % tpr) * 4; z < dpad; z += tpr * 4)
@@ -1397,9 +1466,11 @@ __global__ void bwd_postprocess_kernel(const BwdArgs a, int dpad) {
   *reinterpret_cast<uint4*>(dst) = out;
 }
 
-template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BS>
+template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BS, bool ONE_LAUNCH = false>
 cudaError_t launch_main(const BwdLaunch& l, cudaStream_t stream) {
-  auto kernel = fa_bwd_kernel<D, BF16, CAUSAL, DROPOUT, BS>;
+  if constexpr (!BS && !ONE_LAUNCH)
+    if (l.args.one_launch) return launch_main<D, BF16, CAUSAL, DROPOUT, BS, true>(l, stream);
+  auto kernel = fa_bwd_kernel<D, BF16, CAUSAL, DROPOUT, BS, ONE_LAUNCH>;
   using Cfg = BwdCfg<D, BS, DROPOUT>;
   constexpr int smem = Cfg::kSmemBytes;
   static SmemLimitFlags smem_limit_set;  // one per template instantiation of this function
@@ -1438,7 +1509,7 @@ cudaError_t launch_bwd(const BwdLaunch& l, cudaStream_t stream) {
   const int d = a.k.head_dim;
   const int stages = l.stage_mask == 0 ? 7 : l.stage_mask;
   // 1. preprocess
-  if (stages & 1) {
+  if ((stages & 1) && !a.one_launch) {
     const int tpr = d / 8;
     const int threads = 256;
     const int rows_per_block = threads / tpr;
@@ -1465,7 +1536,7 @@ cudaError_t launch_bwd(const BwdLaunch& l, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
   }
   // 3. postprocess
-  if (stages & 4) {
+  if ((stages & 4) && !a.one_launch) {
     const int64_t total = static_cast<int64_t>(a.total_q) * a.k.heads * (d / 8);
     if (total > 0) {
       const int threads = 256;

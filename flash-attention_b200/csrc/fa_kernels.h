@@ -144,6 +144,9 @@ struct BwdArgs {
   // Deterministic mode: one ticket per (batch, head, 128-row query tile) = number of key tiles
   // that have added their dQ tile so far; nullptr = add in arrival order.
   int32_t* dq_tickets;
+  // One query and one key tile per sequence: a block's dQ is the whole of it, which goes straight to dq, and softmax_d is its own
+  // affair too; no accumulator, no other launch (see one_launch).
+  bool one_launch;
   bool take_over;  // the grid has more blocks than SMs: a CTA goes on with blocks that have not started
   int32_t ticket_stride;  // tickets per (batch, head): ceil(max_seqlen_q / 128)
   int32_t total_q, total_k, max_seqlen_q, max_seqlen_k;
@@ -184,6 +187,16 @@ bool decode_serves(const FwdLaunch& l);  // whether launch_decode takes the call
 cudaError_t launch_decode(const FwdLaunch& l, cudaStream_t stream);
 // Columns of dK and dV that a warp of the backward's epilogue stores at once (see its kBoxColumns).
 inline int grad_box_columns(int dpad, bool is_dropout) { return dpad == 64 && is_dropout ? 32 : 64; }
+// Whether the backward of a call is the main kernel alone, which then needs no workspace: one query tile, one key tile and no more
+// blocks than SMs.  Such calls wait for the host and for launches.  Backward on the device, us, three kernels -> one: 12 x 128
+// (d = 64) 19.5 -> 13.3, 12 x 12 x 128 causal (d = 128) 25.6 -> 19.4, 8 x 12 x 128 with dropout 23.5 -> 19.4; a training pass
+// of the last 66.5 -> 60.2.  softmax_d and dq, made beside each tile, are what the tile then waits for: with several query tiles
+// (12 x 2048 queries, 100 keys 44 -> 95) or more blocks than SMs (32 x 12 x 128 with dropout 34 -> 44) three kernels are
+// faster.  Block-sparse calls and single stages keep the three.
+constexpr int kOneLaunchBlocks = 148;
+inline bool one_launch(int max_seqlen_q, int max_seqlen_k, int64_t pairs, bool sparse, int stage_mask) {
+  return max_seqlen_q <= 128 && max_seqlen_k <= 128 && pairs <= kOneLaunchBlocks && !sparse && stage_mask == 0;
+}
 cudaError_t launch_bwd(const BwdLaunch& l, cudaStream_t stream);
 cudaError_t launch_sdmask(void* s_out, int64_t s_rows, int64_t s_cols, const void* q, const void* k,
                           int64_t q_row_stride, int64_t q_head_stride, int64_t k_row_stride,

@@ -279,12 +279,18 @@ struct BwdCall {
 void run_bwd(const Dims& s, const View& q, const View& k, const View& v, const at::Tensor& dout, const at::Tensor& out,
              const at::Tensor& lse, const View& dq, const View& dk, const View& dv, float* softmax_d,
              const at::Tensor& cu_q, const at::Tensor& cu_k, const at::Tensor* blockmask, const BwdCall& c) {
+  const bool scratch = fa_bwd_needs_workspace(static_cast<int32_t>(s.batch), static_cast<int32_t>(s.heads),
+                                              static_cast<int32_t>(c.max_q), static_cast<int32_t>(c.max_k), blockmask != nullptr ? 1 : 0,
+                                              static_cast<int32_t>(c.stage_mask)) != 0;
   // fp32 dQ accumulator (and the ticket words of the deterministic mode) from the caching allocator,
   // per call, like the reference's dq_tmp (:402-404)
-  const size_t nbytes = fa_bwd_workspace_bytes_ex(static_cast<int32_t>(s.total_q), static_cast<int32_t>(s.heads),
-                                                  static_cast<int32_t>(s.d), static_cast<int32_t>(s.batch),
-                                                  static_cast<int32_t>(c.max_q), c.deterministic ? 1 : 0);
-  at::Tensor ws = at::empty({static_cast<int64_t>(nbytes < 16 ? 16 : nbytes)}, lse.options().dtype(at::kByte));
+  at::Tensor ws;
+  if (scratch) {
+    const size_t nbytes = fa_bwd_workspace_bytes_ex(static_cast<int32_t>(s.total_q), static_cast<int32_t>(s.heads),
+                                                    static_cast<int32_t>(s.d), static_cast<int32_t>(s.batch),
+                                                    static_cast<int32_t>(c.max_q), c.deterministic ? 1 : 0);
+    ws = at::empty({static_cast<int64_t>(nbytes < 16 ? 16 : nbytes)}, lse.options().dtype(at::kByte));
+  }
   fa_bwd_params p = {};
   fill_fwd(p.fwd, s, q, k, v, out, lse, cu_q, cu_k, c.max_q, c.max_k, c.p_dropout, c.scale, c.causal, c.seed, c.offset,
            c.mask_heads_total, c.mask_head_offset, c.status_ptr);
@@ -296,8 +302,10 @@ void run_bwd(const Dims& s, const View& q, const View& k, const View& v, const a
   p.dq_row_stride = dq.row_stride; p.dq_head_stride = dq.head_stride;
   p.dk_row_stride = dk.row_stride; p.dk_head_stride = dk.head_stride;
   p.dv_row_stride = dv.row_stride; p.dv_head_stride = dv.head_stride;
-  p.workspace = ws.data_ptr();
-  p.workspace_bytes = static_cast<size_t>(ws.numel());
+  if (scratch) {
+    p.workspace = ws.data_ptr();
+    p.workspace_bytes = static_cast<size_t>(ws.numel());
+  }
   p.stage_mask = static_cast<int32_t>(c.stage_mask);
   p.deterministic = c.deterministic ? 1 : 0;
   at::Tensor bs_ws;
@@ -305,7 +313,8 @@ void run_bwd(const Dims& s, const View& q, const View& k, const View& v, const a
     check_blockmask(*blockmask, q, c.max_q, c.max_k);
     bs_ws = attach_blockmask(p.fwd, *blockmask, s.batch);
   }
-  check_rc(fa_bwd(&p, at::cuda::getCurrentCUDAStream().stream()));
+  const auto stream = at::cuda::getCurrentCUDAStream().stream();
+  check_rc(scratch ? fa_bwd(&p, stream) : fa_bwd_one_launch(&p, stream));
 }
 
 py::list bwd(const at::Tensor& dout, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,

@@ -21,6 +21,8 @@ EXPORTED_SYMBOLS = (
     "fa_fwd_ex",
     "fa_bwd",
     "fa_bwd_static_scratch",
+    "fa_bwd_needs_workspace",
+    "fa_bwd_one_launch",
     "fa_bwd_workspace_bytes",
     "fa_bwd_workspace_bytes_ex",
     "fa_blocksparse_workspace_bytes",
@@ -123,6 +125,10 @@ def _load():
     lib.fa_bwd.restype = ctypes.c_int
     lib.fa_bwd_static_scratch.argtypes = [ctypes.POINTER(BwdParams), ctypes.c_void_p]
     lib.fa_bwd_static_scratch.restype = ctypes.c_int
+    lib.fa_bwd_needs_workspace.argtypes = [ctypes.c_int32] * 6
+    lib.fa_bwd_needs_workspace.restype = ctypes.c_int
+    lib.fa_bwd_one_launch.argtypes = [ctypes.POINTER(BwdParams), ctypes.c_void_p]
+    lib.fa_bwd_one_launch.restype = ctypes.c_int
     lib.fa_bwd_workspace_bytes.argtypes = [ctypes.c_int32, ctypes.c_int32, ctypes.c_int32]
     lib.fa_bwd_workspace_bytes.restype = ctypes.c_size_t
     lib.fa_bwd_workspace_bytes_ex.argtypes = [ctypes.c_int32] * 6

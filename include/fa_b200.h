@@ -154,6 +154,13 @@ size_t fa_bwd_workspace_bytes(int32_t total_q, int32_t heads, int32_t head_dim);
 size_t fa_bwd_workspace_bytes_ex(int32_t total_q, int32_t heads, int32_t head_dim, int32_t batch,
                                  int32_t max_seqlen_q, int32_t deterministic);
 
+/* Whether a backward call uses the workspace: not with sequences of at most 128 queries and keys and 148 (batch, head) pairs, where
+ * dQ leaves the main kernel as it is.  fa_bwd asks for the workspace all the same; fa_bwd_one_launch is fa_bwd for the
+ * calls that use none (it refuses the others) and reads neither workspace nor workspace_bytes. */
+int fa_bwd_needs_workspace(int32_t batch, int32_t heads, int32_t max_seqlen_q, int32_t max_seqlen_k, int32_t is_blocksparse,
+                           int32_t stage_mask);
+int fa_bwd_one_launch(const fa_bwd_params* params, void* cuda_stream);
+
 /* Scratch a block-sparse call needs (fa_fwd_params.bs_workspace): one int32 per (batch entry,
  * blockmask row, blockmask column).  The reference keeps this walk implicit in its kernels
  * (csrc/flash_attn/src/fmha_block_fprop_kernel_1xN.h:205-232). */
