@@ -898,10 +898,14 @@ cudaError_t launch_groups(const FwdLaunch& l, cudaStream_t stream) {
 //   1024, 1024                0.91           0.93            0.98            0.96
 //   1024, 8192                1.02           1.02            1.14            1.13
 //   4096, 4096 (4 x 16)       0.96           0.99            1.13            1.10
-// so d = 64 takes single tiles at every length (causal calls too: 0.95-0.98), and d = 128 up to 1024 queries and keys
-// (causal calls count the keys up to the longest query).  d = 128 with dropout, 12 heads, 64 x 300 (an odd number of tiles)
-// 164 -> 130 us, 64 x 256 92 -> 80, 32 x 512 ragged 107 -> 92, 16 x 1000 199 -> 178, causal 139 -> 123; 16 x 16 heads, 300
-// queries, 900 keys 115 -> 99, 256 queries, 1024 keys 73 -> 71.
+// so d = 64 takes single tiles at every length (causal calls too: 0.95-0.98).  (The table was taken before the first loads moved
+// ahead of the set-up and the output rows into shared memory, which made single tiles cheaper.)
+// d = 128, one / two now: up to 1024 keys (causal calls count those up to the longest query) 0.91-0.99 (12 heads of 16 sequences:
+// 2000 queries, 256 keys 138 -> 126 us, 8 of 4096 and 512 148 -> 146; dropout 171 -> 156, 201 -> 183).  Beyond, causal:
+// 1100 tokens 0.87, 1300 0.9, 1800 0.92, 2000 0.97, 2500 0.99, 3000 1.00, 4096 1.02, with dropout 2000 0.93, 4096 0.98, 8192 1.03.
+// Not causal: 1500 1.04, 2000 0.99, 4096 1.02, 1024 queries and 2048 keys 1.06, but an odd number of query tiles leaves half of
+// a pair empty: 384 queries, 2048 keys 0.88, 1100 tokens 0.93, 1800 0.95.  Not causal with dropout: 1500 0.99, 3000 1.00, 4096 0.94,
+// 8192 0.95, 384 queries and 2048 keys 0.87; few queries and many keys (256 and 4096, 1024 and 8192) 1.01-1.02.
 // A grid of single tiles that fits one per SM spreads over twice the SMs: 16 heads, 1024 queries, 8192 keys 0.72 (d = 64),
 // 0.92 (d = 128), 0.63 and 0.78 with dropout.
 // A grid of pairs that fills between half of the SMs and all of them runs in one round either way and reads K and
@@ -911,19 +915,26 @@ cudaError_t launch_groups(const FwdLaunch& l, cudaStream_t stream) {
 // share an SM: 192 pairs 85 us, 128 with two.
 // Uneven batches (see `uneven`) announced with more than 4096 tokens take pairs at d = 64 too, which halves their empty blocks:
 // 31 x 256 and 1 x 8192, 12 heads 405 -> 363 us, 2 x 16384 and 126 x 64, 4 heads 935 -> 843.
-constexpr int kOneTileMaxD128 = 1024, kOneTileMaxUneven = 4096;  // queries and keys
+constexpr int kOneTileMaxD128 = 1024, kOneTileMaxOdd = 2048, kOneTileMaxCausal = 2560, kOneTileMaxCausalDropout = 4096;  // keys
+constexpr int kOneTileMaxUneven = 4096;  // queries and keys, d = 64
 
 template <int D, bool CAUSAL, bool DROPOUT>
 bool one_tile_per_cta(const FwdLaunch& l) {
   const int64_t heads = static_cast<int64_t>(l.args.heads) * l.args.batch;
-  const int64_t tiles = (l.max_seqlen_q + kBlockM - 1) / kBlockM * heads;
-  const int64_t pairs = (l.max_seqlen_q + 2 * kBlockM - 1) / (2 * kBlockM) * heads;
+  const int64_t q_tiles = (l.max_seqlen_q + kBlockM - 1) / kBlockM;
+  const int64_t tiles = q_tiles * heads, pairs = (q_tiles + 1) / 2 * heads;
   const int keys = CAUSAL ? min(l.max_seqlen_k, l.max_seqlen_q) : l.max_seqlen_k;
   const bool one_round = pairs > kSms / 2 && pairs <= kSms;
   if (l.max_seqlen_q <= kBlockM) return D == 64 || DROPOUT || keys <= kOneTileMaxD128 || pairs > kSms;
   if (one_round) return false;
   if (D == 64) return !(uneven(l) && max(l.max_seqlen_q, keys) > kOneTileMaxUneven);
-  return l.max_seqlen_q <= kOneTileMaxD128 && (tiles <= kSms || keys <= kOneTileMaxD128);
+  if (l.max_seqlen_q <= kOneTileMaxD128 && (tiles <= kSms || keys <= kOneTileMaxD128)) return true;
+  if (uneven(l)) return false;  // (twice the empty blocks)
+  if (keys <= kOneTileMaxD128) return true;
+  if (CAUSAL) return keys <= (DROPOUT ? kOneTileMaxCausalDropout : kOneTileMaxCausal);
+  const bool odd = q_tiles % 2 != 0;
+  if (DROPOUT) return odd || l.max_seqlen_q > kOneTileMaxD128;
+  return odd && max(l.max_seqlen_q, keys) <= kOneTileMaxOdd;
 }
 
 // Rows for d = 128 without dropout, and for d = 64 without dropout up to 512 keys: there the ends of a CTA's
