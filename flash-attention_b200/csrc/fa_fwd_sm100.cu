@@ -355,9 +355,9 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 
       bool ok = true;
       for (int g = 0; g < G && ok; ++g)
-        if (n_tiles[g] > 0) ok = mbar_wait_warp(smem_u32(&sh.q_full[g]), 0, abort_flag);
+        if (n_tiles[g] > 0) ok = mbar_wait_warp<true>(smem_u32(&sh.q_full[g]), 0, abort_flag);
       if (ok && n_max > 0) {
-        ok = mbar_wait_warp(smem_u32(&sh.k_full[0]), 0, abort_flag);
+        ok = mbar_wait_warp<true>(smem_u32(&sh.k_full[0]), 0, abort_flag);
         if (ok) {
           tc_fence_after();
 #pragma unroll
@@ -370,7 +370,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         const int s = j % Cfg::kStages;
         const int sn = (j + 1) % Cfg::kStages;
         const bool has_next = j + 1 < n_max;
-        auto wait_k = [&]() { ok = mbar_wait_warp(smem_u32(&sh.k_full[sn]), ((j + 1) / Cfg::kStages) & 1, abort_flag); };
+        auto wait_k = [&]() { ok = mbar_wait_warp<true>(smem_u32(&sh.k_full[sn]), ((j + 1) / Cfg::kStages) & 1, abort_flag); };
         if constexpr (Cfg::kSeparateP) {
           // this warp issues only the score products; the next one issues P*V
           if (has_next) wait_k();
@@ -378,7 +378,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 #pragma unroll
           for (int g = 0; g < G; ++g) {
             if (ok && j + 1 < n_tiles[g]) {
-              ok = mbar_wait_warp(smem_u32(&sh.s_free[g]), j & 1, abort_flag);
+              ok = mbar_wait_warp<true>(smem_u32(&sh.s_free[g]), j & 1, abort_flag);
               if (ok) {
                 tc_fence_after();
                 issue_qk(g, sn);
@@ -387,7 +387,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           }
           if (!ok) break;
         } else {
-          ok = mbar_wait_warp(smem_u32(&sh.v_full[s]), (j / Cfg::kStages) & 1, abort_flag);
+          ok = mbar_wait_warp<true>(smem_u32(&sh.v_full[s]), (j / Cfg::kStages) & 1, abort_flag);
           if (PADDED && ok && (j + 1) * kBlockN > sk)
             clear_v_rows<Cfg::kPanels>(smem + (smem_v - smem_q) + s * Cfg::kTileBytes, sk - j * kBlockN, lane);
           // K of the next tile is waited for behind P V of this one, which does not need it (its load takes about 2000 clk where
@@ -398,13 +398,13 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             if (ok && j < n_tiles[g]) {
               constexpr int kFirst = Cfg::kHalfP ? kBlockN / 32 : 0;
               if constexpr (Cfg::kHalfP) {
-                ok = mbar_wait_warp(smem_u32(&sh.p_half[g]), j & 1, abort_flag);
+                ok = mbar_wait_warp<true>(smem_u32(&sh.p_half[g]), j & 1, abort_flag);
                 if (ok) {
                   tc_fence_after();
                   issue_pv(g, s, j > 0, 0, kFirst);
                 }
               }
-              if (ok) ok = mbar_wait_warp(smem_u32(&sh.p_full[g]), j & 1, abort_flag);
+              if (ok) ok = mbar_wait_warp<true>(smem_u32(&sh.p_full[g]), j & 1, abort_flag);
               if (ok) {
                 tc_fence_after();
                 issue_pv(g, s, j > 0, kFirst, kBlockN / 16);
@@ -433,7 +433,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       bool ok = true;
       for (int j = 0; j < n_max && ok; ++j) {
         const int s = j % Cfg::kStages;
-        ok = mbar_wait_warp(smem_u32(&sh.v_full[s]), (j / Cfg::kStages) & 1, abort_flag);
+        ok = mbar_wait_warp<true>(smem_u32(&sh.v_full[s]), (j / Cfg::kStages) & 1, abort_flag);
         if (!ok) break;
         if (PADDED && (j + 1) * kBlockN > sk)
           clear_v_rows<Cfg::kPanels>(smem + (smem_v - smem_q) + s * Cfg::kTileBytes, sk - j * kBlockN, lane);
@@ -441,7 +441,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 #pragma unroll
         for (int g = 0; g < G; ++g) {
           if (ok && j < n_tiles[g]) {
-            ok = mbar_wait_warp(smem_u32(&sh.p_full[g]), j & 1, abort_flag);
+            ok = mbar_wait_warp<true>(smem_u32(&sh.p_full[g]), j & 1, abort_flag);
             if (ok) {
               tc_fence_after();
               const uint32_t tO = tmem + (g == 0 ? Cfg::kTmemO0 : Cfg::kTmemO1);
@@ -486,8 +486,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         bs_it = (ig >> 4) < a.bs_rows16
                     ? a.bs_iter[(static_cast<int64_t>(b) * a.bs_kblocks + (col0 >> 8)) * a.bs_rows16 + (ig >> 4)]
                     : -1;
-      ok = mbar_wait(smem_u32(&sh.s_full[g]), j & 1, abort_flag);
-      ok = __all_sync(0xffffffffu, ok);
+      ok = mbar_wait_warp<true>(smem_u32(&sh.s_full[g]), j & 1, abort_flag);
       if (!ok) break;
       tc_fence_after();
       uint32_t sr[4][32];
@@ -564,8 +563,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       // P*V of the previous tile must have finished before O is rescaled or its P buffer reused.  (Half of the
       // exponentials are still to come: by now it has, as a rule.)
       if (j > 0) {
-        ok = mbar_wait(smem_u32(&sh.o_full[g]), (j - 1) & 1, abort_flag);
-        ok = __all_sync(0xffffffffu, ok);
+        ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), (j - 1) & 1, abort_flag);
         if (!ok) break;
         tc_fence_after();
         if (__any_sync(0xffffffffu, grow)) {
@@ -608,8 +606,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     // ---------------- epilogue: O = acc / (sum * p_keep), LSE
     if (active) {
       if (n > 0 && ok) {
-        ok = mbar_wait(smem_u32(&sh.o_full[g]), (n - 1) & 1, abort_flag);
-        ok = __all_sync(0xffffffffu, ok);
+        ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), (n - 1) & 1, abort_flag);
         tc_fence_after();
       }
       // every product that reads this group's Q has finished: its tile takes the output
@@ -677,7 +674,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           if (!valid) s[i] = __float_as_uint(-INFINITY);
         }
       };
-      ok = mbar_wait_warp(smem_u32(&sh.s_full[g]), j & 1, abort_flag);
+      ok = mbar_wait_warp<true>(smem_u32(&sh.s_full[g]), j & 1, abort_flag);
       if (!ok) break;
       tc_fence_after();
       uint32_t sr[64];
@@ -716,7 +713,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         }
         if (j > 0) {
           // P*V of the previous tile must have finished before O is rescaled
-          ok = mbar_wait_warp(smem_u32(&sh.o_full[g]), (j - 1) & 1, abort_flag);
+          ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), (j - 1) & 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
           const uint64_t al[2] = {pack_f2(alpha[0], alpha[0]), pack_f2(alpha[1], alpha[1])};
@@ -798,7 +795,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         }
         if (half == 0 && j > 0) {
           // P*V of the previous tile must have finished before its P buffer is reused
-          ok = mbar_wait_warp(smem_u32(&sh.o_full[g]), (j - 1) & 1, abort_flag);
+          ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), (j - 1) & 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
         }
@@ -830,7 +827,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       }
       named_barrier_sync(1 + g, 32 * Cfg::kGroupWarps);  // every warp of the group comes here, also after an abandoned wait
       if (n > 0 && ok) {
-        ok = mbar_wait_warp(smem_u32(&sh.o_full[g]), (n - 1) & 1, abort_flag);
+        ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), (n - 1) & 1, abort_flag);
         tc_fence_after();
       }
       const float2 st = sh.row_stats[g][wq * 32 + lane];
