@@ -370,6 +370,10 @@ static int run_fwd(const fa_fwd_params* p, bool zero_unused, const int32_t* boun
                              p->k_row_stride, p->k_head_stride, 128)) return rc;
   if (int rc = make_tile_map(&l.tm_v, p->v, l.is_bf16, p->total_k, p->heads, p->head_dim,
                              p->v_row_stride, p->v_head_stride, 128)) return rc;
+  const bool decode = !bounds && fa::decode_serves(l);
+  if (!decode)
+    if (int rc = make_tile_map(&l.tm_o, p->o, l.is_bf16, p->total_q, p->heads, p->head_dim, p->o_row_stride, p->o_head_stride,
+                               32, true, fa::out_box_columns(l))) return rc;
   if (bounds) {
     l.args.cu_seqlens_q = l.args.cu_seqlens_k = bounds;
     l.args.pad_rows = p->max_seqlen_q;
@@ -379,7 +383,7 @@ static int run_fwd(const fa_fwd_params* p, bool zero_unused, const int32_t* boun
   // A few query rows per sequence: the decoding kernel where it is the faster one.  Dropout and block-sparse
   // calls keep the tile kernel (their mask is tied to its tiles), and so do causal ones, which see no more
   // keys than they have query rows.
-  if (fa::decode_serves(l)) {
+  if (decode) {
     l.decode = fa::DecodeArgs{p->q, p->k, p->v, p->q_row_stride, p->q_head_stride, p->k_row_stride, p->k_head_stride,
                               p->v_row_stride, p->v_head_stride, p->total_q, p->total_k};
     FA_CUDA(fa::launch_decode(l, static_cast<cudaStream_t>(cuda_stream)));

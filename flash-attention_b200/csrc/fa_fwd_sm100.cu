@@ -97,7 +97,7 @@ __device__ __forceinline__ void reg_dealloc() {
 // gets zeros and -inf.  `piece`: the warp's NC * 2048 bytes of shared memory, for the way out (see stage_offset).
 // ig: first query row of the warp.
 template <bool BF16, int NC>
-__device__ __forceinline__ void store_rows(const KernelArgs& a, uint32_t tO, int c0, bool have_acc, bool ok, int ig, int lane,
+__device__ __forceinline__ void store_rows(const KernelArgs& a, const CUtensorMap* tm_o, uint32_t tO, int c0, bool have_acc, bool ok, int ig, int lane,
                                            int sq, int q_start, int b, int h, float m_run, float l_run, uint8_t* piece) {
   constexpr int CH = NC == 1 ? 4 : 8;  // 16-byte chunks of a row in one panel of the piece
   const bool bad_sum = (l_run == 0.f) || (l_run != l_run);
@@ -122,17 +122,31 @@ __device__ __forceinline__ void store_rows(const KernelArgs& a, uint32_t tO, int
       *reinterpret_cast<uint4*>(panel + stage_offset<CH>(lane, (i & 1) * 4 + v)) = make_uint4(w[0], w[1], w[2], w[3]);
     }
   }
+  fence_async_smem();
   __syncwarp();
   if (!ok) return;
+  if (ig + lane < sq && c0 == 0) {
+    const float lse = bad_sum ? -INFINITY : (m_run * a.scale + __logf(l_run));
+    a.lse[(static_cast<int64_t>(b) * a.heads + h) * a.lse_stride + ig + lane] = lse;
+  }
+  // Whole rows by TMA (by the LSU before: 64 x 12 x 512, d = 64, 104.4 us, now 102.4; d = 128: 32 x 12 x 300 causal 51.2 -> 49.2,
+  // 32 x 12 x 512 84 -> 81, 4 x 32 x 3000 causal 342 -> 335).  The warp that holds the sequence's end stores its rows itself: those
+  // behind it are the next sequence's.
+  if (ig + 32 <= sq) {
+    if (lane == 0) {
+#pragma unroll
+      for (int p = 0; p < (NC + 1) / 2; ++p)
+        if (c0 * 32 + p * 64 < a.head_dim) tma_store_3d(tm_o, smem_u32(piece) + p * 4096, c0 * 32 + p * 64, q_start + ig, h);
+      bulk_commit();
+      bulk_wait_read();
+    }
+    return;
+  }
   uint16_t* orow = reinterpret_cast<uint16_t*>(a.o) + static_cast<int64_t>(q_start + ig) * a.o_row_stride +
                    static_cast<int64_t>(h) * a.o_head_stride + c0 * 32;
 #pragma unroll
   for (int p = 0; p < (NC + 1) / 2; ++p)
     stage_copy_out<CH>(piece + p * 4096, orow + p * 64, a.o_row_stride, sq - ig, a.head_dim / 8 - c0 * 4 - p * 8, lane);
-  if (ig + lane < sq && c0 == 0) {
-    const float lse = bad_sum ? -INFINITY : (m_run * a.scale + __logf(l_run));
-    a.lse[(static_cast<int64_t>(b) * a.heads + h) * a.lse_stride + ig + lane] = lse;
-  }
 }
 
 // Padded batches.  A V tile that reaches behind its sequence's last token holds whatever the padding holds, and its
@@ -165,7 +179,7 @@ __device__ __forceinline__ void zero_padding(const KernelArgs& a, int b, int h, 
 template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BLOCKSPARSE, int G, bool ROWS, bool ORDERED, bool PADDED>
 __global__ void __launch_bounds__(FwdCfg<D, G, ROWS>::kThreads, G == 1 ? 2 : 1)
 fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-              const __grid_constant__ CUtensorMap tm_v, const KernelArgs a) {
+              const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const KernelArgs a) {
   using Cfg = FwdCfg<D, G, ROWS>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ FwdShared sh;
@@ -610,7 +624,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         tc_fence_after();
       }
       // every product that reads this group's Q has finished: its tile takes the output
-      store_rows<BF16, D / 32>(a, tO, 0, n > 0 && ok, ok, m0[g] + (warp & 3) * 32, lane, sq, q_start, b, h, m_run, l_run,
+      store_rows<BF16, D / 32>(a, &tm_o, tO, 0, n > 0 && ok, ok, m0[g] + (warp & 3) * 32, lane, sq, q_start, b, h, m_run, l_run,
                                smem + g * Cfg::kTileBytes + (warp & 3) * (D * 64));
     }
   } else if (warp < Cfg::kSoftmaxWarps) {
@@ -831,7 +845,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         tc_fence_after();
       }
       const float2 st = sh.row_stats[g][wq * 32 + lane];
-      store_rows<BF16, D / 64>(a, tO - (static_cast<uint32_t>(hh * 16) << 16), hh * (D / 64), n > 0 && ok, ok,
+      store_rows<BF16, D / 64>(a, &tm_o, tO - (static_cast<uint32_t>(hh * 16) << 16), hh * (D / 64), n > 0 && ok, ok,
                                m_first + wq * 32, lane, sq, q_start, b, h, st.x, st.y,
                                smem + g * Cfg::kTileBytes + (wq * 2 + hh) * (D * 32));
     }
@@ -880,7 +894,7 @@ cudaError_t launch_groups(const FwdLaunch& l, cudaStream_t stream) {
     set_tail_grid(&args, grid.x, int64_t(4) * D * l.max_seqlen_k);  // K and V
     grid = dim3(grid.x * grid.y * grid.z, 1, 1);
   }
-  kernel<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(l.tm_q, l.tm_k, l.tm_v, args);
+  kernel<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(l.tm_q, l.tm_k, l.tm_v, l.tm_o, args);
   return cudaGetLastError();
 }
 
@@ -969,6 +983,10 @@ cudaError_t launch_d(const FwdLaunch& l, cudaStream_t stream) {
 }
 
 }  // namespace
+
+int out_box_columns(const FwdLaunch& l) {
+  return l.dpad == 64 && (l.is_dropout || l.max_seqlen_k > kRowsMaxD64) ? 32 : 64;  // quads: half of a row a warp
+}
 
 cudaError_t launch_fwd(const FwdLaunch& l, cudaStream_t stream) {
   if (l.args.bs_iter != nullptr) {

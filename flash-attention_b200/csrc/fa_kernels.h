@@ -163,6 +163,7 @@ struct DecodeArgs {
 
 struct FwdLaunch {
   CUtensorMap tm_q, tm_k, tm_v;
+  CUtensorMap tm_o;  // output, boxes of 32 rows and out_box_columns columns
   KernelArgs args;
   DecodeArgs decode;
   int32_t max_seqlen_q, max_seqlen_k, total_q;
@@ -182,6 +183,7 @@ struct BwdLaunch {
 };
 
 cudaError_t launch_fwd(const FwdLaunch& l, cudaStream_t stream);
+int out_box_columns(const FwdLaunch& l);  // of the output that a warp of the tile kernel stores at once
 cudaError_t launch_fwd_padded(const FwdLaunch& l, cudaStream_t stream);
 bool decode_serves(const FwdLaunch& l);  // whether launch_decode takes the call (l.decode apart)
 cudaError_t launch_decode(const FwdLaunch& l, cudaStream_t stream);
