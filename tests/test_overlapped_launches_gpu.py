@@ -1,0 +1,70 @@
+"""The backward's three kernels overlap at their ends (programmatic dependent launch, grids of more blocks than SMs): the same
+results in a captured graph, on new inputs, and with calls on two streams at once.  The deterministic mode makes dq
+comparable bit for bit."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _call(batch, seqlen, heads, d, dtype, causal, p, seed):
+    from flash_attn_b200 import flash_attn_cuda as fc
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    cu = torch.arange(0, (batch + 1) * seqlen, seqlen, dtype=torch.int32, device="cuda")
+    q, k, v, dout = (torch.randn(batch * seqlen, heads, d, device="cuda", generator=g).to(dtype) for _ in range(4))
+    out, lse, seed, offset = fc.fwd(q, k, v, cu, cu, seqlen, seqlen, p, d ** -0.5, False, causal, False, g, return_philox=True)
+    grads = [torch.empty_like(x) for x in (q, k, v)]
+
+    def backward():
+        fc.bwd(dout, q, k, v, out, lse, *grads, cu, cu, seqlen, seqlen, p, d ** -0.5, False, causal, None, philox=(seed, offset))
+        return grads
+    return backward, dout
+
+
+CASES = [(4, 700, 12, 64, torch.float16, False, 0.1), (4, 515, 12, 64, torch.bfloat16, True, 0.0),
+         (3, 640, 12, 128, torch.bfloat16, True, 0.0), (20, 130, 8, 64, torch.float16, False, 0.0)]
+
+
+@pytest.fixture
+def deterministic():
+    from flash_attn_b200 import flash_attn_cuda as fc
+    fc.options.deterministic = True
+    yield
+    fc.options.deterministic = False
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_backward_in_a_captured_graph(deterministic, case):
+    backward, dout = _call(*case, seed=1)
+    first = [x.clone() for x in backward()]
+    new = torch.randn(dout.shape, device="cuda", generator=torch.Generator(device="cuda").manual_seed(2)).to(dout.dtype)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = backward()
+    for x in captured:
+        x.zero_()
+    graph.replay()
+    for a, b in zip(captured, first):
+        assert torch.equal(a, b)
+    dout.copy_(new)
+    for _ in range(3):
+        graph.replay()
+    got = [x.clone() for x in captured]
+    for a, b in zip(got, backward()):
+        assert torch.equal(a, b)
+
+
+def test_backward_on_two_streams(deterministic):
+    calls = [_call(*case, seed=3)[0] for case in CASES[:2]]
+    want = [[x.clone() for x in call()] for call in calls]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    got = [[], []]
+    for _ in range(10):
+        for i, (call, stream) in enumerate(zip(calls, streams)):
+            with torch.cuda.stream(stream):
+                got[i] = call()
+    torch.cuda.synchronize()
+    for a, b in zip(got, want):
+        for x, y in zip(a, b):
+            assert torch.equal(x, y)
