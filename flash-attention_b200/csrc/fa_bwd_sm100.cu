@@ -166,9 +166,10 @@ __device__ __forceinline__ void reg_dealloc() {
 // first tiles while the last blocks of the preprocess run, and the postprocess is on the SMs when the last main CTA
 // leaves.  What a kernel takes from the one before it (softmax_d, the cleared accumulator, tickets | the accumulator) comes behind
 // grid_dep_wait, which waits for all of that kernel's blocks and their writes.  Whole backward with its autograd call, us,
-// before -> now: 8 x 12 x 512 with dropout 51 -> 49, 16 x 12 x 1024 187 -> 183, 64 x 12 x 512 244 -> 241; the
-// preprocess behind whatever is ahead of it: training passes of 16 x 8 heads, 200 queries, 1500 keys 80.6 -> 78.4, 8 x 12 x 512 67.6 -> 66.4.  A launch of this kind takes the
-// host longer, so grids that leave SMs idle, whose calls wait for the host, keep ordinary ones (8 x 12 x 128: 21.5 -> 25.8).
+// before -> now: 8 x 12 x 512 with dropout 51 -> 49, 16 x 12 x 1024 187 -> 183, 64 x 12 x 512 244 -> 241; the preprocess behind
+// whatever is ahead of it: training passes of 16 x 8 heads, 200 queries, 1500 keys 80.6 -> 78.4, 8 x 12 x 512 67.6 -> 66.4.
+// A launch of this kind takes the host longer, so grids that leave SMs idle, whose calls wait for the host, keep ordinary ones
+// (8 x 12 x 128: 21.5 -> 25.8).
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
