@@ -56,10 +56,13 @@ class FlashAttention(nn.Module):
             return out.reshape(batch, seqlen, heads, d), None
 
         mask = _mask_matrix(key_padding_mask)
-        # without gradient and dropout: on the batch as it stands
-        native = flash_attn_cuda.compiled_attention(qkv) if p == 0.0 and runs_now(qkv) and runs_now(mask) else None
+        native = flash_attn_cuda.compiled_attention(qkv) if runs_now(qkv) and runs_now(mask) else None
         if native is not None:
-            out = native.attn_padded_qkv(qkv, mask, self.softmax_scale, bool(causal))
+            # without gradient and dropout: on the batch as it stands, else the three steps below as one function
+            if p == 0.0 and not (torch.is_grad_enabled() and qkv.requires_grad):
+                out = native.attn_padded_qkv(qkv, mask, self.softmax_scale, bool(causal))
+            else:
+                out = native.attn_padded_train(qkv, mask, float(p), self.softmax_scale, bool(causal))
             if out is not None:
                 return out, None
         x_unpad, indices, cu, max_len = unpad_input(qkv.reshape(batch, seqlen, three * heads * d), mask)

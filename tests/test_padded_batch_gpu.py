@@ -75,6 +75,51 @@ def test_masks_with_holes_and_calls_left_to_the_packed_way():
         assert torch.all(got[~holes] == 0) and float((got.double() - want).abs().max()) <= 2 ** -10 * float(qkv.abs().max())
     assert native.attn_padded_qkv(qkv, torch.zeros_like(mask), None, False) is None  # no token at all: refused by the packed way
     assert native.attn_padded_qkv(qkv.clone().requires_grad_(), mask, None, False) is None
+    assert native.attn_padded_train(qkv, torch.zeros_like(mask), 0.1, None, False) is None
     assert native.attn_padded_qkv(qkv, mask.int(), None, False) is None
     assert native.attn_padded_qkv(qkv[:, :, :, :, :32], mask, None, False) is None  # not contiguous
     assert native.attn_padded_qkv(qkv.bfloat16(), mask, None, False) is None
+
+
+@pytest.mark.parametrize("batch,seqlen,heads,d,causal,kind,p", [
+    (3, 40, 2, 64, False, "back", 0.0), (5, 128, 12, 64, False, "front", 0.1), (4, 300, 3, 32, True, "both", 0.1),
+    (4, 520, 2, 128, False, "back", 0.2), (3, 257, 4, 64, True, "holes", 0.0)])
+@pytest.mark.parametrize("compiled_autograd", [False, True])
+def test_training_equals_the_three_functions(batch, seqlen, heads, d, causal, kind, p, compiled_autograd):
+    """Output, gradient and generator state, bit for bit (dq in the deterministic mode)."""
+    from flash_attn_b200 import flash_attn_cuda as fc
+    from flash_attn_b200.bert_padding import pad_input, unpad_input
+    from flash_attn_b200.flash_attention import FlashAttention
+    from flash_attn_b200.flash_attn_interface import flash_attn_unpadded_qkvpacked_func
+    g = torch.Generator(device="cuda").manual_seed(seqlen)
+    qkv = torch.randn(batch, seqlen, 3, heads, d, device="cuda", generator=g).half().requires_grad_()
+    dout = torch.randn(batch, seqlen, heads, d, device="cuda", generator=g).half()
+    mask = _mask("back" if kind == "holes" else kind, batch, seqlen, seqlen)
+    if kind == "holes":
+        mask[0, 3::7] = False
+
+    def three():
+        x, idx, cu, longest = unpad_input(qkv.reshape(batch, seqlen, -1), mask)
+        o = flash_attn_unpadded_qkvpacked_func(x.reshape(-1, 3, heads, d), cu, longest, p, causal=causal)
+        return pad_input(o.reshape(-1, heads * d), idx, batch, seqlen).reshape(batch, seqlen, heads, d)
+
+    attn = FlashAttention(attention_dropout=p).train()
+    state = torch.cuda.get_rng_state()
+    fc.options.deterministic = True
+    try:
+        got = []
+        for f in (lambda: attn(qkv, key_padding_mask=mask, causal=causal)[0], three):
+            torch.cuda.manual_seed(7)
+            out = f().mul_(1)  # (the output may be changed in place)
+            if compiled_autograd and not got:
+                with torch._dynamo.compiled_autograd._enable(torch.compile(backend="eager")):
+                    out.backward(dout)
+                grad, qkv.grad = qkv.grad, None
+            else:
+                grad, = torch.autograd.grad(out, qkv, dout)
+            got.append((out.detach(), grad, torch.cuda.get_rng_state()))
+    finally:
+        fc.options.deterministic = False
+        torch.cuda.set_rng_state(state)
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
