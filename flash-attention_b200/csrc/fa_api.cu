@@ -69,6 +69,9 @@ int make_tile_map(CUtensorMap* tm, const void* base, bool bf16, int64_t rows, in
   FA_REQUIRE((reinterpret_cast<uintptr_t>(base) & 15) == 0, "tensor base must be 16-byte aligned");
   FA_REQUIRE((row_stride * 2) % 16 == 0 && (head_stride * 2) % 16 == 0,
              "row and head strides must be multiples of 8 elements");
+  // the stride of a dimension of one element, which addresses nothing, may be anything (0, too, which the driver refuses)
+  if (rows == 1) row_stride = static_cast<int64_t>(heads) * head_dim;
+  if (heads == 1) head_stride = head_dim;
   // A descriptor is a pure function of these nine values, and a training loop presents the same
   // ones again and again (the caching allocator hands back the same blocks): a small per-thread
   // cache saves the driver call, which is a large share of the host time of a short-sequence call.

@@ -6,7 +6,7 @@
 //   first    TMA producer (Q once, K/V ring)
 //   second   tcgen05.mma issuer (d = 128: every product; d = 64: S = Q K^T only)
 //   third    d = 64: second issuer, O += P V (two issuers keep S ahead)
-//   fourth   idle
+//   fourth   padded batches: zeros in the output rows without a token; else idle
 // Tensor memory per query tile: 128 columns of fp32 scores S, D of fp32 output O, and at d = 64 64 of the 16-bit
 // probabilities P, which feed the P*V product straight from tensor memory.  At d = 128 P overwrites the first 64
 // columns of S; at d = 64 the next score product starts as soon as the group has read its scores.

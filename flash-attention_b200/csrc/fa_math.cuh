@@ -56,7 +56,8 @@ __device__ __forceinline__ uint32_t pack_lowp(float lo, float hi) {
 
 // A tile of 32 rows whose threads hold one row each leaves through shared memory: stored straight from the registers, every
 // 16-byte store of a warp touches 32 rows, one L1 tag cycle each.  The rows are put in a warp's own piece of shared memory
-// (32 rows of CH 16-byte chunks, swizzled so that neither side has bank conflicts) and read back CH lanes to a row.  dK and dV
+// (32 rows of CH 16-byte chunks, in the 64- or 128-byte swizzle of a tensor map: neither side has bank conflicts) and leave by
+// TMA, or read back CH lanes to a row where TMA would write rows that are not the warp's.  dK and dV
 // of a block of 128 keys: 4096 (d = 128) and 2048 (d = 64) tag cycles -> 512 and 256, which counts where a block has few query
 // tiles.  Whole backward, us, before -> now: 64 x 12 x 512 (d = 64) 305 -> 278, 16 x 12 x 1024 230 -> 218, 8 x 12 x 4096 1185
 // -> 1135, with dropout 1343 -> 1330; 16 x 12 x 1000 causal (d = 128) 287 -> 271.
