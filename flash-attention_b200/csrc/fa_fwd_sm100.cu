@@ -62,9 +62,10 @@ struct FwdCfg {
   // S = Q K^T can be issued as soon as the softmax group has read the current S into registers.
   // At d = 128 the 512 columns are full and P overwrites the first 64 columns of its S buffer.
   static constexpr bool kSeparateP = (D == 64);
-  // d = 128 without dropout: P is handed over in two halves, so that P*V of the first 64 keys runs while the
-  // other half is exponentiated; S of the next tile waits for P*V there.
+  // d = 128 without dropout: P is handed over in two parts, so that P*V of the first 96 keys runs while the
+  // rest is exponentiated; S of the next tile waits for P*V there, and so tells that it is over.
   static constexpr bool kHalfP = kRows && !kSeparateP;
+  static constexpr int kFirstSteps = kHalfP ? 6 : 0;  // of 16 keys, in the first part
   static constexpr uint32_t kTmemP0 = kSeparateP ? 192 * G : kTmemS0, kTmemP1 = kSeparateP ? 192 * G + 64 : kTmemS1;
   // register split (per thread) of the 128 or 168 (rows), 80 or 96 (quads) a thread is launched with
   static constexpr int kSoftmaxRegs = kRows ? ((G == 1) ? 208 : 224) : ((G == 1) ? 96 : 104);
@@ -384,7 +385,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           mma_commit(smem_u32(&sh.s_full[g]));
         }
       };
-      // key steps [k0, k1) of 16; the last part reports the product
+      // key steps [k0, k1) of 16; the last part reports the product, unless P comes in parts
       auto issue_pv = [&](int g, int stage, bool accumulate, int k0, int k1) {
         const uint64_t va = desc_here(desc_at(desc_v, stage * Cfg::kTileBytes));
         const uint32_t tO = tmem + (g == 0 ? Cfg::kTmemO0 : Cfg::kTmemO1);
@@ -393,7 +394,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 #pragma unroll
           for (int ks = k0; ks < k1; ++ks)
             mma_ts(tO, tP + ks * 8, desc_at(va, ks * 2048), idesc_pv, accumulate || ks > 0);
-          if (k1 == kBlockN / 16) mma_commit(smem_u32(&sh.o_full[g]));
+          if (!Cfg::kHalfP && k1 == kBlockN / 16) mma_commit(smem_u32(&sh.o_full[g]));
         }
       };
 
@@ -446,22 +447,23 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 #pragma unroll
           for (int g = 0; g < G; ++g) {
             if (ok && j < n_tiles[g]) {
-              constexpr int kFirst = Cfg::kHalfP ? kBlockN / 32 : 0;
               if constexpr (Cfg::kHalfP) {
                 ok = mbar_wait_warp<true>(smem_u32(&sh.p_half[g]), j & 1, abort_flag);
                 if (ok) {
                   tc_fence_after();
-                  issue_pv(g, s, j > 0, 0, kFirst);
+                  issue_pv(g, s, j > 0, 0, Cfg::kFirstSteps);
                 }
               }
               if (ok) ok = mbar_wait_warp<true>(smem_u32(&sh.p_full[g]), j & 1, abort_flag);
               if (ok) {
                 tc_fence_after();
-                issue_pv(g, s, j > 0, kFirst, kBlockN / 16);
+                issue_pv(g, s, j > 0, Cfg::kFirstSteps, kBlockN / 16);
                 if (j + 1 < n_tiles[g]) {
                   if (!k_here) wait_k();
                   k_here = true;
                   if (ok) issue_qk(g, sn);
+                } else if (Cfg::kHalfP) {  // (S of the next tile reports the others)
+                  if (elect_one()) mma_commit(smem_u32(&sh.o_full[g]));
                 }
               }
             }
@@ -595,29 +597,30 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       // p = exp2(s * c - m * c): packed fma, one ex2 per element, packed row sum, 16-bit pack
       uint32_t pk[64];
       uint64_t sum_a = 0ull, sum_b = 0ull;
-      auto expo_half = [&](int half) {
+      auto expo = [&](int from, int to) {
 #pragma unroll
-        for (int c = 2 * half; c < 2 * half + 2; ++c)
-#pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            float p0, p1, p2, p3;
-            unpack_f2(fma2(pack_f2(__uint_as_float(sr[c][i]), __uint_as_float(sr[c][i + 1])), c2, nmc2), p0, p1);
-            unpack_f2(fma2(pack_f2(__uint_as_float(sr[c][i + 2]), __uint_as_float(sr[c][i + 3])), c2, nmc2), p2, p3);
-            p0 = ex2f(p0); p1 = ex2f(p1); p2 = ex2f(p2); p3 = ex2f(p3);
-            const uint64_t p01 = pack_f2(p0, p1), p23 = pack_f2(p2, p3);
-            sum_a = add2(sum_a, p01);
-            sum_b = add2(sum_b, p23);
-            pk[c * 16 + i / 2] = pack_lowp<BF16>(p0, p1);
-            pk[c * 16 + i / 2 + 1] = pack_lowp<BF16>(p2, p3);
-          }
+        for (int e = from; e < to; e += 4) {
+          const int c = e / 32, i = e % 32;
+          float p0, p1, p2, p3;
+          unpack_f2(fma2(pack_f2(__uint_as_float(sr[c][i]), __uint_as_float(sr[c][i + 1])), c2, nmc2), p0, p1);
+          unpack_f2(fma2(pack_f2(__uint_as_float(sr[c][i + 2]), __uint_as_float(sr[c][i + 3])), c2, nmc2), p2, p3);
+          p0 = ex2f(p0); p1 = ex2f(p1); p2 = ex2f(p2); p3 = ex2f(p3);
+          const uint64_t p01 = pack_f2(p0, p1), p23 = pack_f2(p2, p3);
+          sum_a = add2(sum_a, p01);
+          sum_b = add2(sum_b, p23);
+          pk[c * 16 + i / 2] = pack_lowp<BF16>(p0, p1);
+          pk[c * 16 + i / 2 + 1] = pack_lowp<BF16>(p2, p3);
+        }
       };
-      expo_half(0);
-      // P*V of the previous tile must have finished before O is rescaled or its P buffer reused.  (Half of the
-      // exponentials are still to come: by now it has, as a rule.)
+      expo(0, 64);
+      // P*V of the previous tile must have finished before O is rescaled or its P buffer reused.  With P over S (d = 128) it has: these
+      // scores were issued behind it.  (Else: half of the exponentials are still to come, and by now it has, as a rule.)
       if (j > 0) {
-        ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), (j - 1) & 1, abort_flag);
-        if (!ok) break;
-        tc_fence_after();
+        if constexpr (Cfg::kSeparateP) {
+          ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), (j - 1) & 1, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+        }
         if (__any_sync(0xffffffffu, grow)) {
           const uint64_t alpha2 = pack_f2(alpha, alpha);
 #pragma unroll
@@ -636,20 +639,31 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           }
         }
       }
-      // hand P to the tensor core through tensor memory, in two halves (64 keys each)
+      // Hand P to the tensor core through tensor memory.  In parts: three quarters first, and reported behind the next eight
+      // exponentials, when the stores have been taken.  us, halves that are reported at once and a wait for P V ahead of the first -> no
+      // wait -> now: 4 x 12 x 4096 354 -> 342 -> 342, 4 x 12 x 8192 causal 660 -> 639 -> 637, 16 x 12 x 1000 120 -> 117 -> 115, 64 x 12 x
+      // 300 92.3 -> 91.0 -> 90.5.  (Traces, 4 x 12 x 4096: a group's 3560 clk a tile are 200 for the scores, 300 for the maximum, 1500
+      // exponentials beside the other group's, 170 of that wait, 1070 from P to the next S.)
       tmem_st32(tP, reinterpret_cast<uint32_t(&)[32]>(pk[0]));
       if constexpr (Cfg::kHalfP) {
+        static_assert(Cfg::kFirstSteps == 6, "96 keys");
+        expo(64, 96);
+        tmem_st16(tP + 32, reinterpret_cast<uint32_t(&)[16]>(pk[32]));
+        expo(96, 104);
         tmem_wait_st();
         tc_fence_before();
         mbar_arrive(smem_u32(&sh.p_half[g]));
+        expo(104, 128);
+      } else {
+        expo(64, 128);
       }
-      expo_half(1);
       {
         float s0, s1;
         unpack_f2(add2(sum_a, sum_b), s0, s1);
         l_run = l_run * alpha + (s0 + s1);
       }
-      tmem_st32(tP + 32, reinterpret_cast<uint32_t(&)[32]>(pk[32]));
+      if constexpr (Cfg::kHalfP) tmem_st16(tP + 48, reinterpret_cast<uint32_t(&)[16]>(pk[48]));
+      else tmem_st32(tP + 32, reinterpret_cast<uint32_t(&)[32]>(pk[32]));
       tmem_wait_st();
       tc_fence_before();
       mbar_arrive(smem_u32(&sh.p_full[g]));
@@ -658,7 +672,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     // ---------------- epilogue: O = acc / (sum * p_keep), LSE
     if (active) {
       if (n > 0 && ok) {
-        ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), (n - 1) & 1, abort_flag);
+        ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), Cfg::kHalfP ? 0 : (n - 1) & 1, abort_flag);
         tc_fence_after();
       }
       // every product that reads this group's Q has finished: its tile takes the output
