@@ -28,7 +28,9 @@
 // LSE = max*scale + ln(sum), -inf for a row without any valid key.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <climits>
 #include <cstddef>
+#include <type_traits>
 #include "fa_kernels.h"
 #include "fa_math.cuh"
 #include "sm100_prims.cuh"
@@ -43,7 +45,7 @@ constexpr int kBlockN = 128;
 // G: query tiles (softmax groups) per CTA.  Two share every K / V tile, and one such CTA fills an SM.  One leaves
 // room for a second CTA on the SM, whose loads, first products and epilogue run under the tiles of the other:
 // for short sequences, where those are a third of a CTA's time (see one_tile_per_cta).
-template <int D, int G, bool ROWS>
+template <int D, int G, bool ROWS, bool TAKE = false>
 struct FwdCfg {
   // Softmax layout.  Rows: a warpgroup per query tile, one thread per row.  Quads: eight warps per query tile, 16
   // rows each (see the softmax code for both).
@@ -55,17 +57,18 @@ struct FwdCfg {
   static constexpr int kStages = (G == 1) ? ((D == 64) ? 2 : 1) : ((D == 64) ? 3 : 2);
   static constexpr int kPanels = D / 64;
   static constexpr int kTileBytes = kBlockM * D * 2;
-  static constexpr int kSmemBytes = (G + 2 * kStages) * kTileBytes + 1024;
+  // Where the output rows pass through: Q's tile, or where a CTA goes on with another block (TAKE), whose Q is loaded ahead, a
+  // place of their own, at d = 128 with one tile V's, which is needed last of the next block's operands.
+  static constexpr bool kOutInV = TAKE && D == 128 && G == 1;  // (rows)
+  static constexpr int kOutPiece = kOutInV ? kTileBytes / kSoftmaxWarps : ROWS ? 4096 : 2048;  // of a softmax warp
+  static constexpr int kOutBytes = TAKE && !kOutInV && (ROWS || G == 1) ? kSoftmaxWarps * kOutPiece : 0;  // beside Q, K and V
+  static constexpr int kSmemBytes = (G + 2 * kStages) * kTileBytes + kOutBytes + 1024;
   static constexpr uint32_t kTmemCols = 256 * G;
   static constexpr uint32_t kTmemS0 = 0, kTmemS1 = 128, kTmemO0 = 128 * G, kTmemO1 = 128 * G + D;
   // d = 64 leaves 128 tensor-memory columns free: P gets its own columns there, so the next
   // S = Q K^T can be issued as soon as the softmax group has read the current S into registers.
   // At d = 128 the 512 columns are full and P overwrites the first 64 columns of its S buffer.
   static constexpr bool kSeparateP = (D == 64);
-  // d = 128 without dropout: P is handed over in two parts, so that P*V of the first 96 keys runs while the
-  // rest is exponentiated; S of the next tile waits for P*V there, and so tells that it is over.
-  static constexpr bool kHalfP = kRows && !kSeparateP;
-  static constexpr int kFirstSteps = kHalfP ? 6 : 0;  // of 16 keys, in the first part
   static constexpr uint32_t kTmemP0 = kSeparateP ? 192 * G : kTmemS0, kTmemP1 = kSeparateP ? 192 * G + 64 : kTmemS1;
   // register split (per thread) of the 128 or 168 (rows), 80 or 96 (quads) a thread is launched with
   static constexpr int kSoftmaxRegs = kRows ? ((G == 1) ? 208 : 224) : ((G == 1) ? 96 : 104);
@@ -81,19 +84,34 @@ struct FwdCfg {
 
 constexpr int kMaxSparseTiles = 1024;  // key tiles of 128 per sequence in block-sparse mode
 
+// What a CTA works on: the query tiles [mp * G, mp * G + G) of one (batch, head) pair; n(g): key tiles of each.  mp < 0: behind the
+// last block
+struct FwdBlock {
+  int q_start, sq, k_start, sk, h, b, mp, n0, n1;
+  __device__ __forceinline__ int n(int g) const { return g == 0 ? n0 : n1; }  // (an array would go to local memory)
+};
+
+template <int STATS>
 struct FwdShared {
   uint64_t q_full[2];
   uint64_t k_full[3], k_empty[3], v_full[3], v_empty[3];
   uint64_t s_full[2], s_free[2], p_half[2], p_full[2], o_full[2];
   uint64_t drained[2];  // of the two issuing warps, at their end
-  float2 row_stats[2][kBlockM];  // (max, sum) of every query row, for the epilogue
+  // from here on: CTAs that take over blocks
+  uint64_t q_empty[2];
+  uint64_t next_full;                 // the answer to a request for another block is in `next`
+  uint64_t blk_full[2], blk_done[2];  // the block after is in `blk`; every role has finished the one there
+  uint64_t out_free;                  // the rows of a block have left the place they pass through
+  uint64_t stats_full[2];             // a group's row statistics are written (bounded, unlike bar.sync)
+  float2 row_stats[STATS][kBlockM];  // (max, sum) of every query row, for the epilogue; taking over: two of a group, by the block's parity
+  alignas(16) uint4 next;
+  FwdBlock blk[2];  // block k in entry k % 2
   uint32_t tmem_base;
   int abort_flag;
   int stop;  // a CTA of this launch has abandoned a wait
 };
-constexpr int kBarriers = 26;  // at the head of FwdShared; those from 16 to 21 (s_free, p_half, p_full) belong to a softmax group
-static_assert(offsetof(FwdShared, s_free) == 16 * 8 && offsetof(FwdShared, o_full) == 22 * 8 && offsetof(FwdShared, row_stats) == kBarriers * 8,
-              "order of the barriers");
+constexpr int kBarriers = 26, kTakeBarriers = 36;  // at the head of FwdShared
+static_assert(offsetof(FwdShared<1>, q_empty) == kBarriers * 8 && offsetof(FwdShared<1>, row_stats) == kTakeBarriers * 8, "order of the barriers");
 
 template <int N>
 __device__ __forceinline__ void reg_alloc() {
@@ -107,8 +125,9 @@ __device__ __forceinline__ void reg_dealloc() {
 // Epilogue of 32 query rows (a warp, thread = row, 32x32b shape), NC 32-column groups from c0 on: O = acc / (sum * p_keep)
 // in the 16-bit type; the warp of the first group also writes LSE = max * scale + ln(sum).  A row without any valid key
 // gets zeros and -inf.  Out through `piece`, the warp's NC * 2048 bytes of shared memory (see stage_offset), in boxes of BOX columns;
-// 0: from the registers.  ig: first query row of the warp.
-template <bool BF16, int NC, int BOX>
+// 0: from the registers.  ig: first query row of the warp.  REUSE: the piece holds one panel, and what was stored from it before
+// (by lane 0) has to be read first; else this waits until its own stores have read it.
+template <bool BF16, int NC, int BOX, bool REUSE>
 __device__ __forceinline__ void store_rows(const KernelArgs& a, const CUtensorMap* tm_o, uint32_t tO, int c0, bool have_acc, bool ok, int ig, int lane,
                                            int sq, int q_start, int b, int h, float m_run, float l_run, uint8_t* piece) {
   constexpr bool STAGED = BOX != 0;
@@ -120,6 +139,21 @@ __device__ __forceinline__ void store_rows(const KernelArgs& a, const CUtensorMa
     return reinterpret_cast<uint16_t*>(a.o) + static_cast<int64_t>(q_start + row) * a.o_row_stride +
            static_cast<int64_t>(h) * a.o_head_stride + column;
   };
+  // Whole rows by TMA (by the LSU before: 64 x 12 x 512, d = 64, 104.4 us, now 102.4; d = 128: 32 x 12 x 300 causal 51.2 -> 49.2,
+  // 32 x 12 x 512 84 -> 81, 4 x 32 x 3000 causal 342 -> 335).  The warp that holds the sequence's end stores its rows itself: those
+  // behind it are the next sequence's.
+  const bool whole = ig + 32 <= sq;
+  auto send = [&](int p) {
+    if (whole) {
+      if (lane == 0 && c0 * 32 + p * 64 < a.head_dim) {
+        tma_store_3d(tm_o, smem_u32(piece) + (REUSE ? 0 : p * 4096), c0 * 32 + p * 64, q_start + ig, h);
+        bulk_commit();
+      }
+    } else {
+      stage_copy_out<CH>(piece + (REUSE ? 0 : p * 4096), out(ig, c0 * 32 + p * 64), a.o_row_stride, sq - ig,
+                         a.head_dim / 8 - c0 * 4 - p * 8, lane);
+    }
+  };
 #pragma unroll
   for (int i = 0; i < NC; ++i) {
     uint32_t orr[32];
@@ -130,6 +164,10 @@ __device__ __forceinline__ void store_rows(const KernelArgs& a, const CUtensorMa
 #pragma unroll
       for (int k = 0; k < 32; ++k) orr[k] = 0u;
     }
+    if (STAGED && REUSE && i % 2 == 0) {
+      if (lane == 0) bulk_wait_read();
+      __syncwarp();
+    }
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
       uint32_t w[4];
@@ -137,12 +175,19 @@ __device__ __forceinline__ void store_rows(const KernelArgs& a, const CUtensorMa
       for (int k = 0; k < 4; ++k)
         w[k] = pack_lowp<BF16>(__uint_as_float(orr[8 * v + 2 * k]) * inv, __uint_as_float(orr[8 * v + 2 * k + 1]) * inv);
       if constexpr (STAGED)
-        *reinterpret_cast<uint4*>(piece + (i / 2) * 4096 + stage_offset<CH>(lane, (i & 1) * 4 + v)) = make_uint4(w[0], w[1], w[2], w[3]);
+        *reinterpret_cast<uint4*>(piece + (REUSE ? 0 : i / 2) * 4096 + stage_offset<CH>(lane, (i & 1) * 4 + v)) = make_uint4(w[0], w[1], w[2], w[3]);
       else if (ok && ig + lane < sq && (c0 + i) * 32 + v * 8 < a.head_dim)
         *reinterpret_cast<uint4*>(out(ig + lane, (c0 + i) * 32 + v * 8)) = make_uint4(w[0], w[1], w[2], w[3]);
     }
+    if constexpr (STAGED && REUSE) {
+      if (i % 2 == 1 || i + 1 == NC) {
+        fence_async_smem();
+        __syncwarp();
+        if (ok) send(i / 2);
+      }
+    }
   }
-  if constexpr (STAGED) {
+  if constexpr (STAGED && !REUSE) {
     fence_async_smem();
     __syncwarp();
   }
@@ -151,23 +196,11 @@ __device__ __forceinline__ void store_rows(const KernelArgs& a, const CUtensorMa
     const float lse = bad_sum ? -INFINITY : (m_run * a.scale + __logf(l_run));
     a.lse[(static_cast<int64_t>(b) * a.heads + h) * a.lse_stride + ig + lane] = lse;
   }
-  if constexpr (!STAGED) return;
-  // Whole rows by TMA (by the LSU before: 64 x 12 x 512, d = 64, 104.4 us, now 102.4; d = 128: 32 x 12 x 300 causal 51.2 -> 49.2,
-  // 32 x 12 x 512 84 -> 81, 4 x 32 x 3000 causal 342 -> 335).  The warp that holds the sequence's end stores its rows itself: those
-  // behind it are the next sequence's.
-  if (ig + 32 <= sq) {
-    if (lane == 0) {
+  if constexpr (STAGED && !REUSE) {
 #pragma unroll
-      for (int p = 0; p < (NC + 1) / 2; ++p)
-        if (c0 * 32 + p * 64 < a.head_dim) tma_store_3d(tm_o, smem_u32(piece) + p * 4096, c0 * 32 + p * 64, q_start + ig, h);
-      bulk_commit();
-      bulk_wait_read();
-    }
-    return;
+    for (int p = 0; p < (NC + 1) / 2; ++p) send(p);
+    if (lane == 0 && whole) bulk_wait_read();
   }
-#pragma unroll
-  for (int p = 0; p < (NC + 1) / 2; ++p)
-    stage_copy_out<CH>(piece + p * 4096, out(ig, c0 * 32 + p * 64), a.o_row_stride, sq - ig, a.head_dim / 8 - c0 * 4 - p * 8, lane);
 }
 
 // Padded batches.  A V tile that reaches behind its sequence's last token holds whatever the padding holds, and its
@@ -196,14 +229,23 @@ __device__ __forceinline__ void zero_padding(const KernelArgs& a, int b, int h, 
   }
 }
 
-// ORDERED: causal grids with the order of set_tail_grid.  PADDED: see KernelArgs::pad_rows
-template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BLOCKSPARSE, int G, bool ROWS, bool ORDERED, bool PADDED>
+// How a grid is laid out and worked on.  kPlain: (tiles, heads, batch).  kLinear: one-dimensional, causal ones with the order of
+// set_tail_grid.  kTake: kLinear, and a CTA goes on with blocks that have not started (see take_over_pays).
+enum Order { kPlain, kLinear, kTake };
+
+// PADDED: see KernelArgs::pad_rows
+template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BLOCKSPARSE, int G, bool ROWS, Order ORDER, bool PADDED>
 __global__ void __launch_bounds__(FwdCfg<D, G, ROWS>::kThreads, G == 1 ? 2 : 1)
 fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
               const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const KernelArgs a) {
-  using Cfg = FwdCfg<D, G, ROWS>;
+  constexpr bool TAKE = ORDER == kTake, LINEAR = ORDER != kPlain;
+  using Cfg = FwdCfg<D, G, ROWS, TAKE>;
+  // d = 128 without dropout: P is handed over in two parts, so that P*V of the first 96 keys runs while the
+  // rest is exponentiated; S of the next tile waits for P*V there, and so tells that it is over.
+  constexpr bool kHalfP = Cfg::kRows && !Cfg::kSeparateP;
+  constexpr int kFirstSteps = kHalfP ? 6 : 0;  // of 16 keys, in the first part
   extern __shared__ uint8_t smem_raw[];
-  __shared__ FwdShared sh;
+  __shared__ FwdShared<ROWS ? 1 : TAKE ? 2 * G : G> sh;
   // block-sparse: key tiles this CTA visits (ascending), built from the layout table
   __shared__ uint16_t tile_list[BLOCKSPARSE ? kMaxSparseTiles : 1];
   __shared__ int tile_count;
@@ -212,35 +254,64 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);  // known to be the same in all lanes
   const int lane = tid & 31;
 
-  int b = blockIdx.z, h = blockIdx.y, mp = CAUSAL ? gridDim.x - 1 - blockIdx.x : blockIdx.x;  // heavy tiles first
-  if constexpr (ORDERED) tail_block(a, blockIdx.x, mp, h, b);
-  const int q_start = a.cu_seqlens_q[PADDED ? 2 * b : b];
-  const int sq = a.cu_seqlens_q[PADDED ? 2 * b + 1 : b + 1] - q_start;
-  const int k_start = PADDED ? q_start : a.cu_seqlens_k[b];
-  const int sk = PADDED ? sq : a.cu_seqlens_k[b + 1] - k_start;
-  if constexpr (ORDERED) {
-    mp = (sq + G * kBlockM - 1) / (G * kBlockM) - 1 - mp;  // of the sequence's own tiles; empty blocks last
-    if (mp < 0) return;
-  }
+  auto decode = [&](uint32_t block) -> FwdBlock {
+    FwdBlock x;
+    if constexpr (LINEAR) tail_block(a, block, x.mp, x.h, x.b);
+    else { x.b = blockIdx.z; x.h = blockIdx.y; x.mp = CAUSAL ? gridDim.x - 1 - blockIdx.x : blockIdx.x; }  // heavy tiles first
+    x.q_start = a.cu_seqlens_q[PADDED ? 2 * x.b : x.b];
+    x.sq = a.cu_seqlens_q[PADDED ? 2 * x.b + 1 : x.b + 1] - x.q_start;
+    x.k_start = PADDED ? x.q_start : a.cu_seqlens_k[x.b];
+    x.sk = PADDED ? x.sq : a.cu_seqlens_k[x.b + 1] - x.k_start;
+    if constexpr (LINEAR && CAUSAL) {
+      const int mp = (x.sq + G * kBlockM - 1) / (G * kBlockM) - 1 - x.mp;  // of the sequence's own tiles; empty blocks last
+      if (!PADDED || mp >= 0) x.mp = mp;
+    }
+    return x;
+  };
+  auto without_queries = [&](const FwdBlock& x) -> bool { return LINEAR && CAUSAL && !PADDED ? x.mp < 0 : x.mp * G * kBlockM >= x.sq; };
+  auto count_tiles = [&](FwdBlock& x) {
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      const int m0 = (x.mp * G + g) * kBlockM;
+      int n = (x.sk + kBlockN - 1) / kBlockN;
+      if (CAUSAL) n = min(n, m0 / kBlockN + 1);
+      (g == 0 ? x.n0 : x.n1) = m0 < x.sq ? n : 0;
+    }
+    if (G == 1) x.n1 = 0;
+  };
+  FwdBlock first = decode(blockIdx.x);
   if constexpr (PADDED) {
-    if (q_start < 0) return;
-    if (mp * G * kBlockM >= sq)
-      zero_padding(a, b, h, mp * G * kBlockM, (mp + 1) * G * kBlockM, q_start - b * a.pad_rows, sq, tid, Cfg::kThreads);
+    if (first.q_start < 0) return;
+    if (without_queries(first))
+      zero_padding(a, first.b, first.h, first.mp * G * kBlockM, (first.mp + 1) * G * kBlockM, first.q_start - first.b * a.pad_rows, first.sq,
+                   tid, Cfg::kThreads);
   }
   // On the lengths alone: a grid announced with a long sequence consists mostly of blocks without queries, and everything ahead of
   // this line is their time.  With the status word and the barriers ahead of it too, which saves the others 0.1 us, us of an SM for such a
   // block 0.93-1.0 (d = 64), now 0.67-0.73; 0.47-0.58 (d = 128), now 0.39-0.48.  1 x 4096 and 63 x 128, 12 heads, d = 64: 232 -> 183 us.
-  if (mp * G * kBlockM >= sq) return;
-  if (warp == Cfg::kSoftmaxWarps) {  // a lane per barrier
-    if (lane == 0) sh.abort_flag = 0;
-    if (lane < kBarriers) mbar_init(smem_u32(&sh.q_full[0]) + lane * 8, lane >= 16 && lane < 22 ? Cfg::kArrivals : 1);
+  if (without_queries(first)) return;
+  count_tiles(first);
+  if (warp == Cfg::kSoftmaxWarps) {
+    if (lane == 0) {
+      sh.abort_flag = 0;
+      if (TAKE) sh.blk[0] = first;
+    }
+    for (int i = lane; i < (TAKE ? kTakeBarriers : kBarriers); i += 32) {
+      const uint64_t* bar = &sh.q_full[0] + i;
+      const uint32_t count = bar >= &sh.s_free[0] && bar < &sh.o_full[0] ? Cfg::kArrivals
+                             : bar >= &sh.blk_done[0] && bar < &sh.out_free ? Cfg::kSoftmaxWarps + 1 + (Cfg::kSeparateP ? 1 : 0) + (PADDED ? 1 : 0)  // all but the producer
+                             : bar == &sh.out_free ? Cfg::kSoftmaxWarps
+                             : bar >= &sh.stats_full[0] ? Cfg::kGroupWarps : 1;
+      mbar_init(smem_u32(bar), count);
+    }
     fence_mbar_init();
     fence_async_smem();
     __syncwarp();
   }
 
-  int n_kv_total = (sk + kBlockN - 1) / kBlockN;
   if constexpr (BLOCKSPARSE) {
+    const int mp = first.mp, sq = first.sq, b = first.b;
+    int n_kv_total = (first.sk + kBlockN - 1) / kBlockN;
     // A key tile is visited when any 16-row block of this CTA's 128 * G query rows has its 256-column
     // key block in the layout; rows whose block is absent are masked inside the tile.
     uint8_t* flags = reinterpret_cast<uint8_t*>(smem_raw);
@@ -267,37 +338,36 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     // flags live in the tile buffers: their ordinary accesses are over, for the async proxy too, before TMA writes there
     fence_async_smem();
     __syncthreads();
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      const int m0 = (mp * G + g) * kBlockM;
+      int n = n_kv_total;
+      if constexpr (CAUSAL) {
+        // listed key tiles (ascending) up to the one that holds this query tile's diagonal
+        n = 0;
+        while (n < n_kv_total && tile_list[n] <= m0 / kBlockN) ++n;
+      }
+      (g == 0 ? first.n0 : first.n1) = m0 < sq ? n : 0;
+    }
   }
   auto kv_tile = [&](int j) -> int {
     if constexpr (BLOCKSPARSE) return tile_list[j];
     else return j;
   };
-  int m0[G], n_tiles[G];
-#pragma unroll
-  for (int g = 0; g < G; ++g) {
-    m0[g] = (mp * G + g) * kBlockM;
-    const bool active = m0[g] < sq;
-    int n = n_kv_total;
-    if constexpr (CAUSAL && BLOCKSPARSE) {
-      // listed key tiles (ascending) up to the one that holds this query tile's diagonal
-      n = 0;
-      while (n < n_kv_total && tile_list[n] <= m0[g] / kBlockN) ++n;
-    } else if (CAUSAL) {
-      n = min(n, m0[g] / kBlockN + 1);
-    }
-    n_tiles[g] = active ? n : 0;
-  }
-  const int n_max = max(n_tiles[0], n_tiles[G - 1]);
 
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   const uint32_t smem_q = smem_u32(smem);
   const uint32_t smem_k = smem_q + G * Cfg::kTileBytes;
   const uint32_t smem_v = smem_k + Cfg::kStages * Cfg::kTileBytes;
+  const uint32_t smem_out = smem_v + Cfg::kStages * Cfg::kTileBytes;
   // the 128 rows from `row` on of one operand (one thread)
-  auto load_tile = [&](uint32_t dst, const CUtensorMap* map, uint64_t& bar, int row) {
+  auto load_tile = [&](uint32_t dst, const CUtensorMap* map, uint64_t& bar, int row, int h) {
     mbar_expect_tx(smem_u32(&bar), Cfg::kTileBytes);
     for (int p = 0; p < Cfg::kPanels; ++p) tma_load_3d(dst + p * 16384, map, smem_u32(&bar), p * 64, row, h);
+  };
+  auto load_q = [&](const FwdBlock& x, int g) {
+    load_tile(smem_q + g * Cfg::kTileBytes, &tm_q, sh.q_full[g], x.q_start + (x.mp * G + g) * kBlockM, x.h);
   };
 
   // The producer asks for Q and the first K and V at once, ahead of everything else a CTA does: behind
@@ -306,11 +376,12 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   // is used (issuer) and the rows stored through shared memory (store_rows, 3500 clk before), us, before -> now: 16 x 12 x 1000
   // causal (d = 128) 97 -> 83; d = 64: 64 x 12 x 512 100 -> 95, 16 x 12 x 1024 87 -> 80, 8 x 12 x 4096 479 -> 465, 2 x 4 x 16384
   // causal 310 -> 307.
-  if (tid == 32 * Cfg::kSoftmaxWarps && n_max > 0) {
+  const int first_max = max(first.n(0), first.n(G - 1));
+  if (tid == 32 * Cfg::kSoftmaxWarps && first_max > 0) {
     for (int g = 0; g < G; ++g)
-      if (n_tiles[g] > 0) load_tile(smem_q + g * Cfg::kTileBytes, &tm_q, sh.q_full[g], q_start + m0[g]);
-    load_tile(smem_k, &tm_k, sh.k_full[0], k_start + kv_tile(0) * kBlockN);
-    load_tile(smem_v, &tm_v, sh.v_full[0], k_start + kv_tile(0) * kBlockN);
+      if (first.n(g) > 0) load_q(first, g);
+    load_tile(smem_k, &tm_k, sh.k_full[0], first.k_start + kv_tile(0) * kBlockN, first.h);
+    load_tile(smem_v, &tm_v, sh.v_full[0], first.k_start + kv_tile(0) * kBlockN, first.h);
   }
   // Fail fast: once a CTA of this launch has abandoned a wait, those that start after it do not go on.  Quads look here and leave behind
   // the barrier, with their first loads ended.  In rows and padded batches, whose shorter walks would wait for the word, the idle warp
@@ -329,9 +400,9 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   tc_fence_after();
   const uint32_t tmem = sh.tmem_base;
   if (!kLateLook && sh.stop) {
-    if (tid == 32 * Cfg::kSoftmaxWarps && n_max > 0) {
+    if (tid == 32 * Cfg::kSoftmaxWarps && first_max > 0) {
       for (int g = 0; g < G; ++g)
-        if (n_tiles[g] > 0) mbar_drain(smem_u32(&sh.q_full[g]), 0);
+        if (first.n(g) > 0) mbar_drain(smem_u32(&sh.q_full[g]), 0);
       mbar_drain(smem_u32(&sh.k_full[0]), 0);
       mbar_drain(smem_u32(&sh.v_full[0]), 0);
     }
@@ -340,101 +411,175 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   }
   volatile int* abort_flag = &sh.abort_flag;
 
+  // Block k of this CTA.  The softmax warps read it where they use it, to hold few registers across the tiles.
+  auto block_at = [&](uint32_t k) -> std::conditional_t<TAKE, const FwdBlock&, FwdBlock> {
+    if constexpr (TAKE) return sh.blk[k & 1];
+    else return first;
+  };
+  // A warp has finished block k: waits for the next one, if any (or until a wait is abandoned).
+  auto next_block = [&](uint32_t k) -> bool {
+    if constexpr (!TAKE) return false;
+    __syncwarp();
+    if (elect_one()) mbar_arrive(smem_u32(&sh.blk_done[k & 1]));
+    return mbar_wait_warp<true>(smem_u32(&sh.blk_full[(k + 1) & 1]), (k >> 1) & 1, abort_flag) && sh.blk[(k + 1) & 1].mp >= 0;
+  };
+
   if (warp >= Cfg::kSoftmaxWarps) reg_dealloc<Cfg::kOtherRegs>();
   if (warp == Cfg::kSoftmaxWarps) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
       bool ok = true;
-      int loads_k = min(n_max, 1), loads_v = loads_k;  // so far
-      for (int j = 1; j < n_max && ok; ++j) {
-        const int s = j % Cfg::kStages;
-        const uint32_t ph = ((j / Cfg::kStages) & 1) ^ 1;
-        if (j >= Cfg::kStages) ok = mbar_wait(smem_u32(&sh.k_empty[s]), ph, abort_flag);
+      int loads_k = 0, loads_v = 0, loads_q[G] = {};  // so far
+      uint32_t asked = 0;                             // requests so far
+      // asked for with the loads of the last key tile: a block taken earlier would wait here while other SMs run dry
+      auto take_next = [&]() {
+        mbar_expect_tx(smem_u32(&sh.next_full), 16);
+        clc_try_cancel(smem_u32(&sh.next), smem_u32(&sh.next_full));
+        ++asked;
+      };
+      FwdBlock x = first;
+      for (uint32_t k = 0; ok; ++k) {
+        const int n_max = max(x.n(0), x.n(G - 1));
+        for (int g = 0; g < G && ok; ++g) {
+          if (x.n(g) == 0) continue;
+          if (k > 0) {
+            if (loads_q[g] > 0) ok = mbar_wait(smem_u32(&sh.q_empty[g]), (loads_q[g] & 1) ^ 1, abort_flag);
+            if (!ok) break;
+            load_q(x, g);
+          }
+          ++loads_q[g];
+        }
+        for (int j = 0; j < n_max && ok; ++j) {
+          const int s = loads_k % Cfg::kStages;
+          const uint32_t ph = ((loads_k / Cfg::kStages) & 1) ^ 1;
+          const int row = x.k_start + kv_tile(j) * kBlockN;
+          if (k > 0 || j > 0) {  // (the first ones are under way)
+            if (loads_k >= Cfg::kStages) ok = mbar_wait(smem_u32(&sh.k_empty[s]), ph, abort_flag);
+            if (!ok) break;
+            load_tile(smem_k + s * Cfg::kTileBytes, &tm_k, sh.k_full[s], row, x.h);
+          }
+          ++loads_k;
+          if (TAKE && j + 1 == n_max) take_next();
+          if (k > 0 || j > 0) {
+            if (loads_v >= Cfg::kStages) ok = mbar_wait(smem_u32(&sh.v_empty[s]), ph, abort_flag);
+            if (ok && Cfg::kOutInV && j == 0) ok = mbar_wait(smem_u32(&sh.out_free), (k & 1) ^ 1, abort_flag);
+            if (!ok) break;
+            load_tile(smem_v + s * Cfg::kTileBytes, &tm_v, sh.v_full[s], row, x.h);
+          }
+          ++loads_v;
+        }
+        if (!TAKE || !ok) break;
+        if (n_max == 0) take_next();
+        // The next block with queries.  (Padded batches pass the others on too: their rows get zeros.)
+        bool more = false;
+        while (true) {
+          ok = mbar_wait(smem_u32(&sh.next_full), (asked - 1) & 1, abort_flag);
+          if (!ok) break;
+          uint32_t block;
+          more = clc_answer(smem_u32(&sh.next), block);
+          fence_async_smem();
+          if (!more) break;
+          more = !launch_failed();
+          x = decode(block);
+          if (!more || PADDED || !without_queries(x)) break;
+          take_next();
+        }
         if (!ok) break;
-        load_tile(smem_k + s * Cfg::kTileBytes, &tm_k, sh.k_full[s], k_start + kv_tile(j) * kBlockN);
-        loads_k = j + 1;
-        if (j >= Cfg::kStages) ok = mbar_wait(smem_u32(&sh.v_empty[s]), ph, abort_flag);
+        if (!more) x.mp = -1;
+        count_tiles(x);
+        // its place is free once every role has finished block k - 1
+        if (k >= 1) ok = mbar_wait(smem_u32(&sh.blk_done[(k + 1) & 1]), ((k - 1) >> 1) & 1, abort_flag);
         if (!ok) break;
-        load_tile(smem_v + s * Cfg::kTileBytes, &tm_v, sh.v_full[s], k_start + kv_tile(j) * kBlockN);
-        loads_v = j + 1;
+        sh.blk[(k + 1) & 1] = x;
+        mbar_arrive(smem_u32(&sh.blk_full[(k + 1) & 1]));
+        if (!more) break;
       }
-      for (int g = 0; g < G; ++g)
-        if (n_tiles[g] > 0) mbar_drain(smem_u32(&sh.q_full[g]), 0);
+      for (int g = 0; g < G; ++g) mbar_drain_ring(&sh.q_full[g], 1, loads_q[g]);
       mbar_drain_ring(sh.k_full, Cfg::kStages, loads_k);
       mbar_drain_ring(sh.v_full, Cfg::kStages, loads_v);
+      if (TAKE) mbar_drain_ring(&sh.next_full, 1, asked);
     }
   } else if (warp == Cfg::kSoftmaxWarps + 1) {
     // ------------------------------------------------------------------ MMA issuer
     // all 32 lanes run the loop, one elected lane issues (see mma_ss)
-    {
-      constexpr uint32_t idesc_qk = make_idesc(BF16, false, false, kBlockM, kBlockN);
-      constexpr uint32_t idesc_pv = make_idesc(BF16, false, true, kBlockM, D);
-      const uint64_t desc_q = make_smem_desc(smem_q, 16, 1024);
-      const uint64_t desc_k = make_smem_desc(smem_k, 16, 1024);
-      const uint64_t desc_v = make_smem_desc(smem_v, 16384, 1024);
-      auto issue_qk = [&](int g, int stage) {
-        const uint64_t qa = desc_here(desc_at(desc_q, g * Cfg::kTileBytes));
-        const uint64_t ka = desc_here(desc_at(desc_k, stage * Cfg::kTileBytes));
-        const uint32_t tS = tmem + (g == 0 ? Cfg::kTmemS0 : Cfg::kTmemS1);
-        if (elect_one()) {
+    constexpr uint32_t idesc_qk = make_idesc(BF16, false, false, kBlockM, kBlockN);
+    constexpr uint32_t idesc_pv = make_idesc(BF16, false, true, kBlockM, D);
+    const uint64_t desc_q = make_smem_desc(smem_q, 16, 1024);
+    const uint64_t desc_k = make_smem_desc(smem_k, 16, 1024);
+    const uint64_t desc_v = make_smem_desc(smem_v, 16384, 1024);
+    // last: the block's last product of this group, which frees its Q
+    auto issue_qk = [&](int g, int stage, bool last) {
+      const uint64_t qa = desc_here(desc_at(desc_q, g * Cfg::kTileBytes));
+      const uint64_t ka = desc_here(desc_at(desc_k, stage * Cfg::kTileBytes));
+      const uint32_t tS = tmem + (g == 0 ? Cfg::kTmemS0 : Cfg::kTmemS1);
+      if (elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < D / 16; ++ks) {
-            const uint32_t off = (ks >> 2) * 16384 + (ks & 3) * 32;
-            mma_ss(tS, desc_at(qa, off), desc_at(ka, off), idesc_qk, ks > 0);
-          }
-          mma_commit(smem_u32(&sh.s_full[g]));
+        for (int ks = 0; ks < D / 16; ++ks) {
+          const uint32_t off = (ks >> 2) * 16384 + (ks & 3) * 32;
+          mma_ss(tS, desc_at(qa, off), desc_at(ka, off), idesc_qk, ks > 0);
         }
-      };
-      // key steps [k0, k1) of 16; the last part reports the product, unless P comes in parts
-      auto issue_pv = [&](int g, int stage, bool accumulate, int k0, int k1) {
-        const uint64_t va = desc_here(desc_at(desc_v, stage * Cfg::kTileBytes));
-        const uint32_t tO = tmem + (g == 0 ? Cfg::kTmemO0 : Cfg::kTmemO1);
-        const uint32_t tP = tmem + (g == 0 ? Cfg::kTmemP0 : Cfg::kTmemP1);
-        if (elect_one()) {
+        mma_commit(smem_u32(&sh.s_full[g]));
+        if (TAKE && last) mma_commit(smem_u32(&sh.q_empty[g]));
+      }
+    };
+    // key steps [k0, k1) of 16; the last part reports the product, unless P comes in parts
+    auto issue_pv = [&](int g, int stage, bool accumulate, int k0, int k1) {
+      const uint64_t va = desc_here(desc_at(desc_v, stage * Cfg::kTileBytes));
+      const uint32_t tO = tmem + (g == 0 ? Cfg::kTmemO0 : Cfg::kTmemO1);
+      const uint32_t tP = tmem + (g == 0 ? Cfg::kTmemP0 : Cfg::kTmemP1);
+      if (elect_one()) {
 #pragma unroll
-          for (int ks = k0; ks < k1; ++ks)
-            mma_ts(tO, tP + ks * 8, desc_at(va, ks * 2048), idesc_pv, accumulate || ks > 0);
-          if (!Cfg::kHalfP && k1 == kBlockN / 16) mma_commit(smem_u32(&sh.o_full[g]));
-        }
-      };
+        for (int ks = k0; ks < k1; ++ks)
+          mma_ts(tO, tP + ks * 8, desc_at(va, ks * 2048), idesc_pv, accumulate || ks > 0);
+        if (!kHalfP && k1 == kBlockN / 16) mma_commit(smem_u32(&sh.o_full[g]));
+      }
+    };
 
-      bool ok = true;
-      for (int g = 0; g < G && ok; ++g)
-        if (n_tiles[g] > 0) ok = mbar_wait_warp<true>(smem_u32(&sh.q_full[g]), 0, abort_flag);
-      if (ok && n_max > 0) {
-        ok = mbar_wait_warp<true>(smem_u32(&sh.k_full[0]), 0, abort_flag);
+    bool ok = true;
+    int kv = 0, c[G] = {};         // key tiles of the blocks before; products of each group
+    uint32_t k = 0, c_q[G] = {};   // block; blocks whose Q was loaded
+    do {
+      const FwdBlock x = block_at(k);
+      int n_tiles[G];
+      for (int g = 0; g < G; ++g) n_tiles[g] = __shfl_sync(0xffffffffu, x.n(g), 0);
+      const int n_max = max(n_tiles[0], n_tiles[G - 1]);
+      for (int g = 0; g < G; ++g)
+        if (ok && n_tiles[g] > 0) ok = mbar_wait_warp<true>(smem_u32(&sh.q_full[g]), c_q[g]++ & 1, abort_flag);
+      if constexpr (Cfg::kSeparateP) {
+        // this warp issues only the score products; the next one issues P*V
+        for (int j = 0; j < n_max && ok; ++j) {
+          const int s = (kv + j) % Cfg::kStages;
+          ok = mbar_wait_warp<true>(smem_u32(&sh.k_full[s]), ((kv + j) / Cfg::kStages) & 1, abort_flag);
+#pragma unroll
+          for (int g = 0; g < G; ++g) {
+            if (ok && j < n_tiles[g]) {
+              if (c[g] > 0) ok = mbar_wait_warp<true>(smem_u32(&sh.s_free[g]), (c[g] & 1) ^ 1, abort_flag);
+              if (ok) {
+                tc_fence_after();
+                issue_qk(g, s, j + 1 == n_tiles[g]);
+                ++c[g];
+              }
+            }
+          }
+          if (ok && elect_one()) mma_commit(smem_u32(&sh.k_empty[s]));
+        }
+      } else if (n_max > 0) {
+        if (ok) ok = mbar_wait_warp<true>(smem_u32(&sh.k_full[kv % Cfg::kStages]), (kv / Cfg::kStages) & 1, abort_flag);
         if (ok) {
           tc_fence_after();
 #pragma unroll
           for (int g = 0; g < G; ++g)
-            if (n_tiles[g] > 0) issue_qk(g, 0);
-          if (elect_one()) mma_commit(smem_u32(&sh.k_empty[0]));
+            if (n_tiles[g] > 0) issue_qk(g, kv % Cfg::kStages, n_tiles[g] == 1);
+          if (elect_one()) mma_commit(smem_u32(&sh.k_empty[kv % Cfg::kStages]));
         }
-      }
-      for (int j = 0; j < n_max && ok; ++j) {
-        const int s = j % Cfg::kStages;
-        const int sn = (j + 1) % Cfg::kStages;
-        const bool has_next = j + 1 < n_max;
-        auto wait_k = [&]() { ok = mbar_wait_warp<true>(smem_u32(&sh.k_full[sn]), ((j + 1) / Cfg::kStages) & 1, abort_flag); };
-        if constexpr (Cfg::kSeparateP) {
-          // this warp issues only the score products; the next one issues P*V
-          if (has_next) wait_k();
-          if (!ok) break;
-#pragma unroll
-          for (int g = 0; g < G; ++g) {
-            if (ok && j + 1 < n_tiles[g]) {
-              ok = mbar_wait_warp<true>(smem_u32(&sh.s_free[g]), j & 1, abort_flag);
-              if (ok) {
-                tc_fence_after();
-                issue_qk(g, sn);
-              }
-            }
-          }
-          if (!ok) break;
-        } else {
-          ok = mbar_wait_warp<true>(smem_u32(&sh.v_full[s]), (j / Cfg::kStages) & 1, abort_flag);
-          if (PADDED && ok && (j + 1) * kBlockN > sk)
-            clear_v_rows<Cfg::kPanels>(smem + (smem_v - smem_q) + s * Cfg::kTileBytes, sk - j * kBlockN, lane);
+        for (int j = 0; j < n_max && ok; ++j) {
+          const int s = (kv + j) % Cfg::kStages;
+          const int sn = (kv + j + 1) % Cfg::kStages;
+          const bool has_next = j + 1 < n_max;
+          auto wait_k = [&]() { ok = mbar_wait_warp<true>(smem_u32(&sh.k_full[sn]), ((kv + j + 1) / Cfg::kStages) & 1, abort_flag); };
+          ok = mbar_wait_warp<true>(smem_u32(&sh.v_full[s]), ((kv + j) / Cfg::kStages) & 1, abort_flag);
+          if (PADDED && ok && (j + 1) * kBlockN > x.sk)
+            clear_v_rows<Cfg::kPanels>(smem + (smem_v - smem_q) + s * Cfg::kTileBytes, x.sk - j * kBlockN, lane);
           // K of the next tile is waited for behind P V of this one, which does not need it (its load takes about 2000 clk where
           // two CTAs with a stage each share an SM).  Pairs with dropout and without a causal mask wait ahead of it: their two groups
           // then take turns better (us: 2 x 16384 and 126 x 64 tokens, 4 heads 1603 -> 1486, 16 x 256 queries, 4096 keys, 16 heads
@@ -447,100 +592,121 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 #pragma unroll
           for (int g = 0; g < G; ++g) {
             if (ok && j < n_tiles[g]) {
-              if constexpr (Cfg::kHalfP) {
-                ok = mbar_wait_warp<true>(smem_u32(&sh.p_half[g]), j & 1, abort_flag);
+              const bool more = j + 1 < n_tiles[g];
+              if constexpr (kHalfP) {
+                ok = mbar_wait_warp<true>(smem_u32(&sh.p_half[g]), c[g] & 1, abort_flag);
                 if (ok) {
                   tc_fence_after();
-                  issue_pv(g, s, j > 0, 0, Cfg::kFirstSteps);
+                  issue_pv(g, s, j > 0, 0, kFirstSteps);
                 }
               }
-              if (ok) ok = mbar_wait_warp<true>(smem_u32(&sh.p_full[g]), j & 1, abort_flag);
+              if (ok) ok = mbar_wait_warp<true>(smem_u32(&sh.p_full[g]), c[g] & 1, abort_flag);
               if (ok) {
                 tc_fence_after();
-                issue_pv(g, s, j > 0, Cfg::kFirstSteps, kBlockN / 16);
-                if (j + 1 < n_tiles[g]) {
+                issue_pv(g, s, j > 0, kFirstSteps, kBlockN / 16);
+                ++c[g];
+                if (more) {
                   if (!k_here) wait_k();
                   k_here = true;
-                  if (ok) issue_qk(g, sn);
-                } else if (Cfg::kHalfP) {  // (S of the next tile reports the others)
+                  if (ok) issue_qk(g, sn, j + 2 == n_tiles[g]);
+                } else if (kHalfP) {  // (S of the next tile reports the others)
                   if (elect_one()) mma_commit(smem_u32(&sh.o_full[g]));
                 }
               }
             }
           }
-        }
-        if (!ok) break;
-        if (elect_one()) {
-          if (!Cfg::kSeparateP) mma_commit(smem_u32(&sh.v_empty[s]));
-          if (has_next) mma_commit(smem_u32(&sh.k_empty[sn]));
+          if (!ok) break;
+          if (elect_one()) {
+            mma_commit(smem_u32(&sh.v_empty[s]));
+            if (has_next) mma_commit(smem_u32(&sh.k_empty[sn]));
+          }
         }
       }
-      mma_drain(smem_u32(&sh.drained[0]));
-    }
+      kv += n_max;
+    } while (ok && next_block(k++));
+    mma_drain(smem_u32(&sh.drained[0]));
   } else if (warp == Cfg::kSoftmaxWarps + 2) {
     // ------------------------------------------------------------------ second MMA issuer (d = 64): P*V
     if constexpr (Cfg::kSeparateP) {
       constexpr uint32_t idesc_pv = make_idesc(BF16, false, true, kBlockM, D);
       const uint64_t desc_v = make_smem_desc(smem_v, 16384, 1024);
       bool ok = true;
-      for (int j = 0; j < n_max && ok; ++j) {
-        const int s = j % Cfg::kStages;
-        ok = mbar_wait_warp<true>(smem_u32(&sh.v_full[s]), (j / Cfg::kStages) & 1, abort_flag);
-        if (!ok) break;
-        if (PADDED && (j + 1) * kBlockN > sk)
-          clear_v_rows<Cfg::kPanels>(smem + (smem_v - smem_q) + s * Cfg::kTileBytes, sk - j * kBlockN, lane);
-        const uint64_t va = desc_here(desc_at(desc_v, s * Cfg::kTileBytes));
+      int kv = 0, c[G] = {};  // as above
+      uint32_t k = 0;
+      do {
+        const FwdBlock x = block_at(k);
+        int n_tiles[G];
+        for (int g = 0; g < G; ++g) n_tiles[g] = __shfl_sync(0xffffffffu, x.n(g), 0);
+        const int n_max = max(n_tiles[0], n_tiles[G - 1]);
+        for (int j = 0; j < n_max && ok; ++j, ++kv) {
+          const int s = kv % Cfg::kStages;
+          ok = mbar_wait_warp<true>(smem_u32(&sh.v_full[s]), (kv / Cfg::kStages) & 1, abort_flag);
+          if (!ok) break;
+          if (PADDED && (j + 1) * kBlockN > x.sk)
+            clear_v_rows<Cfg::kPanels>(smem + (smem_v - smem_q) + s * Cfg::kTileBytes, x.sk - j * kBlockN, lane);
+          const uint64_t va = desc_here(desc_at(desc_v, s * Cfg::kTileBytes));
 #pragma unroll
-        for (int g = 0; g < G; ++g) {
-          if (ok && j < n_tiles[g]) {
-            ok = mbar_wait_warp<true>(smem_u32(&sh.p_full[g]), j & 1, abort_flag);
-            if (ok) {
-              tc_fence_after();
-              const uint32_t tO = tmem + (g == 0 ? Cfg::kTmemO0 : Cfg::kTmemO1);
-              const uint32_t tP = tmem + (g == 0 ? Cfg::kTmemP0 : Cfg::kTmemP1);
-              if (elect_one()) {
+          for (int g = 0; g < G; ++g) {
+            if (ok && j < n_tiles[g]) {
+              ok = mbar_wait_warp<true>(smem_u32(&sh.p_full[g]), c[g] & 1, abort_flag);
+              if (ok) {
+                tc_fence_after();
+                ++c[g];
+                const uint32_t tO = tmem + (g == 0 ? Cfg::kTmemO0 : Cfg::kTmemO1);
+                const uint32_t tP = tmem + (g == 0 ? Cfg::kTmemP0 : Cfg::kTmemP1);
+                if (elect_one()) {
 #pragma unroll
-                for (int ks = 0; ks < kBlockN / 16; ++ks)
-                  mma_ts(tO, tP + ks * 8, desc_at(va, ks * 2048), idesc_pv, j > 0 || ks > 0);
-                mma_commit(smem_u32(&sh.o_full[g]));
+                  for (int ks = 0; ks < kBlockN / 16; ++ks)
+                    mma_ts(tO, tP + ks * 8, desc_at(va, ks * 2048), idesc_pv, j > 0 || ks > 0);
+                  mma_commit(smem_u32(&sh.o_full[g]));
+                }
               }
             }
           }
+          if (!ok) break;
+          if (elect_one()) mma_commit(smem_u32(&sh.v_empty[s]));
         }
-        if (!ok) break;
-        if (elect_one()) mma_commit(smem_u32(&sh.v_empty[s]));
-      }
+      } while (ok && next_block(k++));
       mma_drain(smem_u32(&sh.drained[1]));
     }
   } else if (kLateLook && warp == Cfg::kSoftmaxWarps + 3) {
-    if constexpr (PADDED)
-      zero_padding(a, b, h, mp * G * kBlockM, (mp + 1) * G * kBlockM, q_start - b * a.pad_rows, sq, lane, 32);
     if (lane == 0 && launch_failed()) *abort_flag = 1;
+    if constexpr (PADDED) {
+      uint32_t k = 0;
+      do {
+        const FwdBlock x = block_at(k);
+        zero_padding(a, x.b, x.h, x.mp * G * kBlockM, (x.mp + 1) * G * kBlockM, x.q_start - x.b * a.pad_rows, x.sq, lane, 32);
+      } while (next_block(k++));
+    }
   } else if (Cfg::kRows && warp < Cfg::kSoftmaxWarps) {
     // ------------------------------------------------------------------ softmax groups, one thread per query row
     reg_alloc<Cfg::kSoftmaxRegs>();
-    const int g = warp >> 2;
+    const int g = (G == 1) ? 0 : warp >> 2;
     const int row = tid & 127;
-    const int ig = m0[g] + row;  // query index within the sequence
     const uint32_t lane_sel = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t tS = tmem + (g == 0 ? Cfg::kTmemS0 : Cfg::kTmemS1) + lane_sel;
     const uint32_t tO = tmem + (g == 0 ? Cfg::kTmemO0 : Cfg::kTmemO1) + lane_sel;
     const uint32_t tP = tmem + (g == 0 ? Cfg::kTmemP0 : Cfg::kTmemP1) + lane_sel;
-    const int n = n_tiles[g];
-    const bool active = m0[g] < sq;
-
-    float m_run = -INFINITY, l_run = 0.f;
     bool ok = true;
     const uint64_t c2 = pack_f2(a.scale_log2, a.scale_log2);
+    int t = 0;                // key tiles so far
+    uint32_t k = 0, c_o = 0;  // block; blocks with key tiles before
+    do {
+    const FwdBlock& x = block_at(k);
+    const int n = x.n(g);
+    float m_run = -INFINITY, l_run = 0.f;
+    const int free_tiles = CAUSAL ? min(x.sk / kBlockN, x.mp * G + g) : x.sk / kBlockN;  // key tiles without a mask
 
-    for (int j = 0; j < n && ok; ++j) {
+    for (int j = 0; j < n && ok; ++j, ++t) {
       const int col0 = kv_tile(j) * kBlockN;
       int32_t bs_it = 0;
-      if constexpr (BLOCKSPARSE)
+      if constexpr (BLOCKSPARSE) {
+        const int b = x.b, ig = (x.mp * G + g) * kBlockM + row;
         bs_it = (ig >> 4) < a.bs_rows16
                     ? a.bs_iter[(static_cast<int64_t>(b) * a.bs_kblocks + (col0 >> 8)) * a.bs_rows16 + (ig >> 4)]
                     : -1;
-      ok = mbar_wait_warp<true>(smem_u32(&sh.s_full[g]), j & 1, abort_flag);
+      }
+      ok = mbar_wait_warp<true>(smem_u32(&sh.s_full[g]), t & 1, abort_flag);
       if (!ok) break;
       tc_fence_after();
       uint32_t sr[4][32];
@@ -552,9 +718,8 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         mbar_arrive(smem_u32(&sh.s_free[g]));
       }
 
-      bool need_mask = (col0 + kBlockN > sk);
-      if (CAUSAL) need_mask = need_mask || (col0 + kBlockN - 1 > m0[g]);
-      if (need_mask) {
+      if (kv_tile(j) >= free_tiles) {
+        const int ig = (x.mp * G + g) * kBlockM + row, sk = x.sk;  // query index within the sequence
 #pragma unroll
         for (int c = 0; c < 4; ++c)
 #pragma unroll
@@ -617,7 +782,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       // scores were issued behind it.  (Else: half of the exponentials are still to come, and by now it has, as a rule.)
       if (j > 0) {
         if constexpr (Cfg::kSeparateP) {
-          ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), (j - 1) & 1, abort_flag);
+          ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), (t & 1) ^ 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
         }
@@ -645,8 +810,8 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       // 300 92.3 -> 91.0 -> 90.5.  (Traces, 4 x 12 x 4096: a group's 3560 clk a tile are 200 for the scores, 300 for the maximum, 1500
       // exponentials beside the other group's, 170 of that wait, 1070 from P to the next S.)
       tmem_st32(tP, reinterpret_cast<uint32_t(&)[32]>(pk[0]));
-      if constexpr (Cfg::kHalfP) {
-        static_assert(Cfg::kFirstSteps == 6, "96 keys");
+      if constexpr (kHalfP) {
+        static_assert(kFirstSteps == 6, "96 keys");
         expo(64, 96);
         tmem_st16(tP + 32, reinterpret_cast<uint32_t(&)[16]>(pk[32]));
         expo(96, 104);
@@ -662,7 +827,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         unpack_f2(add2(sum_a, sum_b), s0, s1);
         l_run = l_run * alpha + (s0 + s1);
       }
-      if constexpr (Cfg::kHalfP) tmem_st16(tP + 48, reinterpret_cast<uint32_t(&)[16]>(pk[48]));
+      if constexpr (kHalfP) tmem_st16(tP + 48, reinterpret_cast<uint32_t(&)[16]>(pk[48]));
       else tmem_st32(tP + 32, reinterpret_cast<uint32_t(&)[32]>(pk[32]));
       tmem_wait_st();
       tc_fence_before();
@@ -670,15 +835,24 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     }
 
     // ---------------- epilogue: O = acc / (sum * p_keep), LSE
-    if (active) {
+    const int m_first = (x.mp * G + g) * kBlockM, sq = x.sq;
+    if (m_first < sq) {
       if (n > 0 && ok) {
-        ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), Cfg::kHalfP ? 0 : (n - 1) & 1, abort_flag);
+        ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), (kHalfP ? c_o : t - 1) & 1, abort_flag);
         tc_fence_after();
       }
-      // every product that reads this group's Q has finished: its tile takes the output
-      store_rows<BF16, D / 32, Cfg::kBoxRows>(a, &tm_o, tO, 0, n > 0 && ok, ok, m0[g] + (warp & 3) * 32, lane, sq, q_start, b, h, m_run, l_run,
-                               smem + g * Cfg::kTileBytes + (warp & 3) * (D * 64));
+      // (every product that reads this group's Q has finished: without other blocks its tile takes the output)
+      store_rows<BF16, D / 32, Cfg::kBoxRows, TAKE && !Cfg::kOutInV>(a, &tm_o, tO, 0, n > 0 && ok, ok, m_first + (warp & 3) * 32, lane, sq, x.q_start, x.b, x.h,
+                               m_run, l_run, TAKE ? smem + ((Cfg::kOutInV ? smem_v : smem_out) - smem_q) + warp * Cfg::kOutPiece
+                                                  : smem + g * Cfg::kTileBytes + (warp & 3) * (D * 64));
     }
+    if (n > 0) ++c_o;
+    if constexpr (Cfg::kOutInV) {
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&sh.out_free));
+    }
+    } while (ok && next_block(k++));
+    if (TAKE && lane == 0) bulk_wait_read();
   } else if (warp < Cfg::kSoftmaxWarps) {
     // ------------------------------------------------------------------ softmax warps
     // A warp owns 16 query rows.  It reads their scores with the 16x256b shape, in which a thread holds rows r8 and
@@ -688,24 +862,23 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     const int g = (G == 1) ? 0 : warp >> 3;
     const int hh = (warp >> 2) & 1, wq = warp & 3;
     const int r8 = lane >> 2, q4 = lane & 3;
-    const int m_first = m0[G == 1 ? 0 : g];
-    const int row0 = m_first + wq * 32 + hh * 16;  // of the warp; query index within the sequence
     const uint32_t lane_sel = static_cast<uint32_t>(wq * 32 + hh * 16) << 16;
     const uint32_t tS = tmem + (g == 0 ? Cfg::kTmemS0 : Cfg::kTmemS1) + lane_sel;
     const uint32_t tO = tmem + (g == 0 ? Cfg::kTmemO0 : Cfg::kTmemO1) + lane_sel;
     const uint32_t tP = tmem + (g == 0 ? Cfg::kTmemP0 : Cfg::kTmemP1) + lane_sel;
-    const int n = n_tiles[G == 1 ? 0 : g];
-    const bool active = m_first < sq;
-
-    // rows r8 (u = 0) and r8 + 8 (u = 1); l_run: this thread's share of the row sum (its 32 columns per tile)
-    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
     bool ok = true;
     const uint64_t c2 = pack_f2(a.scale_log2, a.scale_log2);
+    int t = 0;                // key tiles so far
+    uint32_t k = 0, c_s = 0;  // block; blocks with queries before
+    do {
+    const FwdBlock& x = block_at(k);
+    const int n = x.n(g);
+    // rows r8 (u = 0) and r8 + 8 (u = 1); l_run: this thread's share of the row sum (its 32 columns per tile)
+    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
+    const int free_tiles = CAUSAL ? min(x.sk / kBlockN, x.mp * G + g) : x.sk / kBlockN;  // key tiles without a mask
 
     const int64_t bh_sub =
-        (static_cast<int64_t>(b) * a.drop.heads_total + a.drop.head_offset + h) * 256;
-    const int L16 = (sq + 15) >> 4;
-    const int i16 = row0 >> 4;
+        (static_cast<int64_t>(x.b) * a.drop.heads_total + a.drop.head_offset + x.h) * 256;
     QuadPhilox<8> qp;
     float thr_term = 0.f;
     if constexpr (DROPOUT) {
@@ -718,19 +891,23 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       if (lane == 0) mbar_arrive(smem_u32(&bar));
     };
 
-    for (int j = 0; j < n && ok; ++j) {
+    for (int j = 0; j < n && ok; ++j, ++t) {
       const int col0 = kv_tile(j) * kBlockN;
       int32_t bs_it = 0;
-      if constexpr (BLOCKSPARSE)
+      if constexpr (BLOCKSPARSE) {
+        const int i16 = ((x.mp * G + g) * kBlockM + wq * 32 + hh * 16) >> 4;
         bs_it = i16 < a.bs_rows16
-                    ? a.bs_iter[(static_cast<int64_t>(b) * a.bs_kblocks + (col0 >> 8)) * a.bs_rows16 + i16]
+                    ? a.bs_iter[(static_cast<int64_t>(x.b) * a.bs_kblocks + (col0 >> 8)) * a.bs_rows16 + i16]
                     : -1;
-      const bool need_mask = (col0 + kBlockN > sk) || (CAUSAL && (col0 + kBlockN - 1 > m_first)) ||
-                             (BLOCKSPARSE && bs_it < 0);
+      }
+      const bool need_mask = TAKE ? j >= free_tiles
+                                  : (col0 + kBlockN > x.sk) || (CAUSAL && (col0 + kBlockN - 1 > (x.mp * G + g) * kBlockM)) ||
+                                        (BLOCKSPARSE && bs_it < 0);
       // -inf for columns without a key, keys behind the diagonal and 16-row blocks that are not in the layout; s[]
       // holds the units from unit0 on, s[4 * unit + 2 * u + c] = (row r8 + 8 u, column 8 unit + 2 q4 + c)
       auto mask = [&](auto& s, int unit0) {
         constexpr int kValues = sizeof(s) / 4;
+        const int sk = x.sk, row0 = (x.mp * G + g) * kBlockM + wq * 32 + hh * 16;  // of the warp; query index within the sequence
 #pragma unroll
         for (int i = 0; i < kValues; ++i) {
           const int col = col0 + (unit0 + (i >> 2)) * 8 + 2 * q4 + (i & 1);
@@ -740,7 +917,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           if (!valid) s[i] = __float_as_uint(-INFINITY);
         }
       };
-      ok = mbar_wait_warp<true>(smem_u32(&sh.s_full[g]), j & 1, abort_flag);
+      ok = mbar_wait_warp<true>(smem_u32(&sh.s_full[g]), t & 1, abort_flag);
       if (!ok) break;
       tc_fence_after();
       uint32_t sr[64];
@@ -779,14 +956,14 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         }
         if (j > 0) {
           // P*V of the previous tile must have finished before O is rescaled
-          ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), (j - 1) & 1, abort_flag);
+          ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), (t & 1) ^ 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
           const uint64_t al[2] = {pack_f2(alpha[0], alpha[0]), pack_f2(alpha[1], alpha[1])};
 #pragma unroll 1
-          for (int c = 0; c < D; c += 32) {
+          for (int col = 0; col < D; col += 32) {
             uint32_t orr[16];
-            tmem_ld_quad16(tO + c, orr);
+            tmem_ld_quad16(tO + col, orr);
             tmem_wait_ld();
 #pragma unroll
             for (int i = 0; i < 16; i += 2) {
@@ -795,7 +972,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
               orr[i] = __float_as_uint(lo);
               orr[i + 1] = __float_as_uint(hi);
             }
-            tmem_st_quad16(tO + c, orr);
+            tmem_st_quad16(tO + col, orr);
           }
           tmem_wait_st();
         }
@@ -813,7 +990,8 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       if constexpr (DROPOUT) {
         int64_t it_index;
         if constexpr (BLOCKSPARSE) it_index = bs_it;
-        else it_index = fa_iter_index(CAUSAL, col0 >> a.drop.n_shift, i16, L16, a.drop.n_shift);
+        else it_index = fa_iter_index(CAUSAL, col0 >> a.drop.n_shift, ((x.mp * G + g) * kBlockM + wq * 32 + hh * 16) >> 4,
+                                      (x.sq + 15) >> 4, a.drop.n_shift);
         qp.set_tile(a.drop, it_index, col0);
       }
 #pragma unroll
@@ -861,7 +1039,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         }
         if (half == 0 && j > 0) {
           // P*V of the previous tile must have finished before its P buffer is reused
-          ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), (j - 1) & 1, abort_flag);
+          ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), (t & 1) ^ 1, abort_flag);
           if (!ok) break;
           tc_fence_after();
         }
@@ -883,24 +1061,34 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 
     // ---------------- epilogue: O = acc / (sum * p_keep), LSE.  One thread per query row (32 rows per warp, half of the
     // columns): the statistics of a row pass through shared memory.
-    if (active) {
+    const int m_first = (x.mp * G + g) * kBlockM;
+    if (m_first < x.sq) {
+      float2* stats = sh.row_stats[TAKE ? 2 * g + (k & 1) : g];
 #pragma unroll
       for (int u = 0; u < 2; ++u) {
         float l = l_run[u];
         l += __shfl_xor_sync(0xffffffffu, l, 1);
         l += __shfl_xor_sync(0xffffffffu, l, 2);
-        if (q4 == 0) sh.row_stats[g][wq * 32 + hh * 16 + u * 8 + r8] = make_float2(m_run[u], l);
+        if (q4 == 0) stats[wq * 32 + hh * 16 + u * 8 + r8] = make_float2(m_run[u], l);
       }
-      named_barrier_sync(1 + g, 32 * Cfg::kGroupWarps);  // every warp of the group comes here, also after an abandoned wait
+      if constexpr (TAKE) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&sh.stats_full[g]));
+        if (ok) ok = mbar_wait_warp<true>(smem_u32(&sh.stats_full[g]), c_s++ & 1, abort_flag);
+      } else {
+        named_barrier_sync(1 + g, 32 * Cfg::kGroupWarps);  // every warp of the group comes here, also after an abandoned wait
+      }
       if (n > 0 && ok) {
-        ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), (n - 1) & 1, abort_flag);
+        ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), (t - 1) & 1, abort_flag);
         tc_fence_after();
       }
-      const float2 st = sh.row_stats[g][wq * 32 + lane];
-      store_rows<BF16, D / 64, Cfg::kBoxQuads>(a, &tm_o, tO - (static_cast<uint32_t>(hh * 16) << 16), hh * (D / 64), n > 0 && ok, ok,
-                               m_first + wq * 32, lane, sq, q_start, b, h, st.x, st.y,
-                               smem + g * Cfg::kTileBytes + (wq * 2 + hh) * (D * 32));
+      const float2 st = stats[wq * 32 + lane];
+      uint8_t* piece = TAKE ? smem + (smem_out - smem_q) + warp * Cfg::kOutPiece : smem + g * Cfg::kTileBytes + (wq * 2 + hh) * (D * 32);
+      store_rows<BF16, D / 64, Cfg::kBoxQuads, TAKE>(a, &tm_o, tO - (static_cast<uint32_t>(hh * 16) << 16), hh * (D / 64),
+                               n > 0 && ok, ok, m_first + wq * 32, lane, x.sq, x.q_start, x.b, x.h, st.x, st.y, piece);
     }
+    } while (ok && next_block(k++));
+    if (TAKE && lane == 0) bulk_wait_read();
   }
 
   tc_fence_before();
@@ -914,36 +1102,57 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   }
 }
 
-// Announced lengths above twice the actual ones on average: the grid consists mostly of blocks without queries.
-inline bool uneven(const FwdLaunch& l) {
-  return static_cast<int64_t>(l.args.batch) * l.max_seqlen_q > 2 * static_cast<int64_t>(l.total_q);
+// Announced lengths above `times` the actual ones on average: the grid consists mostly of blocks without queries.
+inline bool uneven(const FwdLaunch& l, int times = 2) {
+  return static_cast<int64_t>(l.args.batch) * l.max_seqlen_q > times * static_cast<int64_t>(l.total_q);
 }
 
 constexpr int kSms = 148;
 
-// Causal grids with their last tiles in order of weight (set_tail_grid): where the blocks do not all start at once,
-// and not up to 512 queries (four tiles: nothing to gain, and a place that is computed takes registers that blockIdx does not:
-// us, pair by pair -> ordered, d = 128, 64 x 12 x 256 60 -> 65, 64 x 12 x 300 86 -> 91, 32 x 12 x 512 ragged 56 -> 59, 4 x 4 x
-// 600 ragged (80 blocks) 12.0 -> 13.0).
+// Blocks that start at once
 template <int G>
-bool tail_order(const FwdLaunch& l, int tiles) {
-  return l.max_seqlen_q > 512 && linear_grid(tiles, l.args.heads, l.args.batch) &&
-         static_cast<int64_t>(tiles) * l.args.heads * l.args.batch > (G == 1 ? 2 : 1) * kSms;
-}
+constexpr int kSlots = (G == 1 ? 2 : 1) * kSms;
 
-template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BS, int G, bool ROWS, bool ORDERED = false, bool PADDED = false>
+// Causal grids with their last tiles in order of weight (set_tail_grid): where the blocks do not all start at once, and not up to 512
+// queries (four tiles: nothing to gain, and with a CTA per block a place that is computed cost 5-8 %).
+inline bool tail_order(const FwdLaunch& l) { return l.max_seqlen_q > 512; }
+
+// Whether a CTA goes on with blocks that have not started (cluster launch control, in the order of the grid) where there are more
+// than start at once.  The next block's Q, K and V load and its first scores are made while the rows of the one before leave; a CTA
+// of its own began with barriers, tensor memory and 3500 clk for its first scores, about two key tiles.  us, a CTA per block -> now:
+// d = 128, 16 x 12 x 1000 causal 85.5 -> 77.7, 64 x 12 x 256 59.4 -> 49.1, 32 x 12 x 512 ragged 61.4 -> 54.7, in pairs of tiles 4 x 32 x
+// 3000 causal 293 -> 269, 4 x 12 x 4096 343 -> 328, 16 x 12 x 8192 causal 2570 -> 2490; d = 64, 64 x 12 x 300 69.7 -> 59.3, padded
+// 64 x 12 x 512 ragged 92 -> 82; blocks without queries, which the producer passes over: 1 x 4096 and 63 x 128 tokens, 12 heads 182 ->
+// 116 (d = 64), 172 -> 128.
+// Quads of d = 64 up to some length alone: their two CTAs on an SM take longer for a tile, most of all in long walks (32 768 tokens, 12 heads,
+// not causal / causal, over a CTA per block: 600 0.95 / 0.87, 1024 0.96 / 0.92, 1500 0.99 / 0.95, 2048 1.02 / 0.96, 2560 1.01 / 0.99, 3000
+// 1.02 / 1.00, 4096 1.08 / 1.02, 1 x 2 x 65536 causal 1.09), unless most blocks are empty (31 x 256 and 1 x 8192: 0.97 / 0.91; announced with 2.5
+// times their tokens, 2 x 16384 and 3 x 1, 1.04).  Not with dropout: the loop has no registers left for it (8-14 % slower).
+template <int D, bool ROWS, bool CAUSAL>
+constexpr int kTakeMaxKeys = D == 64 && !ROWS ? (CAUSAL ? 2560 : 1536) : INT_MAX;
+
+template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BS, int G, bool ROWS, bool PADDED = false, Order ORDER = kPlain>
 cudaError_t launch_groups(const FwdLaunch& l, cudaStream_t stream) {
   dim3 grid((l.max_seqlen_q + G * kBlockM - 1) / (G * kBlockM), l.args.heads, l.args.batch);
-  if constexpr (CAUSAL && !ORDERED && !PADDED)
-    if (tail_order<G>(l, grid.x)) return launch_groups<D, BF16, CAUSAL, DROPOUT, BS, G, ROWS, true>(l, stream);
-  auto kernel = fa_fwd_kernel<D, BF16, CAUSAL, DROPOUT, BS, G, ROWS, ORDERED, PADDED>;
-  using Cfg = FwdCfg<D, G, ROWS>;
+  if constexpr (ORDER == kPlain) {
+    if (linear_grid(grid.x, grid.y, grid.z) && int64_t(grid.x) * grid.y * grid.z > kSlots<G>) {
+      constexpr bool kCanTake = !BS && !DROPOUT;
+      constexpr int kMaxKeys = kTakeMaxKeys<D, ROWS, CAUSAL>;
+      if constexpr (kCanTake)
+        if (l.max_seqlen_k <= kMaxKeys || uneven(l, 3))
+          return launch_groups<D, BF16, CAUSAL, DROPOUT, BS, G, ROWS, PADDED, kTake>(l, stream);
+      if constexpr (CAUSAL && !(kCanTake && kMaxKeys == INT_MAX))
+        if (tail_order(l)) return launch_groups<D, BF16, CAUSAL, DROPOUT, BS, G, ROWS, PADDED, kLinear>(l, stream);
+    }
+  }
+  auto kernel = fa_fwd_kernel<D, BF16, CAUSAL, DROPOUT, BS, G, ROWS, ORDER, PADDED>;
+  using Cfg = FwdCfg<D, G, ROWS, ORDER == kTake>;
   static SmemLimitFlags smem_limit_set;  // one per template instantiation of this function
   cudaError_t e = set_smem_limit_once(kernel, Cfg::kSmemBytes, smem_limit_set);
   if (e != cudaSuccess) return e;
   KernelArgs args = l.args;
-  if constexpr (ORDERED) {
-    set_tail_grid(&args, grid.x, int64_t(4) * D * l.max_seqlen_k);  // K and V
+  if constexpr (ORDER != kPlain) {
+    set_tail_grid(&args, grid.x, CAUSAL && tail_order(l) ? int64_t(4) * D * l.max_seqlen_k : 0);  // K and V
     grid = dim3(grid.x * grid.y * grid.z, 1, 1);
   }
   kernel<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(l.tm_q, l.tm_k, l.tm_v, l.tm_o, args);
@@ -1019,12 +1228,12 @@ cudaError_t launch_one(const FwdLaunch& l, cudaStream_t stream) {
   const bool one_tile = one_tile_per_cta<D, CAUSAL, DROPOUT>(l);
   if constexpr (!DROPOUT) {
     if (rows_layout<D, DROPOUT>(l))
-      return one_tile ? launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 1, true, false, PADDED>(l, stream)
-                      : launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 2, true, false, PADDED>(l, stream);
+      return one_tile ? launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 1, true, PADDED>(l, stream)
+                      : launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 2, true, PADDED>(l, stream);
   }
   if constexpr (D == 64 || DROPOUT) {
-    return one_tile ? launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 1, false, false, PADDED>(l, stream)
-                    : launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 2, false, false, PADDED>(l, stream);
+    return one_tile ? launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 1, false, PADDED>(l, stream)
+                    : launch_groups<D, BF16, CAUSAL, DROPOUT, BS, 2, false, PADDED>(l, stream);
   }
   return cudaErrorInvalidValue;
 }

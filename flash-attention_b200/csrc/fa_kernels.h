@@ -109,7 +109,8 @@ __host__ __device__ __forceinline__ void causal_block(const KernelArgs& a, uint3
 constexpr int64_t kTailBlocks = 1024, kTailBytes = 64 << 20;
 inline void set_tail_grid(KernelArgs* a, int tiles, int64_t bytes_per_pair) {
   const int64_t pairs = static_cast<int64_t>(a->heads) * a->batch;
-  int64_t last = kTailBlocks / tiles < kTailBytes / bytes_per_pair ? kTailBlocks / tiles : kTailBytes / bytes_per_pair;
+  int64_t last = 1;  // (bytes_per_pair = 0: all pair by pair, which with one last pair comes to the same)
+  if (bytes_per_pair > 0) last = kTailBlocks / tiles < kTailBytes / bytes_per_pair ? kTailBlocks / tiles : kTailBytes / bytes_per_pair;
   if (last > pairs) last = pairs;
   if (last < 1) last = 1;
   a->tail_tiles = fast_div(tiles);
