@@ -240,10 +240,11 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
               const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_o, const KernelArgs a) {
   constexpr bool TAKE = ORDER == kTake, LINEAR = ORDER != kPlain;
   using Cfg = FwdCfg<D, G, ROWS, TAKE>;
-  // d = 128 without dropout: P is handed over in two parts, so that P*V of the first 96 keys runs while the
-  // rest is exponentiated; S of the next tile waits for P*V there, and so tells that it is over.
-  constexpr bool kHalfP = Cfg::kRows && !Cfg::kSeparateP;
-  constexpr int kFirstSteps = kHalfP ? 6 : 0;  // of 16 keys, in the first part
+  // d = 128: P is handed over in two parts, so that P*V of the first 96 keys (64 in quads) runs while the rest is exponentiated; S of
+  // the next tile waits for P*V there, and so tells that it is over.  Quads, us, whole and waited for -> now: 4 x 12 x 4096 causal with
+  // dropout 298 -> 290, 2 x 16384 and 126 x 64, 4 heads 1486 -> 1450, causal 922 -> 892, 16 x 256 queries, 4096 keys 198 -> 190.
+  constexpr bool kHalfP = !Cfg::kSeparateP;
+  constexpr int kFirstSteps = kHalfP ? (Cfg::kRows ? 6 : 4) : 0;  // of 16 keys, in the first part
   extern __shared__ uint8_t smem_raw[];
   __shared__ FwdShared<ROWS ? 1 : TAKE ? 2 * G : G> sh;
   // block-sparse: key tiles this CTA visits (ascending), built from the layout table
@@ -811,7 +812,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       // exponentials beside the other group's, 170 of that wait, 1070 from P to the next S.)
       tmem_st32(tP, reinterpret_cast<uint32_t(&)[32]>(pk[0]));
       if constexpr (kHalfP) {
-        static_assert(kFirstSteps == 6, "96 keys");
+        static_assert(!Cfg::kRows || kFirstSteps == 6, "96 keys");
         expo(64, 96);
         tmem_st16(tP + 32, reinterpret_cast<uint32_t(&)[16]>(pk[32]));
         expo(96, 104);
@@ -869,7 +870,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     bool ok = true;
     const uint64_t c2 = pack_f2(a.scale_log2, a.scale_log2);
     int t = 0;                // key tiles so far
-    uint32_t k = 0, c_s = 0;  // block; blocks with queries before
+    uint32_t k = 0, c_o = 0, c_s = 0;  // block; blocks with key tiles before, with queries before
     do {
     const FwdBlock& x = block_at(k);
     const int n = x.n(g);
@@ -955,10 +956,12 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           l_run[u] *= alpha[u];
         }
         if (j > 0) {
-          // P*V of the previous tile must have finished before O is rescaled
-          ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), (t & 1) ^ 1, abort_flag);
-          if (!ok) break;
-          tc_fence_after();
+          // P*V of the previous tile must have finished before O is rescaled (with P in parts: see the rows)
+          if constexpr (!kHalfP) {
+            ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), (t & 1) ^ 1, abort_flag);
+            if (!ok) break;
+            tc_fence_after();
+          }
           const uint64_t al[2] = {pack_f2(alpha[0], alpha[0]), pack_f2(alpha[1], alpha[1])};
 #pragma unroll 1
           for (int col = 0; col < D; col += 32) {
@@ -1037,7 +1040,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             pk[2 * unit + 2 + u] = pack_lowp<BF16>(p2, p3);
           }
         }
-        if (half == 0 && j > 0) {
+        if (!kHalfP && half == 0 && j > 0) {
           // P*V of the previous tile must have finished before its P buffer is reused
           ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), (t & 1) ^ 1, abort_flag);
           if (!ok) break;
@@ -1045,6 +1048,10 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         }
         // hand P to the tensor core through tensor memory
         tmem_st_pair16(tP + half * 32, pk);
+        if (kHalfP && half == 0) {
+          tmem_wait_st();
+          arrive_warp(sh.p_half[g]);
+        }
       }
       if (ok) {
         tmem_wait_st();
@@ -1079,7 +1086,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         named_barrier_sync(1 + g, 32 * Cfg::kGroupWarps);  // every warp of the group comes here, also after an abandoned wait
       }
       if (n > 0 && ok) {
-        ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), (t - 1) & 1, abort_flag);
+        ok = mbar_wait_warp<true>(smem_u32(&sh.o_full[g]), (kHalfP ? c_o : t - 1) & 1, abort_flag);
         tc_fence_after();
       }
       const float2 st = stats[wq * 32 + lane];
@@ -1087,6 +1094,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       store_rows<BF16, D / 64, Cfg::kBoxQuads, TAKE>(a, &tm_o, tO - (static_cast<uint32_t>(hh * 16) << 16), hh * (D / 64),
                                n > 0 && ok, ok, m_first + wq * 32, lane, x.sq, x.q_start, x.b, x.h, st.x, st.y, piece);
     }
+    if (n > 0) ++c_o;
     } while (ok && next_block(k++));
     if (TAKE && lane == 0) bulk_wait_read();
   }
