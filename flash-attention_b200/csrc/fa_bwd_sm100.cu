@@ -93,9 +93,10 @@ struct BwdCfg {
   static constexpr uint32_t kTmemDS = 256 + 3 * D;
 };
 
-// What a block works on: key tile n0 / 128 of one (batch, head) pair.  nm: query tiles to walk, -1 behind the last block
+// What a block works on: key tile n0 / 128 of one (batch, head) pair.  nm: query tiles to walk, -1 behind the last block; list: which of
+// the CTA's lists holds them (block-sparse)
 struct BlockInfo {
-  int q_start, sq, k_start, sk, n0, h, b, nm;
+  int q_start, sq, k_start, sk, n0, h, b, nm, list;
 };
 
 struct BwdShared {
@@ -229,14 +230,14 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   // key tile.  Every role walks the same blocks; c counts the key tiles with work, g the query tiles walked so far,
   // which give the phases of the barriers.  Main kernel, us, a CTA per block -> now: 16 x 8 heads, 200 queries, 1500
   // keys 72.5 -> 52.5; 64 x 12 x 512 227 -> 170; 16 x 12 x 1000 causal (d = 128) 249 -> 205; 8 x 12 x 512 with dropout
-  // 41.6 -> 36.9; 2 x 4 x 16384 causal 711 -> 689; 4 x 12 x 8192 causal (d = 128) 2199 -> 2131.
-  constexpr bool kTakeOver = !BLOCKSPARSE;
+  // 41.6 -> 36.9; 2 x 4 x 16384 causal 711 -> 689; 4 x 12 x 8192 causal (d = 128) 2199 -> 2131.  Block-sparse, whole backward, 4 x
+  // 16 x 4096 with 25 % of the blocks 398 -> 334, with dropout 442 -> 385, 16 x 12 x 2048 ragged 260 -> 199.
   auto decode = [&](uint32_t block) -> BlockInfo {
     BlockInfo x;
     int nt;
     if (CAUSAL && gridDim.y == 1 && gridDim.z == 1) {
       causal_block(ka, block, nt, x.h, x.b);
-    } else if (kTakeOver && a.take_over) {
+    } else if (a.take_over) {
       const uint32_t pair = block / ka.grid_tiles;
       nt = block - pair * ka.grid_tiles;
       x.b = pair / ka.heads;
@@ -249,6 +250,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     x.k_start = ka.cu_seqlens_k[x.b];
     x.sk = ka.cu_seqlens_k[x.b + 1] - x.k_start;
     x.n0 = nt * kBN;
+    x.list = 0;
     const int m_tiles = (x.sq + kBM - 1) / kBM;
     // (a call of one launch also writes dq = 0 for a sequence without keys)
     x.nm = x.n0 < x.sk || ONE_LAUNCH ? m_tiles - (CAUSAL ? min(m_tiles, x.n0 / kBM) : 0) : 0;
@@ -259,7 +261,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   BlockInfo first = decode(blockIdx.x);
   // (not in the deterministic mode, whose blocks wait for blocks of smaller index: those start first only as the
   // hardware launches them; and not where every block has an SM at once)
-  const bool take_over = kTakeOver && a.take_over;
+  const bool take_over = a.take_over;
   // a block behind its sequence's last key.  A CTA of its own leaves here, before it takes tensor memory and sets up its
   // barriers: 1 x 4096 and 63 x 128, 12 heads, deterministic, us, through the whole kernel -> here: 869 -> 642 (d = 64),
   // 1311 -> 1044 (d = 128)
@@ -279,50 +281,51 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     return;
   }
 
-  // block-sparse: query tiles that have at least one 16-row block in this key block's list
-  __shared__ uint16_t qtile_list[BLOCKSPARSE ? kMaxSparseTiles : 1];
+  // Block-sparse: the query tiles that have at least one 16-row block in this key block's list, in ascending order; those of block k
+  // in list k % 2.  The whole CTA makes the first list, the producer's warp those of blocks taken over.
+  constexpr int kListTiles = BLOCKSPARSE ? kMaxSparseTiles : 1;
+  __shared__ uint16_t qtile_list[BLOCKSPARSE ? 2 : 1][kListTiles];
   // deterministic mode: how many key tiles before this one add into the same query tile
-  __shared__ uint16_t qtile_order[BLOCKSPARSE ? kMaxSparseTiles : 1];
-  __shared__ int qtile_count;
+  __shared__ uint16_t qtile_order[kListTiles];
+  __shared__ uint32_t qtile_bits[(kListTiles + 31) / 32];
+  // a bit for each of the query tiles [32 c, 32 c + 32) of key block kb (one warp)
+  auto list_bits = [&](const BlockInfo& x, int kb, int c, int mt) -> uint32_t {
+    const int m = c * 32 + lane, rb_end = min(ka.bs_rows16, (x.sq + 15) >> 4);
+    const int32_t* brow = ka.bs_iter + (static_cast<int64_t>(x.b) * ka.bs_kblocks + kb) * ka.bs_rows16;
+    bool any = false;
+    if (m < mt && !(CAUSAL && m < x.n0 / kBM))  // (query tiles entirely before this key tile see none of it)
+#pragma unroll
+      for (int i = 0; i < kBM / 16; ++i)
+        if (m * (kBM / 16) + i < rb_end) any = any || (brow[m * (kBM / 16) + i] >= 0);
+    return __ballot_sync(0xffffffffu, any);
+  };
+  auto list_tiles = [&](const BlockInfo& x) -> int { return min((x.sq + kBM - 1) / kBM, kMaxSparseTiles); };
+  auto put_in_list = [&](uint16_t* list, int c, uint32_t bits, int before) {
+    if (bits >> lane & 1) list[before + __popc(bits & ((1u << lane) - 1))] = static_cast<uint16_t>(c * 32 + lane);
+  };
   if constexpr (BLOCKSPARSE) {
-    const int b = first.b, sq = first.sq, n0 = first.n0, nt = n0 / kBN;
-    const int m_tiles = (sq + kBM - 1) / kBM, m_begin = CAUSAL ? min(m_tiles, n0 / kBM) : 0;
-    uint8_t* flags = reinterpret_cast<uint8_t*>(smem_raw);
-    const int32_t* brow = ka.bs_iter + (static_cast<int64_t>(b) * ka.bs_kblocks + (n0 >> 8)) * ka.bs_rows16;
-    const int rb_end = min(ka.bs_rows16, (sq + 15) >> 4);
-    const int mt = min(m_tiles, kMaxSparseTiles);
-    uint16_t* order_all = reinterpret_cast<uint16_t*>(smem_raw + kMaxSparseTiles);
-    for (int m = threadIdx.x; m < mt; m += Cfg::kThreads) {
-      bool any = false;
-      for (int rb = m * (kBM / 16); rb < min((m + 1) * (kBM / 16), rb_end); ++rb) any = any || (brow[rb] >= 0);
-      if (CAUSAL && m < m_begin) any = false;  // query tiles entirely before this key tile see none of it
-      flags[m] = any ? 1 : 0;
-      if (a.dq_tickets != nullptr && any) {
-        // the two 128-row key tiles of a 256-row key block visit the same query tiles
-        int before = 0;
-        for (int kb = 0; kb < (n0 >> 8); ++kb) {
-          const int32_t* prow = ka.bs_iter + (static_cast<int64_t>(b) * ka.bs_kblocks + kb) * ka.bs_rows16;
-          bool hit = false;
-          for (int rb = m * (kBM / 16); rb < min((m + 1) * (kBM / 16), rb_end); ++rb) hit = hit || (prow[rb] >= 0);
-          before += hit ? 2 : 0;
+    const int mt = list_tiles(first);
+    for (int c = warp; c * 32 < mt; c += Cfg::kThreads / 32) {
+      const uint32_t bits = list_bits(first, first.n0 >> 8, c, mt);
+      if (lane == 0) qtile_bits[c] = bits;
+    }
+    __syncthreads();
+    int total = 0;
+    for (int c = 0; c * 32 < mt; ++c) {
+      const uint32_t bits = qtile_bits[c];
+      if (c % (Cfg::kThreads / 32) == warp) {
+        put_in_list(qtile_list[0], c, bits, total);
+        if (a.dq_tickets != nullptr) {
+          // the two 128-row key tiles of a 256-row key block visit the same query tiles
+          int before = 0;
+          for (int kb = 0; kb < first.n0 >> 8; ++kb) before += (list_bits(first, kb, c, mt) >> lane & 1) * 2;
+          if (bits >> lane & 1)
+            qtile_order[total + __popc(bits & ((1u << lane) - 1))] = static_cast<uint16_t>(before + (first.n0 / kBN & 1));
         }
-        order_all[m] = static_cast<uint16_t>(before + ((nt & 1) ? 1 : 0));
       }
+      total += __popc(bits);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int n = 0;
-      for (int m = 0; m < mt; ++m)
-        if (flags[m]) {
-          if (a.dq_tickets != nullptr) qtile_order[n] = order_all[m];
-          qtile_list[n++] = static_cast<uint16_t>(m);
-        }
-      qtile_count = n;
-    }
-    __syncthreads();
-    first.nm = qtile_count;
-    fence_async_smem();  // (of the accesses to the lists above, which TMA overwrites)
-    __syncthreads();
+    first.nm = first.n0 < first.sk ? total : 0;  // (the list is read behind the barrier below)
   }
   // Deterministic mode: the key tiles of one (batch, head) add into a query tile in ascending
   // key-tile order.  Dense causal grids then walk the query tiles from the last one down, so that
@@ -331,7 +334,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   const bool deterministic = a.dq_tickets != nullptr;
   const bool walk_down = CAUSAL && !BLOCKSPARSE && deterministic;
   auto q_tile = [&](const BlockInfo& x, int t) -> int {
-    if constexpr (BLOCKSPARSE) return qtile_list[t];
+    if constexpr (BLOCKSPARSE) return qtile_list[x.list][t];
     const int m_tiles = (x.sq + kBM - 1) / kBM;
     return walk_down ? m_tiles - 1 - t : m_tiles - x.nm + t;  // causal: from the tile of the first key on
   };
@@ -457,8 +460,17 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 
   if (warp >= kProducer) {
     reg_dealloc<Cfg::kOtherRegs>();
-    if (warp == kProducer && lane == 0) {
+    if (warp == kProducer && (BLOCKSPARSE || lane == 0)) {
       // -------------------------------------------------------------- TMA producer
+      // (one lane; block-sparse: the warp stays together, to make the lists of blocks taken over, and one lane issues)
+      const bool lead = lane == 0;
+      auto wait = [&](uint64_t& bar, uint32_t parity) -> bool {
+        const bool done = mbar_wait(smem_u32(&bar), parity, abort_flag);
+        return BLOCKSPARSE ? __all_sync(0xffffffffu, done) : done;
+      };
+      auto load = [&](uint32_t dst, const CUtensorMap* map, uint64_t& bar, int row, int h) {
+        for (int p = 0; p < D / 64; ++p) tma_load_3d(dst + p * 16384, map, smem_u32(&bar), p * 64, row, h);
+      };
       tma_prefetch_desc(&tm_q);
       tma_prefetch_desc(&tm_k);
       tma_prefetch_desc(&tm_v);
@@ -473,8 +485,10 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         // asked for when the last query tile is under way: a block taken earlier would wait here while other SMs run dry
         auto take_next = [&]() {
           if (!take_over) return;
-          mbar_expect_tx(smem_u32(&sh.next_full), 16);
-          clc_try_cancel(smem_u32(&sh.next), smem_u32(&sh.next_full));
+          if (lead) {
+            mbar_expect_tx(smem_u32(&sh.next_full), 16);
+            clc_try_cancel(smem_u32(&sh.next), smem_u32(&sh.next_full));
+          }
           ++asked;
         };
         if (nm <= 0) take_next();
@@ -482,46 +496,45 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           const int s = loads_q % Cfg::kQStages;
           const int row = x.q_start + q_tile(x, t) * kBM;
           auto load_k = [&]() {
-            if (loads_k > 0) ok = mbar_wait(smem_u32(&sh.k_empty), (loads_k & 1) ^ 1, abort_flag);
+            if (loads_k > 0) ok = wait(sh.k_empty, (loads_k & 1) ^ 1);
             if (!ok) return;
-            mbar_expect_tx(smem_u32(&sh.k_full), Cfg::kTileBytes);
-            for (int p = 0; p < D / 64; ++p)
-              tma_load_3d(smem_k + p * 16384, &tm_k, smem_u32(&sh.k_full), p * 64, x.k_start + x.n0, h);
+            if (lead) {
+              mbar_expect_tx(smem_u32(&sh.k_full), Cfg::kTileBytes);
+              load(smem_k, &tm_k, sh.k_full, x.k_start + x.n0, h);
+            }
             ++loads_k;
           };
           const bool first_k = loads_k == 0;
           if (first_k) load_k();
           if (t == 0) {
             // V is free after the last dP of the key tile before, K after its last dQ
-            if (loads_v > 0) ok = mbar_wait(smem_u32(&sh.v_empty), (loads_v & 1) ^ 1, abort_flag);
+            if (loads_v > 0) ok = wait(sh.v_empty, (loads_v & 1) ^ 1);
             if (!ok) break;
-            mbar_expect_tx(smem_u32(&sh.v_full), Cfg::kTileBytes);
-            for (int p = 0; p < D / 64; ++p)
-              tma_load_3d(smem_v + p * 16384, &tm_v, smem_u32(&sh.v_full), p * 64, x.k_start + x.n0, h);
+            if (lead) {
+              mbar_expect_tx(smem_u32(&sh.v_full), Cfg::kTileBytes);
+              load(smem_v, &tm_v, sh.v_full, x.k_start + x.n0, h);
+            }
             ++loads_v;
           }
           if constexpr (Cfg::kTwoPhase) {
             // dO(g) follows dV(g - 1), Q(g) follows dK(g - 1): the order in which they finish
-            if (loads_do > 0) ok = mbar_wait(smem_u32(&sh.do_empty), (loads_do & 1) ^ 1, abort_flag);
+            if (loads_do > 0) ok = wait(sh.do_empty, (loads_do & 1) ^ 1);
             if (!ok) break;
-            const uint32_t bar_do = smem_u32(&sh.do_full);
-            mbar_expect_tx(bar_do, Cfg::kTileBytes);
-            for (int p = 0; p < D / 64; ++p) tma_load_3d(smem_do + p * 16384, &tm_do, bar_do, p * 64, row, h);
+            mbar_expect_tx(smem_u32(&sh.do_full), Cfg::kTileBytes);
+            load(smem_do, &tm_do, sh.do_full, row, h);
             ++loads_do;
-            if (loads_q > 0) ok = mbar_wait(smem_u32(&sh.q_empty[0]), (loads_q & 1) ^ 1, abort_flag);
+            if (loads_q > 0) ok = wait(sh.q_empty[0], (loads_q & 1) ^ 1);
             if (!ok) break;
-            const uint32_t bar = smem_u32(&sh.q_full[0]);
-            mbar_expect_tx(bar, Cfg::kTileBytes);
-            for (int p = 0; p < D / 64; ++p) tma_load_3d(smem_q + p * 16384, &tm_q, bar, p * 64, row, h);
+            mbar_expect_tx(smem_u32(&sh.q_full[0]), Cfg::kTileBytes);
+            load(smem_q, &tm_q, sh.q_full[0], row, h);
           } else {
             if (loads_q >= Cfg::kQStages)
-              ok = mbar_wait(smem_u32(&sh.q_empty[s]), ((loads_q / Cfg::kQStages) & 1) ^ 1, abort_flag);
+              ok = wait(sh.q_empty[s], ((loads_q / Cfg::kQStages) & 1) ^ 1);
             if (!ok) break;
-            const uint32_t bar = smem_u32(&sh.q_full[s]);
-            mbar_expect_tx(bar, 2 * Cfg::kTileBytes);
-            for (int p = 0; p < D / 64; ++p) {
-              tma_load_3d(smem_q + s * Cfg::kTileBytes + p * 16384, &tm_q, bar, p * 64, row, h);
-              tma_load_3d(smem_do + s * Cfg::kTileBytes + p * 16384, &tm_do, bar, p * 64, row, h);
+            if (lead) {
+              mbar_expect_tx(smem_u32(&sh.q_full[s]), 2 * Cfg::kTileBytes);
+              load(smem_q + s * Cfg::kTileBytes, &tm_q, sh.q_full[s], row, h);
+              load(smem_do + s * Cfg::kTileBytes, &tm_do, sh.q_full[s], row, h);
             }
           }
           ++loads_q;
@@ -534,13 +547,14 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         // keys: a CTA each 0.72, passed on 0.82-0.93, here 0.52-0.65; 1 x 8192 and 31 x 256, 12 heads 771 -> 712 (d = 64).
         bool more = false;
         while (true) {
-          ok = mbar_wait(smem_u32(&sh.next_full), (asked - 1) & 1, abort_flag);
+          ok = wait(sh.next_full, (asked - 1) & 1);
           if (!ok) break;
           uint32_t block;
           more = clc_answer(smem_u32(&sh.next), block);
           fence_async_smem();
           if (!more) break;
           more = !launch_failed();
+          if (BLOCKSPARSE) more = __all_sync(0xffffffffu, more);
           x = decode(block);
           if (!more || x.n0 < x.sk) break;
           take_next();
@@ -548,10 +562,25 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         if (!ok) break;
         if (!more) x.nm = -1;
         // its place is free once every role has finished block k - 1
-        if (k >= 1) ok = mbar_wait(smem_u32(&sh.blk_done[(k + 1) & 1]), ((k - 1) >> 1) & 1, abort_flag);
+        if (k >= 1) ok = wait(sh.blk_done[(k + 1) & 1], ((k - 1) >> 1) & 1);
         if (!ok) break;
-        sh.blk[(k + 1) & 1] = x;
-        mbar_arrive(smem_u32(&sh.blk_full[(k + 1) & 1]));
+        if constexpr (BLOCKSPARSE) {
+          if (more) {
+            const int mt = list_tiles(x);
+            x.list = (k + 1) & 1;
+            x.nm = 0;
+            for (int c = 0; c * 32 < mt; ++c) {
+              const uint32_t bits = list_bits(x, x.n0 >> 8, c, mt);
+              put_in_list(qtile_list[x.list], c, bits, x.nm);
+              x.nm += __popc(bits);
+            }
+          }
+          __syncwarp();
+        }
+        if (lead) {
+          sh.blk[(k + 1) & 1] = x;
+          mbar_arrive(smem_u32(&sh.blk_full[(k + 1) & 1]));
+        }
         if (!more) break;
       }
       mbar_drain_ring(&sh.k_full, 1, loads_k);
@@ -1496,7 +1525,7 @@ cudaError_t launch_main(const BwdLaunch& l, cudaStream_t stream) {
   // (causal, us: 4 x 4 x 600 ragged 28.8 -> 28.3 at d = 128, 12 x 12 x 128 16.1 -> 16.0 at d = 64).
   const bool linear = linear_grid(grid.x, grid.y, grid.z) && int64_t(grid.x) * grid.y * grid.z > kSms;
   args.k.grid_tiles = grid.x;
-  args.take_over = !BS && linear && l.args.dq_tickets == nullptr;
+  args.take_over = linear && l.args.dq_tickets == nullptr;
   if constexpr (CAUSAL) set_causal_grid(&args.k, grid.x, int64_t(8) * D * args.max_seqlen_q);  // Q, dO and the fp32 dQ
   if (linear && (CAUSAL || args.take_over)) grid = dim3(grid.x * grid.y * grid.z, 1, 1);
   // (not the main kernel of d = 128, causal, with dropout: its grid is slower when it starts beside the preprocess.  Whole backward
