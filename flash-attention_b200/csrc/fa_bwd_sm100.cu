@@ -53,7 +53,8 @@ constexpr int kSms = 148;
 constexpr int kMaxSparseTiles = 1024;  // query tiles of 128 per sequence in block-sparse mode
 
 // BS: block-sparse variant (its tile list takes shared memory that the third Q / dO stage would need)
-template <int D, bool BS = false, bool DROPOUT = false>
+// SHORT: see short_queries
+template <int D, bool BS = false, bool DROPOUT = false, bool SHORT = false>
 struct BwdCfg {
   // d = 128 runs a different schedule: shared memory holds a single stage of Q and of dO, each
   // with its own barriers, and the compute groups work in two phases (P~ from S, then dS from dP)
@@ -63,7 +64,8 @@ struct BwdCfg {
   // the refill takes about 1500 clk to land, so with two stages the S / dP products of the next
   // tile start late and the compute groups wait; the third stage lets the load run a whole tile
   // ahead.
-  static constexpr int kQStages = (D == 64) ? (BS ? 2 : 3) : 1;
+  static constexpr int kQStages = (D == 64) ? (BS || SHORT ? 2 : 3) : 1;
+  static constexpr int kKvStages = SHORT ? 2 : 1;
   // Compute warps.  d = 64 with dropout: sixteen of one 16-row block and one half of the keys each (quad layout), four
   // per scheduler, which cover each other's waits and generator chains; else eight, a thread per row and half.
   static constexpr bool kQuad = DROPOUT && !kTwoPhase;
@@ -80,8 +82,8 @@ struct BwdCfg {
   static constexpr int kTileBytes = 128 * D * 2;
   static constexpr int kPdsBytes = 128 * 128 * 2;
   static constexpr int kDqStageBytes = 2 * 16384;  // two [128 rows x 32 fp32] boxes
-  // K, V, (Q, dO) x stages, P~, dS, dQ staging
-  static constexpr int kSmemBytes = (2 + 2 * kQStages) * kTileBytes + 2 * kPdsBytes + kDqStageBytes + 1024;
+  // (K, V) x stages, (Q, dO) x stages, P~, dS, dQ staging
+  static constexpr int kSmemBytes = 2 * (kKvStages + kQStages) * kTileBytes + 2 * kPdsBytes + kDqStageBytes + 1024;
   static constexpr uint32_t kTmemS = 0, kTmemDP = 128, kTmemDV = 256, kTmemDK = 256 + D;
   static constexpr uint32_t kTmemDQ = kAliasDq ? 128 : 256 + 2 * D;
   // d = 64 leaves 64 tensor-memory columns free: a second copy of the 16-bit dS can go there and feed
@@ -100,7 +102,7 @@ struct BlockInfo {
 };
 
 struct BwdShared {
-  uint64_t k_full, v_full, k_empty, v_empty;  // the key tile's operands, once per key tile
+  uint64_t k_full[2], v_full[2], k_empty[2], v_empty[2];  // the key tile's operands, once per key tile
   uint64_t acc_free;                          // dV and dK read out, once per key tile
   uint64_t next_full;                         // the answer to a request for another block is in `next`
   uint64_t blk_full[2], blk_done[2];          // the block after is in `blk`; every role has finished the one there
@@ -199,13 +201,13 @@ cudaError_t launch(bool overlap, void (*kernel)(P...), dim3 grid, int threads, i
 
 // ------------------------------------------------------------------------------------------------
 // ONE_LAUNCH: see one_launch()
-template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BLOCKSPARSE, bool ONE_LAUNCH>
-__global__ void __launch_bounds__(BwdCfg<D, BLOCKSPARSE, DROPOUT>::kThreads, 1)
+template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BLOCKSPARSE, bool ONE_LAUNCH, bool SHORT>
+__global__ void __launch_bounds__(BwdCfg<D, BLOCKSPARSE, DROPOUT, SHORT>::kThreads, 1)
 fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
               const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
               const __grid_constant__ CUtensorMap tm_dq, const __grid_constant__ CUtensorMap tm_dk,
               const __grid_constant__ CUtensorMap tm_dv, const BwdArgs a) {
-  using Cfg = BwdCfg<D, BLOCKSPARSE, DROPOUT>;
+  using Cfg = BwdCfg<D, BLOCKSPARSE, DROPOUT, SHORT>;
   constexpr int kDqWarp = Cfg::kComputeWarps, kProducer = kDqWarp + 4;  // first warp of the dQ group, of the last four
   constexpr bool kVote = Cfg::kQuad && !ONE_LAUNCH;  // (see mbar_wait_warp)
   constexpr int kBoxColumns = grad_box_columns(D, CAUSAL, DROPOUT);
@@ -359,22 +361,25 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
   const uint32_t smem_k = smem_u32(smem);
-  const uint32_t smem_v = smem_k + Cfg::kTileBytes;
-  const uint32_t smem_q = smem_v + Cfg::kTileBytes;                       // stages of Q
+  const uint32_t smem_v = smem_k + Cfg::kTileBytes;  // of the first stage
+  auto kv_at = [&](int c) -> uint32_t { return c % Cfg::kKvStages * (2 * Cfg::kTileBytes); };  // of key tile c
+  const uint32_t smem_q = smem_k + 2 * Cfg::kKvStages * Cfg::kTileBytes;  // stages of Q
   const uint32_t smem_do = smem_q + Cfg::kQStages * Cfg::kTileBytes;      // stages of dO
   const uint32_t smem_p = smem_do + Cfg::kQStages * Cfg::kTileBytes;
   const uint32_t smem_ds = smem_p + Cfg::kPdsBytes;
-  uint8_t* p_ptr = smem + (2 + 2 * Cfg::kQStages) * Cfg::kTileBytes;
+  uint8_t* p_ptr = smem + 2 * (Cfg::kKvStages + Cfg::kQStages) * Cfg::kTileBytes;
   uint8_t* ds_ptr = p_ptr + Cfg::kPdsBytes;
   uint8_t* dq_stage = ds_ptr + Cfg::kPdsBytes;
 
   if (tid == 0) {
     sh.abort_flag = 0;
-    mbar_init(smem_u32(&sh.k_full), 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_u32(&sh.k_full[i]), 1);
+      mbar_init(smem_u32(&sh.v_full[i]), 1);
+      mbar_init(smem_u32(&sh.k_empty[i]), 1);
+      mbar_init(smem_u32(&sh.v_empty[i]), 1);
+    }
     mbar_init(smem_u32(&sh.stat_ready), 4);
-    mbar_init(smem_u32(&sh.v_full), 1);
-    mbar_init(smem_u32(&sh.k_empty), 1);
-    mbar_init(smem_u32(&sh.v_empty), 1);
     mbar_init(smem_u32(&sh.acc_free), Cfg::kComputeWarps);
     mbar_init(smem_u32(&sh.next_full), 1);
     for (int i = 0; i < 2; ++i) {
@@ -496,23 +501,25 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           const int s = loads_q % Cfg::kQStages;
           const int row = x.q_start + q_tile(x, t) * kBM;
           auto load_k = [&]() {
-            if (loads_k > 0) ok = wait(sh.k_empty, (loads_k & 1) ^ 1);
+            const int stage = loads_k % Cfg::kKvStages;
+            if (loads_k >= Cfg::kKvStages) ok = wait(sh.k_empty[stage], ((loads_k / Cfg::kKvStages) & 1) ^ 1);
             if (!ok) return;
             if (lead) {
-              mbar_expect_tx(smem_u32(&sh.k_full), Cfg::kTileBytes);
-              load(smem_k, &tm_k, sh.k_full, x.k_start + x.n0, h);
+              mbar_expect_tx(smem_u32(&sh.k_full[stage]), Cfg::kTileBytes);
+              load(smem_k + kv_at(loads_k), &tm_k, sh.k_full[stage], x.k_start + x.n0, h);
             }
             ++loads_k;
           };
-          const bool first_k = loads_k == 0;
+          const bool first_k = t == 0 && (SHORT || loads_k == 0);
           if (first_k) load_k();
           if (t == 0) {
             // V is free after the last dP of the key tile before, K after its last dQ
-            if (loads_v > 0) ok = wait(sh.v_empty, (loads_v & 1) ^ 1);
+            const int stage = loads_v % Cfg::kKvStages;
+            if (ok && loads_v >= Cfg::kKvStages) ok = wait(sh.v_empty[stage], ((loads_v / Cfg::kKvStages) & 1) ^ 1);
             if (!ok) break;
             if (lead) {
-              mbar_expect_tx(smem_u32(&sh.v_full), Cfg::kTileBytes);
-              load(smem_v, &tm_v, sh.v_full, x.k_start + x.n0, h);
+              mbar_expect_tx(smem_u32(&sh.v_full[stage]), Cfg::kTileBytes);
+              load(smem_v + kv_at(loads_v), &tm_v, sh.v_full[stage], x.k_start + x.n0, h);
             }
             ++loads_v;
           }
@@ -583,8 +590,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         }
         if (!more) break;
       }
-      mbar_drain_ring(&sh.k_full, 1, loads_k);
-      mbar_drain_ring(&sh.v_full, 1, loads_v);
+      mbar_drain_ring(sh.k_full, Cfg::kKvStages, loads_k);
+      mbar_drain_ring(sh.v_full, Cfg::kKvStages, loads_v);
       mbar_drain_ring(sh.q_full, Cfg::kQStages, loads_q);
       mbar_drain_ring(&sh.do_full, 1, loads_do);
       mbar_drain_ring(&sh.next_full, 1, asked);
@@ -596,7 +603,9 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       do {
       const int nm = __shfl_sync(0xffffffffu, sh.blk[k & 1].nm, 0);
       if (nm <= 0) continue;
-      ok = mbar_wait_warp<kVote>(smem_u32(&sh.k_full), c & 1, abort_flag);
+      const int kv = c % Cfg::kKvStages;
+      const uint32_t smem_kc = smem_k + kv_at(c), smem_vc = smem_v + kv_at(c);
+      ok = mbar_wait_warp<kVote>(smem_u32(&sh.k_full[kv]), (c / Cfg::kKvStages) & 1, abort_flag);
       if constexpr (Cfg::kTwoPhase) {
         // d = 128: every product, issued by this thread in the order
         //   dV(t) | dK(t), dQ(t) | S(t+1) | dP(t+1)
@@ -610,7 +619,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           if (!ok) return;
           tc_fence_after();
           if (elect_one()) {
-            issue_kk(tS_, smem_q, smem_k);
+            issue_kk(tS_, smem_q, smem_kc);
             mma_commit(smem_u32(&sh.s_full));
           }
         };
@@ -620,13 +629,13 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           if (!ok) return;
           tc_fence_after();
           if (elect_one()) {
-            issue_kk(tDP_, smem_do, smem_v);
+            issue_kk(tDP_, smem_do, smem_vc);
             mma_commit(smem_u32(&sh.sdp_full));
-            if (last) mma_commit(smem_u32(&sh.v_empty));
+            if (last) mma_commit(smem_u32(&sh.v_empty[kv]));
           }
         };
         if (ok) scores(g0);
-        if (ok) ok = mbar_wait_warp(smem_u32(&sh.v_full), c & 1, abort_flag);
+        if (ok) ok = mbar_wait_warp(smem_u32(&sh.v_full[kv]), (c / Cfg::kKvStages) & 1, abort_flag);
         if (ok) grad_p(g0, nm == 1);
         for (int t = 0; t < nm && ok; ++t) {
           const int g = g0 + t;
@@ -649,10 +658,10 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           if (elect_one()) {
             issue_tt(tDK_, smem_ds, smem_q, t > 0);
             mma_commit(smem_u32(&sh.q_empty[0]));
-            issue_dq(tDQ_, smem_ds, smem_k);
+            issue_dq(tDQ_, smem_ds, smem_kc);
             mma_commit(smem_u32(&sh.dq_full));
             mma_commit(smem_u32(&sh.ds_free));
-            if (!has_next) mma_commit(smem_u32(&sh.k_empty));
+            if (!has_next) mma_commit(smem_u32(&sh.k_empty[kv]));
           }
           if (has_next) {
             scores(g + 1);
@@ -668,13 +677,13 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           if (!ok) return;
           tc_fence_after();
           if (elect_one()) {
-            issue_kk(tS_, smem_q + s * Cfg::kTileBytes, smem_k);
-            issue_kk(tDP_, smem_do + s * Cfg::kTileBytes, smem_v);
+            issue_kk(tS_, smem_q + s * Cfg::kTileBytes, smem_kc);
+            issue_kk(tDP_, smem_do + s * Cfg::kTileBytes, smem_vc);
             mma_commit(smem_u32(&sh.sdp_full));
-            if (last) mma_commit(smem_u32(&sh.v_empty));
+            if (last) mma_commit(smem_u32(&sh.v_empty[kv]));
           }
         };
-        if (ok) ok = mbar_wait_warp<kVote>(smem_u32(&sh.v_full), c & 1, abort_flag);
+        if (ok) ok = mbar_wait_warp<kVote>(smem_u32(&sh.v_full[kv]), (c / Cfg::kKvStages) & 1, abort_flag);
         if (ok) scores(g0, nm == 1);
         for (int t = 0; t < nm && ok; ++t) {
           const int g = g0 + t;
@@ -685,11 +694,11 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           tc_fence_after();
           // its tile is read out of tensor memory while dV / dK are still running
           if (elect_one()) {
-            if constexpr (kDsInTmem) issue_dq_t(tDQ_, tDS_, smem_k);
-            else issue_dq(tDQ_, smem_ds, smem_k);
+            if constexpr (kDsInTmem) issue_dq_t(tDQ_, tDS_, smem_kc);
+            else issue_dq(tDQ_, smem_ds, smem_kc);
             mma_commit(smem_u32(&sh.dq_full));
             mma_commit(smem_u32(&sh.pds_free));
-            if (t + 1 == nm) mma_commit(smem_u32(&sh.k_empty));
+            if (t + 1 == nm) mma_commit(smem_u32(&sh.k_empty[kv]));
           }
         }
       }
@@ -1509,12 +1518,23 @@ __global__ void bwd_postprocess_kernel(const BwdArgs a, int dpad) {
   *reinterpret_cast<uint4*>(dst) = out;
 }
 
-template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BS, bool ONE_LAUNCH = false>
+// Calls with few query tiles at d = 64: a block's K and V are then a good part of its loads and are waited for at its start, so two
+// stages hold them, and two (not three) Q and dO.  Whole backward, 12 heads, 32 768 tokens, us, one stage of K and V -> two: 64 x 512
+// 239 -> 247, 85 x 384 212 -> 213, 128 x 256 182 -> 171, 163 x 200 212 -> 206, 256 x 128 155 -> 149, with dropout (ragged) up to 256
+// 239 -> 234, up to 384 261 -> 266; 16 x 8 heads, up to 256 queries, 1500 keys 67.4 -> 63.6, 300 queries 67.5 -> 67.6.
+constexpr int kShortQueries = 256;
+inline bool short_queries(const BwdLaunch& l) { return l.args.max_seqlen_q <= kShortQueries; }
+
+template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BS, bool ONE_LAUNCH = false, bool SHORT = false>
 cudaError_t launch_main(const BwdLaunch& l, cudaStream_t stream) {
-  if constexpr (!BS && !ONE_LAUNCH)
+  if constexpr (!BS && !ONE_LAUNCH && !SHORT) {
     if (l.args.one_launch) return launch_main<D, BF16, CAUSAL, DROPOUT, BS, true>(l, stream);
-  auto kernel = fa_bwd_kernel<D, BF16, CAUSAL, DROPOUT, BS, ONE_LAUNCH>;
-  using Cfg = BwdCfg<D, BS, DROPOUT>;
+    if constexpr (D == 64)
+      if (short_queries(l) && int64_t((l.args.max_seqlen_k + kBN - 1) / kBN) * l.args.k.heads * l.args.k.batch > kSms)
+        return launch_main<D, BF16, CAUSAL, DROPOUT, BS, false, true>(l, stream);
+  }
+  auto kernel = fa_bwd_kernel<D, BF16, CAUSAL, DROPOUT, BS, ONE_LAUNCH, SHORT>;
+  using Cfg = BwdCfg<D, BS, DROPOUT, SHORT>;
   constexpr int smem = Cfg::kSmemBytes;
   static SmemLimitFlags smem_limit_set;  // one per template instantiation of this function
   cudaError_t e = set_smem_limit_once(kernel, smem, smem_limit_set);
