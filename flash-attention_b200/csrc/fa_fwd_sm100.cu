@@ -1183,11 +1183,14 @@ cudaError_t launch_groups(const FwdLaunch& l, cudaStream_t stream) {
 //   1024, 8192                1.03       1.04           1.17       1.09
 //   4096, 4096 (4 x 16)       1.00       1.01           1.16       1.08
 // so d = 64 takes single tiles at every length (causal calls too: 0.95-0.98).
-// d = 128, one / two: up to 1024 keys (causal calls count those up to the longest query) 0.91-1.02 (12 heads of 16 sequences:
-// 2000 queries, 256 keys 138 -> 126 us, 8 of 4096 and 512 148 -> 146; dropout 171 -> 156, 201 -> 183).  Beyond, causal:
-// 1100 tokens 0.87, 1300 0.9, 1800 0.92, 2000 0.97, 2500 0.99, 3000 1.00, 4096 1.02, with dropout 2000 0.96, 4096 1.00, 8192 1.01.
-// Not causal: 1500 1.04, 2000 0.99, 4096 1.02, 1024 queries and 2048 keys 1.06, but an odd number of query tiles leaves half of
-// a pair empty: 384 queries, 2048 keys 0.88, 1100 tokens 0.93, 1800 0.95.  Not causal with dropout (8 x 12 / 4 x 16 heads): 1100 0.84 / 0.83,
+// d = 128 without dropout, whose CTAs go on with other blocks, so that the ends of a walk count for less (one / two, 12 heads, 16 384
+// tokens): not causal 200 tokens 1.08, 300 0.94, 512 1.14, 700 1.11, 1000 1.09, 1100 1.08, 1500 1.14, 1800 1.07, 3000 1.16, ragged 200 0.98,
+// 512 1.04, 1000 1.07, 2000 1.11; 16 x 256 queries, 512 and 1024 keys 1.09 and 1.16, 600 and 900 1.10, 2000 and 256 1.07, but three query
+// tiles, which leave a quarter of their pairs empty, 384 and 2048 0.97.  Causal, where the tiles of a pair differ by one in their keys
+// (even / ragged): 512 0.90 / 0.85, 1000 0.97 / 0.91, 1300 0.94 / 0.96, 1500 1.03 / 0.96, 1800 0.98 / 0.99, 2000 1.06 / 1.01, 2500 1.06 / 1.02,
+// 4096 1.07 / 1.03.
+// d = 128 with dropout: up to 1024 keys (causal calls count those up to the longest query) one (2000 queries, 256 keys 171 -> 156, 8 of 4096
+// and 512 201 -> 183).  Beyond, causal: 2000 0.96, 4096 1.00, 8192 1.01.  Not causal (8 x 12 / 4 x 16 heads): 1100 0.84 / 0.83,
 // 1500 1.00 / 1.03, 2000 0.94 / 0.94, 2500 0.97 / 0.97, 3000 1.04 / 0.97, 4096 1.04 / 1.07 (4 x 12 0.97), 6000 1.05 / 1.02, 8192 1.07 / 1.08, 384
 // queries and 2048 keys 0.66 / 1.07, 1100 and 4096 0.87 / 0.79: how the last round of CTAs falls decides, and the rule stays.
 // A grid of single tiles that fits one per SM spreads over twice the SMs: 16 heads, 1024 queries, 8192 keys 0.72 (d = 64),
@@ -1199,7 +1202,7 @@ cudaError_t launch_groups(const FwdLaunch& l, cudaStream_t stream) {
 // share an SM: 192 pairs 85 us, 128 with two.
 // Uneven batches (see `uneven`) announced with more than 4096 tokens take pairs at d = 64 too, which halves their empty blocks:
 // 31 x 256 and 1 x 8192, 12 heads 431 -> 374 us, 2 x 16384 and 126 x 64, 4 heads 948 -> 865.
-constexpr int kOneTileMaxD128 = 1024, kOneTileMaxOdd = 2048, kOneTileMaxCausal = 2560, kOneTileMaxCausalDropout = 4096;  // keys
+constexpr int kOneTileMaxD128 = 1024, kOneTileMaxCausal = 1920, kOneTileMaxCausalDropout = 4096;  // keys
 constexpr int kOneTileMaxUneven = 4096;  // queries and keys, d = 64
 
 template <int D, bool CAUSAL, bool DROPOUT>
@@ -1212,13 +1215,12 @@ bool one_tile_per_cta(const FwdLaunch& l) {
   if (l.max_seqlen_q <= kBlockM) return D == 64 || DROPOUT || keys <= kOneTileMaxD128 || pairs > kSms;
   if (one_round) return false;
   if (D == 64) return !(uneven(l) && max(l.max_seqlen_q, keys) > kOneTileMaxUneven);
-  if (l.max_seqlen_q <= kOneTileMaxD128 && (tiles <= kSms || keys <= kOneTileMaxD128)) return true;
-  if (uneven(l)) return false;  // (twice the empty blocks)
+  const bool pairs_at_once = !CAUSAL && !DROPOUT && q_tiles != 3;  // (at any length)
+  if (l.max_seqlen_q <= kOneTileMaxD128 && (tiles <= kSms || (keys <= kOneTileMaxD128 && !pairs_at_once))) return true;
+  if (uneven(l) || pairs_at_once) return false;  // (uneven: twice the empty blocks)
   if (keys <= kOneTileMaxD128) return true;
   if (CAUSAL) return keys <= (DROPOUT ? kOneTileMaxCausalDropout : kOneTileMaxCausal);
-  const bool odd = q_tiles % 2 != 0;
-  if (DROPOUT) return odd || l.max_seqlen_q > kOneTileMaxD128;
-  return odd && max(l.max_seqlen_q, keys) <= kOneTileMaxOdd;
+  return !DROPOUT || q_tiles % 2 != 0 || l.max_seqlen_q > kOneTileMaxD128;
 }
 
 // Rows for d = 128 without dropout, and for d = 64 without dropout up to 512 keys: there the ends of a CTA's
