@@ -95,12 +95,20 @@ struct BwdCfg {
   static constexpr uint32_t kTmemDS = 256 + 3 * D;
 };
 
-// What a block works on: key tile n0 / 128 of one (batch, head) pair.  nm: query tiles to walk, -1 behind the last block.  (32 bytes: with
-// a ninth word 2 x 4 x 16384 causal, d = 64, took 712 us instead of 703)
-struct BlockInfo {
+// What a block works on: key tile n0 / 128 of one (batch, head) pair.  nm: query tiles to walk, -1 behind the last block.  The size of the
+// record decides how the compiler reads it from shared memory: in 32 bytes two wide loads, best with a causal mask (d = 64, 2 x 4 x
+// 16384: 703 us, in 36 bytes 712), in 36 bytes each word where it is used, best without (4 x 12 x 4096 561 and 554 us, ragged batches up to
+// 512 tokens with dropout 306 and 303).
+template <bool CAUSAL>
+struct BlockRecord {
   int q_start, sq, k_start, sk, n0, h, b, nm;
 };
+template <>
+struct BlockRecord<false> {
+  int q_start, sq, k_start, sk, n0, h, b, nm, unused;
+};
 
+template <bool CAUSAL>
 struct BwdShared {
   uint64_t k_full[2], v_full[2], k_empty[2], v_empty[2];  // the key tile's operands, once per key tile
   uint64_t acc_free;                          // dV and dK read out, once per key tile
@@ -108,7 +116,7 @@ struct BwdShared {
   uint64_t blk_full[2], blk_done[2];          // the block after is in `blk`; every role has finished the one there
   uint64_t drained[3];                        // of the issuing warps, at their end
   alignas(16) uint4 next;
-  alignas(16) BlockInfo blk[2];               // block k in entry k % 2
+  alignas(16) BlockRecord<CAUSAL> blk[2];               // block k in entry k % 2
   uint64_t q_full[3], q_empty[3];
   uint64_t do_full, do_empty;  // dO ring of the two-phase schedule (one stage)
   // d = 64: S and dP together / P~ and dS together.  Two-phase schedule: sdp_full = dP landed,
@@ -214,7 +222,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   constexpr bool kTmaRows = kBoxColumns != 0;
   constexpr bool kDsInTmem = Cfg::kDsInTmemCapable && !DROPOUT;
   extern __shared__ uint8_t smem_raw[];
-  __shared__ BwdShared sh;
+  using BlockInfo = BlockRecord<CAUSAL>;
+  __shared__ BwdShared<CAUSAL> sh;
 
   const int tid = threadIdx.x;
   // Known to be the same in all lanes, for the issuing warps (see mma_ss).  The compute and dQ groups take
@@ -252,6 +261,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     x.k_start = ka.cu_seqlens_k[x.b];
     x.sk = ka.cu_seqlens_k[x.b + 1] - x.k_start;
     x.n0 = nt * kBN;
+    if constexpr (!CAUSAL) x.unused = 0;
     const int m_tiles = (x.sq + kBM - 1) / kBM;
     // (a call of one launch also writes dq = 0 for a sequence without keys)
     x.nm = x.n0 < x.sk || ONE_LAUNCH ? m_tiles - (CAUSAL ? min(m_tiles, x.n0 / kBM) : 0) : 0;
