@@ -86,13 +86,15 @@ struct BwdCfg {
   static constexpr int kSmemBytes = 2 * (kKvStages + kQStages) * kTileBytes + 2 * kPdsBytes + kDqStageBytes + 1024;
   static constexpr uint32_t kTmemS = 0, kTmemDP = 128, kTmemDV = 256, kTmemDK = 256 + D;
   static constexpr uint32_t kTmemDQ = kAliasDq ? 128 : 256 + 2 * D;
-  // d = 64 leaves 64 tensor-memory columns free: a second copy of the 16-bit dS can go there and feed
+  // A second copy of the 16-bit dS goes to tensor memory and feeds
   // dQ = dS K as the A operand (its M dimension is the query row, like the lanes of S), so that
   // product does not read dS from shared memory; dK = dS^T Q still takes the shared-memory copy.
-  // Used without dropout, where shared-memory bandwidth is the bound (8 x 12 x 4096: 1.49 -> 1.39 ms);
-  // with dropout the compute groups are the bound and the extra stores cost 2 %.
-  static constexpr bool kDsInTmemCapable = !kTwoPhase;
-  static constexpr uint32_t kTmemDS = 256 + 3 * D;
+  // Used without dropout, where shared-memory bandwidth is the bound (d = 64, 8 x 12 x 4096: 1.49 -> 1.39 ms);
+  // with dropout the compute groups are the bound and the extra stores cost 2 %.  d = 64 leaves 64 columns free for it; at d = 128 it takes
+  // the place of the scores, 32 columns in each half of them: a thread overwrites what it has read itself, and the next S is issued behind dQ.
+  // There, us: 4 x 12 x 4096 1155 -> 1147 (causal 607 -> 603), 16 x 12 x 1000 causal 241.7 -> 240.4, back to back under the power
+  // limit 16 x 12 x 8192 causal 9860 -> 9817.
+  static constexpr uint32_t kTmemDS = kTwoPhase ? kTmemS : 256 + 3 * D;
 };
 
 // What a block works on: key tile n0 / 128 of one (batch, head) pair.  nm: query tiles to walk, -1 behind the last block.  The size of the
@@ -220,7 +222,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   constexpr bool kVote = Cfg::kQuad && !ONE_LAUNCH;  // (see mbar_wait_warp)
   constexpr int kBoxColumns = grad_box_columns(D, CAUSAL, DROPOUT);
   constexpr bool kTmaRows = kBoxColumns != 0;
-  constexpr bool kDsInTmem = Cfg::kDsInTmemCapable && !DROPOUT;
+  constexpr bool kDsInTmem = !DROPOUT;
   extern __shared__ uint8_t smem_raw[];
   using BlockInfo = BlockRecord<CAUSAL>;
   __shared__ BwdShared<CAUSAL> sh;
@@ -461,7 +463,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     const uint64_t db = desc_here(make_smem_desc(b_base, 16384, 1024));
 #pragma unroll
     for (int ks = 0; ks < kBN / 16; ++ks)
-      mma_ts(dst, a_tmem + ks * 8, desc_at(db, ks * 2048), idesc_dq, ks > 0);
+      mma_ts(dst, a_tmem + (Cfg::kTwoPhase ? (ks >> 2) * 64 + (ks & 3) * 8 : ks * 8), desc_at(db, ks * 2048), idesc_dq, ks > 0);
   };
 
   // A warp has finished block k: waits for the next one, if any (or until a wait is abandoned).
@@ -666,7 +668,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           if (elect_one()) {
             issue_tt(tDK_, smem_ds, smem_q, t > 0);
             mma_commit(smem_u32(&sh.q_empty[0]));
-            issue_dq(tDQ_, smem_ds, smem_kc);
+            if constexpr (kDsInTmem) issue_dq_t(tDQ_, tDS_, smem_kc);
+            else issue_dq(tDQ_, smem_ds, smem_kc);
             mma_commit(smem_u32(&sh.dq_full));
             mma_commit(smem_u32(&sh.ds_free));
             if (!has_next) mma_commit(smem_u32(&sh.k_empty[kv]));
@@ -1083,6 +1086,8 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             *reinterpret_cast<uint4*>(ds_ptr + off) =
                 make_uint4(pds[4 * ch4], pds[4 * ch4 + 1], pds[4 * ch4 + 2], pds[4 * ch4 + 3]);
           }
+          // second copy of dS for the dQ product, over this group's own scores, which every thread of it has read
+          if constexpr (kDsInTmem) tmem_st16(tDS_ + lane_sel + w * 64 + c * 16, pds);
         }
         tc_fence_before();  // the dP columns are about to be overwritten by dQ
       } else {
