@@ -322,13 +322,12 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     for (int c = warp; c * 32 < n_kv; c += kWarps) {
       const int j = c * 32 + lane;
       const int32_t* row = a.bs_iter + (static_cast<int64_t>(b) * a.bs_kblocks + (j >> 1)) * a.bs_rows16;
-      bool any = false;
+      int most = -1;  // (all loads at once: none decides about the next)
       // (causal: a key tile that starts behind the CTA's last query row is masked entirely)
-      if (j < n_kv && !(CAUSAL && j * kBlockN > mp * G * kBlockM + G * kBlockM - 1))
+      if (j < n_kv && rb0 < rb1 && !(CAUSAL && j * kBlockN > mp * G * kBlockM + G * kBlockM - 1))
 #pragma unroll
-        for (int i = 0; i < G * kBlockM / 16; ++i)
-          if (rb0 + i < rb1) any = any || (row[rb0 + i] >= 0);
-      const uint32_t bits = __ballot_sync(0xffffffffu, any);
+        for (int i = 0; i < G * kBlockM / 16; ++i) most = max(most, row[min(rb0 + i, rb1 - 1)]);
+      const uint32_t bits = __ballot_sync(0xffffffffu, most >= 0);
       if (lane == 0) tile_bits[c] = bits;
     }
     __syncthreads();
