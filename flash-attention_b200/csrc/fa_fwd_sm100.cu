@@ -106,6 +106,7 @@ struct FwdShared {
   float2 row_stats[STATS][kBlockM];  // (max, sum) of every query row, for the epilogue; taking over: two of a group, by the block's parity
   alignas(16) uint4 next;
   FwdBlock blk[2];  // block k in entry k % 2
+  uint32_t alive;   // changes as the producer gets on (see mbar_wait_warp_alive)
   uint32_t tmem_base;
   int abort_flag;
   int stop;  // a CTA of this launch has abandoned a wait
@@ -419,7 +420,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     if constexpr (!TAKE) return false;
     __syncwarp();
     if (elect_one()) mbar_arrive(smem_u32(&sh.blk_done[k & 1]));
-    return mbar_wait_warp<true>(smem_u32(&sh.blk_full[(k + 1) & 1]), (k >> 1) & 1, abort_flag) && sh.blk[(k + 1) & 1].mp >= 0;
+    return mbar_wait_warp_alive<true>(smem_u32(&sh.blk_full[(k + 1) & 1]), (k >> 1) & 1, abort_flag, &sh.alive) && sh.blk[(k + 1) & 1].mp >= 0;
   };
 
   if (warp >= Cfg::kSoftmaxWarps) reg_dealloc<Cfg::kOtherRegs>();
@@ -429,11 +430,12 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       bool ok = true;
       int loads_k = 0, loads_v = 0, loads_q[G] = {};  // so far
       uint32_t asked = 0;                             // requests so far
+      auto still_alive = [&](uint32_t count) { *const_cast<volatile uint32_t*>(&sh.alive) = count; };
       // asked for with the loads of the last key tile: a block taken earlier would wait here while other SMs run dry
       auto take_next = [&]() {
         mbar_expect_tx(smem_u32(&sh.next_full), 16);
         clc_try_cancel(smem_u32(&sh.next), smem_u32(&sh.next_full));
-        ++asked;
+        still_alive(++asked + loads_k);
       };
       FwdBlock x = first;
       for (uint32_t k = 0; ok; ++k) {
@@ -457,6 +459,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             load_tile(smem_k + s * Cfg::kTileBytes, &tm_k, sh.k_full[s], row, x.h);
           }
           ++loads_k;
+          if (TAKE) still_alive(asked + loads_k);
           if (TAKE && j + 1 == n_max) take_next();
           if (k > 0 || j > 0) {
             if (loads_v >= Cfg::kStages) ok = mbar_wait(smem_u32(&sh.v_empty[s]), ph, abort_flag);

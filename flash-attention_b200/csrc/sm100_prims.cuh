@@ -100,6 +100,26 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
 
+// The same where the wait spans another role's work of any length (the producer passes over thousands of blocks without work, or one
+// group walks a long sequence while the other has no rows): `alive` is a word which that role changes as it gets on, and the
+// wait is abandoned where it has stood still for the limit.
+template <bool VOTE_FIRST = false>
+__device__ __forceinline__ bool mbar_wait_warp_alive(uint32_t bar, uint32_t parity, volatile int* abort_flag, const volatile uint32_t* alive) {
+  if constexpr (VOTE_FIRST)
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  uint32_t seen = *alive;
+  long long t0 = clock64();
+  bool done;
+  while (!(done = mbar_try_wait(bar, parity)) && !*abort_flag) {
+    if (clock64() - t0 <= WAIT_LIMIT_CYCLES) continue;
+    const uint32_t now = *alive;
+    if (now == seen) *abort_flag = 1;
+    seen = now;
+    t0 = clock64();
+  }
+  return __all_sync(0xffffffffu, done);
+}
+
 // What a role has under way (a copy into shared memory, products in tensor memory) ends before the CTA does, also after an
 // abandoned wait: waits, with the same limit, for the phase of `bar` with this parity.
 __device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity) {
