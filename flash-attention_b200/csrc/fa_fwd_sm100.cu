@@ -28,19 +28,16 @@
 // LSE = max*scale + ln(sum), -inf for a row without any valid key.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
-#include <climits>
 #include <cstddef>
 #include <type_traits>
 #include "fa_kernels.h"
 #include "fa_math.cuh"
+#include "fa_rules.h"
 #include "sm100_prims.cuh"
 
 namespace fa {
 
 namespace {
-
-constexpr int kBlockM = 128;
-constexpr int kBlockN = 128;
 
 // G: query tiles (softmax groups) per CTA.  Two share every K / V tile, and one such CTA fills an SM.  One leaves
 // room for a second CTA on the SM, whose loads, first products and epilogue run under the tiles of the other:
@@ -229,10 +226,6 @@ __device__ __forceinline__ void zero_padding(const KernelArgs& a, int b, int h, 
       *reinterpret_cast<uint4*>(o + r * a.o_row_stride + (i - r * chunks) * 8) = make_uint4(0, 0, 0, 0);
   }
 }
-
-// How a grid is laid out and worked on.  kPlain: (tiles, heads, batch).  kLinear: one-dimensional, causal ones with the order of
-// set_tail_grid.  kTake: kLinear, and a CTA goes on with blocks that have not started (see take_over_pays).
-enum Order { kPlain, kLinear, kTake };
 
 // PADDED: see KernelArgs::pad_rows
 template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BLOCKSPARSE, int G, bool ROWS, Order ORDER, bool PADDED>
@@ -1116,48 +1109,15 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
   }
 }
 
-// Announced lengths above `times` the actual ones on average: the grid consists mostly of blocks without queries.
-inline bool uneven(const FwdLaunch& l, int times = 2) {
-  return static_cast<int64_t>(l.args.batch) * l.max_seqlen_q > times * static_cast<int64_t>(l.total_q);
-}
-
-constexpr int kSms = 148;
-
-// Blocks that start at once
-template <int G>
-constexpr int kSlots = (G == 1 ? 2 : 1) * kSms;
-
-// Causal grids with their last tiles in order of weight (set_tail_grid): where the blocks do not all start at once, and not up to 512
-// queries (four tiles: nothing to gain, and with a CTA per block a place that is computed cost 5-8 %).
-inline bool tail_order(const FwdLaunch& l) { return l.max_seqlen_q > 512; }
-
-// Whether a CTA goes on with blocks that have not started (cluster launch control, in the order of the grid) where there are more
-// than start at once.  The next block's Q, K and V load and its first scores are made while the rows of the one before leave; a CTA
-// of its own began with barriers, tensor memory and 3500 clk for its first scores, about two key tiles.  us, a CTA per block -> now:
-// d = 128, 16 x 12 x 1000 causal 85.5 -> 77.7, 64 x 12 x 256 59.4 -> 49.1, 32 x 12 x 512 ragged 61.4 -> 54.7, in pairs of tiles 4 x 32 x
-// 3000 causal 293 -> 269, 4 x 12 x 4096 343 -> 328, 16 x 12 x 8192 causal 2570 -> 2490; d = 64, 64 x 12 x 300 69.7 -> 59.3, padded
-// 64 x 12 x 512 ragged 92 -> 82; blocks without queries, which the producer passes over: 1 x 4096 and 63 x 128 tokens, 12 heads 182 ->
-// 116 (d = 64), 172 -> 128.
-// Quads of d = 64 up to some length alone: their two CTAs on an SM take longer for a tile, most of all in long walks (32 768 tokens, 12 heads,
-// not causal / causal, over a CTA per block: 600 0.95 / 0.87, 1024 0.96 / 0.92, 1500 0.99 / 0.95, 2048 1.02 / 0.96, 2560 1.01 / 0.99, 3000
-// 1.02 / 1.00, 4096 1.08 / 1.02, 1 x 2 x 65536 causal 1.09), unless most blocks are empty (31 x 256 and 1 x 8192: 0.97 / 0.91; announced with 2.5
-// times their tokens, 2 x 16384 and 3 x 1, 1.04).  Not with dropout: the loop has no registers left for it (8-14 % slower).
-template <int D, bool ROWS, bool CAUSAL>
-constexpr int kTakeMaxKeys = D == 64 && !ROWS ? (CAUSAL ? 2560 : 1536) : INT_MAX;
-
 template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BS, int G, bool ROWS, bool PADDED = false, Order ORDER = kPlain>
 cudaError_t launch_groups(const FwdLaunch& l, cudaStream_t stream) {
   dim3 grid((l.max_seqlen_q + G * kBlockM - 1) / (G * kBlockM), l.args.heads, l.args.batch);
   if constexpr (ORDER == kPlain) {
-    if (linear_grid(grid.x, grid.y, grid.z) && int64_t(grid.x) * grid.y * grid.z > kSlots<G>) {
-      constexpr bool kCanTake = !BS && !DROPOUT;
-      constexpr int kMaxKeys = kTakeMaxKeys<D, ROWS, CAUSAL>;
-      if constexpr (kCanTake)
-        if (l.max_seqlen_k <= kMaxKeys || uneven(l, 3))
-          return launch_groups<D, BF16, CAUSAL, DROPOUT, BS, G, ROWS, PADDED, kTake>(l, stream);
-      if constexpr (CAUSAL && !(kCanTake && kMaxKeys == INT_MAX))
-        if (tail_order(l)) return launch_groups<D, BF16, CAUSAL, DROPOUT, BS, G, ROWS, PADDED, kLinear>(l, stream);
-    }
+    const Order order = grid_order<D, CAUSAL, DROPOUT, BS, G, ROWS>(l);
+    if constexpr (kCanTake<DROPOUT, BS>)
+      if (order == kTake) return launch_groups<D, BF16, CAUSAL, DROPOUT, BS, G, ROWS, PADDED, kTake>(l, stream);
+    if constexpr (CAUSAL && !(kCanTake<DROPOUT, BS> && kTakeMaxKeys<D, ROWS, CAUSAL> == INT_MAX))
+      if (order == kLinear) return launch_groups<D, BF16, CAUSAL, DROPOUT, BS, G, ROWS, PADDED, kLinear>(l, stream);
   }
   auto kernel = fa_fwd_kernel<D, BF16, CAUSAL, DROPOUT, BS, G, ROWS, ORDER, PADDED>;
   using Cfg = FwdCfg<D, G, ROWS, ORDER == kTake>;
@@ -1172,66 +1132,6 @@ cudaError_t launch_groups(const FwdLaunch& l, cudaStream_t stream) {
   kernel<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(l.tm_q, l.tm_k, l.tm_v, l.tm_o, args);
   return cudaGetLastError();
 }
-
-// One query tile per CTA (two CTAs per SM) or two.  What one tile gains lies at the two ends of a CTA's walk over the
-// keys, which run under the tiles of the SM's other CTA.  What it loses is a share per key tile: two CTAs each read the K
-// and V that a pair reads once, and at d = 128 a single stage holds them.
-// Time with one tile / with two, 16 x 16 heads, not causal:
-//                        d = 64   dropout d = 64   d = 128   dropout d = 128
-//   128 queries, 512 keys     0.75       0.85           0.87       0.78
-//   256, 512                  0.88       0.94           1.00       0.87
-//   256, 4096                 1.06       1.01           1.16       1.07
-//   1024, 1024                0.91       0.92           1.02       0.97
-//   1024, 8192                1.03       1.04           1.17       1.09
-//   4096, 4096 (4 x 16)       1.00       1.01           1.16       1.08
-// so d = 64 takes single tiles at every length (causal calls too: 0.95-0.98).
-// d = 128 without dropout, whose CTAs go on with other blocks, so that the ends of a walk count for less (one / two, 12 heads, 16 384
-// tokens): not causal 200 tokens 1.08, 300 0.94, 512 1.14, 700 1.11, 1000 1.09, 1100 1.08, 1500 1.14, 1800 1.07, 3000 1.16, ragged 200 0.98,
-// 512 1.04, 1000 1.07, 2000 1.11; 16 x 256 queries, 512 and 1024 keys 1.09 and 1.16, 600 and 900 1.10, 2000 and 256 1.07, but three query
-// tiles, which leave a quarter of their pairs empty, 384 and 2048 0.97.  Causal, where the tiles of a pair differ by one in their keys
-// (even / ragged): 512 0.90 / 0.85, 1000 0.97 / 0.91, 1300 0.94 / 0.96, 1500 1.03 / 0.96, 1800 0.98 / 0.99, 2000 1.06 / 1.01, 2500 1.06 / 1.02,
-// 4096 1.07 / 1.03.
-// d = 128 with dropout: up to 1024 keys (causal calls count those up to the longest query) one (2000 queries, 256 keys 171 -> 156, 8 of 4096
-// and 512 201 -> 183).  Beyond, causal: 2000 0.96, 4096 1.00, 8192 1.01.  Not causal (8 x 12 / 4 x 16 heads): 1100 0.84 / 0.83,
-// 1500 1.00 / 1.03, 2000 0.94 / 0.94, 2500 0.97 / 0.97, 3000 1.04 / 0.97, 4096 1.04 / 1.07 (4 x 12 0.97), 6000 1.05 / 1.02, 8192 1.07 / 1.08, 384
-// queries and 2048 keys 0.66 / 1.07, 1100 and 4096 0.87 / 0.79: how the last round of CTAs falls decides, and the rule stays.
-// A grid of single tiles that fits one per SM spreads over twice the SMs: 16 heads, 1024 queries, 8192 keys 0.72 (d = 64),
-// 0.92 (d = 128), 0.63 and 0.78 with dropout.
-// A grid of pairs that fills between half of the SMs and all of them runs in one round either way and reads K and
-// V once per pair: 80-140 pairs of 200-4000 queries 1.02-1.13, with dropout 0.99-1.15.
-// Up to 128 queries both grids have as many CTAs; with long keys at d = 128 one alone on its SM then wants the second
-// stage (16 queries, 4096 keys, one -> two: 96 (batch, head) pairs 69 -> 52 us, 144 pairs 80 -> 58).  From 149 on two
-// share an SM: 192 pairs 85 us, 128 with two.
-// Uneven batches (see `uneven`) announced with more than 4096 tokens take pairs at d = 64 too, which halves their empty blocks:
-// 31 x 256 and 1 x 8192, 12 heads 431 -> 374 us, 2 x 16384 and 126 x 64, 4 heads 948 -> 865.
-constexpr int kOneTileMaxD128 = 1024, kOneTileMaxCausal = 1920, kOneTileMaxCausalDropout = 4096;  // keys
-constexpr int kOneTileMaxUneven = 4096;  // queries and keys, d = 64
-
-template <int D, bool CAUSAL, bool DROPOUT>
-bool one_tile_per_cta(const FwdLaunch& l) {
-  const int64_t heads = static_cast<int64_t>(l.args.heads) * l.args.batch;
-  const int64_t q_tiles = (l.max_seqlen_q + kBlockM - 1) / kBlockM;
-  const int64_t tiles = q_tiles * heads, pairs = (q_tiles + 1) / 2 * heads;
-  const int keys = CAUSAL ? min(l.max_seqlen_k, l.max_seqlen_q) : l.max_seqlen_k;
-  const bool one_round = pairs > kSms / 2 && pairs <= kSms;
-  if (l.max_seqlen_q <= kBlockM) return D == 64 || DROPOUT || keys <= kOneTileMaxD128 || pairs > kSms;
-  if (one_round) return false;
-  if (D == 64) return !(uneven(l) && max(l.max_seqlen_q, keys) > kOneTileMaxUneven);
-  const bool pairs_at_once = !CAUSAL && !DROPOUT && q_tiles != 3;  // (at any length)
-  if (l.max_seqlen_q <= kOneTileMaxD128 && (tiles <= kSms || (keys <= kOneTileMaxD128 && !pairs_at_once))) return true;
-  if (uneven(l) || pairs_at_once) return false;  // (uneven: twice the empty blocks)
-  if (keys <= kOneTileMaxD128) return true;
-  if (CAUSAL) return keys <= (DROPOUT ? kOneTileMaxCausalDropout : kOneTileMaxCausal);
-  return !DROPOUT || q_tiles % 2 != 0 || l.max_seqlen_q > kOneTileMaxD128;
-}
-
-// Rows for d = 128 without dropout, and for d = 64 without dropout up to 512 keys: there the ends of a CTA's
-// walk are most of it, and twelve warps take longer through them than eight (quads / rows: 12 heads of 128 queries and
-// keys 5.9 / 5.7 us, 16 x 16 heads, 128 queries, 512 keys 12.5 / 11.8, 1024 keys and queries 0.98).
-constexpr int kRowsMaxD64 = 512;  // keys
-
-template <int D, bool DROPOUT>
-bool rows_layout(const FwdLaunch& l) { return !DROPOUT && (D == 128 || l.max_seqlen_k <= kRowsMaxD64); }
 
 template <int D, bool CAUSAL, bool DROPOUT>
 int box_columns(const FwdLaunch& l) {
