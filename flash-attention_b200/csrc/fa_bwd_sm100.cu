@@ -119,7 +119,6 @@ struct BwdShared {
   uint64_t drained[3];                        // of the issuing warps, at their end
   alignas(16) uint4 next;
   alignas(16) BlockRecord<CAUSAL> blk[2];               // block k in entry k % 2
-  uint32_t alive;                             // changes as the producer gets on (see mbar_wait_warp_alive)
   uint64_t q_full[3], q_empty[3];
   uint64_t do_full, do_empty;  // dO ring of the two-phase schedule (one stage)
   // d = 64: S and dP together / P~ and dS together.  Two-phase schedule: sdp_full = dP landed,
@@ -472,7 +471,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     if (!take_over) return false;
     __syncwarp();
     if (elect_one()) mbar_arrive(smem_u32(&sh.blk_done[k & 1]));
-    return mbar_wait_warp_alive<kVote>(smem_u32(&sh.blk_full[(k + 1) & 1]), (k >> 1) & 1, abort_flag, &sh.alive) && sh.blk[(k + 1) & 1].nm >= 0;
+    return mbar_wait_warp<kVote>(smem_u32(&sh.blk_full[(k + 1) & 1]), (k >> 1) & 1, abort_flag) && sh.blk[(k + 1) & 1].nm >= 0;
   };
 
   if (warp >= kProducer) {
@@ -505,7 +504,6 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           if (lead) {
             mbar_expect_tx(smem_u32(&sh.next_full), 16);
             clc_try_cancel(smem_u32(&sh.next), smem_u32(&sh.next_full));
-            *const_cast<volatile uint32_t*>(&sh.alive) = asked;
           }
           ++asked;
         };
@@ -576,7 +574,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           more = !launch_failed();
           if (BLOCKSPARSE) more = __all_sync(0xffffffffu, more);
           x = decode(block);
-          if (!more || x.n0 < x.sk) break;
+          if (!more || x.n0 < x.sk || asked % kPassOnEvery == 0) break;  // (the last: see kPassOnEvery)
           take_next();
         }
         if (!ok) break;
@@ -585,7 +583,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         if (k >= 1) ok = wait(sh.blk_done[(k + 1) & 1], ((k - 1) >> 1) & 1);
         if (!ok) break;
         if constexpr (BLOCKSPARSE) {
-          if (more) {
+          if (more && x.n0 < x.sk) {
             const int mt = list_tiles(x);
             x.nm = 0;
             for (int c = 0; c * 32 < mt; ++c) {
@@ -1167,7 +1165,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 
     // ---------------- epilogue: group 0 writes dV = acc / p_keep, group 1 writes dK = acc * scale / p_keep
     if (ok && take_over) {
-      ok = mbar_wait_warp_alive<kVote>(smem_u32(&sh.blk_full[(k + 1) & 1]), (k >> 1) & 1, abort_flag, &sh.alive);
+      ok = mbar_wait_warp<kVote>(smem_u32(&sh.blk_full[(k + 1) & 1]), (k >> 1) & 1, abort_flag);
       fetched = ok && sh.blk[(k + 1) & 1].nm > 0;
       if (fetched) fetch_stats(sh.blk[(k + 1) & 1], 0, k + 1);
     }

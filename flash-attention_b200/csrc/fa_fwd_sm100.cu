@@ -103,7 +103,7 @@ struct FwdShared {
   float2 row_stats[STATS][kBlockM];  // (max, sum) of every query row, for the epilogue; taking over: two of a group, by the block's parity
   alignas(16) uint4 next;
   FwdBlock blk[2];  // block k in entry k % 2
-  uint32_t alive;   // changes as the producer gets on (see mbar_wait_warp_alive)
+  uint32_t alive;   // pairs: changes as the producer gets on (see mbar_wait_alive)
   uint32_t tmem_base;
   int abort_flag;
   int stop;  // a CTA of this launch has abandoned a wait
@@ -409,11 +409,13 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     else return first;
   };
   // A warp has finished block k: waits for the next one, if any (or until a wait is abandoned).
-  auto next_block = [&](uint32_t k) -> bool {
+  // idle: a softmax group without rows has no part in the block, which the others may be at for any time.
+  auto next_block = [&](uint32_t k, bool idle = false) -> bool {
     if constexpr (!TAKE) return false;
     __syncwarp();
     if (elect_one()) mbar_arrive(smem_u32(&sh.blk_done[k & 1]));
-    return mbar_wait_warp_alive<true>(smem_u32(&sh.blk_full[(k + 1) & 1]), (k >> 1) & 1, abort_flag, &sh.alive) && sh.blk[(k + 1) & 1].mp >= 0;
+    if (G == 2 && idle) mbar_wait_alive(smem_u32(&sh.blk_full[(k + 1) & 1]), (k >> 1) & 1, abort_flag, &sh.alive);
+    return mbar_wait_warp<true>(smem_u32(&sh.blk_full[(k + 1) & 1]), (k >> 1) & 1, abort_flag) && sh.blk[(k + 1) & 1].mp >= 0;
   };
 
   if (warp >= Cfg::kSoftmaxWarps) reg_dealloc<Cfg::kOtherRegs>();
@@ -423,12 +425,11 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       bool ok = true;
       int loads_k = 0, loads_v = 0, loads_q[G] = {};  // so far
       uint32_t asked = 0;                             // requests so far
-      auto still_alive = [&](uint32_t count) { *const_cast<volatile uint32_t*>(&sh.alive) = count; };
       // asked for with the loads of the last key tile: a block taken earlier would wait here while other SMs run dry
       auto take_next = [&]() {
         mbar_expect_tx(smem_u32(&sh.next_full), 16);
         clc_try_cancel(smem_u32(&sh.next), smem_u32(&sh.next_full));
-        still_alive(++asked + loads_k);
+        ++asked;
       };
       FwdBlock x = first;
       for (uint32_t k = 0; ok; ++k) {
@@ -452,7 +453,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
             load_tile(smem_k + s * Cfg::kTileBytes, &tm_k, sh.k_full[s], row, x.h);
           }
           ++loads_k;
-          if (TAKE) still_alive(asked + loads_k);
+          if (TAKE && G == 2) *const_cast<volatile uint32_t*>(&sh.alive) = loads_k;
           if (TAKE && j + 1 == n_max) take_next();
           if (k > 0 || j > 0) {
             if (loads_v >= Cfg::kStages) ok = mbar_wait(smem_u32(&sh.v_empty[s]), ph, abort_flag);
@@ -464,7 +465,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
         }
         if (!TAKE || !ok) break;
         if (n_max == 0) take_next();
-        // The next block with queries.  (Padded batches pass the others on too: their rows get zeros.)
+        // The next block with queries.  (Padded batches pass the others on too: their rows get zeros.  Else see kPassOnEvery.)
         bool more = false;
         while (true) {
           ok = mbar_wait(smem_u32(&sh.next_full), (asked - 1) & 1, abort_flag);
@@ -476,6 +477,10 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
           more = !launch_failed();
           x = decode(block);
           if (!more || PADDED || !without_queries(x)) break;
+          if (asked % kPassOnEvery == 0) {
+            x.mp = x.sq = 0;
+            break;
+          }
           take_next();
         }
         if (!ok) break;
@@ -683,11 +688,11 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     const uint32_t tP = tmem + (g == 0 ? Cfg::kTmemP0 : Cfg::kTmemP1) + lane_sel;
     bool ok = true, s_early = false;
     const uint64_t c2 = pack_f2(a.scale_log2, a.scale_log2);
-    int t = 0;                // key tiles so far
+    int t = 0, n;             // key tiles so far, of the block
     uint32_t k = 0, c_o = 0;  // block; blocks with key tiles before
     do {
     const FwdBlock& x = block_at(k);
-    const int n = x.n(g);
+    n = x.n(g);
     float m_run = -INFINITY, l_run = 0.f;
     const int free_tiles = CAUSAL ? min(x.sk / kBlockN, x.mp * G + g) : x.sk / kBlockN;  // key tiles without a mask
 
@@ -851,7 +856,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&sh.out_free));
     }
-    } while (ok && next_block(k++));
+    } while (ok && next_block(k++, n == 0));
     if (TAKE && lane == 0) bulk_wait_read();
   } else if (warp < Cfg::kSoftmaxWarps) {
     // ------------------------------------------------------------------ softmax warps
@@ -868,11 +873,11 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     const uint32_t tP = tmem + (g == 0 ? Cfg::kTmemP0 : Cfg::kTmemP1) + lane_sel;
     bool ok = true;
     const uint64_t c2 = pack_f2(a.scale_log2, a.scale_log2);
-    int t = 0;                // key tiles so far
+    int t = 0, n;             // key tiles so far, of the block
     uint32_t k = 0, c_o = 0, c_s = 0;  // block; blocks with key tiles before, with queries before
     do {
     const FwdBlock& x = block_at(k);
-    const int n = x.n(g);
+    n = x.n(g);
     // rows r8 (u = 0) and r8 + 8 (u = 1); l_run: this thread's share of the row sum (its 32 columns per tile)
     float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
     const int free_tiles = CAUSAL ? min(x.sk / kBlockN, x.mp * G + g) : x.sk / kBlockN;  // key tiles without a mask
@@ -1094,7 +1099,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
                                n > 0 && ok, ok, m_first + wq * 32, lane, x.sq, x.q_start, x.b, x.h, st.x, st.y, piece);
     }
     if (n > 0) ++c_o;
-    } while (ok && next_block(k++));
+    } while (ok && next_block(k++, n == 0));
     if (TAKE && lane == 0) bulk_wait_read();
   }
 

@@ -33,6 +33,9 @@ __device__ __forceinline__ bool elect_one() {
 // mbarrier
 // ---------------------------------------------------------------------------------------------
 constexpr long long WAIT_LIMIT_CYCLES = 200000000LL;  // about 0.1 s at 2 GHz; a healthy wait lasts microseconds
+// Where CTAs take over blocks, the others of its roles wait while the producer passes over blocks without work, 0.4-0.7 us each: every 4096th
+// goes through all roles, so that no such wait comes near the limit.
+constexpr uint32_t kPassOnEvery = 4096;
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -100,24 +103,18 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
 
-// The same where the wait spans another role's work of any length (the producer passes over thousands of blocks without work, or one
-// group walks a long sequence while the other has no rows): `alive` is a word which that role changes as it gets on, and the
-// wait is abandoned where it has stood still for the limit.
-template <bool VOTE_FIRST = false>
-__device__ __forceinline__ bool mbar_wait_warp_alive(uint32_t bar, uint32_t parity, volatile int* abort_flag, const volatile uint32_t* alive) {
-  if constexpr (VOTE_FIRST)
-    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+// Ahead of a wait that spans another role's work of any length (one group walks a long sequence while the other has no rows): until the
+// phase is over or `alive`, a word which that role changes as it gets on, has stood still for the limit.
+__device__ __forceinline__ void mbar_wait_alive(uint32_t bar, uint32_t parity, const volatile int* abort_flag, const volatile uint32_t* alive) {
   uint32_t seen = *alive;
   long long t0 = clock64();
-  bool done;
-  while (!(done = mbar_try_wait(bar, parity)) && !*abort_flag) {
+  while (!mbar_try_wait(bar, parity) && !*abort_flag) {
     if (clock64() - t0 <= WAIT_LIMIT_CYCLES) continue;
     const uint32_t now = *alive;
-    if (now == seen) *abort_flag = 1;
+    if (now == seen) return;
     seen = now;
     t0 = clock64();
   }
-  return __all_sync(0xffffffffu, done);
 }
 
 // What a role has under way (a copy into shared memory, products in tensor memory) ends before the CTA does, also after an
