@@ -39,7 +39,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <type_traits>
-#include "fa_kernels.h"
+#include "fa_rules.h"
 #include "fa_math.cuh"
 #include "sm100_prims.cuh"
 
@@ -49,7 +49,6 @@ namespace {
 
 constexpr int kBM = 128;  // query rows per tile
 constexpr int kBN = 128;  // key rows per tile
-constexpr int kSms = 148;
 constexpr int kMaxSparseTiles = 1024;  // query tiles of 128 per sequence in block-sparse mode
 
 // BS: block-sparse variant (its tile list takes shared memory that the third Q / dO stage would need)
@@ -384,7 +383,7 @@ fa_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 
   if (tid == 0) {
     sh.abort_flag = 0;
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < Cfg::kKvStages; ++i) {
       mbar_init(smem_u32(&sh.k_full[i]), 1);
       mbar_init(smem_u32(&sh.v_full[i]), 1);
       mbar_init(smem_u32(&sh.k_empty[i]), 1);
@@ -1531,20 +1530,12 @@ __global__ void bwd_postprocess_kernel(const BwdArgs a, int dpad) {
   *reinterpret_cast<uint4*>(dst) = out;
 }
 
-// Calls with few query tiles at d = 64: a block's K and V are then a good part of its loads and are waited for at its start, so two
-// stages hold them, and two (not three) Q and dO.  Whole backward, 12 heads, 32 768 tokens, us, one stage of K and V -> two: 64 x 512
-// 239 -> 247, 85 x 384 212 -> 213, 128 x 256 182 -> 171, 163 x 200 212 -> 206, 256 x 128 155 -> 149, with dropout (ragged) up to 256
-// 239 -> 234, up to 384 261 -> 266; 16 x 8 heads, up to 256 queries, 1500 keys 67.4 -> 63.6, 300 queries 67.5 -> 67.6.
-constexpr int kShortQueries = 256;
-inline bool short_queries(const BwdLaunch& l) { return l.args.max_seqlen_q <= kShortQueries; }
-
 template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BS, bool ONE_LAUNCH = false, bool SHORT = false>
 cudaError_t launch_main(const BwdLaunch& l, cudaStream_t stream) {
   if constexpr (!BS && !ONE_LAUNCH && !SHORT) {
     if (l.args.one_launch) return launch_main<D, BF16, CAUSAL, DROPOUT, BS, true>(l, stream);
     if constexpr (D == 64)
-      if (short_queries(l) && int64_t((l.args.max_seqlen_k + kBN - 1) / kBN) * l.args.k.heads * l.args.k.batch > kSms)
-        return launch_main<D, BF16, CAUSAL, DROPOUT, BS, false, true>(l, stream);
+      if (short_queries(l)) return launch_main<D, BF16, CAUSAL, DROPOUT, BS, false, true>(l, stream);
   }
   auto kernel = fa_bwd_kernel<D, BF16, CAUSAL, DROPOUT, BS, ONE_LAUNCH, SHORT>;
   using Cfg = BwdCfg<D, BS, DROPOUT, SHORT>;

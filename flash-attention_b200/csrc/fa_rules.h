@@ -113,4 +113,17 @@ constexpr int kRowsMaxD64 = 512;  // keys
 template <int D, bool DROPOUT>
 bool rows_layout(const FwdLaunch& l) { return !DROPOUT && (D == 128 || l.max_seqlen_k <= kRowsMaxD64); }
 
+// Backward.  Calls with few query tiles at d = 64: a block's K and V are then a good part of its loads and are waited for at its start, so two
+// stages hold them, and two (not three) Q and dO.  Whole backward, us, one stage of K and V -> two: 32 x 12 heads, 256 queries, 500 keys
+// 76.3 -> 72.8, 1500 178.4 -> 169.4, with dropout 86.9 -> 84.4 and 209.4 -> 204.8; 128 x 12 x 128 80.9 -> 77.1; 64 x 12 x 512 239 -> 247, 85 x
+// 384 212 -> 213, with dropout (ragged) up to 384 261 -> 266.  With a causal mask, 128 x 12 x 256 180.9 -> 171.3, with dropout 192 -> 186, but
+// not where keys lie behind the last query, whose blocks store zeros and little else: 32 x 12, 40 queries, 1500 keys 52.2 -> 53.3, with
+// dropout (28 bytes of spills) 57.7 -> 62.6, 200 queries 83.5 -> 88.0.
+constexpr int kShortQueries = 256;
+inline bool short_queries(const BwdLaunch& l) {
+  const int q_tiles = (l.args.max_seqlen_q + kBlockM - 1) / kBlockM, k_tiles = (l.args.max_seqlen_k + kBlockN - 1) / kBlockN;
+  return l.dpad == 64 && l.args.max_seqlen_q <= kShortQueries && int64_t(k_tiles) * l.args.k.heads * l.args.k.batch > kSms &&
+         (!l.is_causal || k_tiles <= q_tiles);
+}
+
 }  // namespace fa

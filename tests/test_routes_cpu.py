@@ -1,5 +1,5 @@
 """CPU test of the rules that choose a kernel for a call, on the functions that the launches use (compiled for the host): query tiles
-per CTA, softmax layout and order of the forward's grid.  The cases are those of the GPU tests that aim at a kernel, and the calls on
+per CTA, softmax layout and order of the forward's grid, stages of the backward.  The cases are those of the GPU tests that aim at a kernel, and the calls on
 either side of a rule's line."""
 import os
 import shutil
@@ -44,8 +44,17 @@ bool pair_by_pair() {
 }
 int main(int argc, char**) {
   if (argc > 1) return pair_by_pair() ? 0 : 1;
+  char kind;
   int d, batch, heads, mq, mk, total, causal, dropout, bs;
-  while (scanf("%d %d %d %d %d %d %d %d %d", &d, &batch, &heads, &mq, &mk, &total, &causal, &dropout, &bs) == 9) {
+  while (scanf(" %c %d %d %d %d %d %d %d %d %d", &kind, &d, &batch, &heads, &mq, &mk, &total, &causal, &dropout, &bs) == 10) {
+    if (kind == 'b') {
+      fa::BwdLaunch w;
+      std::memset(&w, 0, sizeof w);
+      w.dpad = d; w.is_causal = causal; w.is_dropout = dropout;
+      w.args.k.batch = batch; w.args.k.heads = heads; w.args.max_seqlen_q = mq; w.args.max_seqlen_k = mk;
+      puts(fa::short_queries(w) ? "short" : "long");
+      continue;
+    }
     fa::FwdLaunch l;
     std::memset(&l, 0, sizeof l);
     l.args.batch = batch; l.args.heads = heads;
@@ -62,7 +71,7 @@ int main(int argc, char**) {
 def call(d, q_lens, heads, max_k=None, causal=False, dropout=False, sparse=False, max_q=None):
     """(d is the padded head size, 64 or 128)"""
     max_q = max_q or max(q_lens)
-    return (d, len(q_lens), heads, max_q, max_k or max_q, sum(q_lens), int(causal), int(dropout), int(sparse))
+    return ("f", d, len(q_lens), heads, max_q, max_k or max_q, sum(q_lens), int(causal), int(dropout), int(sparse))
 
 
 # d = 128, one query tile per CTA (the GPU test of these compares each with 64 bits)
@@ -73,6 +82,10 @@ LIMIT_D128 = ([1900, 1700, 1919, 1601], 12)
 # forwards that take blocks over
 TAKE_OVER = [(128, [1000] * 40, 12, False, 2), (128, [300, 256] * 60, 8, True, 1), (64, [300, 512] * 40, 12, False, 1), (64, [1000, 700] * 30, 12, True, 1)]
 
+def backward(d, batch, heads, max_q, max_k, causal=False, dropout=False):
+    return ("b", d, batch, heads, max_q, max_k, batch * max_q, int(causal), int(dropout), 0)
+
+
 CASES = (
     [(call(128, q, h, max(k or q), c), ("1", "rows")) for q, h, k, c in SINGLE_TILES_D128[:2] + SINGLE_TILES_D128[3:]]
     + [(call(128, LIMIT_D128[0], LIMIT_D128[1], n, True, max_q=n), (tiles, "rows")) for n, tiles in ((1920, "1"), (1921, "2"))]
@@ -82,7 +95,13 @@ CASES = (
        (call(64, [1000] * 40, 12, causal=True, dropout=True), ("1", "quads", "linear")),
        (call(64, [4096] * 4, 16, causal=True, sparse=True), ("1", "quads", "linear")),
        (call(64, [4096] * 8, 12, causal=True), ("1", "quads", "linear")), (call(64, [4096] * 8, 12), ("1", "quads", "plain")),
-       (call(128, [4096] * 8, 12, dropout=True), ("1", "quads", "plain"))])
+       (call(128, [4096] * 8, 12, dropout=True), ("1", "quads", "plain"))]
+    # two stages of K and V in the backward: not with a causal mask and keys that no query sees
+    + [(backward(64, 16, 8, 200, 1500), ("short",)), (backward(64, 16, 8, 257, 1500), ("long",)), (backward(64, 32, 12, 40, 1500, dropout=True), ("short",)),
+       (backward(64, 12, 12, 200, 128), ("long",)), (backward(64, 64, 12, 256, 256, causal=True), ("short",)),
+       (backward(64, 64, 12, 128, 128, causal=True, dropout=True), ("short",)), (backward(64, 32, 12, 40, 1500, causal=True, dropout=True), ("long",)),
+       (backward(64, 32, 12, 200, 500, causal=True), ("long",)), (backward(64, 32, 12, 200, 257, causal=True), ("long",)),
+       (backward(128, 16, 8, 200, 1500), ("long",))])
 
 
 @pytest.fixture(scope="module")
