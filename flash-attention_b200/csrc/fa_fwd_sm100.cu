@@ -1121,7 +1121,7 @@ cudaError_t launch_groups(const FwdLaunch& l, cudaStream_t stream) {
     const Order order = grid_order<D, CAUSAL, DROPOUT, BS, G, ROWS>(l);
     if constexpr (kCanTake<DROPOUT, BS>)
       if (order == kTake) return launch_groups<D, BF16, CAUSAL, DROPOUT, BS, G, ROWS, PADDED, kTake>(l, stream);
-    if constexpr (CAUSAL && !(kCanTake<DROPOUT, BS> && kTakeMaxKeys<D, ROWS, CAUSAL> == INT_MAX))
+    if constexpr (CAUSAL)
       if (order == kLinear) return launch_groups<D, BF16, CAUSAL, DROPOUT, BS, G, ROWS, PADDED, kLinear>(l, stream);
   }
   auto kernel = fa_fwd_kernel<D, BF16, CAUSAL, DROPOUT, BS, G, ROWS, ORDER, PADDED>;

@@ -20,6 +20,15 @@ inline bool uneven(const FwdLaunch& l, int times = 2) {
 
 constexpr int kSms = 148;
 
+// Groups of g query tiles that hold rows of a sequence, over all heads, as far as the lengths on the host tell: all of them where every
+// sequence is as long as announced, else the rows' share and half a group at the end of each sequence.
+inline bool even_batch(const FwdLaunch& l) { return static_cast<int64_t>(l.args.batch) * l.max_seqlen_q <= l.total_q; }
+inline int64_t groups_with_rows(const FwdLaunch& l, int g) {
+  const int64_t rows = g * kBlockM, all = (l.max_seqlen_q + rows - 1) / rows * l.args.batch;
+  const int64_t some = l.total_q / rows + (l.args.batch + 1) / 2;
+  return (even_batch(l) || some > all ? all : some) * l.args.heads;
+}
+
 // Blocks that start at once
 template <int G>
 constexpr int kSlots = (G == 1 ? 2 : 1) * kSms;
@@ -39,17 +48,37 @@ inline bool tail_order(const FwdLaunch& l) { return l.max_seqlen_q > 512; }
 // not causal / causal, over a CTA per block: 600 0.95 / 0.87, 1024 0.96 / 0.92, 1500 0.99 / 0.95, 2048 1.02 / 0.96, 2560 1.01 / 0.99, 3000
 // 1.02 / 1.00, 4096 1.08 / 1.02, 1 x 2 x 65536 causal 1.09), unless most blocks are empty (31 x 256 and 1 x 8192: 0.97 / 0.91; announced with 2.5
 // times their tokens, 2 x 16384 and 3 x 1, 1.04).  Not with dropout: the loop has no registers left for it (8-14 % slower).
+// Nor in grids of few rounds, where little is taken over and a block that was asked for early waits for its CTA while others end.  Time
+// over that of a CTA per block, 12 heads, by rounds (announced blocks over those that start at once):
+//   quads, not causal    6 x 600 ragged 1.14 (1.2), 5 x 1500 ragged 1.15 (2.4), 14 x 600 1.10 (2.8), 11 x 1000 ragged 1.08 (3.6), 25 x 600 0.94 (5); even
+//                        batches 0.96-0.97 up to 1.5
+//   quads, causal        7 x 700 1.07 (1.7), 5 x 900 1.09, 9 x 1000 1.03 (2.9), 17 x 600 0.97 (3.4), 11 x 1000 0.98 (3.6), 21 x 700 0.94 (5)
+//   rows (d = 64), single tiles (d = 128)   even batches 0.9-0.98 from one round on; where the blocks with rows start at once, 14 x 200 of 1 to 200
+//                        tokens 1.19-1.23, 9 x 300 ragged 1.04-1.12, and at d = 64 or without a causal mask up to 1.5 rounds of those (14 x 500 of 1 to
+//                        500 tokens 1.06-1.11)
+//   d = 128, causal, up to 512 queries (no order of weight)   15 x 300 1.12 (1.8), 18 x 300 ragged 1.15, 17 x 200 of 1 to 200 tokens 1.25; from 3.5
+//                        rounds of blocks with rows on 0.94-1.0
+// Up to 128 queries, and in pairs of query tiles, it pays at any size (0.9, 0.93-0.97 just above one round).
 template <int D, bool ROWS, bool CAUSAL>
 constexpr int kTakeMaxKeys = D == 64 && !ROWS ? (CAUSAL ? 2560 : 1536) : INT_MAX;
+template <int D, int G, bool ROWS, bool CAUSAL>
+bool take_over_pays(const FwdLaunch& l, int64_t blocks) {
+  if (uneven(l, 3)) return true;
+  if (l.max_seqlen_k > kTakeMaxKeys<D, ROWS, CAUSAL>) return false;
+  if (l.max_seqlen_q <= kBlockM || (ROWS && G == 2)) return true;
+  if (!ROWS) return 4 * blocks > (CAUSAL ? 13 : 16) * kSlots<G> || (!CAUSAL && even_batch(l) && 2 * blocks <= 3 * kSlots<G>);
+  const int quarter_rounds = D == 128 && CAUSAL ? (tail_order(l) ? 4 : 13) : even_batch(l) ? 4 : 6;  // of blocks with rows
+  return 4 * groups_with_rows(l, G) > quarter_rounds * kSlots<G>;
+}
 
 template <bool DROPOUT, bool BS>
 constexpr bool kCanTake = !BS && !DROPOUT;
 
 template <int D, bool CAUSAL, bool DROPOUT, bool BS, int G, bool ROWS>
 Order grid_order(const FwdLaunch& l) {
-  const int64_t tiles = (l.max_seqlen_q + G * kBlockM - 1) / (G * kBlockM);
-  if (!linear_grid(tiles, l.args.heads, l.args.batch) || tiles * l.args.heads * l.args.batch <= kSlots<G>) return kPlain;
-  if (kCanTake<DROPOUT, BS> && (l.max_seqlen_k <= kTakeMaxKeys<D, ROWS, CAUSAL> || uneven(l, 3))) return kTake;
+  const int64_t tiles = (l.max_seqlen_q + G * kBlockM - 1) / (G * kBlockM), blocks = tiles * l.args.heads * l.args.batch;
+  if (!linear_grid(tiles, l.args.heads, l.args.batch) || blocks <= kSlots<G>) return kPlain;
+  if (kCanTake<DROPOUT, BS> && take_over_pays<D, G, ROWS, CAUSAL>(l, blocks)) return kTake;
   return CAUSAL && tail_order(l) ? kLinear : kPlain;
 }
 

@@ -96,6 +96,14 @@ CASES = (
        (call(64, [4096] * 4, 16, causal=True, sparse=True), ("1", "quads", "linear")),
        (call(64, [4096] * 8, 12, causal=True), ("1", "quads", "linear")), (call(64, [4096] * 8, 12), ("1", "quads", "plain")),
        (call(128, [4096] * 8, 12, dropout=True), ("1", "quads", "plain"))]
+    # grids of few rounds: a CTA per block
+    + [(call(64, [600, 450, 300, 560, 420, 330], 12), ("1", "quads", "plain")), (call(64, [600] * 12, 12), ("1", "quads", "plain")),
+       (call(64, [600] * 5, 12), ("1", "quads", "take")), (call(64, [600] * 25, 12), ("1", "quads", "take")),
+       (call(64, [900] * 5, 12, causal=True), ("1", "quads", "linear")), (call(64, [700] * 21, 12, causal=True), ("1", "quads", "take")),
+       (call(64, [200] + [100] * 13, 12), ("1", "rows", "plain")), (call(64, [200] * 14, 12), ("1", "rows", "take")),
+       (call(128, [300] * 16, 12, causal=True), ("1", "rows", "plain")), (call(128, [300] * 41, 12, causal=True), ("1", "rows", "take")),
+       (call(128, [700] * 7, 12, causal=True), ("1", "rows", "take")), (call(128, [700] + [300] * 5, 12, causal=True), ("1", "rows", "linear")),
+       (call(64, [128] * 30, 12), ("1", "rows", "take")), (call(64, [8192] + [256] * 31, 12), ("2", "quads", "take"))]
     # two stages of K and V in the backward: not with a causal mask and keys that no query sees
     + [(backward(64, 16, 8, 200, 1500), ("short",)), (backward(64, 16, 8, 257, 1500), ("long",)), (backward(64, 32, 12, 40, 1500, dropout=True), ("short",)),
        (backward(64, 12, 12, 200, 128), ("long",)), (backward(64, 64, 12, 256, 256, causal=True), ("short",)),
