@@ -54,8 +54,7 @@ inline bool tail_order(const FwdLaunch& l) { return l.max_seqlen_q > 512; }
 //                        batches 0.96-0.97 up to 1.5
 //   quads, causal        7 x 700 1.07 (1.7), 5 x 900 1.09, 9 x 1000 1.03 (2.9), 17 x 600 0.97 (3.4), 11 x 1000 0.98 (3.6), 21 x 700 0.94 (5)
 //   rows (d = 64), single tiles (d = 128)   even batches 0.9-0.98 from one round on; where the blocks with rows start at once, 14 x 200 of 1 to 200
-//                        tokens 1.19-1.23, 9 x 300 ragged 1.04-1.12, and at d = 64 or without a causal mask up to 1.5 rounds of those (14 x 500 of 1 to
-//                        500 tokens 1.06-1.11)
+//                        tokens 1.19-1.23, 9 x 300 ragged 1.04-1.12
 //   d = 128, causal, up to 512 queries (no order of weight)   15 x 300 1.12 (1.8), 18 x 300 ragged 1.15, 17 x 200 of 1 to 200 tokens 1.25; from 3.5
 //                        rounds of blocks with rows on 0.94-1.0
 // Up to 128 queries, and in pairs of query tiles, it pays at any size (0.9, 0.93-0.97 just above one round).
@@ -67,8 +66,7 @@ bool take_over_pays(const FwdLaunch& l, int64_t blocks) {
   if (l.max_seqlen_k > kTakeMaxKeys<D, ROWS, CAUSAL>) return false;
   if (l.max_seqlen_q <= kBlockM || (ROWS && G == 2)) return true;
   if (!ROWS) return 4 * blocks > (CAUSAL ? 13 : 16) * kSlots<G> || (!CAUSAL && even_batch(l) && 2 * blocks <= 3 * kSlots<G>);
-  const int quarter_rounds = D == 128 && CAUSAL ? (tail_order(l) ? 4 : 13) : even_batch(l) ? 4 : 6;  // of blocks with rows
-  return 4 * groups_with_rows(l, G) > quarter_rounds * kSlots<G>;
+  return 40 * groups_with_rows(l, G) > (D == 128 && CAUSAL && !tail_order(l) ? 130 : even_batch(l) ? 40 : 44) * kSlots<G>;
 }
 
 template <bool DROPOUT, bool BS>
@@ -96,8 +94,8 @@ Order grid_order(const FwdLaunch& l) {
 // so d = 64 takes single tiles at every length (causal calls too: 0.95-0.98).
 // d = 128 without dropout, whose CTAs go on with other blocks, so that the ends of a walk count for less (one / two, 12 heads, 16 384
 // tokens): not causal 200 tokens 1.08, 300 0.94, 512 1.14, 700 1.11, 1000 1.09, 1100 1.08, 1500 1.14, 1800 1.07, 3000 1.16, ragged 200 0.98,
-// 512 1.04, 1000 1.07, 2000 1.11; 16 x 256 queries, 512 and 1024 keys 1.09 and 1.16, 600 and 900 1.10, 2000 and 256 1.07, but three query
-// tiles, which leave a quarter of their pairs empty, 384 and 2048 0.97.  Causal, where the tiles of a pair differ by one in their keys
+// 512 1.04, 1000 1.07, 2000 1.11; 16 x 256 queries, 512 and 1024 keys 1.09 and 1.16, 600 and 900 1.10, 2000 and 256 1.07 (see
+// pairs_fall_short for the others).  Causal, where the tiles of a pair differ by one in their keys
 // (even / ragged): 512 0.90 / 0.85, 1000 0.97 / 0.91, 1300 0.94 / 0.96, 1500 1.03 / 0.96, 1800 0.98 / 0.99, 2000 1.06 / 1.01, 2500 1.06 / 1.02,
 // 4096 1.07 / 1.03.
 // d = 128 with dropout: up to 1024 keys (causal calls count those up to the longest query) one (2000 queries, 256 keys 171 -> 156, 8 of 4096
@@ -113,8 +111,28 @@ Order grid_order(const FwdLaunch& l) {
 // share an SM: 192 pairs 85 us, 128 with two.
 // Uneven batches (see `uneven`) announced with more than 4096 tokens take pairs at d = 64 too, which halves their empty blocks:
 // 31 x 256 and 1 x 8192, 12 heads 431 -> 374 us, 2 x 16384 and 126 x 64, 4 heads 948 -> 865.
-constexpr int kOneTileMaxD128 = 1024, kOneTileMaxCausal = 1920, kOneTileMaxCausalDropout = 4096;  // keys
+constexpr int kPairsMaxKeys = 640, kOneTileMaxOdd = 2048, kOneTileMaxD128 = 1024, kOneTileMaxCausal = 1920, kOneTileMaxCausalDropout = 4096;  // keys
 constexpr int kOneTileMaxUneven = 4096;  // queries and keys, d = 64
+
+// d = 128, not causal, no dropout, where pairs serve most calls (at any length): the calls that single tiles serve better.  Time with
+// pairs over that with one tile, 12 heads:
+//   three query tiles, a quarter of whose pairs is empty: 384 queries and 2048 keys 1.03
+//   pairs begin a second round and single tiles almost fit one: 15 x 256 1.09, 7 x 450 ragged 1.17, 6 x 640 ragged 1.18, 4 x 1100 ragged 1.28, 15 x
+//     150 ragged and 1000 keys 1.13 (18 x 256 1.10; beyond 1.5 rounds of single tiles, 1.25 in ragged batches, 0.86-1.05).  Not where the
+//     pairs with rows fit one round (5 x 700 ragged 0.91, 5 x 900 of 1 to 900 tokens 0.93), nor where pairs served the call without
+//     blocks being taken over (even numbers of tiles beyond 1024 queries: 2 x 2000 0.84)
+//   few keys, and second tiles that are often empty: 43 x 150 of 1 to 150 tokens 1.09, 62 x 150 1.11, 14 x 450 ragged 1.12 (sequences of
+//     1000 keys 0.89-1.03)
+inline bool pairs_fall_short(const FwdLaunch& l) {
+  const int q_tiles = (l.max_seqlen_q + kBlockM - 1) / kBlockM;
+  if (q_tiles == 3) return true;
+  const int64_t tiles = groups_with_rows(l, 1), pairs = groups_with_rows(l, 2);
+  if (100 * pairs <= 92 * kSms && 100 * tiles >= 87 * 2 * pairs) return false;
+  const bool few = l.max_seqlen_q <= kOneTileMaxD128 || (q_tiles % 2 != 0 && std::max(l.max_seqlen_q, l.max_seqlen_k) <= kOneTileMaxOdd);
+  if (few && 4 * tiles <= (even_batch(l) ? 6 : 5) * kSlots<1>) return true;
+  return l.max_seqlen_k <= kPairsMaxKeys && !even_batch(l) &&
+         (10 * tiles < 8 * 2 * pairs || (100 * tiles < 89 * 2 * pairs && tiles <= 2 * kSlots<1>));
+}
 
 template <int D, bool CAUSAL, bool DROPOUT>
 bool one_tile_per_cta(const FwdLaunch& l) {
@@ -126,7 +144,7 @@ bool one_tile_per_cta(const FwdLaunch& l) {
   if (l.max_seqlen_q <= kBlockM) return D == 64 || DROPOUT || keys <= kOneTileMaxD128 || pairs > kSms;
   if (one_round) return false;
   if (D == 64) return !(uneven(l) && std::max(l.max_seqlen_q, keys) > kOneTileMaxUneven);
-  const bool pairs_at_once = !CAUSAL && !DROPOUT && q_tiles != 3;  // (at any length)
+  const bool pairs_at_once = !CAUSAL && !DROPOUT && !pairs_fall_short(l);
   if (l.max_seqlen_q <= kOneTileMaxD128 && (tiles <= kSms || (keys <= kOneTileMaxD128 && !pairs_at_once))) return true;
   if (uneven(l) || pairs_at_once) return false;  // (uneven: twice the empty blocks)
   if (keys <= kOneTileMaxD128) return true;

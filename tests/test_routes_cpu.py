@@ -104,6 +104,12 @@ CASES = (
        (call(128, [300] * 16, 12, causal=True), ("1", "rows", "plain")), (call(128, [300] * 41, 12, causal=True), ("1", "rows", "take")),
        (call(128, [700] * 7, 12, causal=True), ("1", "rows", "take")), (call(128, [700] + [300] * 5, 12, causal=True), ("1", "rows", "linear")),
        (call(64, [128] * 30, 12), ("1", "rows", "take")), (call(64, [8192] + [256] * 31, 12), ("2", "quads", "take"))]
+    # d = 128, not causal: pairs, but not where they need a second round that single tiles do not, or are half empty
+    + [(call(128, [256] * 15, 12), ("1", "rows")), (call(128, [256] * 22, 12), ("2", "rows")), (call(128, [640, 400, 500, 350, 480, 540], 12), ("1", "rows")),
+       (call(128, [1100, 570, 630, 730], 12), ("1", "rows")), (call(128, [1100] * 8, 12), ("2", "rows")), (call(128, [2000, 900], 12), ("2", "rows")),
+       (call(128, [374, 406, 386, 631, 465], 12, max_q=700), ("2", "rows")), (call(128, [150] + [60, 90] * 21, 12), ("1", "rows")),
+       (call(128, [150] + [60, 90] * 21, 12, max_k=1000), ("2", "rows")), (call(128, [512] * 40, 12), ("2", "rows")),
+       (call(128, [384] * 40, 12), ("1", "rows")), (call(128, [5000] + [700] * 30, 12), ("2", "rows"))]
     # two stages of K and V in the backward: not with a causal mask and keys that no query sees
     + [(backward(64, 16, 8, 200, 1500), ("short",)), (backward(64, 16, 8, 257, 1500), ("long",)), (backward(64, 32, 12, 40, 1500, dropout=True), ("short",)),
        (backward(64, 12, 12, 200, 128), ("long",)), (backward(64, 64, 12, 256, 256, causal=True), ("short",)),
