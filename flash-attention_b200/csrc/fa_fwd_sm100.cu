@@ -1117,11 +1117,13 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
 template <int D, bool BF16, bool CAUSAL, bool DROPOUT, bool BS, int G, bool ROWS, bool PADDED = false, Order ORDER = kPlain>
 cudaError_t launch_groups(const FwdLaunch& l, cudaStream_t stream) {
   dim3 grid((l.max_seqlen_q + G * kBlockM - 1) / (G * kBlockM), l.args.heads, l.args.batch);
-  if constexpr (ORDER == kPlain) {
+  // (padded batches take pairs at d = 64 only where all blocks start at once: no batch of theirs is uneven)
+  if constexpr (ORDER == kPlain && !(PADDED && D == 64 && G == 2)) {
     const Order order = grid_order<D, CAUSAL, DROPOUT, BS, G, ROWS>(l);
     if constexpr (kCanTake<DROPOUT, BS>)
       if (order == kTake) return launch_groups<D, BF16, CAUSAL, DROPOUT, BS, G, ROWS, PADDED, kTake>(l, stream);
-    if constexpr (CAUSAL)
+    // (in rows, pairs and padded batches beyond 512 tokens always take over: see take_over_pays)
+    if constexpr (CAUSAL && !(kCanTake<DROPOUT, BS> && ROWS && (G == 2 || PADDED)))
       if (order == kLinear) return launch_groups<D, BF16, CAUSAL, DROPOUT, BS, G, ROWS, PADDED, kLinear>(l, stream);
   }
   auto kernel = fa_fwd_kernel<D, BF16, CAUSAL, DROPOUT, BS, G, ROWS, ORDER, PADDED>;

@@ -1,7 +1,9 @@
 """CPU test of the rules that choose a kernel for a call, on the functions that the launches use (compiled for the host): query tiles
 per CTA, softmax layout and order of the forward's grid, stages of the backward.  The cases are those of the GPU tests that aim at a kernel, and the calls on
 either side of a rule's line."""
+import math
 import os
+import random
 import shutil
 import subprocess
 
@@ -144,3 +146,25 @@ def test_routes(routes):
 
 def test_order_without_a_tail(routes):
     routes([], "pair_by_pair")
+
+
+def test_kernels_that_no_call_reaches(routes):
+    """The launches leave out: in padded batches (all rows are there) at d = 64 pairs in more than one round; in order of weight without taking
+    over, pairs in rows, and padded batches in rows."""
+    rng = random.Random(1)
+
+    def log_int(lo, hi):
+        return int(round(math.exp(rng.uniform(math.log(lo), math.log(hi)))))
+
+    calls = []
+    for _ in range(20000):
+        batch, heads, longest = log_int(1, 4000), rng.choice((1, 2, 4, 12, 16, 32)), log_int(1, 70000)
+        total = batch * longest if rng.random() < 0.5 else max(1, int(batch * longest * rng.random()))
+        max_k = longest if rng.random() < 0.7 else log_int(1, 70000)
+        calls.append(("f", rng.choice((64, 128)), batch, heads, longest, max_k, total, rng.randint(0, 1), 0, 0))
+    got = routes(calls)
+    for c, (tiles, layout, order) in zip(calls, got):
+        padded = c[6] == c[2] * c[4] and c[4] == c[5]
+        assert not (padded and c[1] == 64 and tiles == "2" and order != "plain"), c
+        assert not (layout == "rows" and order == "linear" and (tiles == "2" or padded)), c
+    assert {g[0] for g in got} == {"1", "2"} and {g[2] for g in got} == {"plain", "linear", "take"}
