@@ -29,8 +29,8 @@
 //   last four   TMA producer, MMA issuer (S, dP, dQ; everything at d = 128), second and third issuer (dV | dK) at d = 64
 // The compute warps write dV and dK at the end.
 //
-// Schedules.  d = 64: Q and dO travel together through a three-stage ring; S and dP of tile t + 1
-// are issued as soon as the compute groups have read tile t into registers.  d = 128: shared
+// Schedules.  d = 64: Q and dO travel together through a three-stage ring (two stages for block-sparse calls, and for few queries, which
+// hold two stages of K and V instead: short_queries in fa_rules.h); S and dP of tile t + 1 are issued as soon as the compute groups have read tile t into registers.  d = 128: shared
 // memory holds one stage of Q and one of dO, each with its own barriers.  The compute groups work
 // in two phases, P~ from S and then dS from dP; dV(t) is issued after phase one and releases dO
 // for its refill, dK(t) and dQ(t) follow phase two and dK releases Q; S(t + 1) is issued when Q
@@ -108,6 +108,7 @@ template <>
 struct BlockRecord<false> {
   int q_start, sq, k_start, sk, n0, h, b, nm, unused;
 };
+static_assert(sizeof(BlockRecord<true>) == 32 && sizeof(BlockRecord<false>) == 36, "sizes that were measured");
 
 template <bool CAUSAL>
 struct BwdShared {

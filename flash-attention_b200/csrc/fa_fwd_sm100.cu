@@ -1,9 +1,10 @@
 // FlashAttention forward for sm_100a.
 //
-// One CTA owns G = 1 or 2 consecutive 128-row query tiles of one (batch, head) pair and walks the key /
-// value sequence in 128-row tiles; one_tile_per_cta says which G serves which call.  With G = 1 two CTAs share an
-// SM.  Warp roles: G softmax groups, then four warps:
-//   first    TMA producer (Q once, K/V ring)
+// A block is G = 1 or 2 consecutive 128-row query tiles of one (batch, head) pair, whose key / value sequence is walked in
+// 128-row tiles; one_tile_per_cta (fa_rules.h) says which G serves which call.  A CTA works on one block, or goes on with blocks that
+// have not started (kTake, see take_over_pays): the producer asks for the next and publishes it, every role walks the same blocks.
+// With G = 1 two CTAs share an SM.  Warp roles: G softmax groups, then four warps:
+//   first    TMA producer (Q once per block, K/V ring; taking over: the next block)
 //   second   tcgen05.mma issuer (d = 128: every product; d = 64: S = Q K^T only)
 //   third    d = 64: second issuer, O += P V (two issuers keep S ahead)
 //   fourth   padded batches: zeros in the output rows without a token; rows and padded batches: a look at the status word; else idle
@@ -50,7 +51,8 @@ struct FwdCfg {
   static constexpr int kGroupWarps = kRows ? 4 : 8;
   static constexpr int kSoftmaxWarps = G * kGroupWarps;
   static constexpr int kThreads = 32 * kSoftmaxWarps + 128;  // + 1 warpgroup (producer, MMA issuers, idle)
-  // G = 1: 80 KB (d = 64: Q, two stages) or 96 KB (d = 128: Q, one stage), so that two CTAs fit
+  // G = 1: 80 KB (d = 64: Q, two stages; 96 KB with a place for the output rows, kOutBytes) or 96 KB (d = 128: Q, one stage), so that
+  // two CTAs fit
   static constexpr int kStages = (G == 1) ? ((D == 64) ? 2 : 1) : ((D == 64) ? 3 : 2);
   static constexpr int kPanels = D / 64;
   static constexpr int kTileBytes = kBlockM * D * 2;
