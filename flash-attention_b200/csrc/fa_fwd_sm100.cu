@@ -420,7 +420,13 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     return mbar_wait_warp<true>(smem_u32(&sh.blk_full[(k + 1) & 1]), (k >> 1) & 1, abort_flag) && sh.blk[(k + 1) & 1].mp >= 0;
   };
 
-  if (warp >= Cfg::kSoftmaxWarps) reg_dealloc<Cfg::kOtherRegs>();
+  // Causal calls with dropout in single tiles (quads) spilled 20-80 bytes with 96 and 48 registers; the four other warps do with 32 (104 x 256
+  // + 32 x 128 = 80 x 384, what the CTA is launched with).  us: block-sparse, 25 % of the
+  // blocks, 4 x 16 x 4096 151.6 -> 145.2, 16 x 12 x 2048 ragged 138.8 -> 130.1; dense 16 x 12 x 1000 86.1 -> 84.1, 4 x 12 x 4096 243.4 -> 239.2,
+  // d = 128 100.7 -> 99.2 and 298.0 -> 296.8.
+  // Without a causal mask the same made them 1-2.5 % slower (4 x 12 x 4096 442 -> 449, d = 128 544 -> 555).
+  constexpr bool kMoreRegs = CAUSAL && DROPOUT && G == 1;
+  if (warp >= Cfg::kSoftmaxWarps) reg_dealloc<kMoreRegs ? 32 : Cfg::kOtherRegs>();
   if (warp == Cfg::kSoftmaxWarps) {
     // ------------------------------------------------------------------ TMA producer
     if (lane == 0) {
@@ -865,7 +871,7 @@ fa_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ 
     // A warp owns 16 query rows.  It reads their scores with the 16x256b shape, in which a thread holds rows r8 and
     // r8 + 8 and, of every 8-column unit, two adjacent columns: the ownership pattern of the reference's mask
     // generator (one Philox call covers exactly one thread's part of a 16 x 16 patch, QuadPhilox).
-    reg_alloc<Cfg::kSoftmaxRegs>();
+    reg_alloc<kMoreRegs ? 104 : Cfg::kSoftmaxRegs>();
     const int g = (G == 1) ? 0 : warp >> 3;
     const int hh = (warp >> 2) & 1, wq = warp & 3;
     const int r8 = lane >> 2, q4 = lane & 3;
