@@ -55,8 +55,8 @@ inline bool tail_order(const FwdLaunch& l) { return l.max_seqlen_q > 512; }
 //   quads, causal        7 x 700 1.07 (1.7), 5 x 900 1.09, 9 x 1000 1.03 (2.9), 17 x 600 0.97 (3.4), 11 x 1000 0.98 (3.6), 21 x 700 0.94 (5)
 //   rows (d = 64), single tiles (d = 128)   even batches 0.9-0.98 from one round on; where the blocks with rows start at once, 14 x 200 of 1 to 200
 //                        tokens 1.19-1.23, 9 x 300 ragged 1.04-1.12
-//   d = 128, causal, up to 512 queries (no order of weight)   15 x 300 1.12 (1.8), 18 x 300 ragged 1.15, 17 x 200 of 1 to 200 tokens 1.25; from 3.5
-//                        rounds of blocks with rows on 0.94-1.0
+//   d = 128, causal, up to 512 queries (no order of weight)   15 x 300 1.12 (1.8), 18 x 300 ragged 1.15, 17 x 200 of 1 to 200 tokens 1.25; from 3.25
+//                        rounds of blocks with rows on 0.94-1.0, even batches of four tiles 1.05 (1.8), 16 x 512 0.96 (2.6)
 // Up to 128 queries, and in pairs of query tiles, it pays at any size (0.9, 0.93-0.97 just above one round).
 template <int D, bool ROWS, bool CAUSAL>
 constexpr int kTakeMaxKeys = D == 64 && !ROWS ? (CAUSAL ? 2560 : 1536) : INT_MAX;
@@ -66,7 +66,9 @@ bool take_over_pays(const FwdLaunch& l, int64_t blocks) {
   if (l.max_seqlen_k > kTakeMaxKeys<D, ROWS, CAUSAL>) return false;
   if (l.max_seqlen_q <= kBlockM || (ROWS && G == 2)) return true;
   if (!ROWS) return 4 * blocks > (CAUSAL ? 13 : 16) * kSlots<G> || (!CAUSAL && even_batch(l) && 2 * blocks <= 3 * kSlots<G>);
-  return 40 * groups_with_rows(l, G) > (D == 128 && CAUSAL && !tail_order(l) ? 130 : even_batch(l) ? 40 : 44) * kSlots<G>;
+  const bool even = even_batch(l);
+  const int rounds40 = D == 128 && CAUSAL && !tail_order(l) ? (even && l.max_seqlen_q > 3 * kBlockM ? 96 : 130) : even ? 40 : 44;  // in fortieths
+  return 40 * groups_with_rows(l, G) > rounds40 * kSlots<G>;
 }
 
 template <bool DROPOUT, bool BS>

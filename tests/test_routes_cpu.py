@@ -103,7 +103,8 @@ CASES = (
        (call(64, [600] * 5, 12), ("1", "quads", "take")), (call(64, [600] * 25, 12), ("1", "quads", "take")),
        (call(64, [900] * 5, 12, causal=True), ("1", "quads", "linear")), (call(64, [700] * 21, 12, causal=True), ("1", "quads", "take")),
        (call(64, [200] + [100] * 13, 12), ("1", "rows", "plain")), (call(64, [200] * 14, 12), ("1", "rows", "take")),
-       (call(128, [300] * 16, 12, causal=True), ("1", "rows", "plain")), (call(128, [300] * 41, 12, causal=True), ("1", "rows", "take")),
+       (call(128, [300] * 16, 12, causal=True), ("1", "rows", "plain")), (call(128, [512] * 16, 12, causal=True), ("1", "rows", "take")),
+       (call(128, [512] * 11, 12, causal=True), ("1", "rows", "plain")), (call(128, [300] * 41, 12, causal=True), ("1", "rows", "take")),
        (call(128, [700] * 7, 12, causal=True), ("1", "rows", "take")), (call(128, [700] + [300] * 5, 12, causal=True), ("1", "rows", "linear")),
        (call(64, [128] * 30, 12), ("1", "rows", "take")), (call(64, [8192] + [256] * 31, 12), ("2", "quads", "take"))]
     # d = 128, not causal: pairs, but not where they need a second round that single tiles do not, or are half empty
