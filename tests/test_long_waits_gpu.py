@@ -44,6 +44,32 @@ def test_backward_of_sequences_without_keys(d, causal):
     torch.testing.assert_close(got[0].float(), want[0].float(), rtol=2.0 ** -10, atol=1e-5 * want[0].float().abs().max().item())
 
 
+def test_block_sparse_backward_of_sequences_without_keys():
+    """2048 x 16 x 1024 blocks, whose lists are made for those with keys alone."""
+    from flash_attn_b200 import flash_attn_cuda as fc
+    from flash_attn_b200.flash_blocksparse_attn_interface import convert_blockmask
+    batch, heads, longest = 2048, 16, 131072
+    lens = LENS * 2
+    q, k, v, dout, cu, _ = U.make_varlen(lens, lens, heads, 64, torch.float16, seed=1)
+    layout = torch.ones(32, longest // 256, dtype=torch.int32, device="cuda")
+    layout[3, 0], layout[7, 1] = 0, 0
+    wide_mask, mask = convert_blockmask(layout, False), convert_blockmask(layout[:, :2].contiguous(), False)
+    out, lse = fc.fwd_block(q, k, v, cu, cu, mask, 300, 300, 0.0, 0.125, False, False, None)
+
+    def run(cu, stats, mask, longest):
+        grads = [torch.full_like(t, float("nan")) for t in (q, k, v)]
+        fc.bwd_block(dout, q, k, v, out, stats, *grads, cu, cu, mask, 300, longest, 0.0, 0.125, False, None)
+        fc.check_device_status()
+        return grads
+
+    want = run(cu, lse, mask, 300)
+    wide = torch.zeros(batch, heads, lse.shape[2], device="cuda")
+    wide[:4], wide[-4:] = lse[:4], lse[4:]
+    got = run(torch.tensor([0] + _announced(batch)).cumsum(0).int().cuda(), wide, wide_mask, longest)
+    assert torch.equal(got[1], want[1]) and torch.equal(got[2], want[2])
+    torch.testing.assert_close(got[0].float(), want[0].float(), rtol=2.0 ** -10, atol=1e-5 * want[0].float().abs().max().item())
+
+
 @pytest.mark.parametrize("d", [64, 128])
 def test_forward_of_sequences_without_queries(d):
     """8192 x 16 x 256 pairs of tiles; the softmax_lse of the announced lengths takes 34 GB."""
